@@ -16,6 +16,7 @@
 // walking the nonzeros of A (CSR, read through the read-only cache and
 // broadcast across the warp).  Structural zeros of A cost nothing, so the
 // sparse tensor-product operators run at their nonzero count.
+#include <math.h>
 #include <stdlib.h>
 #include <string.h>
 #include <vector>
@@ -34,6 +35,11 @@ struct MulHandle {
     int *colidx;     // device, nnz
     double *val64;   // device, nnz
     float *val32;    // device, nnz
+    // The fixed-point form of the operator (FP64 applies; null when the
+    // operator does not fit it): per row (first entry, end, scale s, 0), per
+    // entry (column, high part, low part, 0)
+    int4 *fxrow;     // device, m
+    int4 *fxval;     // device, nnz
 };
 
 template <typename T>
@@ -118,6 +124,282 @@ mul_csr_kernel(MulHandle h, const T *__restrict__ b, int64_t ldb, T *__restrict_
     }
 }
 
+// ---- FP64 applies in fixed point ---------------------------------------
+//
+// The FP64 unit issues 2 FMAs per clock per SM here; the 32-bit integer
+// multiply-add with a 64-bit sum (IMAD.WIDE) issues about 56, on another
+// pipe (a probe's rates at 1.92 GHz; both run side by side undisturbed).  A
+// dot product of doubles over a common exponent is a dot product of
+// integers, so a row of the operator times a column of B is formed as
+//
+//     B[k, n] = (bh 2^31 + bl) 2^-sb,  |bh| <= 2^30, |bl| <= 2^30
+//     A[m, k] = (ah 2^26 + al) 2^-(s + 26),  sum_k |ah| ~ 2^30, |al| <= 2^25
+//     hh = sum ah bh,  u = sum ah bl,  v = sum al bh    (64-bit, exact)
+//     A B = (hh + u/2^31 + v/2^26 + O(2^-2)) 2^(31 - s - sb)
+//
+// three IMAD.WIDE per nonzero, and the sum is rounded to FP64 once.  sb is
+// the column's own (its largest exponent), s the row's.  B keeps 61 bits
+// below the column's largest value and A 57 below the row's absolute sum,
+// so the result is within 1.5 2^-59 of (row sum)(column maximum), which is
+// below the rounding of an FP64 dot product unless every B value the row
+// touches is small against the column's largest.  That is tested per output
+// (the OR of the |bh| over the row's support against 2^23, the column's
+// largest being in [2^29, 2^30]): such outputs, and those of columns with
+// infinities, NaNs or exponents near the ends of the range, are formed again
+// with FP64 FMAs from global memory by the whole warp.
+//
+// Bounds: hh, u <= 2^61 by the row sums; v <= nnz 2^55, nnz <= 64 (FX_MAXNNZ),
+// so no sum overflows.
+
+constexpr int FX_MAXNNZ = 64;
+constexpr int FX_THR = 1 << 23;
+
+// Columns per lane: 2 (64 columns a CTA, 16-byte accesses) or 1
+template <int CPL>
+struct FxPair;
+template <>
+struct FxPair<1> { using I = int2; using D = double; };
+template <>
+struct FxPair<2> { using I = int4; using D = double2; };
+
+// The exponent field of the largest value; whether anything but zero is
+// there (hi the absolute high word, or 1 for a subnormal below it)
+__device__ __forceinline__ int fx_mag(double x) {
+    const int hi = __double2hiint(x) & 0x7fffffff;
+    return hi | (__double2loint(x) != 0);
+}
+
+// (bh, bl) of x for a column whose largest exponent field is emax
+__device__ __forceinline__ int2 fx_split(double x, int emax) {
+    const int hi = __double2hiint(x);
+    const int e = (hi >> 20) & 0x7ff;
+    const int d = min(emax - e, 63);
+    // 53-bit mantissa over 8 zero bits, shifted down by the exponent
+    // difference (values below 2^-61 of the largest become zero; a zero or
+    // subnormal value always does)
+    unsigned long long q =
+        ((unsigned long long)((hi & 0xfffff) | 0x100000) << 32) | (unsigned)__double2loint(x);
+    q = (q << 8) >> d;
+    long long b = hi < 0 ? -(long long)q : (long long)q;
+    b += 1ll << 30;
+    int2 r;
+    r.x = (int)(b >> 31);
+    r.y = (int)((unsigned)b & 0x7fffffffu) - (1 << 30);
+    return r;
+}
+
+template <int EPI, int CPL>
+__global__ void __launch_bounds__(MUL_WARPS * 32)
+mul_fx_kernel(MulHandle h, const double *__restrict__ b, int64_t ldb, double *__restrict__ c,
+              int64_t ldc, int64_t ncol, double alpha, double beta, int vec) {
+    using I = typename FxPair<CPL>::I;
+    constexpr int NC = 32 * CPL;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    I *bs = reinterpret_cast<I *>(smem_raw);             // [k][32]
+    __shared__ int cmax[MUL_WARPS][NC];
+
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t col = (int64_t)blockIdx.x * NC + lane * CPL;
+    bool ok[CPL];
+#pragma unroll
+    for (int j = 0; j < CPL; j++) ok[j] = col + j < ncol;
+    const bool full = ok[CPL - 1];
+
+    // Load the tile, every warp its rows, eight rows in flight per thread;
+    // the largest magnitude of each column over the warp's rows
+    int mag[CPL];
+#pragma unroll
+    for (int j = 0; j < CPL; j++) mag[j] = 0;
+    constexpr int UNR = 8;
+    for (int r0 = warp; r0 < h.k; r0 += UNR * MUL_WARPS) {
+        double x[UNR][CPL];
+#pragma unroll
+        for (int q = 0; q < UNR; q++) {
+            const int r = r0 + q * MUL_WARPS;
+            const double *src = b + r * ldb + col;
+#pragma unroll
+            for (int j = 0; j < CPL; j++) x[q][j] = 0.0;
+            if (r < h.k) {
+                if (CPL == 2 && vec && full) {
+                    const double2 t = *reinterpret_cast<const double2 *>(src);
+                    x[q][0] = t.x;
+                    x[q][CPL - 1] = t.y;
+                } else {
+#pragma unroll
+                    for (int j = 0; j < CPL; j++)
+                        if (ok[j]) x[q][j] = src[j];
+                }
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < UNR; q++) {
+            const int r = r0 + q * MUL_WARPS;
+            if (r < h.k) {
+                double *dst = reinterpret_cast<double *>(bs + r * 32 + lane);
+#pragma unroll
+                for (int j = 0; j < CPL; j++) {
+                    dst[j] = x[q][j];
+                    mag[j] = max(mag[j], fx_mag(x[q][j]));
+                }
+            }
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < CPL; j++) cmax[warp][lane * CPL + j] = mag[j];
+    __syncthreads();
+
+    // Column exponents; the threshold of the support test (0: a column of
+    // zeros needs none; the largest int: every output of the column by FP64)
+    int emax[CPL], thr[CPL];
+#pragma unroll
+    for (int j = 0; j < CPL; j++) {
+        int mx = cmax[0][lane * CPL + j];
+#pragma unroll
+        for (int w = 1; w < MUL_WARPS; w++) mx = max(mx, cmax[w][lane * CPL + j]);
+        // (at least 64 for the splits: then zeros have an exponent
+        // difference that makes them zero)
+        emax[j] = max(mx >> 20, 64);
+        thr[j] = mx == 0 ? 0 : (emax[j] < 128 || emax[j] > 1900) ? 0x7fffffff : FX_THR;
+    }
+
+    // Split in place (each thread the values that it stored)
+    for (int r = warp; r < h.k; r += MUL_WARPS) {
+        double *src = reinterpret_cast<double *>(bs + r * 32 + lane);
+        int2 *dst = reinterpret_cast<int2 *>(src);
+        int2 t[CPL];
+#pragma unroll
+        for (int j = 0; j < CPL; j++) t[j] = fx_split(src[j], emax[j]);
+#pragma unroll
+        for (int j = 0; j < CPL; j++) dst[j] = t[j];
+    }
+    __syncthreads();
+
+    for (int row = warp; row < h.m; row += MUL_WARPS) {
+        double *crow = c + row * ldc + col;
+        const int4 ri = __ldg(h.fxrow + row);
+        double cin[CPL];
+        if (EPI == EPI_ADD || EPI == EPI_GENERAL) {
+#pragma unroll
+            for (int j = 0; j < CPL; j++) cin[j] = ok[j] ? crow[j] : 0.0;
+        }
+        // (u and v start at half a unit of hh: the final shifts round)
+        long long hh[CPL], u[CPL], v[CPL];
+        int m[CPL];
+#pragma unroll
+        for (int j = 0; j < CPL; j++) {
+            hh[j] = 0;
+            u[j] = 1ll << 30;
+            v[j] = 1ll << 25;
+            m[j] = 0;
+        }
+#pragma unroll 4
+        for (int p = ri.x; p < ri.y; p++) {
+            const int4 a = __ldg(h.fxval + p);
+            const I t = bs[a.x * 32 + lane];
+            const int *tb = reinterpret_cast<const int *>(&t);
+#pragma unroll
+            for (int j = 0; j < CPL; j++) {
+                const int bh = tb[2 * j], bl = tb[2 * j + 1];
+                hh[j] += (long long)a.y * bh;
+                u[j] += (long long)a.y * bl;
+                v[j] += (long long)a.z * bh;
+                m[j] |= bh ^ (bh >> 31);
+            }
+        }
+
+        double r[CPL];
+        bool small = false;
+#pragma unroll
+        for (int j = 0; j < CPL; j++) {
+            const long long t = hh[j] + (u[j] >> 31) + (v[j] >> 26);
+            r[j] = (double)t;
+            // times 2^(31 - s - sb), sb = 1083 - emax: an exponent sum, in
+            // the normal range by the limits on emax and s
+            if (t != 0)
+                r[j] = __hiloint2double(__double2hiint(r[j]) +
+                                            (emax[j] - 1052 - ri.z) * (1 << 20),
+                                        __double2loint(r[j]));
+            small |= m[j] < thr[j];
+        }
+        if (__any_sync(0xffffffffu, small)) {
+            const int p0 = __ldg(h.rowptr + row), p1 = __ldg(h.rowptr + row + 1);
+            double acc[CPL];
+#pragma unroll
+            for (int j = 0; j < CPL; j++) acc[j] = 0.0;
+            for (int p = p0; p < p1; p++) {
+                const double a = __ldg(h.val64 + p);
+                const double *src = b + __ldg(h.colidx + p) * ldb + col;
+#pragma unroll
+                for (int j = 0; j < CPL; j++)
+                    if (ok[j]) acc[j] = fma(a, src[j], acc[j]);
+            }
+#pragma unroll
+            for (int j = 0; j < CPL; j++)
+                if (m[j] < thr[j]) r[j] = acc[j];
+        }
+#pragma unroll
+        for (int j = 0; j < CPL; j++) {
+            if (EPI == EPI_GENERAL) r[j] = alpha * r[j] + beta * cin[j];
+            if (EPI == EPI_ADD) r[j] += cin[j];
+            if (EPI == EPI_SCALE) r[j] *= alpha;
+        }
+        if (CPL == 2 && vec && full) {
+            *reinterpret_cast<double2 *>(crow) = make_double2(r[0], r[CPL - 1]);
+        } else {
+#pragma unroll
+            for (int j = 0; j < CPL; j++)
+                if (ok[j]) crow[j] = r[j];
+        }
+    }
+}
+
+template <int CPL>
+void launch_fx(const MulHandle &h, const double *b, int64_t ldb, double *c, int64_t ldc,
+               int64_t ncol, double alpha, double beta, int vec, cudaStream_t s) {
+    const unsigned grid = b200::ceil_div(ncol, 32 * CPL);
+    const size_t smem = (size_t)h.k * 32 * CPL * sizeof(double);
+    if (alpha == 1.0 && beta == 0.0)
+        mul_fx_kernel<EPI_SET, CPL><<<grid, MUL_WARPS * 32, smem, s>>>(h, b, ldb, c, ldc, ncol, alpha, beta, vec);
+    else if (alpha == 1.0 && beta == 1.0)
+        mul_fx_kernel<EPI_ADD, CPL><<<grid, MUL_WARPS * 32, smem, s>>>(h, b, ldb, c, ldc, ncol, alpha, beta, vec);
+    else if (beta == 0.0)
+        mul_fx_kernel<EPI_SCALE, CPL><<<grid, MUL_WARPS * 32, smem, s>>>(h, b, ldb, c, ldc, ncol, alpha, beta, vec);
+    else
+        mul_fx_kernel<EPI_GENERAL, CPL><<<grid, MUL_WARPS * 32, smem, s>>>(h, b, ldb, c, ldc, ncol, alpha, beta, vec);
+}
+
+// The operator's fixed-point form (rows, entries), or false where it does
+// not fit: a row of more than FX_MAXNNZ entries, or of an absolute sum
+// outside [2^-60, 2^60] (or not finite)
+bool fx_operator(const double *a, int m, int k, std::vector<int4> &rows,
+                 std::vector<int4> &vals) {
+    for (int i = 0; i < m; i++) {
+        const double *ar = a + (size_t)i * k;
+        double l1 = 0.0;
+        int nnz = 0;
+        for (int j = 0; j < k; j++) {
+            l1 += fabs(ar[j]);
+            nnz += ar[j] != 0.0;
+        }
+        if (nnz > FX_MAXNNZ || (nnz && !(l1 >= ldexp(1.0, -60) && l1 <= ldexp(1.0, 60))))
+            return false;
+        // sum |A| 2^s in [2^29, 2^30): with the rounding of every |ah| up
+        // by at most 1 the sum of |ah| stays below 2^30 + FX_MAXNNZ
+        int e = 0;
+        if (nnz) frexp(l1, &e);
+        const int s = 30 - e;
+        const int p0 = (int)vals.size();
+        for (int j = 0; j < k; j++) {
+            if (ar[j] == 0.0) continue;
+            const long long q = llrint(ldexp(ar[j], s + 26));
+            const long long ah = (q + (1ll << 25)) >> 26, al = q - ah * (1ll << 26);
+            vals.push_back(make_int4(j, (int)ah, (int)al, 0));
+        }
+        rows.push_back(make_int4(p0, (int)vals.size(), s, 0));
+    }
+    return true;
+}
+
 template <typename T>
 int launch_mul(const MulHandle *h, const T *b, int64_t ldb, T *c, int64_t ldc, int64_t ncol,
                T alpha, T beta, cudaStream_t s) {
@@ -131,6 +413,32 @@ int launch_mul(const MulHandle *h, const T *b, int64_t ldb, T *c, int64_t ldc, i
     unsigned grid = b200::ceil_div(ncol, MUL_NCOL);
     // 16-byte copies need a 16-byte aligned base and row stride
     const int vec = !((uintptr_t)b & 15) && !((ldb * (int64_t)sizeof(T)) & 15);
+    if constexpr (sizeof(T) == 8) {
+        // (the FP64 FMAs of small outputs read B again, so C must not be B)
+        const bool apart = c + (int64_t)(h->m - 1) * ldc + ncol <= b ||
+                           b + (int64_t)(h->k - 1) * ldb + ncol <= c;
+        // Where the FMAs bound: rows of ten entries and more at every width
+        // (tetrahedra's 20 x 40 lift at 20480 columns 38.5 -> 17.4 us), rows
+        // of four and more once every SM has a tile (hexahedra's 192 x 64
+        // gradient at p = 3: 41.9 -> 25.9 us at 20480 columns, 131 -> 75 us at
+        // 87880; below 9728 columns of rows of four the FP64 form's shorter
+        // chain is up to 10% faster, and for rows of two, 192 x 96, it is
+        // 15-25% faster at every width).  The tile has to leave an SM room
+        // for two CTAs (the 125 x 375 divergence at p = 4: 359 us against
+        // 370).
+        const bool many = h->nnz >= 10 * (int64_t)h->m ||
+                          (h->nnz >= 4 * (int64_t)h->m && ncol > 64 * 152);
+        if (h->fxval && apart && many && smem <= 113 * 1024) {
+            const int vec2 = vec && !((uintptr_t)c & 15) && !(ldc & 1);
+            // One column per lane where two would leave SMs without a tile
+            if (ncol <= 64 * 152)
+                launch_fx<1>(*h, b, ldb, c, ldc, ncol, alpha, beta, vec2, s);
+            else
+                launch_fx<2>(*h, b, ldb, c, ldc, ncol, alpha, beta, vec2, s);
+            B200_CHECK_LAUNCH("mul_fx_kernel");
+            return B200_OK;
+        }
+    }
     if (alpha == T(1) && beta == T(0))
         mul_csr_kernel<T, EPI_SET><<<grid, MUL_WARPS * 32, smem, s>>>(*h, b, ldb, c, ldc, ncol, alpha, beta, vec);
     else if (alpha == T(1) && beta == T(1))
@@ -146,6 +454,21 @@ int launch_mul(const MulHandle *h, const T *b, int64_t ldb, T *c, int64_t ldc, i
 // Opt every instantiation in to the largest tile.  Called from
 // b200_mul_create, which never runs inside a stream capture: changing a
 // function attribute while a capture is open invalidates the capture.
+template <int CPL>
+int opt_in_smem_fx() {
+    void (*fns[4])(MulHandle, const double *, int64_t, double *, int64_t, int64_t, double,
+                   double, int) = {mul_fx_kernel<EPI_SET, CPL>, mul_fx_kernel<EPI_ADD, CPL>,
+                                   mul_fx_kernel<EPI_GENERAL, CPL>,
+                                   mul_fx_kernel<EPI_SCALE, CPL>};
+    // (less the static array of the column maxima)
+    for (auto fn : fns) {
+        cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             224 * 1024);
+        if (e != cudaSuccess) return b200::check_cuda(e, "mul: smem attribute");
+    }
+    return B200_OK;
+}
+
 template <typename T>
 int opt_in_smem() {
     void (*fns[4])(MulHandle, const T *, int64_t, T *, int64_t, int64_t, T, T, int) = {
@@ -159,6 +482,12 @@ int opt_in_smem() {
     return B200_OK;
 }
 
+void free_handle(MulHandle *h) {
+    cudaFree(h->rowptr); cudaFree(h->colidx); cudaFree(h->val64); cudaFree(h->val32);
+    cudaFree(h->fxrow); cudaFree(h->fxval);
+    free(h);
+}
+
 }  // namespace
 
 extern "C" {
@@ -168,6 +497,8 @@ int b200_mul_create(const double *a, int m, int k, void **handle) {
         return b200::set_error(B200_ERR_ARG, "mul_create: bad arguments");
     int orc = opt_in_smem<double>();
     if (!orc) orc = opt_in_smem<float>();
+    if (!orc) orc = opt_in_smem_fx<1>();
+    if (!orc) orc = opt_in_smem_fx<2>();
     if (orc) return orc;
 
     std::vector<int> rowptr(m + 1, 0), colidx;
@@ -205,9 +536,17 @@ int b200_mul_create(const double *a, int m, int k, void **handle) {
         if (!rc) rc = b200::check_cuda(cudaMemcpy(h->val32, v32.data(), sizeof(float) * h->nnz,
                                                   cudaMemcpyHostToDevice), "mul_create");
     }
+    std::vector<int4> fxrow, fxval;
+    if (!rc && h->nnz && fx_operator(a, m, k, fxrow, fxval)) {
+        rc = b200::check_cuda(cudaMalloc(&h->fxrow, sizeof(int4) * m), "mul_create");
+        if (!rc) rc = b200::check_cuda(cudaMalloc(&h->fxval, sizeof(int4) * nz), "mul_create");
+        if (!rc) rc = b200::check_cuda(cudaMemcpy(h->fxrow, fxrow.data(), sizeof(int4) * m,
+                                                  cudaMemcpyHostToDevice), "mul_create");
+        if (!rc) rc = b200::check_cuda(cudaMemcpy(h->fxval, fxval.data(), sizeof(int4) * nz,
+                                                  cudaMemcpyHostToDevice), "mul_create");
+    }
     if (rc) {
-        cudaFree(h->rowptr); cudaFree(h->colidx); cudaFree(h->val64); cudaFree(h->val32);
-        free(h);
+        free_handle(h);
         return rc;
     }
     *handle = h;
@@ -222,9 +561,7 @@ int b200_mul_nnz(void *handle, int *nnz) {
 
 int b200_mul_destroy(void *handle) {
     if (!handle) return B200_OK;
-    MulHandle *h = (MulHandle *)handle;
-    cudaFree(h->rowptr); cudaFree(h->colidx); cudaFree(h->val64); cudaFree(h->val32);
-    free(h);
+    free_handle((MulHandle *)handle);
     return B200_OK;
 }
 
