@@ -139,7 +139,8 @@ def kernel_bytes(k, be):
             per_pt += nd*nv*(2 if m.get('gradwb', True) else 1)
         # Metric terms (nd*nd + 1 values) stored per point or, for affine
         # elements, per element; or the vertices they are rebuilt from
-        geo = {1: (2**nd)*nd*neles, 2: neles*(nd*nd + 1)}.get(
+        geo = {1: (2**nd)*nd*neles, 2: neles*(nd*nd + 1),
+               3: neles*(nd + 1)}.get(
             m.get('geom_mode'), nupts*neles*(nd*nd + 1))
         return (per_pt*nupts*neles + geo)*itemsize
     if kind in ('intcflux_ns', 'intcflux_euler'):

@@ -280,7 +280,9 @@ int b200_mul_tc_terms(void *handle, int *nterms);
  * stored metric terms `smats` (ndims, nupts, ndims, neles) and `rcpdjac`
  * (nupts x neles, leading dimension ldr); 2 reads one stored set per
  * element, smats (ndims, 1, ndims, neles) and rcpdjac (1 x neles), for
- * affine elements whose Jacobian is the same at every point. */
+ * affine elements whose Jacobian is the same at every point; 3 is 2 for
+ * elements whose edges are along the axes: the off-diagonal smats are taken
+ * as zero and not read. */
 
 /* Euler transformed flux; pyfr/solvers/euler/kernels/tflux.mako:8-30,
  * provider call pyfr/solvers/euler/elements.py:149-206. */

@@ -80,7 +80,7 @@ def linear_metrics(verts, upts):
 
 
 # Geometry modes of the element kernels (the C ABI's `linear` argument)
-GEOM_STORED, GEOM_VERTICES, GEOM_PER_ELEMENT = 0, 1, 2
+GEOM_STORED, GEOM_VERTICES, GEOM_PER_ELEMENT, GEOM_DIAGONAL = 0, 1, 2, 3
 
 
 def affine(smats, rtol=1e-13):
@@ -89,6 +89,21 @@ def affine(smats, rtol=1e-13):
     (parallelograms, parallelepipeds, simplices)."""
     dev = np.abs(smats - smats[:, :1]).max(axis=(0, 1, 2))
     return bool(np.all(dev <= rtol*np.abs(smats).max(axis=(0, 1, 2))))
+
+
+def diagonal(smats, rtol=1e-13):
+    """Whether every element's metric terms S (ndims, npts, ndims, neles)
+    are diagonal (to rounding, as ``affine`` takes it): true of elements
+    whose edges are along the axes."""
+    nd = smats.shape[0]
+    off = np.zeros(smats.shape[-1])
+    for i in range(nd):
+        for j in range(nd):
+            if i != j:
+                off = np.maximum(off, np.abs(smats[i, :, j]).max(axis=0))
+    top = np.min([np.abs(smats[i, :, i]).min(axis=0) for i in range(nd)],
+                 axis=0)
+    return bool(np.all(off <= rtol*top))
 
 
 def _host_of(m):
@@ -165,9 +180,9 @@ class PointwiseKernelProvider:
             # one set per element
             m = self._stored_metrics(verts, upts)
             if m is not None:
-                smats, rcpdjac, per_ele = m
-                return (GEOM_PER_ELEMENT if per_ele else GEOM_STORED,
-                        _mat(smats), _mat(rcpdjac), (None, 0), (None, 0))
+                smats, rcpdjac, mode = m
+                return (mode, _mat(smats), _mat(rcpdjac), (None, 0),
+                        (None, 0))
         if linear:
             if not multilin:
                 raise ValueError('Linear-element kernels of this shape need '
@@ -200,12 +215,13 @@ class PointwiseKernelProvider:
         if key not in self._metrics:
             be = self.backend
             sm, rj = linear_metrics(vh, uh)
-            per_ele = self.backend.per_element_metrics and affine(sm)
-            if per_ele:
+            mode = GEOM_STORED
+            if self.backend.per_element_metrics and affine(sm):
                 sm, rj = sm[:, :1], rj[:1]
+                mode = GEOM_DIAGONAL if diagonal(sm) else GEOM_PER_ELEMENT
             self._metrics[key] = (be.const_matrix(sm, tags={'align'}),
                                   be.const_matrix(rj, tags={'align'}),
-                                  per_ele, vh, uh)
+                                  mode, vh, uh)
         return self._metrics[key][:3]
 
     def _tflux_euler(self, tplargs, dims, extrns, u, f, smats=None,

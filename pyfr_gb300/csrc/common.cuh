@@ -69,26 +69,67 @@ __device__ __forceinline__ float narrow_f64(double d) {
     return (float)d;
 }
 
-// 1/d in FP64 without an IEEE division.  A single-precision estimate
-// (rcp.approx.ftz.f32, relative error about 2^-23) refined by two
-// Newton-Raphson steps for f(r) = 1/r - d, r <- r + r*(1 - d*r), each of
-// which squares the relative error (2^-46, then below the rounding of the
-// last step): the result is within about one unit in the last place of
-// the correctly rounded quotient, for 4 FP64 FMAs instead of the several
-// FP64 operations, fix-up tests and slow path of an IEEE division on a GPU
-// whose FP64 unit is narrow.  Operands with |d| outside [2^-100, 2^100]
-// (where the estimate or its reciprocal could leave the binary32 normal
-// range) take the IEEE division.
-__device__ __forceinline__ double rcp_f64(double d) {
-    const uint64_t a = (uint64_t)__double_as_longlong(d) & 0x7fffffffffffffffull;
-    if (a - ((1023ull - 100) << 52) >= (200ull << 52)) return 1.0 / d;
-    float r0;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r0) : "f"(narrow_f64(d)));
-    double r = widen_f32(r0);
-    r = fma(r, fma(-d, r, 1.0), r);
-    r = fma(r, fma(-d, r, 1.0), r);
-    return r;
+// A double in [2^-100, 2^100) by magnitude to a float by truncation, and a
+// normal float to a double, on the integer pipes (the encodings above).
+__device__ __forceinline__ float trunc_f64(double d) {
+    const uint32_t hi = (uint32_t)__double2hiint(d), lo = (uint32_t)__double2loint(d);
+    return __uint_as_float((hi & 0x80000000u) |
+                           (__funnelshift_l(lo, hi & 0x7fffffffu, 3) - (896u << 23)));
 }
+
+__device__ __forceinline__ double widen_normal(float f) {
+    const uint32_t u = __float_as_uint(f);
+    return __hiloint2double((int)((u & 0x80000000u) | (((u & 0x7fffffffu) >> 3) + (896u << 20))),
+                            (int)(u << 29));
+}
+
+// Whether |d| lies in [2^-100, 2^100): there a single-precision estimate of
+// 1/d or 1/sqrt(d) and its argument are normal floats
+__device__ __forceinline__ bool mid_range(double d) {
+    return ((uint32_t)__double2hiint(d) & 0x7fffffffu) - ((1023u - 100) << 20) < (200u << 20);
+}
+
+// 1/d in FP64 without an IEEE division: a single-precision estimate
+// (rcp.approx.ftz.f32 of the truncated operand, relative error e about
+// 2^-22) refined by one step of Chebyshev's third-order iteration,
+// r (1 + e + e^2) with e = 1 - d r, whose error e^3 is below FP64's
+// rounding: 3 FP64 FMAs where an IEEE division spends about ten FP64
+// operations, fix-up tests and a slow path, on a GPU whose FP64 unit is
+// narrow (2 operations per clock and SM).  Operands outside mid_range, zeros,
+// infinities and NaNs take the IEEE division.
+__device__ __forceinline__ double rcp_f64(double d) {
+    if (!mid_range(d)) return 1.0 / d;
+    float r0;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r0) : "f"(trunc_f64(d)));
+    const double r = widen_normal(r0);
+    const double e = fma(-d, r, 1.0);
+    return fma(r, fma(e, e, e), r);
+}
+
+// sqrt(x) in FP64: the single-precision estimate y of 1/sqrt(x), h = x y and
+// two Newton (Heron) steps with the fixed slope y/2, s <- s + (x - s^2) y/2,
+// which take the error from 2^-22 to below FP64's rounding: 5 FP64
+// operations.  Operands outside mid_range, negative ones, zeros, infinities
+// and NaNs take the IEEE square root.
+__device__ __forceinline__ double sqrt_f64(double x) {
+    if (!mid_range(x) || x < 0) return sqrt(x);
+    float y0;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y0) : "f"(trunc_f64(x)));
+    const double y2 = widen_normal(0.5f * y0);
+    double s = x * widen_normal(y0);
+    s = fma(fma(-s, s, x), y2, s);
+    return fma(fma(-s, s, x), y2, s);
+}
+
+// The reciprocal and square root of the flux kernels: in FP64 the forms
+// above, in FP32 the IEEE operations
+__device__ __forceinline__ double rcp(double x) { return rcp_f64(x); }
+__device__ __forceinline__ float rcp(float x) { return 1.0f / x; }
+__device__ __forceinline__ double root(double x) { return sqrt_f64(x); }
+__device__ __forceinline__ float root(float x) { return sqrtf(x); }
+// a/b (in FP64 within one rounding more than the IEEE quotient's)
+__device__ __forceinline__ double quot(double a, double b) { return a * rcp_f64(b); }
+__device__ __forceinline__ float quot(float a, float b) { return a / b; }
 
 }  // namespace b200
 

@@ -93,22 +93,86 @@ template <int ND, typename T>
 __device__ __forceinline__ void inviscid_flux(const T *s, T f[ND][ND + 2], T &p, T v[ND],
                                               T gamma) {
     constexpr int NV = ND + 2;
-    const T invrho = T(1) / s[0], E = s[NV - 1];
+    const T invrho = rcp(s[0]), E = s[NV - 1];
     T rhov[ND];
     T dot = 0;
 #pragma unroll
     for (int i = 0; i < ND; i++) {
         rhov[i] = s[i + 1];
         v[i] = invrho * rhov[i];
-        dot += rhov[i] * rhov[i];
+        dot += rhov[i] * v[i];
     }
-    p = (gamma - T(1)) * (E - T(0.5) * invrho * dot);
+    p = (gamma - T(1)) * (E - T(0.5) * dot);
+    const T h = E + p;
 #pragma unroll
     for (int i = 0; i < ND; i++) {
         f[i][0] = rhov[i];
-        f[i][NV - 1] = (E + p) * v[i];
+        f[i][NV - 1] = h * v[i];
+        f[i][i + 1] = rhov[i] * v[i] + p;
+        // (the momentum flux is symmetric)
 #pragma unroll
-        for (int j = 0; j < ND; j++) f[i][j + 1] = rhov[i] * v[j] + (i == j ? p : T(0));
+        for (int j = i + 1; j < ND; j++) f[i][j + 1] = f[j][i + 1] = rhov[i] * v[j];
+    }
+}
+
+// Dynamic viscosity: constant or Sutherland's law
+// (pyfr/solvers/navstokes/kernels/flux.mako)
+template <int ND, typename T>
+__device__ __forceinline__ T viscosity(const T v[ND], T E_rho, const GasK<T> &g) {
+    if (!g.sutherland) return g.mu;
+    T ke = 0;
+#pragma unroll
+    for (int i = 0; i < ND; i++) ke += v[i] * v[i];
+    const T cpT = g.gamma * (E_rho - T(0.5) * ke);
+    const T Trat = g.rcp_cpTref * cpT;
+    return quot(g.mu_ctt * Trat * root(Trat), cpT + g.cpTs);
+}
+
+// The whole Navier-Stokes flux (inviscid_flux plus viscous_flux_add) of state
+// s with the physical gradient grad, formed together for its operation count
+// (72 FP64 operations in 3-D with the reciprocal, where the two one after the
+// other take about 115; FP64 operations bound the kernel).  With
+// dv_id = grad_d(m_i) - v_i grad_d(rho) = rho d(v_i)/dx_d, mr = -mu/rho and
+// P = p - (2/3) mr div, the momentum flux, which is symmetric, is
+//     f_id = m_i v_d + mr (dv_id + dv_di) + P delta_id,
+// and since sum_i v_i f_id = m.v v_d + p v_d + sum_i v_i tau_id, the energy
+// flux (E + p) v_d + sum_i v_i tau_id - mu gamma/Pr c_v dT/dx_d is
+//     (E - m.v) v_d + sum_i v_i (f_id - kr dv_id)
+//         + kr (grad_d(E) - (E/rho) grad_d(rho)),   kr = mr gamma/Pr.
+template <int ND, typename T>
+__device__ __forceinline__ void ns_flux(const T *s, const T grad[ND][ND + 2], T f[ND][ND + 2],
+                                        const GasK<T> &g) {
+    constexpr int NV = ND + 2;
+    const T inv = rcp(s[0]), E = s[NV - 1], Er = inv * E;
+    T v[ND], dot = 0, dv[ND][ND], div = 0;
+#pragma unroll
+    for (int i = 0; i < ND; i++) {
+        v[i] = inv * s[i + 1];
+        dot += s[i + 1] * v[i];
+    }
+#pragma unroll
+    for (int i = 0; i < ND; i++) {
+#pragma unroll
+        for (int d = 0; d < ND; d++) dv[i][d] = grad[d][i + 1] - v[i] * grad[d][0];
+        div += dv[i][i];
+    }
+    const T mr = -viscosity<ND, T>(v, Er, g) * inv, mr2 = mr + mr, kr = mr * g.gamma_pr;
+    const T P = g.gm1 * (E - T(0.5) * dot) - T(2.0 / 3.0) * mr * div;
+    const T Ed = E - dot;
+#pragma unroll
+    for (int i = 0; i < ND; i++) {
+        f[i][0] = s[i + 1];
+        f[i][i + 1] = s[i + 1] * v[i] + (mr2 * dv[i][i] + P);
+#pragma unroll
+        for (int d = i + 1; d < ND; d++)
+            f[i][d + 1] = f[d][i + 1] = mr * (dv[i][d] + dv[d][i]) + s[i + 1] * v[d];
+    }
+#pragma unroll
+    for (int d = 0; d < ND; d++) {
+        T e = Ed * v[d] + kr * (grad[d][NV - 1] - Er * grad[d][0]);
+#pragma unroll
+        for (int i = 0; i < ND; i++) e += v[i] * (f[d][i + 1] - kr * dv[i][d]);
+        f[d][NV - 1] = e;
     }
 }
 
@@ -119,7 +183,7 @@ __device__ __forceinline__ void viscous_flux_add(const T *uin, const T grad[ND][
                                                  T fout[ND][ND + 2], const GasK<T> &g) {
     constexpr int NV = ND + 2;
     const T rho = uin[0], E = uin[NV - 1];
-    const T rcprho = T(1) / rho;
+    const T rcprho = rcp(rho);
     T vel[ND];
 #pragma unroll
     for (int i = 0; i < ND; i++) vel[i] = rcprho * uin[i + 1];
@@ -131,17 +195,7 @@ __device__ __forceinline__ void viscous_flux_add(const T *uin, const T grad[ND][
 #pragma unroll
         for (int d = 0; d < ND; d++) dv[i][d] = grad[d][i + 1] - vel[i] * grad[d][0];
 
-    T mu_c;
-    if (g.sutherland) {
-        T ke = 0;
-#pragma unroll
-        for (int i = 0; i < ND; i++) ke += vel[i] * vel[i];
-        const T cpT = g.gamma * (rcprho * E - T(0.5) * ke);
-        const T Trat = g.rcp_cpTref * cpT;
-        mu_c = g.mu_ctt * Trat * sqrt(Trat) / (cpT + g.cpTs);
-    } else {
-        mu_c = g.mu;
-    }
+    const T mu_c = viscosity<ND, T>(vel, rcprho * E, g);
 
     // Temperature derivatives (c_v dT/dx_d)
     T dT[ND];
@@ -186,18 +240,20 @@ __device__ __forceinline__ void viscous_flux_add(const T *uin, const T grad[ND][
 // pressure and the normal velocity.  Fewer operations than the full flux
 // followed by its projection, which matters where FP64 throughput bounds.
 template <int ND, typename T>
-__device__ __forceinline__ void inviscid_nflux(const T *s, const T *n, T *fn, T &p, T &vn,
-                                               T gamma) {
+__device__ __forceinline__ void inviscid_nflux(const T *s, const T *n, T *fn, T &p, T &vn, T v[ND],
+                                               T &inv, T gamma) {
     constexpr int NV = ND + 2;
-    const T invrho = T(1) / s[0], E = s[NV - 1];
+    const T E = s[NV - 1];
+    inv = rcp(s[0]);
     T dot = 0, mn = 0;
 #pragma unroll
     for (int i = 0; i < ND; i++) {
-        dot += s[i + 1] * s[i + 1];
+        v[i] = inv * s[i + 1];
+        dot += s[i + 1] * v[i];
         mn += s[i + 1] * n[i];
     }
-    p = (gamma - T(1)) * (E - T(0.5) * invrho * dot);
-    vn = invrho * mn;
+    p = (gamma - T(1)) * (E - T(0.5) * dot);
+    vn = inv * mn;
     fn[0] = mn;
 #pragma unroll
     for (int i = 0; i < ND; i++) fn[i + 1] = s[i + 1] * vn + p * n[i];
@@ -206,9 +262,55 @@ __device__ __forceinline__ void inviscid_nflux(const T *s, const T *n, T *fn, T 
 
 // The (negated-stress) viscous flux of uin along n, formed directly: the
 // normal component of viscous_flux_add's flux, momentum tau.n and energy
-// u.(tau.n) + kcoef dT.n, added to fn (mass untouched).
+// u.(tau.n) + kcoef dT.n, added to fn (mass untouched).  Of the gradient
+// only its normal derivatives g_n = n.grad, the transposed products
+// sum_j n_j grad_i(m_j) and the divergence enter:
+//     (tau.n)_i = mr (g_n(m_i) - v_i g_n(rho)
+//                     + sum_j n_j grad_i(m_j) - v.n grad_i(rho) - 2/3 div n_i)
+// with mr = -mu/rho and div = rho div(v): 60 operations in 3-D where forming
+// every velocity derivative first takes about 75.
 template <int ND, typename T>
 __device__ __forceinline__ void viscous_nflux_add(const T *uin, const T grad[ND][ND + 2],
+                                                  const T *n, T *fn, const GasK<T> &g) {
+    constexpr int NV = ND + 2;
+    const T inv = rcp(uin[0]), Er = inv * uin[NV - 1];
+    T v[ND], vn = 0, gn[NV], div = 0, divr = 0;
+#pragma unroll
+    for (int i = 0; i < ND; i++) {
+        v[i] = inv * uin[i + 1];
+        vn += v[i] * n[i];
+        div += grad[i][i + 1];
+        divr += v[i] * grad[i][0];
+    }
+    div -= divr;
+#pragma unroll
+    for (int q = 0; q < NV; q++) {
+        gn[q] = grad[0][q] * n[0];
+#pragma unroll
+        for (int d = 1; d < ND; d++) gn[q] += grad[d][q] * n[d];
+    }
+    const T mr = -viscosity<ND, T>(v, Er, g) * inv, kr = mr * g.gamma_pr;
+    const T c = T(-2.0 / 3.0) * div;
+    T vt = 0, dT = gn[NV - 1] - Er * gn[0];
+#pragma unroll
+    for (int i = 0; i < ND; i++) {
+        const T dvn = gn[i + 1] - v[i] * gn[0];
+        T t = dvn - vn * grad[i][0];
+#pragma unroll
+        for (int j = 0; j < ND; j++) t += n[j] * grad[i][j + 1];
+        t += c * n[i];
+        fn[i + 1] += mr * t;
+        vt += v[i] * t;
+        dT -= v[i] * dvn;
+    }
+    fn[NV - 1] += mr * vt + kr * dT;
+}
+
+// The same with every velocity derivative formed first: the shifted (mixed-
+// precision) form's, whose FP32 kernels are bound by bandwidth and whose
+// results keep the rounding of this order.
+template <int ND, typename T>
+__device__ __forceinline__ void viscous_nflux_shift_add(const T *uin, const T grad[ND][ND + 2],
                                                   const T *n, T *fn, const GasK<T> &g) {
     constexpr int NV = ND + 2;
     const T rho = uin[0], E = uin[NV - 1];
@@ -223,17 +325,7 @@ __device__ __forceinline__ void viscous_nflux_add(const T *uin, const T grad[ND]
 #pragma unroll
         for (int d = 0; d < ND; d++) dv[i][d] = grad[d][i + 1] - vel[i] * grad[d][0];
 
-    T mu_c;
-    if (g.sutherland) {
-        T ke = 0;
-#pragma unroll
-        for (int i = 0; i < ND; i++) ke += vel[i] * vel[i];
-        const T cpT = g.gamma * (rcprho * E - T(0.5) * ke);
-        const T Trat = g.rcp_cpTref * cpT;
-        mu_c = g.mu_ctt * Trat * sqrt(Trat) / (cpT + g.cpTs);
-    } else {
-        mu_c = g.mu;
-    }
+    const T mu_c = viscosity<ND, T>(vel, rcprho * E, g);
 
     // Normal temperature derivative (c_v dT/dn)
     T dTn = 0;
@@ -265,19 +357,35 @@ __device__ __forceinline__ void viscous_nflux_add(const T *uin, const T grad[ND]
     fn[NV - 1] += e;
 }
 
+// Rusanov flux along n; pen is added to the dissipation's half wave speed
+// (the LDG penalty, which acts on the same difference)
 template <int ND, typename T>
 __device__ __forceinline__ void rsolve_rusanov(const T *ul, const T *ur, const T *n, T *nf,
-                                               T gamma) {
+                                               T gamma, T pen = T(0)) {
     constexpr int NV = ND + 2;
-    T fl[NV], fr[NV], pl, pr, vnl, vnr;
-    inviscid_nflux<ND, T>(ul, n, fl, pl, vnl, gamma);
-    inviscid_nflux<ND, T>(ur, n, fr, pr, vnr, gamma);
-
-    // Maximum wave speed estimate (halved)
-    const T a = sqrt(T(0.25) * gamma * (pl + pr) / (ul[0] + ur[0])) + T(0.25) * fabs(vnl + vnr);
-
+    const T gm1 = gamma - T(1);
+    T mnl = 0, mnr = 0, dl = 0, dr = 0;
 #pragma unroll
-    for (int i = 0; i < NV; i++) nf[i] = T(0.5) * (fl[i] + fr[i]) + a * (ul[i] - ur[i]);
+    for (int i = 0; i < ND; i++) {
+        mnl += ul[i + 1] * n[i];
+        mnr += ur[i + 1] * n[i];
+        dl += ul[i + 1] * ul[i + 1];
+        dr += ur[i + 1] * ur[i + 1];
+    }
+    const T invl = rcp(ul[0]), invr = rcp(ur[0]);
+    const T pl = gm1 * (ul[NV - 1] - T(0.5) * (invl * dl));
+    const T pr = gm1 * (ur[NV - 1] - T(0.5) * (invr * dr));
+    const T vnl = invl * mnl, vnr = invr * mnr, ps = pl + pr;
+
+    // Maximum wave speed estimate (halved), and half normal velocities
+    const T a = root(quot(T(0.25) * gamma * ps, ul[0] + ur[0])) + T(0.25) * fabs(vnl + vnr) + pen;
+    const T hl = T(0.5) * vnl, hr = T(0.5) * vnr, hp = T(0.5) * ps;
+
+    nf[0] = T(0.5) * (mnl + mnr) + a * (ul[0] - ur[0]);
+#pragma unroll
+    for (int i = 0; i < ND; i++)
+        nf[i + 1] = hp * n[i] + hl * ul[i + 1] + hr * ur[i + 1] + a * (ul[i + 1] - ur[i + 1]);
+    nf[NV - 1] = hl * (ul[NV - 1] + pl) + hr * (ur[NV - 1] + pr) + a * (ul[NV - 1] - ur[NV - 1]);
 }
 
 // Inviscid flux, less the reference state's, from the transformed input
@@ -389,39 +497,33 @@ template <int ND, typename T>
 __device__ __forceinline__ void rsolve_hllc(const T *ul, const T *ur, const T *n, T *nf,
                                             T gamma) {
     constexpr int NV = ND + 2;
-    T fl[ND][NV], fr[ND][NV], vl[ND], vr[ND], pl, pr;
-    inviscid_flux<ND, T>(ul, fl, pl, vl, gamma);
-    inviscid_flux<ND, T>(ur, fr, pr, vr, gamma);
+    T fl[NV], fr[NV], vl[ND], vr[ND], pl, pr, nvl, nvr, invl, invr;
+    inviscid_nflux<ND, T>(ul, n, fl, pl, nvl, vl, invl, gamma);
+    inviscid_nflux<ND, T>(ur, n, fr, pr, nvr, vr, invr, gamma);
 
-    T nvl = 0, nvr = 0;
-#pragma unroll
-    for (int i = 0; i < ND; i++) {
-        nvl += n[i] * vl[i];
-        nvr += n[i] * vr[i];
-    }
-    const T al = sqrt(gamma * pl / ul[0]), ar = sqrt(gamma * pr / ur[0]);
-    const T sql = sqrt(ul[0]), sqr = sqrt(ur[0]);
+    const T al = root(gamma * pl * invl), ar = root(gamma * pr * invr);
+    const T sql = root(ul[0]), sqr = root(ur[0]);
 
     // Roe averages of the normal velocity, enthalpy and velocity
-    const T nv = (sql * nvl + sqr * nvr) / (sql + sqr);
-    const T H = (sql * (pr + ur[NV - 1]) + sqr * (pl + ul[NV - 1])) / (sql * ur[0] + sqr * ul[0]);
-    const T inv_rar = T(1) / (sql + sqr);
+    const T inv_rar = rcp(sql + sqr);
+    const T nv = (sql * nvl + sqr * nvr) * inv_rar;
+    const T H = quot(sql * (pr + ur[NV - 1]) + sqr * (pl + ul[NV - 1]), sql * ur[0] + sqr * ul[0]);
     T qq = 0;
 #pragma unroll
     for (int i = 0; i < ND; i++) {
         const T va = (vl[i] * sql + vr[i] * sqr) * inv_rar;
         qq += va * va;
     }
-    const T a = sqrt((gamma - T(1)) * (H - T(0.5) * qq));
+    const T a = root((gamma - T(1)) * (H - T(0.5) * qq));
 
     // Wave speed estimates and the contact speed
     const T sl = fmin(nv - a, nvl - al);
     const T sr = fmax(nv + a, nvr + ar);
-    const T sstar = (pr - pl + ul[0] * nvl * (sl - nvl) - ur[0] * nvr * (sr - nvr)) /
-                    (ul[0] * (sl - nvl) - ur[0] * (sr - nvr));
+    const T sdl = sl - nvl, sdr = sr - nvr;
+    const T sstar = quot(pr - pl + ul[0] * nvl * sdl - ur[0] * nvr * sdr, ul[0] * sdl - ur[0] * sdr);
 
-    const T ul_com = (sl - nvl) / (sl - sstar);
-    const T ur_com = (sr - nvr) / (sr - sstar);
+    const T ul_com = quot(sdl, sl - sstar);
+    const T ur_com = quot(sdr, sr - sstar);
 
     T usl[NV], usr[NV];
     usl[0] = ul_com * ul[0];
@@ -431,17 +533,12 @@ __device__ __forceinline__ void rsolve_hllc(const T *ul, const T *ur, const T *n
         usl[i + 1] = usl[0] * (vl[i] + (sstar - nvl) * n[i]);
         usr[i + 1] = usr[0] * (vr[i] + (sstar - nvr) * n[i]);
     }
-    usl[NV - 1] = ul_com * (ul[NV - 1] + (sstar - nvl) * (ul[0] * sstar + pl / (sl - nvl)));
-    usr[NV - 1] = ur_com * (ur[NV - 1] + (sstar - nvr) * (ur[0] * sstar + pr / (sr - nvr)));
+    usl[NV - 1] = ul_com * (ul[NV - 1] + (sstar - nvl) * (ul[0] * sstar + quot(pl, sdl)));
+    usr[NV - 1] = ur_com * (ur[NV - 1] + (sstar - nvr) * (ur[0] * sstar + quot(pr, sdr)));
 
 #pragma unroll
     for (int i = 0; i < NV; i++) {
-        T nf_fl = 0, nf_fr = 0;
-#pragma unroll
-        for (int j = 0; j < ND; j++) {
-            nf_fl += n[j] * fl[j][i];
-            nf_fr += n[j] * fr[j][i];
-        }
+        const T nf_fl = fl[i], nf_fr = fr[i];
         const T nf_fsl = nf_fl + sl * (usl[i] - ul[i]);
         const T nf_fsr = nf_fr + sr * (usr[i] - ur[i]);
         nf[i] = (T(0) <= sl) ? nf_fl
@@ -458,40 +555,29 @@ template <int ND, typename T>
 __device__ __forceinline__ void rsolve_hll(const T *ul, const T *ur, const T *n, T *nf,
                                            T gamma) {
     constexpr int NV = ND + 2;
-    T fl[ND][NV], fr[ND][NV], vl[ND], vr[ND], pl, pr;
-    inviscid_flux<ND, T>(ul, fl, pl, vl, gamma);
-    inviscid_flux<ND, T>(ur, fr, pr, vr, gamma);
+    T fl[NV], fr[NV], vl[ND], vr[ND], pl, pr, nvl, nvr, invl, invr;
+    inviscid_nflux<ND, T>(ul, n, fl, pl, nvl, vl, invl, gamma);
+    inviscid_nflux<ND, T>(ur, n, fr, pr, nvr, vr, invr, gamma);
 
-    T nvl = 0, nvr = 0;
-#pragma unroll
-    for (int i = 0; i < ND; i++) {
-        nvl += n[i] * vl[i];
-        nvr += n[i] * vr[i];
-    }
-    const T ar = sqrt(gamma * pr / ur[0]);
-    const T sql = sqrt(ul[0]), sqr = sqrt(ur[0]);
-    const T nv = (sql * nvl + sqr * nvr) / (sql + sqr);
-    const T H = (sql * (pr + ur[NV - 1]) + sqr * (pl + ul[NV - 1])) / (sql * ur[0] + sqr * ul[0]);
-    const T inv_rar = T(1) / (sql + sqr);
+    const T ar = root(gamma * pr * invr);
+    const T sql = root(ul[0]), sqr = root(ur[0]);
+    const T inv_rar = rcp(sql + sqr);
+    const T nv = (sql * nvl + sqr * nvr) * inv_rar;
+    const T H = quot(sql * (pr + ur[NV - 1]) + sqr * (pl + ul[NV - 1]), sql * ur[0] + sqr * ul[0]);
     T qq = 0;
 #pragma unroll
     for (int i = 0; i < ND; i++) {
         const T va = (vl[i] * sql + vr[i] * sqr) * inv_rar;
         qq += va * va;
     }
-    const T a = sqrt((gamma - T(1)) * (H - T(0.5) * qq));
+    const T a = root((gamma - T(1)) * (H - T(0.5) * qq));
     const T sl = fmin(nv - a, nvl - ar);
     const T sr = fmax(nv + a, nvr + ar);
-    const T rcpsrsl = T(1) / (sr - sl);
+    const T rcpsrsl = rcp(sr - sl);
 
 #pragma unroll
     for (int i = 0; i < NV; i++) {
-        T nf_fl = 0, nf_fr = 0;
-#pragma unroll
-        for (int j = 0; j < ND; j++) {
-            nf_fl += n[j] * fl[j][i];
-            nf_fr += n[j] * fr[j][i];
-        }
+        const T nf_fl = fl[i], nf_fr = fr[i];
         const T sub = (sr * nf_fl - sl * nf_fr + sl * sr * (ur[i] - ul[i])) * rcpsrsl;
         nf[i] = (T(0) <= sl) ? nf_fl : (T(0) >= sr) ? nf_fr : sub;
     }

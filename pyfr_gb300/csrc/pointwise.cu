@@ -39,23 +39,34 @@ struct ElemGeom {
 };
 
 // Geometry modes (the `linear` argument of the element kernels)
-enum { GEOM_STORED = 0, GEOM_VERTICES = 1, GEOM_PER_ELEMENT = 2 };
+enum { GEOM_STORED = 0, GEOM_VERTICES = 1, GEOM_PER_ELEMENT = 2, GEOM_DIAGONAL = 3 };
 
 // Metric terms at solution point `upt` of element `e`: from the vertices
 // (GEOM_VERTICES, multilinear elements), from the stored per-point smats
 // and 1/|J| (GEOM_STORED), or from one stored set per element
 // (GEOM_PER_ELEMENT: affine elements, whose Jacobian is constant, keep
 // only the rows of their first point: io-shapes (ndims, 1, ndims, neles)
-// and (1, neles)).
-template <int ND, typename T>
+// and (1, neles)).  DIAG (GEOM_DIAGONAL: per-element terms of elements
+// aligned with the axes, whose off-diagonal S are zero) is a compile-time
+// form of the kernels: the two transforms then take 30 FP64 operations a
+// point in 3-D instead of 99 (tflux_ns at 26^3 elements, p = 3: 416 us
+// before both the shared flux expressions and this form).
+template <int ND, typename T, bool DIAG = false>
 __device__ __forceinline__ void elem_metrics(const ElemGeom<T> &g, int nupts, int upt,
                                              int64_t e, T s[ND][ND], T &rcpdjac,
                                              bool need_rcp) {
-    if (g.linear == GEOM_PER_ELEMENT) {
+    if (DIAG || g.linear >= GEOM_PER_ELEMENT) {
         nupts = 1;
         upt = 0;
     }
-    if (g.linear == GEOM_VERTICES) {
+    if (DIAG) {
+#pragma unroll
+        for (int i = 0; i < ND; i++)
+#pragma unroll
+            for (int j = 0; j < ND; j++)
+                s[i][j] = i == j ? g.smats[(int64_t)i * g.lds + soa_off(e, i, ND)] : T(0);
+        rcpdjac = need_rcp ? g.rcpdjac[e] : T(0);
+    } else if (g.linear == GEOM_VERTICES) {
         T V[1 << ND][ND], x[ND], d;
 #pragma unroll
         for (int v = 0; v < (1 << ND); v++)
@@ -75,7 +86,29 @@ __device__ __forceinline__ void elem_metrics(const ElemGeom<T> &g, int nupts, in
     }
 }
 
-template <int ND, typename T>
+// f = S ft, the flux in reference space (DIAG: S is diagonal)
+template <int ND, typename T, bool DIAG>
+__device__ __forceinline__ void store_tflux(T *__restrict__ f, int64_t ldf, int nupts, int upt,
+                                            int64_t e, const T s[ND][ND],
+                                            const T ft[ND][ND + 2]) {
+    constexpr int NV = ND + 2;
+#pragma unroll
+    for (int i = 0; i < ND; i++)
+#pragma unroll
+        for (int j = 0; j < NV; j++) {
+            T acc;
+            if (DIAG) {
+                acc = s[i][i] * ft[i][j];
+            } else {
+                acc = 0;
+#pragma unroll
+                for (int k = 0; k < ND; k++) acc += s[i][k] * ft[k][j];
+            }
+            f[(int64_t)(i * nupts + upt) * ldf + soa_off(e, j, NV)] = acc;
+        }
+}
+
+template <int ND, typename T, bool DIAG>
 __global__ void __launch_bounds__(PW_BLOCK)
 tflux_euler_kernel(int nupts, int64_t neles, T gamma, const T *__restrict__ u, int64_t ldu,
                    T *__restrict__ f, int64_t ldf, ElemGeom<T> geo) {
@@ -85,7 +118,7 @@ tflux_euler_kernel(int nupts, int64_t neles, T gamma, const T *__restrict__ u, i
     if (e >= neles) return;
 
     T s[ND][ND], rcp;
-    elem_metrics<ND, T>(geo, nupts, upt, e, s, rcp, false);
+    elem_metrics<ND, T, DIAG>(geo, nupts, upt, e, s, rcp, false);
 
     T uu[NV];
 #pragma unroll
@@ -94,20 +127,12 @@ tflux_euler_kernel(int nupts, int64_t neles, T gamma, const T *__restrict__ u, i
     T ft[ND][NV], p, vel[ND];
     b200::inviscid_flux<ND, T>(uu, ft, p, vel, gamma);
 
-#pragma unroll
-    for (int i = 0; i < ND; i++)
-#pragma unroll
-        for (int j = 0; j < NV; j++) {
-            T acc = 0;
-#pragma unroll
-            for (int k = 0; k < ND; k++) acc += s[i][k] * ft[k][j];
-            f[(int64_t)(i * nupts + upt) * ldf + soa_off(e, j, NV)] = acc;
-        }
+    store_tflux<ND, T, DIAG>(f, ldf, nupts, upt, e, s, ft);
 }
 
 // Euler transformed flux on shifted inputs q = T(u - u_ref) (b200::Gas):
 // the flux less the reference state's, formed from the perturbation
-template <int ND, typename T, bool MOVING>
+template <int ND, typename T, bool MOVING, bool DIAG>
 __global__ void __launch_bounds__(PW_BLOCK)
 tflux_euler_shift_kernel(int nupts, int64_t neles, b200::GasK<T> gas, const T *__restrict__ u,
                          int64_t ldu, T *__restrict__ f, int64_t ldf, ElemGeom<T> geo) {
@@ -117,7 +142,7 @@ tflux_euler_shift_kernel(int nupts, int64_t neles, b200::GasK<T> gas, const T *_
     if (e >= neles) return;
 
     T s[ND][ND], rcp;
-    elem_metrics<ND, T>(geo, nupts, upt, e, s, rcp, false);
+    elem_metrics<ND, T, DIAG>(geo, nupts, upt, e, s, rcp, false);
 
     T uu[NV];
 #pragma unroll
@@ -126,15 +151,7 @@ tflux_euler_shift_kernel(int nupts, int64_t neles, b200::GasK<T> gas, const T *_
     T ft[ND][NV], p, vel[ND], uf[NV];
     b200::inviscid_flux_shift<ND, T, MOVING>(uu, ft, p, vel, uf, gas);
 
-#pragma unroll
-    for (int i = 0; i < ND; i++)
-#pragma unroll
-        for (int j = 0; j < NV; j++) {
-            T acc = 0;
-#pragma unroll
-            for (int k = 0; k < ND; k++) acc += s[i][k] * ft[k][j];
-            f[(int64_t)(i * nupts + upt) * ldf + soa_off(e, j, NV)] = acc;
-        }
+    store_tflux<ND, T, DIAG>(f, ldf, nupts, upt, e, s, ft);
 }
 
 // Largest characteristic wave speed of each element in reference space,
@@ -192,7 +209,7 @@ wavespeed_kernel(int nupts, int64_t neles, b200::GasK<T> gas, const T *__restric
     wspd[e] = lmax;
 }
 
-template <int ND, typename T>
+template <int ND, typename T, bool DIAG>
 __global__ void __launch_bounds__(PW_BLOCK)
 tflux_ns_kernel(int nupts, int64_t neles, b200::GasK<T> gas, const T *__restrict__ u, int64_t ldu,
                 T *__restrict__ f, int64_t ldf, T *__restrict__ gradu, int64_t ldg,
@@ -209,7 +226,7 @@ tflux_ns_kernel(int nupts, int64_t neles, b200::GasK<T> gas, const T *__restrict
     // flux replaces
     const bool fused = gradu != nullptr;
     T s[ND][ND], rcp;
-    elem_metrics<ND, T>(geo, nupts, upt, e, s, rcp, fused);
+    elem_metrics<ND, T, DIAG>(geo, nupts, upt, e, s, rcp, fused);
 
     T gr[ND][NV];
     if (fused) {
@@ -219,15 +236,27 @@ tflux_ns_kernel(int nupts, int64_t neles, b200::GasK<T> gas, const T *__restrict
 #pragma unroll
             for (int v = 0; v < NV; v++) tg[d][v] = gradu[(int64_t)(d * nupts + upt) * ldg + soa_off(e, v, NV)];
 #pragma unroll
-        for (int i = 0; i < ND; i++)
+        for (int i = 0; i < ND; i++) {
+            // (in FP64 1/|J| goes into the terms, nine products instead of
+            // fifteen; FP32, where bandwidth bounds, scales the sum)
+            constexpr bool PRE = sizeof(T) == 8;
+            T c[ND];
+#pragma unroll
+            for (int k = 0; k < ND; k++) c[k] = DIAG && k != i ? T(0) : PRE ? rcp * s[k][i] : s[k][i];
 #pragma unroll
             for (int j = 0; j < NV; j++) {
-                T acc = 0;
+                T acc;
+                if (DIAG) {
+                    acc = c[i] * tg[i][j];
+                } else {
+                    acc = 0;
 #pragma unroll
-                for (int k = 0; k < ND; k++) acc += s[k][i] * tg[k][j];
-                gr[i][j] = rcp * acc;
+                    for (int k = 0; k < ND; k++) acc += c[k] * tg[k][j];
+                }
+                gr[i][j] = PRE ? acc : rcp * acc;
                 if (gradwb) gradu[(int64_t)(i * nupts + upt) * ldg + soa_off(e, j, NV)] = gr[i][j];
             }
+        }
     } else {
 #pragma unroll
         for (int d = 0; d < ND; d++)
@@ -239,15 +268,14 @@ tflux_ns_kernel(int nupts, int64_t neles, b200::GasK<T> gas, const T *__restrict
 #pragma unroll
     for (int v = 0; v < NV; v++) uu[v] = u[upt * ldu + soa_off(e, v, NV)];
 
-    T ft[ND][NV], p, vel[ND];
+    T ft[ND][NV];
     if (gas.shifted) {
-        T uf[NV], gu[ND][NV];
+        T uf[NV], gu[ND][NV], p, vel[ND];
         b200::inviscid_flux_shift<ND, T>(uu, ft, p, vel, uf, gas);
         b200::unshift_grad<ND, T>(gr, gu, gas);
         b200::viscous_flux_add<ND, T>(uf, gu, ft, gas);
     } else {
-        b200::inviscid_flux<ND, T>(uu, ft, p, vel, gas.gamma);
-        b200::viscous_flux_add<ND, T>(uu, gr, ft, gas);
+        b200::ns_flux<ND, T>(uu, gr, ft, gas);
     }
 
     // Artificial viscosity (pyfr/solvers/baseadvecdiff/kernels/
@@ -260,15 +288,7 @@ tflux_ns_kernel(int nupts, int64_t neles, b200::GasK<T> gas, const T *__restrict
             for (int v = 0; v < NV; v++) ft[d][v] -= a * gr[d][v];
     }
 
-#pragma unroll
-    for (int i = 0; i < ND; i++)
-#pragma unroll
-        for (int j = 0; j < NV; j++) {
-            T acc = 0;
-#pragma unroll
-            for (int k = 0; k < ND; k++) acc += s[i][k] * ft[k][j];
-            f[(int64_t)(i * nupts + upt) * ldf + soa_off(e, j, NV)] = acc;
-        }
+    store_tflux<ND, T, DIAG>(f, ldf, nupts, upt, e, s, ft);
 }
 
 template <int ND, typename T>
@@ -488,8 +508,9 @@ intcflux_euler_kernel(int64_t n, T gamma, T p_min, ScalView<T> vl, ScalView<T> v
 
 #pragma unroll
     for (int v = 0; v < NV; v++) {
-        pl[v * B200_SOASZ] = mag * fn[v];
-        pr[v * B200_SOASZ] = -mag * fn[v];
+        const T fc = mag * fn[v];
+        pl[v * B200_SOASZ] = fc;
+        pr[v * B200_SOASZ] = -fc;
     }
 }
 
@@ -519,8 +540,9 @@ intcflux_euler_shift_kernel(int64_t n, b200::GasK<T> gas, ScalView<T> vl, ScalVi
 
 #pragma unroll
     for (int v = 0; v < NV; v++) {
-        pl[v * B200_SOASZ] = mag * fn[v];
-        pr[v * B200_SOASZ] = -mag * fn[v];
+        const T fc = mag * fn[v];
+        pl[v * B200_SOASZ] = fc;
+        pr[v * B200_SOASZ] = -fc;
     }
 }
 
@@ -592,12 +614,17 @@ intcflux_ns_kernel(int64_t n, b200::GasK<T> gas, T beta, T tau, ScalView<T> vl, 
     const T mag = pair_normal<ND, T>(nl, ldn, i, nl_unit, nn);
 
     // Riemann flux; with a shifted input the viscous terms need the full
-    // states, which the shifted flux reconstructs
+    // states, which the shifted flux reconstructs.  The unshifted Rusanov
+    // flux takes the LDG penalty with its dissipation.
+    const bool penalty = tau != T(0) && (RS != b200::RS_RUSANOV || gas.shifted);
     T fi[NV], ufl[NV], ufr[NV];
     if (RS == b200::RS_RUSANOV && gas.shifted) {
         b200::rsolve_rusanov_shift<ND, T>(ul, ur, nn, fi, ufl, ufr, gas);
     } else {
-        b200::rsolve_t<RS, ND, T>(ul, ur, nn, fi, gas.gamma, gas.p_min);
+        if constexpr (RS == b200::RS_RUSANOV)
+            b200::rsolve_rusanov<ND, T>(ul, ur, nn, fi, gas.gamma, tau);
+        else
+            b200::rsolve_t<RS, ND, T>(ul, ur, nn, fi, gas.gamma, gas.p_min);
 #pragma unroll
         for (int v = 0; v < NV; v++) {
             ufl[v] = ul[v];
@@ -626,7 +653,7 @@ intcflux_ns_kernel(int64_t n, b200::GasK<T> gas, T beta, T tau, ScalView<T> vl, 
         if (gas.shifted) {
             T gu[ND][NV];
             b200::unshift_grad<ND, T>(gg, gu, gas);
-            b200::viscous_nflux_add<ND, T>(ufl, gu, nn, nfl, gas);
+            b200::viscous_nflux_shift_add<ND, T>(ufl, gu, nn, nfl, gas);
         } else {
             b200::viscous_nflux_add<ND, T>(ufl, gg, nn, nfl, gas);
             if (va.base) {
@@ -652,7 +679,7 @@ intcflux_ns_kernel(int64_t n, b200::GasK<T> gas, T beta, T tau, ScalView<T> vl, 
         if (gas.shifted) {
             T gu[ND][NV];
             b200::unshift_grad<ND, T>(gg, gu, gas);
-            b200::viscous_nflux_add<ND, T>(ufr, gu, nn, nfr, gas);
+            b200::viscous_nflux_shift_add<ND, T>(ufr, gu, nn, nfr, gas);
         } else {
             b200::viscous_nflux_add<ND, T>(ufr, gg, nn, nfr, gas);
             if (va.base) {
@@ -676,10 +703,11 @@ intcflux_ns_kernel(int64_t n, b200::GasK<T> gas, T beta, T tau, ScalView<T> vl, 
             fvc = nfl[v];
         else
             fvc = (T(0.5) + beta) * nfl[v] + (T(0.5) - beta) * nfr[v];
-        if (tau != T(0)) fvc += tau * (ul[v] - ur[v]);
+        if (penalty) fvc += tau * (ul[v] - ur[v]);
 
-        pl[v * B200_SOASZ] = mag * (fi[v] + fvc);
-        pr[v * B200_SOASZ] = -mag * (fi[v] + fvc);
+        const T fc = mag * (fi[v] + fvc);
+        pl[v * B200_SOASZ] = fc;
+        pr[v * B200_SOASZ] = -fc;
     }
 }
 
@@ -743,9 +771,29 @@ ElemGeom<T> make_geom(int linear, const T *smats, int64_t lds, const T *rcpdjac,
     return g;
 }
 
+// A launch over the number of dimensions and the diagonal form of the
+// metrics, both compile-time: fn(integral constants); false for ndims other
+// than 2 or 3
+template <typename F>
+bool with_form(int ndims, int linear, F &&fn) {
+    using b2 = std::integral_constant<int, 2>;
+    using b3 = std::integral_constant<int, 3>;
+    if (ndims == 2 && linear == GEOM_DIAGONAL)
+        fn(b2(), std::true_type());
+    else if (ndims == 2)
+        fn(b2(), std::false_type());
+    else if (ndims == 3 && linear == GEOM_DIAGONAL)
+        fn(b3(), std::true_type());
+    else if (ndims == 3)
+        fn(b3(), std::false_type());
+    else
+        return false;
+    return true;
+}
+
 int check_geom(int linear, const void *smats, const void *rcpdjac, const void *verts,
                const void *upts, bool need_rcp) {
-    if (linear < GEOM_STORED || linear > GEOM_PER_ELEMENT)
+    if (linear < GEOM_STORED || linear > GEOM_DIAGONAL)
         return b200::set_error(B200_ERR_ARG, "unknown geometry mode %d", linear);
     if (linear == GEOM_VERTICES && (!verts || !upts))
         return b200::set_error(B200_ERR_ARG, "linear elements need verts and upts");
@@ -763,12 +811,10 @@ int tflux_euler(int ndims, int nupts, int64_t neles, int linear, double gamma, c
     if (rc) return rc;
     auto geo = make_geom<T>(linear, smats, lds, nullptr, 0, verts, ldv, upts, ldup);
     dim3 grid(b200::ceil_div(neles, PW_BLOCK), nupts);
-    if (ndims == 2)
-        tflux_euler_kernel<2, T><<<grid, PW_BLOCK, 0, st>>>(nupts, neles, (T)gamma, u, ldu, f, ldf, geo);
-    else if (ndims == 3)
-        tflux_euler_kernel<3, T><<<grid, PW_BLOCK, 0, st>>>(nupts, neles, (T)gamma, u, ldu, f, ldf, geo);
-    else
-        return b200::set_error(B200_ERR_ARG, "tflux: ndims must be 2 or 3");
+    const bool ok = with_form(ndims, linear, [&](auto nd, auto diag) {
+        tflux_euler_kernel<nd(), T, diag()><<<grid, PW_BLOCK, 0, st>>>(nupts, neles, (T)gamma, u, ldu, f, ldf, geo);
+    });
+    if (!ok) return b200::set_error(B200_ERR_ARG, "tflux: ndims must be 2 or 3");
     B200_CHECK_LAUNCH("tflux_euler");
     return B200_OK;
 }
@@ -815,12 +861,10 @@ int tflux_ns(int ndims, int nupts, int64_t neles, int linear, const b200_gas_t *
         return b200::set_error(B200_ERR_UNSUPPORTED,
                                "tflux_ns: the reference state must be at rest");
     dim3 grid(b200::ceil_div(neles, PW_BLOCK), nupts);
-    if (ndims == 2)
-        tflux_ns_kernel<2, T><<<grid, PW_BLOCK, 0, st>>>(nupts, neles, g, u, ldu, f, ldf, gradu, ldg, geo, av, lda, gradwb);
-    else if (ndims == 3)
-        tflux_ns_kernel<3, T><<<grid, PW_BLOCK, 0, st>>>(nupts, neles, g, u, ldu, f, ldf, gradu, ldg, geo, av, lda, gradwb);
-    else
-        return b200::set_error(B200_ERR_ARG, "tflux_ns: ndims must be 2 or 3");
+    const bool ok = with_form(ndims, linear, [&](auto nd, auto diag) {
+        tflux_ns_kernel<nd(), T, diag()><<<grid, PW_BLOCK, 0, st>>>(nupts, neles, g, u, ldu, f, ldf, gradu, ldg, geo, av, lda, gradwb);
+    });
+    if (!ok) return b200::set_error(B200_ERR_ARG, "tflux_ns: ndims must be 2 or 3");
     B200_CHECK_LAUNCH("tflux_ns");
     return B200_OK;
 }
@@ -876,16 +920,13 @@ int tflux_euler_shift(int ndims, int nupts, int64_t neles, int linear, const b20
     auto geo = make_geom<T>(linear, smats, lds, nullptr, 0, verts, ldv, upts, ldup);
     const auto g = b200::gas_consts<T>(*reinterpret_cast<const Gas *>(gas));
     dim3 grid(b200::ceil_div(neles, PW_BLOCK), nupts);
-    if (ndims == 2 && g.moving)
-        tflux_euler_shift_kernel<2, T, true><<<grid, PW_BLOCK, 0, st>>>(nupts, neles, g, u, ldu, f, ldf, geo);
-    else if (ndims == 2)
-        tflux_euler_shift_kernel<2, T, false><<<grid, PW_BLOCK, 0, st>>>(nupts, neles, g, u, ldu, f, ldf, geo);
-    else if (ndims == 3 && g.moving)
-        tflux_euler_shift_kernel<3, T, true><<<grid, PW_BLOCK, 0, st>>>(nupts, neles, g, u, ldu, f, ldf, geo);
-    else if (ndims == 3)
-        tflux_euler_shift_kernel<3, T, false><<<grid, PW_BLOCK, 0, st>>>(nupts, neles, g, u, ldu, f, ldf, geo);
-    else
-        return b200::set_error(B200_ERR_ARG, "tflux: ndims must be 2 or 3");
+    const bool ok = with_form(ndims, linear, [&](auto nd, auto diag) {
+        if (g.moving)
+            tflux_euler_shift_kernel<nd(), T, true, diag()><<<grid, PW_BLOCK, 0, st>>>(nupts, neles, g, u, ldu, f, ldf, geo);
+        else
+            tflux_euler_shift_kernel<nd(), T, false, diag()><<<grid, PW_BLOCK, 0, st>>>(nupts, neles, g, u, ldu, f, ldf, geo);
+    });
+    if (!ok) return b200::set_error(B200_ERR_ARG, "tflux: ndims must be 2 or 3");
     B200_CHECK_LAUNCH("tflux_euler_shift");
     return B200_OK;
 }
