@@ -284,6 +284,50 @@ int b200_mul_tc_terms(void *handle, int *nterms);
  * elements whose edges are along the axes: the off-diagonal smats are taken
  * as zero and not read. */
 
+/* Tensor-product elements (quadrilaterals, hexahedra) by the lines of their
+ * points: one handle per shape and order from the one-dimensional matrices,
+ * row-major, q points a line (3 to 5): grad (q x (q + 2)), the corrected
+ * derivative of (u, common solution at the low and high end); interp (2 x q),
+ * the values at both ends; div (q x (q + 2)), the derivative less its own
+ * lift and the lift of the common flux at both ends.  fpt[(d*lines + l)*2 + end]
+ * is the flux point at that end of line l of direction d; point i of line l is
+ * l*q + i (d = 0), (l/q)*q*q + l%q + i*q (d = 1), l + i*q*q (d = 2).
+ * te_interp: u -> flux points.  te_gradflux_ns: gradient, its values at the
+ * flux points of the faces in facemask (bit 2d + end; rows k*nfpts + point of
+ * gf; with refgrad in reference space), and r = the divergence of the transformed Navier-Stokes flux less its
+ * own lift; c the common solution, which may be gf's first nfpts rows; r may
+ * be u.  te_lift: r = -rcpdjac (r + lift of fc).  te_euler: r = -(1/|J|) times
+ * the corrected divergence of the Euler flux of u; r may be u.  linear: 0, 2 or
+ * 3 of the geometry modes; ldj = 0 takes one rcpdjac per element. */
+int b200_te_create(int ndims, int q, const double *grad, const double *interp,
+                   const double *div, const int *fpt, void **handle);
+int b200_te_destroy(void *handle);
+int b200_te_interp_f64(void *handle, int64_t neles, const double *u, int64_t ldu, double *f,
+                       int64_t ldf, void *stream);
+int b200_te_interp_f32(void *handle, int64_t neles, const float *u, int64_t ldu, float *f,
+                       int64_t ldf, void *stream);
+int b200_te_gradflux_ns_f64(void *handle, int64_t neles, int linear, const b200_gas_t *gas,
+                            const double *u, int64_t ldu, const double *c, int64_t ldc,
+                            double *gf, int64_t ldg, unsigned facemask, int refgrad,
+                            const double *smats, int64_t lds, const double *rcpdjac, int64_t ldj, double *r,
+                            int64_t ldr, void *stream);
+int b200_te_gradflux_ns_f32(void *handle, int64_t neles, int linear, const b200_gas_t *gas,
+                            const float *u, int64_t ldu, const float *c, int64_t ldc, float *gf,
+                            int64_t ldg, unsigned facemask, int refgrad, const float *smats, int64_t lds,
+                            const float *rcpdjac, int64_t ldj, float *r, int64_t ldr,
+                            void *stream);
+int b200_te_euler_f64(void *handle, int64_t neles, int linear, double gamma, const double *u,
+                      int64_t ldu, const double *fc, int64_t ldf, const double *smats,
+                      int64_t lds, const double *rcpdjac, int64_t ldj, double *r, int64_t ldr,
+                      void *stream);
+int b200_te_euler_f32(void *handle, int64_t neles, int linear, double gamma, const float *u,
+                      int64_t ldu, const float *fc, int64_t ldf, const float *smats, int64_t lds,
+                      const float *rcpdjac, int64_t ldj, float *r, int64_t ldr, void *stream);
+int b200_te_lift_f64(void *handle, int64_t neles, const double *fc, int64_t ldf,
+                     const double *rcpdjac, int64_t ldj, double *r, int64_t ldr, void *stream);
+int b200_te_lift_f32(void *handle, int64_t neles, const float *fc, int64_t ldf,
+                     const float *rcpdjac, int64_t ldj, float *r, int64_t ldr, void *stream);
+
 /* Euler transformed flux; pyfr/solvers/euler/kernels/tflux.mako:8-30,
  * provider call pyfr/solvers/euler/elements.py:149-206. */
 int b200_tflux_euler_f64(int ndims, int nupts, int64_t neles, int linear, double gamma,

@@ -180,12 +180,23 @@ class B200Backend:
         self.ordered_meta_kernel_cls = types.OrderedMetaKernel
         self.unordered_meta_kernel_cls = types.UnorderedMetaKernel
 
-        from pyfr_gb300.backend import blasext, fused, mul, pointwise
+        # Element kernels of tensor-product elements (tensorele.py) where
+        # they apply; 'general': the operator applies and pointwise kernels
+        # one by one
+        self.element_kernels = cfg.get('backend-b200', 'element-kernels',
+                                       'auto')
+        if self.element_kernels not in {'auto', 'general'}:
+            raise ValueError('element-kernels must be auto or general')
+
+        from pyfr_gb300.backend import (blasext, fused, mul, pointwise,
+                                        tensorele)
         self._providers = [pointwise.PointwiseKernelProvider(self),
                            blasext.BlasExtKernels(self),
                            mul.TensorMulKernels(self),
-                           mul.MulKernels(self)]
+                           mul.MulKernels(self),
+                           tensorele.TensorElementKernels(self)]
         self.pointwise = self._providers[0]
+        self.tensor_elements = self._providers[-1]
         self._fuser = fused.Fuser(self)
         self._status = None
 

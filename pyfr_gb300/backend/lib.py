@@ -157,6 +157,12 @@ def _sig_pointwise(fp):
         'entropylocal': [C.POINTER(EF), i64, vp, i64, vp, i64, vp, i64, vp],
         'intcent': [i64, vp, vp, vp, vp, i32, vp],
         'reduce_max': [i64, vp, vp, vp, vp],
+        'te_interp': [vp, i64, vp, i64, vp, i64, vp],
+        'te_gradflux_ns': [vp, i64, i32, C.POINTER(Gas), vp, i64, vp, i64, vp,
+                           i64, C.c_uint, i32, vp, i64, vp, i64, vp, i64, vp],
+        'te_euler': [vp, i64, i32, f64, vp, i64, vp, i64, vp, i64, vp, i64, vp,
+                     i64, vp],
+        'te_lift': [vp, i64, vp, i64, vp, i64, vp, i64, vp],
     }
 
 
@@ -190,6 +196,8 @@ _SIGS = {
     'b200_graph_end_capture': [vp, C.POINTER(vp)],
     'b200_graph_launch': [vp, vp],
     'b200_graph_destroy': [vp],
+    'b200_te_create': [i32, i32, pd, pd, pd, C.POINTER(i32), C.POINTER(vp)],
+    'b200_te_destroy': [vp],
     'b200_mul_create': [pd, i32, i32, C.POINTER(vp)],
     'b200_mul_nnz': [vp, C.POINTER(i32)],
     'b200_mul_destroy': [vp],

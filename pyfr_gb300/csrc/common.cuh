@@ -112,7 +112,7 @@ __device__ __forceinline__ double rcp_f64(double d) {
 // operations.  Operands outside mid_range, negative ones, zeros, infinities
 // and NaNs take the IEEE square root.
 __device__ __forceinline__ double sqrt_f64(double x) {
-    if (!mid_range(x) || x < 0) return sqrt(x);
+    if (!mid_range(x) || __double2hiint(x) < 0) return sqrt(x);
     float y0;
     asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y0) : "f"(trunc_f64(x)));
     const double y2 = widen_normal(0.5f * y0);

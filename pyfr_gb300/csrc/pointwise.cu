@@ -18,73 +18,25 @@
 //   intcflux (NS)      pyfr/solvers/navstokes/kernels/intcflux.mako:10-54
 //   intconu            pyfr/solvers/navstokes/kernels/intconu.mako:4-19
 #include "common.cuh"
+#include "elemgeom.cuh"
 #include "exprprog.cuh"
 #include "physics.cuh"
 #include "../../include/pyfrb200.h"
 
 using b200::Gas;
 using b200::soa_off;
+using b200::ElemGeom;
+using b200::elem_metrics;
+using b200::make_geom;
+using b200::GEOM_DIAGONAL;
+using b200::GEOM_PER_ELEMENT;
+using b200::GEOM_STORED;
+using b200::GEOM_VERTICES;
+using b200::with_form;
 
 namespace {
 
 constexpr int PW_BLOCK = 128;
-
-template <typename T>
-struct ElemGeom {
-    const T *smats;  int64_t lds;
-    const T *rcpdjac; int64_t ldr;
-    const T *verts;  int64_t ldv;
-    const T *upts;   int64_t ldup;
-    int linear;
-};
-
-// Geometry modes (the `linear` argument of the element kernels)
-enum { GEOM_STORED = 0, GEOM_VERTICES = 1, GEOM_PER_ELEMENT = 2, GEOM_DIAGONAL = 3 };
-
-// Metric terms at solution point `upt` of element `e`: from the vertices
-// (GEOM_VERTICES, multilinear elements), from the stored per-point smats
-// and 1/|J| (GEOM_STORED), or from one stored set per element
-// (GEOM_PER_ELEMENT: affine elements, whose Jacobian is constant, keep
-// only the rows of their first point: io-shapes (ndims, 1, ndims, neles)
-// and (1, neles)).  DIAG (GEOM_DIAGONAL: per-element terms of elements
-// aligned with the axes, whose off-diagonal S are zero) is a compile-time
-// form of the kernels: the two transforms then take 30 FP64 operations a
-// point in 3-D instead of 99 (tflux_ns at 26^3 elements, p = 3: 416 us
-// before both the shared flux expressions and this form).
-template <int ND, typename T, bool DIAG = false>
-__device__ __forceinline__ void elem_metrics(const ElemGeom<T> &g, int nupts, int upt,
-                                             int64_t e, T s[ND][ND], T &rcpdjac,
-                                             bool need_rcp) {
-    if (DIAG || g.linear >= GEOM_PER_ELEMENT) {
-        nupts = 1;
-        upt = 0;
-    }
-    if (DIAG) {
-#pragma unroll
-        for (int i = 0; i < ND; i++)
-#pragma unroll
-            for (int j = 0; j < ND; j++)
-                s[i][j] = i == j ? g.smats[(int64_t)i * g.lds + soa_off(e, i, ND)] : T(0);
-        rcpdjac = need_rcp ? g.rcpdjac[e] : T(0);
-    } else if (g.linear == GEOM_VERTICES) {
-        T V[1 << ND][ND], x[ND], d;
-#pragma unroll
-        for (int v = 0; v < (1 << ND); v++)
-#pragma unroll
-            for (int k = 0; k < ND; k++) V[v][k] = g.verts[v * g.ldv + soa_off(e, k, ND)];
-#pragma unroll
-        for (int k = 0; k < ND; k++) x[k] = g.upts[upt * g.ldup + k];
-        b200::linear_smats<ND, T>(V, x, s, d);
-        rcpdjac = need_rcp ? T(1) / d : T(0);
-    } else {
-#pragma unroll
-        for (int i = 0; i < ND; i++)
-#pragma unroll
-            for (int j = 0; j < ND; j++)
-                s[i][j] = g.smats[(int64_t)(i * nupts + upt) * g.lds + soa_off(e, j, ND)];
-        rcpdjac = need_rcp ? g.rcpdjac[(int64_t)upt * g.ldr + e] : T(0);
-    }
-}
 
 // f = S ft, the flux in reference space (DIAG: S is diagonal)
 template <int ND, typename T, bool DIAG>
@@ -590,9 +542,14 @@ __device__ __forceinline__ void face_grad_to_phys(const FaceMetrics<T> &fm, int 
         for (int v = 0; v < NV; v++) gg[i][v] = out[i][v];
 }
 
+// sides: 1 the left gradient, 2 the right one, 3 both (beta between +-1/2); pen:
+// tau is not zero.  (Decided on the host: a comparison of doubles is an operation
+// of the FP64 unit.)  FP64, RUSANOV, one side: about 150 FP64 operations a pair,
+// which bound the kernel.
 template <int RS, int ND, typename T, bool FM>
 __global__ void __launch_bounds__(PW_BLOCK, sizeof(T) == 4 ? 8 : 1)
-intcflux_ns_kernel(int64_t n, b200::GasK<T> gas, T beta, T tau, ScalView<T> vl, ScalView<T> vr,
+intcflux_ns_kernel(int64_t n, b200::GasK<T> gas, T beta, T tau, int sides, int pen,
+                   ScalView<T> vl, ScalView<T> vr,
                    VectView<T> gl, VectView<T> gr, int ix64, const T *__restrict__ nl,
                    int64_t ldn, int nl_unit, ScalView<T> va, FaceMetrics<T> fm) {
     constexpr int NV = ND + 2;
@@ -602,8 +559,8 @@ intcflux_ns_kernel(int64_t n, b200::GasK<T> gas, T beta, T tau, ScalView<T> vl, 
     T *pl = vl.base + b200::load_ix(vl.map, ix64, i);
     T *pr = vr.base + b200::load_ix(vr.map, ix64, i);
     // (the element columns of the face metrics, loaded early)
-    const int kl = FM && beta != T(-0.5) ? fm.il[i] : 0;
-    const int kr = FM && beta != T(0.5) ? fm.ir[i] : 0;
+    const int kl = FM && (sides & 1) ? fm.il[i] : 0;
+    const int kr = FM && (sides & 2) ? fm.ir[i] : 0;
 
     T ul[NV], ur[NV], nn[ND];
 #pragma unroll
@@ -616,7 +573,7 @@ intcflux_ns_kernel(int64_t n, b200::GasK<T> gas, T beta, T tau, ScalView<T> vl, 
     // Riemann flux; with a shifted input the viscous terms need the full
     // states, which the shifted flux reconstructs.  The unshifted Rusanov
     // flux takes the LDG penalty with its dissipation.
-    const bool penalty = tau != T(0) && (RS != b200::RS_RUSANOV || gas.shifted);
+    const bool penalty = pen && (RS != b200::RS_RUSANOV || gas.shifted);
     T fi[NV], ufl[NV], ufr[NV];
     if (RS == b200::RS_RUSANOV && gas.shifted) {
         b200::rsolve_rusanov_shift<ND, T>(ul, ur, nn, fi, ufl, ufr, gas);
@@ -635,13 +592,56 @@ intcflux_ns_kernel(int64_t n, b200::GasK<T> gas, T beta, T tau, ScalView<T> vl, 
     // Artificial viscosity at the point (the left side's value)
     const T a = va.base ? va.base[b200::load_ix(va.map, ix64, i)] : T(0);
 
+    // FP64, where operations bound: one side's viscous flux goes onto the
+    // Riemann flux as it is formed
+    if constexpr (sizeof(T) == 8) {
+        if (sides != 3) {
+            const bool left = sides == 1;
+            const VectView<T> &gv = left ? gl : gr;
+            const T *g = gv.base + b200::load_ix(gv.map, ix64, i);
+            const int64_t rstr = b200::load_ix(gv.rstr, ix64, i);
+            T gg[ND][NV], uf[NV];
+#pragma unroll
+            for (int d = 0; d < ND; d++)
+#pragma unroll
+                for (int v = 0; v < NV; v++) gg[d][v] = g[d * rstr + v * B200_SOASZ];
+#pragma unroll
+            for (int v = 0; v < NV; v++) uf[v] = left ? ufl[v] : ufr[v];
+            if (FM) face_grad_to_phys<ND, NV, T>(fm, left ? kl : kr, gg);
+            if (gas.shifted) {
+                T gu[ND][NV];
+                b200::unshift_grad<ND, T>(gg, gu, gas);
+                b200::viscous_nflux_shift_add<ND, T>(uf, gu, nn, fi, gas);
+            } else {
+                b200::viscous_nflux_add<ND, T>(uf, gg, nn, fi, gas);
+                if (va.base) {
+#pragma unroll
+                    for (int v = 0; v < NV; v++) {
+                        T gn = 0;
+#pragma unroll
+                        for (int d = 0; d < ND; d++) gn += nn[d] * gg[d][v];
+                        fi[v] -= a * gn;
+                    }
+                }
+            }
+#pragma unroll
+            for (int v = 0; v < NV; v++) {
+                if (penalty) fi[v] += tau * (ul[v] - ur[v]);
+                const T fc = mag * fi[v];
+                pl[v * B200_SOASZ] = fc;
+                pr[v * B200_SOASZ] = -fc;
+            }
+            return;
+        }
+    }
+
     // LDG viscous common flux from the left and/or right states, each
     // formed along the normal directly
     T nfl[NV], nfr[NV];
 #pragma unroll
     for (int v = 0; v < NV; v++) nfl[v] = nfr[v] = 0;
 
-    if (beta != T(-0.5)) {
+    if (sides & 1) {
         const T *g = gl.base + b200::load_ix(gl.map, ix64, i);
         const int64_t rstr = b200::load_ix(gl.rstr, ix64, i);
         T gg[ND][NV];
@@ -667,7 +667,7 @@ intcflux_ns_kernel(int64_t n, b200::GasK<T> gas, T beta, T tau, ScalView<T> vl, 
             }
         }
     }
-    if (beta != T(0.5)) {
+    if (sides & 2) {
         const T *g = gr.base + b200::load_ix(gr.map, ix64, i);
         const int64_t rstr = b200::load_ix(gr.rstr, ix64, i);
         T gg[ND][NV];
@@ -697,9 +697,9 @@ intcflux_ns_kernel(int64_t n, b200::GasK<T> gas, T beta, T tau, ScalView<T> vl, 
 #pragma unroll
     for (int v = 0; v < NV; v++) {
         T fvc;
-        if (beta == T(-0.5))
+        if (sides == 2)
             fvc = nfr[v];
-        else if (beta == T(0.5))
+        else if (sides == 1)
             fvc = nfl[v];
         else
             fvc = (T(0.5) + beta) * nfl[v] + (T(0.5) - beta) * nfr[v];
@@ -757,38 +757,6 @@ intconu_kernel(int64_t n, int nvars, T beta, ScalView<T> lin, ScalView<T> rin,
                 pro[v * B200_SOASZ] = x;
             }
     }
-}
-
-template <typename T>
-ElemGeom<T> make_geom(int linear, const T *smats, int64_t lds, const T *rcpdjac, int64_t ldr,
-                      const T *verts, int64_t ldv, const T *upts, int64_t ldup) {
-    ElemGeom<T> g;
-    g.smats = smats; g.lds = lds;
-    g.rcpdjac = rcpdjac; g.ldr = ldr;
-    g.verts = verts; g.ldv = ldv;
-    g.upts = upts; g.ldup = ldup;
-    g.linear = linear;
-    return g;
-}
-
-// A launch over the number of dimensions and the diagonal form of the
-// metrics, both compile-time: fn(integral constants); false for ndims other
-// than 2 or 3
-template <typename F>
-bool with_form(int ndims, int linear, F &&fn) {
-    using b2 = std::integral_constant<int, 2>;
-    using b3 = std::integral_constant<int, 3>;
-    if (ndims == 2 && linear == GEOM_DIAGONAL)
-        fn(b2(), std::true_type());
-    else if (ndims == 2)
-        fn(b2(), std::false_type());
-    else if (ndims == 3 && linear == GEOM_DIAGONAL)
-        fn(b3(), std::true_type());
-    else if (ndims == 3)
-        fn(b3(), std::false_type());
-    else
-        return false;
-    return true;
 }
 
 int check_geom(int linear, const void *smats, const void *rcpdjac, const void *verts,
@@ -981,14 +949,15 @@ int intcflux_ns(int ndims, int64_t n, int rsolver, const b200_gas_t *gas, double
     if (ndims != 2 && ndims != 3)
         return b200::set_error(B200_ERR_ARG, "intcflux_ns: ndims must be 2 or 3");
     unsigned grid = b200::ceil_div(n, PW_BLOCK);
+    const int sides = beta == 0.5 ? 1 : beta == -0.5 ? 2 : 3, pen = tau != 0.0;
     const bool ok = b200::with_rsolver(rsolver, [&](auto rsc) {
         constexpr int RS = decltype(rsc)::value;
         if (ndims == 2)
-            intcflux_ns_kernel<RS, 2, T, false><<<grid, PW_BLOCK, 0, st>>>(n, g, (T)beta, (T)tau, l, r, gl, gr, ix64, nl, ldn, nl_unit, va, fm);
+            intcflux_ns_kernel<RS, 2, T, false><<<grid, PW_BLOCK, 0, st>>>(n, g, (T)beta, (T)tau, sides, pen, l, r, gl, gr, ix64, nl, ldn, nl_unit, va, fm);
         else if (!fm.m)
-            intcflux_ns_kernel<RS, 3, T, false><<<grid, PW_BLOCK, 0, st>>>(n, g, (T)beta, (T)tau, l, r, gl, gr, ix64, nl, ldn, nl_unit, va, fm);
+            intcflux_ns_kernel<RS, 3, T, false><<<grid, PW_BLOCK, 0, st>>>(n, g, (T)beta, (T)tau, sides, pen, l, r, gl, gr, ix64, nl, ldn, nl_unit, va, fm);
         else
-            intcflux_ns_kernel<RS, 3, T, true><<<grid, PW_BLOCK, 0, st>>>(n, g, (T)beta, (T)tau, l, r, gl, gr, ix64, nl, ldn, nl_unit, va, fm);
+            intcflux_ns_kernel<RS, 3, T, true><<<grid, PW_BLOCK, 0, st>>>(n, g, (T)beta, (T)tau, sides, pen, l, r, gl, gr, ix64, nl, ldn, nl_unit, va, fm);
     });
     if (!ok) return b200::set_error(B200_ERR_ARG, "intcflux: unknown Riemann solver %d", rsolver);
     B200_CHECK_LAUNCH("intcflux_ns");

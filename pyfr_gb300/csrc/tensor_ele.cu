@@ -1,0 +1,1016 @@
+// Element kernels of tensor-product elements (quadrilaterals and hexahedra
+// with Gauss-Legendre points), whose operators are one-dimensional matrices
+// applied along the lines of points of each direction:
+//
+//   te_interp     the solution at the flux points (M0)
+//   te_gradflux   Navier-Stokes: the corrected gradient (M4 - M6 M0 and M6),
+//                 its transform, the flux at the solution points, the
+//                 gradient at the flux points (M0) and the divergence of the
+//                 flux less its own lift (M1 - M3 M2), one element's data
+//                 staying in shared memory from the first to the last
+//   te_lift       R = -(1/|J|) (R + M3 Fc)
+//   te_euler      Euler: the flux, its divergence, the lift of the common
+//                 flux and the scaling: R from u and Fc
+//
+// They take the place of the operator applies and pointwise kernels that the
+// systems otherwise run one by one
+// (pyfr/solvers/baseadvec/elements.py:91-120,
+// pyfr/solvers/baseadvecdiff/elements.py:47-116), where the gradient was
+// written once and read three times and the flux written and read.
+//
+// Along a line every operand is used by all of its outputs from registers and
+// the matrices are constants of the launch, where the general sparse apply
+// loads an index, a coefficient and an operand per product.
+//
+// FP64: the products along a line run on the integer pipe, in fixed point over
+// the line's own largest exponent (the arithmetic of the general apply,
+// csrc/mul.cu: IMAD.WIDE issues 56 a clock and SM where the FP64 unit issues
+// 2 FMAs; its support test is not needed, since a line is its support).
+// With B of 58 or 60 bits and A of 60 or 61 below the largest row sum the
+// result is within 2^-56 of (row sum)(largest value), an eighth of the rounding
+// of one FP64 FMA.
+// The FP64 unit is left to the flux, beside which the integer work of the
+// other warps runs.
+#include <math.h>
+#include <stdlib.h>
+#include <string.h>
+
+#include "common.cuh"
+#include "elemgeom.cuh"
+#include "physics.cuh"
+#include "../../include/pyfrb200.h"
+
+using b200::ElemGeom;
+using b200::Gas;
+using b200::soa_off;
+
+namespace {
+
+// ---- matrices of the lines --------------------------------------------------
+
+// The derivative matrices are antisymmetric about the line's middle: with an
+// odd number of points the middle point does not enter its own derivative, and
+// is left out (so that an infinity there has the reach that it has in the
+// general apply, which skips zeros).  te_create checks that the entry is zero.
+template <int NO, int NI>
+__device__ constexpr bool absent(int i, int j) {
+    return NI == NO + 2 && (NO & 1) && i == NO / 2 && j == NO / 2;
+}
+
+template <typename T, int NO, int NI>
+struct Mat;
+
+template <int NO, int NI>
+struct Mat<float, NO, NI> {
+    float d[NO][NI];
+};
+
+// a = (ah, al): A = (ah 2^31 + al) 2^-(s + 31), |al| <= 2^30, every row's sum of
+// |ah| below 2^30 + NI, or below 2^29 + NI (wide: rows of ND directions are
+// summed).  With B of BITS = 60 bits (58 for wide), |bh| < 2^(BITS - 31), |bl| <
+// 2^31, the cross sum of Fx stays below 2^63: 2^61 + 7 2^59 for one line of 7
+// entries, 3 2^60 + 2^60 + 22 2^57 for three of them and a kept value, and the
+// high sum below 2^60.
+template <int NO, int NI>
+struct Mat<double, NO, NI> {
+    double d[NO][NI];
+    int2 a[NO][NI];
+    int s;
+};
+
+template <int NO, int NI>
+void set_mat(Mat<float, NO, NI> &m, const double *a, bool = false) {
+    for (int i = 0; i < NO; i++)
+        for (int j = 0; j < NI; j++) m.d[i][j] = (float)a[i * NI + j];
+}
+
+template <int NO, int NI>
+void set_mat(Mat<double, NO, NI> &m, const double *a, bool wide = false) {
+    double l1 = 0.0;
+    for (int i = 0; i < NO; i++) {
+        double r = 0.0;
+        for (int j = 0; j < NI; j++) r += fabs(a[i * NI + j]);
+        l1 = fmax(l1, r);
+    }
+    int e = 0;
+    if (l1 > 0.0) frexp(l1, &e);
+    m.s = (wide ? 29 : 30) - e;
+    for (int i = 0; i < NO; i++)
+        for (int j = 0; j < NI; j++) {
+            const double x = a[i * NI + j];
+            const long long q = llrint(ldexp(x, m.s + 31));
+            const long long ah = (q + (1ll << 30)) >> 31;
+            m.d[i][j] = x;
+            m.a[i][j] = make_int2((int)ah, (int)(q - ah * (1ll << 31)));
+        }
+}
+
+// ---- fixed point along a line -------------------------------------------------
+
+// The magnitude that the largest exponent is taken from
+__device__ __forceinline__ int hi_abs(double x) { return __double2hiint(x) & 0x7fffffff; }
+
+// Exponents that the fixed-point form does not take (near the ends of the
+// range, infinities, NaNs; zeros it does take)
+__device__ __forceinline__ bool out_of_range(int mx) {
+    return mx != 0 && (unsigned)(mx - (128 << 20)) >= (unsigned)((1900 - 128) << 20);
+}
+
+// x as (bh 2^31 + bl) 2^-(1022 + BITS - emax), |bh| < 2^(BITS - 31), |bl| < 2^31,
+// both of x's sign: with the mantissa's leading one at bit 63 of (vh, vl), bh is
+// vh shifted down by 95 - 32 - BITS and the exponent difference d, bl the 31
+// bits below.  In 32-bit operations throughout (a 64-bit shift by a variable
+// issues as slowly as a quarter of these).
+__device__ __forceinline__ unsigned shr_clamp(unsigned x, unsigned n) {
+    return __funnelshift_rc(x, 0u, n);
+}
+
+template <int BITS>
+__device__ __forceinline__ int2 split(double x, int emax) {
+    const int hi = __double2hiint(x), lo = __double2loint(x);
+    // (zeros and subnormals: a difference of at least 64, so that nothing is
+    // left of them)
+    const int d = emax - ((hi >> 20) & 0x7ff);
+    const unsigned vh = __funnelshift_l(lo, (hi & 0xfffff) | 0x100000, 11), vl = (unsigned)lo << 11;
+    constexpr int DH = 63 - BITS, DL = DH + 1;
+    int bh = (int)shr_clamp(vh, d + DH);
+    int bl = (int)(shr_clamp(__funnelshift_rc(vl, vh, d + DL), max(d + DL - 32, 0)) & 0x7fffffffu);
+    if (hi < 0) {
+        bh = -bh;
+        bl = -bl;
+    }
+    return make_int2(bh, bl);
+}
+
+// t 2^sc rounded to FP64, |t| < 2^61, on the integer pipes: the conversion
+// instruction runs on the FP64 unit, at its rate of 2 a clock and SM
+__device__ __forceinline__ double fixed_to_f64(long long t, int sc) {
+    const int sg = (int)(t >> 63);
+    const unsigned long long mag = (unsigned long long)((t ^ (long long)sg) - (long long)sg);
+    unsigned h = (unsigned)(mag >> 32), l = (unsigned)mag;
+    int e = 1023 + 62 + sc;
+    if (h == 0) {
+        h = l;
+        l = 0;
+        e -= 32;
+    }
+    // The leading one to bit 63; its 53 bits rounded (a carry out of them lands
+    // in the exponent, as it should)
+    const int lz = __clz((int)h);
+    const unsigned nh = __funnelshift_l(l, h, lz), nl = l << (lz & 31);
+    const unsigned long long q =
+        (((unsigned long long)nh << 32 | nl) >> 11) + ((nl >> 10) & 1u);
+    const int hi = (int)(q >> 32) + (e - lz) * (1 << 20) + (sg & (int)0x80000000);
+    return h == 0 ? 0.0 : __hiloint2double(hi, (int)q);
+}
+
+// Sums of products of one output
+struct Fx {
+    long long hh, w;
+    __device__ __forceinline__ void clear() {
+        hh = 0;
+        w = 1ll << 30;
+    }
+    __device__ __forceinline__ void mad(int2 a, int2 b) {
+        hh += (long long)a.x * b.x;
+        w += (long long)a.x * b.y;
+        w += (long long)a.y * b.x;
+    }
+    // sc: emax - s - (991 + BITS)
+    __device__ __forceinline__ double value(int sc) const {
+        return fixed_to_f64(hh + (w >> 31), sc);
+    }
+};
+
+// The operands of a line, as the products take them
+template <typename T, int NI>
+struct Operands;
+
+template <int NI>
+struct Operands<float, NI> {
+    float x[NI];
+    __device__ __forceinline__ explicit Operands(const float (&v)[NI]) {
+#pragma unroll
+        for (int j = 0; j < NI; j++) x[j] = v[j];
+    }
+    template <int NO>
+    __device__ __forceinline__ float row(const Mat<float, NO, NI> &m, int i) const {
+        float acc = m.d[i][0] * x[0];
+#pragma unroll
+        for (int j = 1; j < NI; j++)
+            if (!absent<NO, NI>(i, j)) acc = fmaf(m.d[i][j], x[j], acc);
+        return acc;
+    }
+};
+
+template <int NI>
+struct Operands<double, NI> {
+    int2 b[NI];
+    int emax;
+    bool wild;
+    __device__ __forceinline__ explicit Operands(const double (&v)[NI]) {
+        int mx = hi_abs(v[0]);
+#pragma unroll
+        for (int j = 1; j < NI; j++) mx = max(mx, hi_abs(v[j]));
+        wild = out_of_range(mx);
+        emax = max(mx >> 20, 64);
+#pragma unroll
+        for (int j = 0; j < NI; j++) {
+            b[j] = split<60>(v[j], emax);
+            // (the bits of x itself where they are not split)
+            if (wild) b[j] = make_int2(__double2hiint(v[j]), __double2loint(v[j]));
+        }
+    }
+    template <int NO>
+    __device__ __forceinline__ double row(const Mat<double, NO, NI> &m, int i) const {
+        if (wild) {
+            double y = 0.0;
+#pragma unroll
+            for (int j = 0; j < NI; j++)
+                if (!absent<NO, NI>(i, j)) y = fma(m.d[i][j], __hiloint2double(b[j].x, b[j].y), y);
+            return y;
+        }
+        Fx s;
+        s.clear();
+#pragma unroll
+        for (int j = 0; j < NI; j++)
+            if (!absent<NO, NI>(i, j)) s.mad(m.a[i][j], b[j]);
+        return s.value(emax - m.s - 1051);
+    }
+};
+
+// ---- launch constants -----------------------------------------------------------
+
+constexpr int ipow(int q, int n) { return n == 0 ? 1 : q * ipow(q, n - 1); }
+
+template <typename T, int ND, int Q>
+struct Line {
+    static constexpr int NV = ND + 2, NP = ipow(Q, ND), L = NP / Q, NFP = 2 * ND * L;
+    Mat<T, Q, Q + 2> grad;      // corrected derivative from (u, common lo, hi)
+    Mat<T, 2, Q> interp;        // values at the low and high end
+    Mat<T, 2, Q + 2> gradend;   // interp of grad: the derivative at the ends
+    Mat<T, Q, Q + 2> div;       // derivative less own lift, from (F, Fc lo, hi)
+    unsigned char fpt[ND][L][2];
+
+    // First point of line l of direction d, and the distance of its points
+    __device__ static __forceinline__ int stride(int d) { return d == 0 ? 1 : d == 1 ? Q : Q * Q; }
+    __device__ static __forceinline__ int base(int d, int l) {
+        return d == 0 ? l * Q : d == 1 ? (l / Q) * (Q * Q) + l % Q : l;
+    }
+};
+
+// One thread's outputs of the divergence: the Q points of x-line l, from the
+// fluxes of all directions along their lines, Fc at the lines' ends and (KEEP)
+// a value already there.  Fluxes: f(d, p) gives direction d at point p; ends:
+// c(d, l, end).  The inputs are visited twice, for the largest exponent and for
+// the products, rather than held.
+template <typename T, int ND, int Q, bool FLUX, bool LIFT, bool KEEP, typename V>
+__device__ __forceinline__ void visit(const Line<T, ND, Q> &P, int l, V &&vis) {
+    const int y = l % Q, z = l / Q;
+#pragma unroll
+    for (int j = 0; j < Q; j++)
+        if (FLUX) vis.along(0, l * Q + j, j);
+#pragma unroll
+    for (int e = 0; e < 2; e++)
+        if (LIFT) vis.along_end(0, l, e);
+#pragma unroll
+    for (int d = 1; d < ND; d++) {
+        const int row = d == 1 ? y : z;
+#pragma unroll
+        for (int i = 0; i < Q; i++) {
+            // line of direction d through point i of the x-line
+            const int ld = d == 1 ? (ND == 3 ? z * Q + i : i) : y * Q + i;
+            const int b = P.base(d, ld), st = P.stride(d);
+#pragma unroll
+            for (int j = 0; j < Q; j++)
+                if (FLUX) vis.across(d, b + j * st, i, row, j);
+#pragma unroll
+            for (int e = 0; e < 2; e++)
+                if (LIFT) vis.across_end(d, ld, e, i, row);
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < Q; i++)
+        if (KEEP) vis.keep(l * Q + i, i);
+}
+
+template <typename T, int ND, int Q, typename G>
+struct SumVisit {
+    const Line<T, ND, Q> &P;
+    const G &g;
+    T y[Q];
+    __device__ __forceinline__ void along(int d, int p, int j) {
+        const T x = g.flux(d, p);
+#pragma unroll
+        for (int i = 0; i < Q; i++)
+            if (!absent<Q, Q + 2>(i, j)) y[i] += P.div.d[i][j] * x;
+    }
+    __device__ __forceinline__ void along_end(int d, int l, int e) {
+        const T x = g.end(d, l, e);
+#pragma unroll
+        for (int i = 0; i < Q; i++) y[i] += P.div.d[i][Q + e] * x;
+    }
+    __device__ __forceinline__ void across(int d, int p, int i, int row, int j) {
+        if (!absent<Q, Q + 2>(row, j)) y[i] += P.div.d[row][j] * g.flux(d, p);
+    }
+    __device__ __forceinline__ void across_end(int d, int l, int e, int i, int row) {
+        y[i] += P.div.d[row][Q + e] * g.end(d, l, e);
+    }
+    __device__ __forceinline__ void keep(int p, int i) { y[i] += g.old(p); }
+};
+
+template <typename G>
+struct MaxVisit {
+    const G &g;
+    int mx;
+    __device__ __forceinline__ void along(int d, int p, int) { mx = max(mx, g.flux_hi(d, p)); }
+    __device__ __forceinline__ void along_end(int d, int l, int e) {
+        mx = max(mx, hi_abs(g.end(d, l, e)));
+    }
+    __device__ __forceinline__ void across(int d, int p, int, int, int) {
+        mx = max(mx, g.flux_hi(d, p));
+    }
+    __device__ __forceinline__ void across_end(int d, int l, int e, int, int) {
+        mx = max(mx, hi_abs(g.end(d, l, e)));
+    }
+    __device__ __forceinline__ void keep(int p, int) { mx = max(mx, hi_abs(g.old(p))); }
+};
+
+template <int ND, int Q, typename G>
+struct FxVisit {
+    const Line<double, ND, Q> &P;
+    const G &g;
+    int emax;
+    Fx s[Q];
+    __device__ __forceinline__ void along(int d, int p, int j) {
+        const int2 b = split<58>(g.flux(d, p), emax);
+#pragma unroll
+        for (int i = 0; i < Q; i++)
+            if (!absent<Q, Q + 2>(i, j)) s[i].mad(P.div.a[i][j], b);
+    }
+    __device__ __forceinline__ void along_end(int d, int l, int e) {
+        const int2 b = split<58>(g.end(d, l, e), emax);
+#pragma unroll
+        for (int i = 0; i < Q; i++) s[i].mad(P.div.a[i][Q + e], b);
+    }
+    __device__ __forceinline__ void across(int d, int p, int i, int row, int j) {
+        if (!absent<Q, Q + 2>(row, j)) s[i].mad(P.div.a[row][j], split<58>(g.flux(d, p), emax));
+    }
+    __device__ __forceinline__ void across_end(int d, int l, int e, int i, int row) {
+        s[i].mad(P.div.a[row][Q + e], split<58>(g.end(d, l, e), emax));
+    }
+    // (the coefficient one is 2^s: s is at most 29 for row sums of 1/2 and
+    // more, which te_create asks for, and positive for those it takes)
+    __device__ __forceinline__ void keep(int p, int i) {
+        s[i].mad(make_int2(1 << P.div.s, 0), split<58>(g.old(p), emax));
+    }
+};
+
+// Fluxes that are in fixed point already
+template <int ND, int Q, typename G>
+struct FixedVisit {
+    const Line<double, ND, Q> &P;
+    const G &g;
+    Fx s[Q];
+    __device__ __forceinline__ void along(int d, int p, int j) {
+        const int2 b = *reinterpret_cast<const int2 *>(g.at(d, p));
+#pragma unroll
+        for (int i = 0; i < Q; i++)
+            if (!absent<Q, Q + 2>(i, j)) s[i].mad(P.div.a[i][j], b);
+    }
+    __device__ __forceinline__ void across(int d, int p, int i, int row, int j) {
+        // (an absent entry is zero)
+        s[i].mad(P.div.a[row][j], *reinterpret_cast<const int2 *>(g.at(d, p)));
+    }
+    __device__ __forceinline__ void along_end(int, int, int) {}
+    __device__ __forceinline__ void across_end(int, int, int, int, int) {}
+    __device__ __forceinline__ void keep(int, int) {}
+};
+
+template <bool FLUX, bool LIFT, bool KEEP, int ND, int Q, typename G>
+__device__ __forceinline__ void div_line(const Line<float, ND, Q> &P, const G &g, int l,
+                                         float (&y)[Q]) {
+    SumVisit<float, ND, Q, G> v{P, g, {}};
+    visit<float, ND, Q, FLUX, LIFT, KEEP>(P, l, v);
+#pragma unroll
+    for (int i = 0; i < Q; i++) y[i] = v.y[i];
+}
+
+template <bool FLUX, bool LIFT, bool KEEP, int ND, int Q, typename G>
+__device__ __forceinline__ void div_line(const Line<double, ND, Q> &P, const G &g, int l,
+                                         double (&y)[Q]) {
+    MaxVisit<G> m{g, 0};
+    visit<double, ND, Q, FLUX, LIFT, KEEP>(P, l, m);
+    if (out_of_range(m.mx)) {
+        SumVisit<double, ND, Q, G> v{P, g, {}};
+        visit<double, ND, Q, FLUX, LIFT, KEEP>(P, l, v);
+#pragma unroll
+        for (int i = 0; i < Q; i++) y[i] = v.y[i];
+        return;
+    }
+    FxVisit<ND, Q, G> v{P, g, max(m.mx >> 20, 64), {}};
+#pragma unroll
+    for (int i = 0; i < Q; i++) v.s[i].clear();
+    visit<double, ND, Q, FLUX, LIFT, KEEP>(P, l, v);
+#pragma unroll
+    for (int i = 0; i < Q; i++) y[i] = v.s[i].value(v.emax - P.div.s - 1049);
+}
+
+// ---- kernels ------------------------------------------------------------------
+
+constexpr int TE_BLOCK = 256;
+
+// Elements of a block: 64 bytes of a variable's row, two sectors, so that
+// several blocks' elements fit an SM's shared memory
+template <typename T>
+constexpr int te_elems() { return 64 / (int)sizeof(T); }
+
+// u at both ends of every line.  A warp takes one line and variable of 32
+// elements; the lines of one block of elements are consecutive, so that the
+// three reads of a point are near each other in time.
+template <typename T, int ND, int Q>
+__global__ void __launch_bounds__(TE_BLOCK)
+te_interp_kernel(const __grid_constant__ Line<T, ND, Q> P, int64_t neles, int nchunk,
+                 const T *__restrict__ u, int64_t ldu, T *__restrict__ f, int64_t ldf) {
+    using K = Line<T, ND, Q>;
+    const int lane = threadIdx.x & 31;
+    const int64_t blk = blockIdx.x / nchunk;
+    const int t = (int)(blockIdx.x % nchunk) * (TE_BLOCK / 32) + (threadIdx.x >> 5);
+    if (t >= K::NV * ND * K::L || blk * 32 + lane >= neles) return;
+    const int v = t % K::NV, d = t / K::NV / K::L, l = t / K::NV % K::L;
+    const int p0 = K::base(d, l), st = K::stride(d);
+    const int64_t col = (blk * K::NV + v) * 32 + lane;
+    T x[Q];
+#pragma unroll
+    for (int i = 0; i < Q; i++) x[i] = u[(p0 + i * st) * ldu + col];
+    const Operands<T, Q> b(x);
+#pragma unroll
+    for (int e = 0; e < 2; e++) f[P.fpt[d][l][e] * ldf + col] = b.row(P.interp, e);
+}
+
+// Fluxes of one element in shared memory, component c of point p at
+// sm[(c NPS + p) E]; NPS odd, so that two neighbouring components or points lie
+// in different halves of the banks.  Ends and old values in global memory.
+template <typename T, int ND, int Q, int E>
+struct SmemFlux {
+    static constexpr int NPS = ipow(Q, ND) | 1;
+    const Line<T, ND, Q> &P;
+    const T *sm;            // + element
+    int v;
+    const T *fc;            // + column of the element and variable
+    int64_t ldf;
+    __device__ __forceinline__ const T *at(int d, int p) const {
+        return sm + ((d * (ND + 2) + v) * NPS + p) * E;
+    }
+    __device__ __forceinline__ T flux(int d, int p) const { return *at(d, p); }
+    __device__ __forceinline__ int flux_hi(int d, int p) const {
+        return reinterpret_cast<const int *>(at(d, p))[1] & 0x7fffffff;
+    }
+    __device__ __forceinline__ T end(int d, int l, int e) const {
+        return fc[P.fpt[d][l][e] * ldf];
+    }
+    __device__ __forceinline__ T old(int) const { return T(0); }
+};
+
+// The gradient in physical space, (1/|J|) S^T tg
+template <int ND, typename T>
+__device__ __forceinline__ void grad_to_phys(const T s[ND][ND], T rcp, const T tg[ND][ND + 2],
+                                             T gr[ND][ND + 2]) {
+#pragma unroll
+    for (int i = 0; i < ND; i++) {
+        T k[ND];
+#pragma unroll
+        for (int d = 0; d < ND; d++) k[d] = rcp * s[d][i];
+#pragma unroll
+        for (int v = 0; v < ND + 2; v++) {
+            T acc = k[0] * tg[0][v];
+#pragma unroll
+            for (int d = 1; d < ND; d++) acc += k[d] * tg[d][v];
+            gr[i][v] = acc;
+        }
+    }
+}
+
+// facemask: bit 2 d + end, the faces whose gradient is wanted on any element;
+// refgrad: it stays in reference space (the interface kernels transform it).
+// r may be u, and gf's first component may be c: every element's values are
+// read before they are written.
+template <typename T, int ND, int Q, bool DIAG, int E>
+__global__ void __launch_bounds__(TE_BLOCK)
+te_gradflux_kernel(const __grid_constant__ Line<T, ND, Q> P, int64_t neles, b200::GasK<T> gas,
+                   const T *u, int64_t ldu, const T *c, int64_t ldc, T *gf, int64_t ldg,
+                   unsigned facemask, int refgrad, ElemGeom<T> geo, T *r, int64_t ldr) {
+    using K = Line<T, ND, Q>;
+    constexpr int NV = K::NV, NP = K::NP, L = K::L, NFP = K::NFP, NPS = NP | 1;
+    constexpr int G = TE_BLOCK / E;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    T *sm = reinterpret_cast<T *>(smem_raw);
+
+    constexpr bool FIXED = sizeof(T) == 8;
+    __shared__ int top[NV][E];      // largest flux of each variable
+
+    const int el = threadIdx.x % E, grp = threadIdx.x / E;
+    const int64_t e = (int64_t)blockIdx.x * E + el;
+    const bool live = e < neles;
+    const int64_t col0 = soa_off(live ? e : 0, 0, NV);
+    T *const sme = sm + el;
+    if (FIXED)
+        for (int v = grp; v < NV; v += G) top[v][el] = 0;
+
+    // The corrected gradient along every line; for a diagonal metric, already
+    // in physical space (unless it is wanted in reference space)
+    T sd[ND] = {};
+    if (DIAG && live) {
+#pragma unroll
+        for (int d = 0; d < ND; d++)
+            sd[d] = geo.rcpdjac[e] * geo.smats[(int64_t)d * geo.lds + soa_off(e, d, ND)];
+    }
+    const bool scale = DIAG && !refgrad, own = DIAG || refgrad;
+    for (int t = grp; t < NV * ND * L; t += G) {
+        const int v = t % NV, d = t / NV / L, l = t / NV % L;
+        const int p0 = K::base(d, l), st = K::stride(d);
+        T x[Q + 2];
+#pragma unroll
+        for (int i = 0; i < Q; i++) x[i] = live ? u[(p0 + i * st) * ldu + col0 + v * 32] : T(0);
+#pragma unroll
+        for (int i = 0; i < 2; i++)
+            x[Q + i] = live ? c[P.fpt[d][l][i] * ldc + col0 + v * 32] : T(0);
+        const Operands<T, Q + 2> b(x);
+        const T s = DIAG ? (d == 0 ? sd[0] : d == 1 ? sd[1] : sd[ND - 1]) : T(1);
+#pragma unroll
+        for (int i = 0; i < Q; i++) {
+            T y = b.row(P.grad, i);
+            if (scale) y *= s;
+            sme[((d * NV + v) * NPS + p0 + i * st) * E] = y;
+        }
+        // The derivative along the line at its ends, where the metric leaves
+        // it a component of its own.  (Where the first component's rows are
+        // those of c, this thread alone reads the value that it replaces.)
+        if (own && live) {
+#pragma unroll
+            for (int i = 0; i < 2; i++)
+                if ((facemask >> (2 * d + i)) & 1) {
+                    const T y = b.row(P.gradend, i);
+                    gf[(int64_t)(d * NFP + P.fpt[d][l][i]) * ldg + col0 + v * 32] =
+                        scale ? s * y : y;
+                }
+        }
+    }
+    __syncthreads();
+
+    if (!DIAG && !refgrad) {
+        for (int p = grp; p < NP; p += G) {
+            T s[ND][ND] = {}, rcp = T(0), tg[ND][NV], gr[ND][NV];
+            if (live) b200::elem_metrics<ND, T>(geo, NP, p, e, s, rcp, true);
+#pragma unroll
+            for (int d = 0; d < ND; d++)
+#pragma unroll
+                for (int v = 0; v < NV; v++) tg[d][v] = sme[((d * NV + v) * NPS + p) * E];
+            grad_to_phys<ND, T>(s, rcp, tg, gr);
+#pragma unroll
+            for (int d = 0; d < ND; d++)
+#pragma unroll
+                for (int v = 0; v < NV; v++) sme[((d * NV + v) * NPS + p) * E] = gr[d][v];
+        }
+        __syncthreads();
+    }
+
+    // The gradient at the flux points that are read
+    for (int t = grp; t < NV * ND * ND * L; t += G) {
+        const int v = t % NV, k = t / NV % ND, d = t / (NV * ND) / L, l = t / (NV * ND) % L;
+        const unsigned need = (facemask >> (2 * d)) & 3;
+        if (!need || (own && k == d)) continue;
+        const int p0 = K::base(d, l), st = K::stride(d);
+        T x[Q];
+#pragma unroll
+        for (int i = 0; i < Q; i++) x[i] = sme[((k * NV + v) * NPS + p0 + i * st) * E];
+        const Operands<T, Q> b(x);
+#pragma unroll
+        for (int i = 0; i < 2; i++)
+            if (live && ((need >> i) & 1))
+                gf[(int64_t)(k * NFP + P.fpt[d][l][i]) * ldg + col0 + v * 32] = b.row(P.interp, i);
+    }
+    __syncthreads();
+
+    // The flux in reference space, in the place of the gradient
+    for (int p = grp; p < NP; p += G) {
+        T uu[NV], gr[ND][NV], ft[ND][NV], s[ND][ND] = {}, rcp = T(0);
+        if (live) b200::elem_metrics<ND, T, DIAG>(geo, NP, p, e, s, rcp, !DIAG && refgrad);
+#pragma unroll
+        for (int v = 0; v < NV; v++) uu[v] = live ? u[p * ldu + col0 + v * 32] : T(1);
+#pragma unroll
+        for (int d = 0; d < ND; d++)
+#pragma unroll
+            for (int v = 0; v < NV; v++) gr[d][v] = sme[((d * NV + v) * NPS + p) * E];
+        if (DIAG && refgrad) {
+#pragma unroll
+            for (int d = 0; d < ND; d++)
+#pragma unroll
+                for (int v = 0; v < NV; v++) gr[d][v] *= sd[d];
+        } else if (refgrad) {
+            T tg[ND][NV];
+#pragma unroll
+            for (int d = 0; d < ND; d++)
+#pragma unroll
+                for (int v = 0; v < NV; v++) tg[d][v] = gr[d][v];
+            grad_to_phys<ND, T>(s, rcp, tg, gr);
+        }
+        b200::ns_flux<ND, T>(uu, gr, ft, gas);
+#pragma unroll
+        for (int v = 0; v < NV; v++) {
+            int mx = 0;
+#pragma unroll
+            for (int i = 0; i < ND; i++) {
+                T acc = s[i][DIAG ? i : 0] * ft[DIAG ? i : 0][v];
+#pragma unroll
+                for (int k = 1; k < ND; k++)
+                    if (!DIAG) acc += s[i][k] * ft[k][v];
+                sme[((i * NV + v) * NPS + p) * E] = acc;
+                if constexpr (FIXED) mx = max(mx, hi_abs(acc));
+            }
+            if constexpr (FIXED) atomicMax(&top[v][el], mx);
+        }
+    }
+    __syncthreads();
+
+    // FP64: the fluxes in fixed point over the largest of the element's and
+    // variable's (each is an operand of the lines of Q points, and is split
+    // once), except where that is out of range
+    if constexpr (FIXED) {
+        for (int p = grp; p < NP; p += G) {
+#pragma unroll
+            for (int v = 0; v < NV; v++) {
+                const int mx = top[v][el];
+                if (out_of_range(mx)) continue;
+#pragma unroll
+                for (int i = 0; i < ND; i++) {
+                    double *q = &sme[((i * NV + v) * NPS + p) * E];
+                    *reinterpret_cast<int2 *>(q) = split<58>(*q, max(mx >> 20, 64));
+                }
+            }
+        }
+        __syncthreads();
+    }
+
+    // The divergence along the lines of every direction
+    for (int t = grp; t < NV * L; t += G) {
+        const int v = t % NV, l = t / NV;
+        const SmemFlux<T, ND, Q, E> g{P, sme, v, nullptr, 0};
+        T y[Q];
+        bool done = false;
+        if constexpr (FIXED) {
+            const int mx = top[v][el];
+            if (!out_of_range(mx)) {
+                FixedVisit<ND, Q, SmemFlux<T, ND, Q, E>> f{P, g, {}};
+#pragma unroll
+                for (int i = 0; i < Q; i++) f.s[i].clear();
+                visit<T, ND, Q, true, false, false>(P, l, f);
+#pragma unroll
+                for (int i = 0; i < Q; i++)
+                    y[i] = f.s[i].value(max(mx >> 20, 64) - P.div.s - 1049);
+                done = true;
+            }
+        }
+        if (!done) {
+            SumVisit<T, ND, Q, SmemFlux<T, ND, Q, E>> f{P, g, {}};
+            visit<T, ND, Q, true, false, false>(P, l, f);
+#pragma unroll
+            for (int i = 0; i < Q; i++) y[i] = f.y[i];
+        }
+#pragma unroll
+        for (int i = 0; i < Q; i++)
+            if (live) r[(l * Q + i) * ldr + col0 + v * 32] = y[i];
+    }
+}
+
+// Euler: flux at the points, divergence, lift and scaling.  r may be u.
+template <typename T, int ND, int Q, bool DIAG, int E>
+__global__ void __launch_bounds__(TE_BLOCK)
+te_euler_kernel(const __grid_constant__ Line<T, ND, Q> P, int64_t neles, T gamma, const T *u,
+                int64_t ldu, const T *__restrict__ fc, int64_t ldf, ElemGeom<T> geo, T *r,
+                int64_t ldr) {
+    using K = Line<T, ND, Q>;
+    constexpr int NV = K::NV, NP = K::NP, L = K::L, NPS = NP | 1;
+    constexpr int G = TE_BLOCK / E;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    T *sm = reinterpret_cast<T *>(smem_raw);
+
+    const int el = threadIdx.x % E, grp = threadIdx.x / E;
+    const int64_t e = (int64_t)blockIdx.x * E + el;
+    const bool live = e < neles;
+    const int64_t col0 = soa_off(live ? e : 0, 0, NV);
+    T *const sme = sm + el;
+
+    for (int p = grp; p < NP; p += G) {
+        T uu[NV], ft[ND][NV], s[ND][ND] = {}, rcp, pr, vel[ND];
+        if (live) b200::elem_metrics<ND, T, DIAG>(geo, NP, p, e, s, rcp, false);
+#pragma unroll
+        for (int v = 0; v < NV; v++) uu[v] = live ? u[p * ldu + col0 + v * 32] : T(1);
+        b200::inviscid_flux<ND, T>(uu, ft, pr, vel, gamma);
+#pragma unroll
+        for (int i = 0; i < ND; i++)
+#pragma unroll
+            for (int v = 0; v < NV; v++) {
+                T acc = s[i][DIAG ? i : 0] * ft[DIAG ? i : 0][v];
+#pragma unroll
+                for (int k = 1; k < ND; k++)
+                    if (!DIAG) acc += s[i][k] * ft[k][v];
+                sme[((i * NV + v) * NPS + p) * E] = acc;
+            }
+    }
+    __syncthreads();
+    if (!live) return;
+
+    for (int t = grp; t < NV * L; t += G) {
+        const int v = t % NV, l = t / NV;
+        const SmemFlux<T, ND, Q, E> g{P, sme, v, fc + col0 + v * 32, ldf};
+        T y[Q];
+        div_line<true, true, false>(P, g, l, y);
+#pragma unroll
+        for (int i = 0; i < Q; i++) {
+            const int p = l * Q + i;
+            const T rj = geo.rcpdjac[(geo.linear >= b200::GEOM_PER_ELEMENT ? 0 : p * geo.ldr) + e];
+            r[p * ldr + col0 + v * 32] = -rj * y[i];
+        }
+    }
+}
+
+template <typename T, int ND, int Q>
+struct GlobalEnds {
+    const Line<T, ND, Q> &P;
+    const T *fc, *r;        // + column of the element and variable
+    int64_t ldf, ldr;
+    __device__ __forceinline__ T flux(int, int) const { return T(0); }
+    __device__ __forceinline__ int flux_hi(int, int) const { return 0; }
+    __device__ __forceinline__ T end(int d, int l, int e) const {
+        return fc[P.fpt[d][l][e] * ldf];
+    }
+    __device__ __forceinline__ T old(int p) const { return r[p * ldr]; }
+};
+
+// R = -(1/|J|) (R + M3 Fc): a warp takes an x-line and variable of 32 elements
+template <typename T, int ND, int Q>
+__global__ void __launch_bounds__(TE_BLOCK)
+te_lift_kernel(const __grid_constant__ Line<T, ND, Q> P, int64_t neles, int nchunk,
+               const T *__restrict__ fc, int64_t ldf, const T *__restrict__ rcpdjac, int64_t ldj,
+               T *__restrict__ r, int64_t ldr) {
+    using K = Line<T, ND, Q>;
+    const int lane = threadIdx.x & 31;
+    const int64_t blk = blockIdx.x / nchunk;
+    const int t = (int)(blockIdx.x % nchunk) * (TE_BLOCK / 32) + (threadIdx.x >> 5);
+    if (t >= K::NV * K::L || blk * 32 + lane >= neles) return;
+    const int v = t % K::NV, l = t / K::NV;
+    const int64_t col = (blk * K::NV + v) * 32 + lane;
+    const GlobalEnds<T, ND, Q> g{P, fc + col, r + col, ldf, ldr};
+    T y[Q];
+    div_line<false, true, true>(P, g, l, y);
+#pragma unroll
+    for (int i = 0; i < Q; i++) {
+        const int p = l * Q + i;
+        r[p * ldr + col] = -rcpdjac[p * ldj + blk * 32 + lane] * y[i];
+    }
+}
+
+// ---- host side ----------------------------------------------------------------
+
+constexpr int QMAX = 5;
+
+// The one-dimensional matrices in FP64, and the flux points of the lines
+struct TeHandle {
+    int ndims, q;
+    double grad[QMAX * (QMAX + 2)], interp[2 * QMAX], div[QMAX * (QMAX + 2)];
+    unsigned char fpt[3 * QMAX * QMAX * 2];
+};
+
+template <typename T, int ND, int Q>
+Line<T, ND, Q> line_of(const TeHandle &h) {
+    Line<T, ND, Q> p;
+    set_mat(p.grad, h.grad);
+    set_mat(p.interp, h.interp);
+    double ge[2 * (Q + 2)];
+    for (int e = 0; e < 2; e++)
+        for (int j = 0; j < Q + 2; j++) {
+            double x = 0.0;
+            for (int i = 0; i < Q; i++) x += h.interp[e * Q + i] * h.grad[i * (Q + 2) + j];
+            ge[e * (Q + 2) + j] = x;
+        }
+    set_mat(p.gradend, ge);
+    set_mat(p.div, h.div, true);
+    memcpy(p.fpt, h.fpt, sizeof(p.fpt));
+    return p;
+}
+
+// fn(integral constants ND, Q) for the handle's shape
+template <typename F>
+bool with_shape(const TeHandle &h, F &&fn) {
+#define B200_TE(nd, nq)                                                      \
+    if (h.ndims == nd && h.q == nq) {                                        \
+        fn(std::integral_constant<int, nd>(), std::integral_constant<int, nq>()); \
+        return true;                                                         \
+    }
+    B200_TE(2, 3) B200_TE(2, 4) B200_TE(2, 5)
+    B200_TE(3, 3) B200_TE(3, 4) B200_TE(3, 5)
+#undef B200_TE
+    return false;
+}
+
+template <typename Fn>
+int opt_in(Fn fn, size_t smem) {
+    return b200::check_cuda(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                 (int)smem), "te: smem attribute");
+}
+
+template <typename T, int ND, int Q>
+constexpr size_t te_smem() {
+    return (size_t)ND * (ND + 2) * (ipow(Q, ND) | 1) * te_elems<T>() * sizeof(T);
+}
+
+template <typename T>
+int te_opt_in(const TeHandle &h) {
+    int rc = 0;
+    with_shape(h, [&](auto nd, auto nq) {
+        constexpr int ND = nd(), Q = nq(), E = te_elems<T>();
+        constexpr size_t s = te_smem<T, ND, Q>();
+        rc = opt_in(te_gradflux_kernel<T, ND, Q, true, E>, s);
+        if (!rc) rc = opt_in(te_gradflux_kernel<T, ND, Q, false, E>, s);
+        if (!rc) rc = opt_in(te_euler_kernel<T, ND, Q, true, E>, s);
+        if (!rc) rc = opt_in(te_euler_kernel<T, ND, Q, false, E>, s);
+    });
+    return rc;
+}
+
+int check_te(const void *handle, const char *what, std::initializer_list<const void *> ptrs) {
+    if (!handle) return b200::set_error(B200_ERR_ARG, "%s: null handle", what);
+    for (const void *p : ptrs)
+        if (!p) return b200::set_error(B200_ERR_ARG, "%s: null pointer", what);
+    return B200_OK;
+}
+
+template <typename T>
+int te_interp(void *handle, int64_t neles, const T *u, int64_t ldu, T *f, int64_t ldf,
+              cudaStream_t st) {
+    int rc = check_te(handle, "te_interp", {u, f});
+    if (rc || neles <= 0) return rc;
+    const TeHandle &h = *(const TeHandle *)handle;
+    with_shape(h, [&](auto nd, auto nq) {
+        using K = Line<T, nd(), nq()>;
+        const int nchunk = (int)b200::ceil_div(K::NV * nd() * K::L, TE_BLOCK / 32);
+        te_interp_kernel<T, nd(), nq()><<<b200::ceil_div(neles, 32) * nchunk, TE_BLOCK, 0, st>>>(
+            line_of<T, nd(), nq()>(h), neles, nchunk, u, ldu, f, ldf);
+    });
+    B200_CHECK_LAUNCH("te_interp");
+    return B200_OK;
+}
+
+int te_geom(int linear, const void *smats, const void *rcpdjac) {
+    if (linear != b200::GEOM_STORED && linear != b200::GEOM_PER_ELEMENT &&
+        linear != b200::GEOM_DIAGONAL)
+        return b200::set_error(B200_ERR_ARG, "te: the metric terms must be stored");
+    if (!smats || !rcpdjac) return b200::set_error(B200_ERR_ARG, "te: null metric terms");
+    return B200_OK;
+}
+
+template <typename T>
+int te_gradflux_ns(void *handle, int64_t neles, int linear, const b200_gas_t *gas, const T *u,
+                   int64_t ldu, const T *c, int64_t ldc, T *gf, int64_t ldg, unsigned facemask, int refgrad,
+                   const T *smats, int64_t lds, const T *rcpdjac, int64_t ldj, T *r, int64_t ldr,
+                   cudaStream_t st) {
+    int rc = check_te(handle, "te_gradflux", {gas, u, c, gf, r});
+    if (!rc) rc = te_geom(linear, smats, rcpdjac);
+    if (rc || neles <= 0) return rc;
+    const TeHandle &h = *(const TeHandle *)handle;
+    const auto g = b200::gas_consts<T>(*reinterpret_cast<const Gas *>(gas));
+    if (g.shifted)
+        return b200::set_error(B200_ERR_UNSUPPORTED, "te_gradflux: takes unshifted states");
+    const auto geo = b200::make_geom<T>(linear, smats, lds, rcpdjac, ldj, nullptr, 0, nullptr, 0);
+    with_shape(h, [&](auto nd, auto nq) {
+        constexpr int ND = nd(), Q = nq(), E = te_elems<T>();
+        const unsigned grid = b200::ceil_div(neles, E);
+        constexpr size_t s = te_smem<T, ND, Q>();
+        const auto P = line_of<T, ND, Q>(h);
+        if (linear == b200::GEOM_DIAGONAL)
+            te_gradflux_kernel<T, ND, Q, true, E><<<grid, TE_BLOCK, s, st>>>(P, neles, g, u, ldu, c, ldc, gf, ldg, facemask, refgrad, geo, r, ldr);
+        else
+            te_gradflux_kernel<T, ND, Q, false, E><<<grid, TE_BLOCK, s, st>>>(P, neles, g, u, ldu, c, ldc, gf, ldg, facemask, refgrad, geo, r, ldr);
+    });
+    B200_CHECK_LAUNCH("te_gradflux");
+    return B200_OK;
+}
+
+template <typename T>
+int te_euler(void *handle, int64_t neles, int linear, double gamma, const T *u, int64_t ldu,
+             const T *fc, int64_t ldf, const T *smats, int64_t lds, const T *rcpdjac, int64_t ldj,
+             T *r, int64_t ldr, cudaStream_t st) {
+    int rc = check_te(handle, "te_euler", {u, fc, r});
+    if (!rc) rc = te_geom(linear, smats, rcpdjac);
+    if (rc || neles <= 0) return rc;
+    const TeHandle &h = *(const TeHandle *)handle;
+    const auto geo = b200::make_geom<T>(linear, smats, lds, rcpdjac, ldj, nullptr, 0, nullptr, 0);
+    with_shape(h, [&](auto nd, auto nq) {
+        constexpr int ND = nd(), Q = nq(), E = te_elems<T>();
+        const unsigned grid = b200::ceil_div(neles, E);
+        constexpr size_t s = te_smem<T, ND, Q>();
+        const auto P = line_of<T, ND, Q>(h);
+        if (linear == b200::GEOM_DIAGONAL)
+            te_euler_kernel<T, ND, Q, true, E><<<grid, TE_BLOCK, s, st>>>(P, neles, (T)gamma, u, ldu, fc, ldf, geo, r, ldr);
+        else
+            te_euler_kernel<T, ND, Q, false, E><<<grid, TE_BLOCK, s, st>>>(P, neles, (T)gamma, u, ldu, fc, ldf, geo, r, ldr);
+    });
+    B200_CHECK_LAUNCH("te_euler");
+    return B200_OK;
+}
+
+template <typename T>
+int te_lift(void *handle, int64_t neles, const T *fc, int64_t ldf, const T *rcpdjac, int64_t ldj,
+            T *r, int64_t ldr, cudaStream_t st) {
+    int rc = check_te(handle, "te_lift", {fc, rcpdjac, r});
+    if (rc || neles <= 0) return rc;
+    const TeHandle &h = *(const TeHandle *)handle;
+    with_shape(h, [&](auto nd, auto nq) {
+        using K = Line<T, nd(), nq()>;
+        const int nchunk = (int)b200::ceil_div(K::NV * K::L, TE_BLOCK / 32);
+        te_lift_kernel<T, nd(), nq()><<<b200::ceil_div(neles, 32) * nchunk, TE_BLOCK, 0, st>>>(
+            line_of<T, nd(), nq()>(h), neles, nchunk, fc, ldf, rcpdjac, ldj, r, ldr);
+    });
+    B200_CHECK_LAUNCH("te_lift");
+    return B200_OK;
+}
+
+}  // namespace
+
+extern "C" {
+
+int b200_te_create(int ndims, int q, const double *grad, const double *interp, const double *div,
+                   const int *fpt, void **handle) {
+    if (!grad || !interp || !div || !fpt || !handle)
+        return b200::set_error(B200_ERR_ARG, "te_create: null pointer");
+    TeHandle *h = (TeHandle *)calloc(1, sizeof(TeHandle));
+    if (!h) return b200::set_error(B200_ERR_STATE, "te_create: out of host memory");
+    h->ndims = ndims;
+    h->q = q;
+    if (!with_shape(*h, [](auto, auto) {})) {
+        free(h);
+        return b200::set_error(B200_ERR_UNSUPPORTED, "te_create: %d-D, %d points a line", ndims, q);
+    }
+    // (finite, and with a row sum that the fixed-point form takes)
+    double top = 0.0;
+    for (int i = 0; i < q * (q + 2); i++) top = fmax(top, fmax(fabs(grad[i]), fabs(div[i])));
+    bool fine = top >= 0.5 && top <= 1e6;
+    for (int i = 0; i < q * (q + 2); i++) fine = fine && isfinite(grad[i]) && isfinite(div[i]);
+    for (int i = 0; i < 2 * q; i++) fine = fine && fabs(interp[i]) <= 1e6;
+    const int mid = (q / 2) * (q + 2) + q / 2;
+    if (q & 1) fine = fine && grad[mid] == 0.0 && div[mid] == 0.0;
+    const int nf = 2 * ndims * (ndims == 2 ? q : q * q);
+    for (int i = 0; i < nf; i++) fine = fine && fpt[i] >= 0 && fpt[i] < nf;
+    if (!fine) {
+        free(h);
+        return b200::set_error(B200_ERR_ARG, "te_create: operators out of range");
+    }
+    memcpy(h->grad, grad, sizeof(double) * q * (q + 2));
+    memcpy(h->interp, interp, sizeof(double) * 2 * q);
+    memcpy(h->div, div, sizeof(double) * q * (q + 2));
+    for (int i = 0; i < nf; i++) h->fpt[i] = (unsigned char)fpt[i];
+    int rc = te_opt_in<double>(*h);
+    if (!rc) rc = te_opt_in<float>(*h);
+    if (rc) {
+        free(h);
+        return rc;
+    }
+    *handle = h;
+    return B200_OK;
+}
+
+int b200_te_destroy(void *handle) {
+    free(handle);
+    return B200_OK;
+}
+
+#define B200_TE_API(T, sfx)                                                                     \
+    int b200_te_interp_##sfx(void *h, int64_t neles, const T *u, int64_t ldu, T *f, int64_t ldf, \
+                             void *stream) {                                                    \
+        return te_interp<T>(h, neles, u, ldu, f, ldf, (cudaStream_t)stream);                    \
+    }                                                                                           \
+    int b200_te_gradflux_ns_##sfx(void *h, int64_t neles, int linear, const b200_gas_t *gas,     \
+                                  const T *u, int64_t ldu, const T *c, int64_t ldc, T *gf,      \
+                                  int64_t ldg, unsigned facemask, int refgrad, const T *smats,  \
+                                  int64_t lds, const T *rcpdjac, int64_t ldj, T *r,             \
+                                  int64_t ldr, void *stream) {                                  \
+        return te_gradflux_ns<T>(h, neles, linear, gas, u, ldu, c, ldc, gf, ldg, facemask,       \
+                                 refgrad, smats, lds, rcpdjac, ldj, r, ldr,                     \
+                                 (cudaStream_t)stream);                                         \
+    }                                                                                           \
+    int b200_te_euler_##sfx(void *h, int64_t neles, int linear, double gamma, const T *u,        \
+                            int64_t ldu, const T *fc, int64_t ldf, const T *smats, int64_t lds, \
+                            const T *rcpdjac, int64_t ldj, T *r, int64_t ldr, void *stream) {   \
+        return te_euler<T>(h, neles, linear, gamma, u, ldu, fc, ldf, smats, lds, rcpdjac, ldj, r, \
+                           ldr, (cudaStream_t)stream);                                          \
+    }                                                                                           \
+    int b200_te_lift_##sfx(void *h, int64_t neles, const T *fc, int64_t ldf, const T *rcpdjac,   \
+                           int64_t ldj, T *r, int64_t ldr, void *stream) {                      \
+        return te_lift<T>(h, neles, fc, ldf, rcpdjac, ldj, r, ldr, (cudaStream_t)stream);        \
+    }
+
+B200_TE_API(double, f64)
+B200_TE_API(float, f32)
+
+}  // extern "C"

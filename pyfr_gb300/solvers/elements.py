@@ -345,6 +345,51 @@ class BaseElements:
     def qpts(self):
         return self._be.const_matrix(self.basis.qpts)
 
+    # ---- element kernels (pyfr_gb300/backend/tensorele.py) -----------------
+
+    # The faces (bit 2*direction + end) whose gradient an interface reads,
+    # set by the system
+    te_facemask = 0
+
+    def te_handle(self):
+        """(handle, flux points of the lines) when this type's right-hand
+        side runs on the element kernels: tensor-product elements that are
+        all linear, in the backend's own precision (no tensor-core applies),
+        on unshifted states, with no anti-aliasing, shock capturing or
+        source terms.  None otherwise.  (The state of the system's set-up
+        when its kernels are made decides.)"""
+        be = self._be
+        viscous = 'grad_upts' in self._scratch_bufs
+        if be.element_kernels != 'auto' or be.fuse_operators or \
+                be.ref_state is not None or self.linoff or \
+                not be.precompute_metrics or \
+                getattr(self, 'antialias', False) or \
+                self._srctplargs is not None or \
+                self.cfg.get('solver', 'shock-capturing', 'none') != 'none':
+            return None
+        return be.tensor_elements.handle(self.basis, viscous)
+
+    def _te_mats(self):
+        return dict(verts=self.ploc_at('linspts', 'linear'), upts=self.upts)
+
+    def set_te_faces(self, fidxs):
+        """Have the gradient formed at the flux points of these faces."""
+        fpt = self.te_handle()[1]
+        self.te_facemask = 0
+        for d, e in np.ndindex(self.ndims, 2):
+            pts = set(fpt[d, :, e].tolist())
+            if any(pts == set(np.asarray(self.basis.facefpts[f]).tolist())
+                   for f in fidxs):
+                self.te_facemask |= 1 << (2*d + e)
+
+    def _disu_kernel(self, uin):
+        te = self.te_handle()
+        if te:
+            return self._be.kernel('te_interp', te[0], self.scal_upts[uin],
+                                   self._scal_fpts, self.neles)
+        return self._be.kernel('mul', self.opmat('M0'), self.scal_upts[uin],
+                               out=self._scal_fpts)
+
     # ---- interface helpers (pyfr/solvers/base/elements.py:446-469) --------
 
     def get_ploc_for_inters(self, eidxs, fidx):
@@ -528,8 +573,7 @@ class EulerElements(_WavespeedMixin, _DivergenceMixin, FluidElements,
         be.pointwise.register('pyfr.solvers.euler.kernels.tflux')
 
         # Interpolate the solution to the flux points
-        kernels['disu'] = lambda uin: be.kernel(
-            'mul', self.opmat('M0'), self.scal_upts[uin], out=self._scal_fpts)
+        kernels['disu'] = lambda uin: self._disu_kernel(uin)
 
         # Transformed flux, at the solution points or, with flux
         # anti-aliasing, at the quadrature points
@@ -577,6 +621,14 @@ class EulerElements(_WavespeedMixin, _DivergenceMixin, FluidElements,
         # Divergence of the partially corrected flux and the correction
         self._divergence_kernels()
 
+        def te_euler(uin, fout):
+            te = self.te_handle()
+            return be.kernel(
+                'te_euler', te[0], tplargs | {'ktype': 'linear'}, self.neles,
+                self.scal_upts[uin], self._scal_fpts, self.scal_upts[fout],
+                **self._te_mats()) if te else NullKernel()
+        self.te_rhs = te_euler
+
 
 class NavierStokesElements(_WavespeedMixin, _DivergenceMixin, FluidElements,
                            BaseElements):
@@ -614,8 +666,7 @@ class NavierStokesElements(_WavespeedMixin, _DivergenceMixin, FluidElements,
         be.pointwise.register('pyfr.solvers.baseadvecdiff.kernels.gradcoru')
         be.pointwise.register('pyfr.solvers.navstokes.kernels.tflux')
 
-        kernels['disu'] = lambda uin: be.kernel(
-            'mul', self.opmat('M0'), self.scal_upts[uin], out=self._scal_fpts)
+        kernels['disu'] = lambda uin: self._disu_kernel(uin)
 
         # (not needed when the interfaces write the common solution to
         # both sides of every flux point: comm_covered, set by the system)
@@ -751,3 +802,22 @@ class NavierStokesElements(_WavespeedMixin, _DivergenceMixin, FluidElements,
                 for kt, n, rgn, kw in tdisf)
 
         self._divergence_kernels()
+
+        # (the flux at the solution points, the divergence and, at the flux
+        # points, the gradient, in one kernel; then the correction)
+        def te_gradflux(uin, fout):
+            te = self.te_handle()
+            return be.kernel(
+                'te_gradflux', te[0], tplargs | {'ktype': 'linear-fused'},
+                self.neles, self.scal_upts[uin], self._comm_fpts,
+                self._vect_fpts, self.te_facemask, self.scal_upts[fout],
+                refgrad=not self.grad_writeback, **self._te_mats()) if te else NullKernel()
+        self.te_rhs = te_gradflux
+
+        def te_lift(fout):
+            te = self.te_handle()
+            return be.kernel(
+                'te_lift', te[0], tplargs | {'ktype': 'linear'}, self.neles,
+                self._scal_fpts, self.scal_upts[fout],
+                **self._te_mats()) if te else NullKernel()
+        kernels['te_lift'] = te_lift

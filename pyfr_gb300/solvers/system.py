@@ -249,6 +249,28 @@ class BaseSystem:
                 kernels[kn].extend(k)
         return kernels
 
+    # The kernels of a right-hand side that an element type's own kernel
+    # (te_rhs, tensorele.py) takes the place of
+    _general_kernels = ('tgradpcoru_upts', 'tgradcoru_upts', 'tdisf_fused',
+                        'gradcoru_fpts', 'tdisf', 'tdivtpcorf', 'tdivtconf',
+                        'negdivconf')
+
+    def _get_rhs_kernels(self, uinbank, foutbank):
+        """The kernels of one right-hand side: for the element types that
+        have one their own kernel, te_rhs, else the general ones."""
+        k = self._get_kernels(uinbank, foutbank)
+        for e in self.ele_map.values():
+            if not e.te_handle():
+                continue
+            tag = f'eles/{id(e)}'
+            for n in self._general_kernels:
+                k[f'eles/{n}'] = [l for l in k[f'eles/{n}']
+                                  if self._ktags[l] != tag]
+            l = e.te_rhs(uinbank, foutbank)
+            self._ktags[l] = tag
+            k['eles/te_rhs'].append(l)
+        return k
+
     def _kdeps(self, kdict, kern, *dnames):
         return [k for n in dnames for k in kdict[n]
                 if self._ktags[kern] == self._ktags[k]]
@@ -457,7 +479,7 @@ class EulerSystem(BaseSystem):
     bcinterscls = EulerBCInters
 
     def _rhs_graphs(self, uinbank, foutbank):
-        k = self._get_kernels(uinbank, foutbank)
+        k = self._get_rhs_kernels(uinbank, foutbank)
 
         def deps(dk, *names):
             return self._kdeps(k, dk, *names)
@@ -480,6 +502,7 @@ class EulerSystem(BaseSystem):
         g_intf.commit()
 
         g_flux_div = self.backend.graph()
+        g_flux_div.add_all(k['eles/te_rhs'])
         # (flux anti-aliasing: the solution at the quadrature points first)
         g_flux_div.add_all(k['eles/qptsu'])
         for l in k['eles/tdisf']:
@@ -515,9 +538,26 @@ class NavierStokesSystem(BaseSystem):
     mpiinterscls = NavierStokesMPIInters
     bcinterscls = NavierStokesBCInters
 
-    def __init__(self, *args, **kwargs):
-        super().__init__(*args, **kwargs)
+    def commit(self):
+        self._setup_element_kernels()
         self._setup_face_gradients()
+        super().commit()
+
+    def _setup_element_kernels(self):
+        """Tell the element types that run on their own kernels which
+        faces' gradients are read: with ldg-beta = +-1/2 the interfaces
+        take one side's."""
+        beta = self.cfg.getfloat('solver-interfaces', 'ldg-beta')
+        read = defaultdict(set)
+        for i in self._sided_inters:
+            sides = [i.lhs] if beta == 0.5 or i.rhs is None else \
+                [i.rhs] if beta == -0.5 else [i.lhs, i.rhs]
+            for s in sides:
+                for et, fidx, _ in s.items():
+                    read[et].add(fidx)
+        for et, e in self.ele_map.items():
+            if e.te_handle():
+                e.set_te_faces(read[et])
 
     def _setup_face_gradients(self):
         """With single-precision state and every element affine, the flux
@@ -562,7 +602,7 @@ class NavierStokesSystem(BaseSystem):
         be.commit()
 
     def _rhs_graphs(self, uinbank, foutbank):
-        k = self._get_kernels(uinbank, foutbank)
+        k = self._get_rhs_kernels(uinbank, foutbank)
 
         def deps(dk, *names):
             return self._kdeps(k, dk, *names)
@@ -598,6 +638,7 @@ class NavierStokesSystem(BaseSystem):
         # Graph 2: corrected gradient, fused flux, face gradients, common
         # flux and the divergence of the partially corrected flux
         g_grad_flux = self.backend.graph()
+        g_grad_flux.add_all(k['eles/te_rhs'])
         g_grad_flux.add_all(k['eles/tgradpcoru_upts'])
         for l in k['eles/tgradcoru_upts']:
             g_grad_flux.add(l, deps=deps(l, 'eles/tgradpcoru_upts'))
@@ -605,8 +646,9 @@ class NavierStokesSystem(BaseSystem):
             g_grad_flux.add(l, deps=deps(l, 'eles/tgradcoru_upts'))
         for l in k['eles/gradcoru_fpts']:
             g_grad_flux.add(l, deps=deps(l, 'eles/tdisf_fused'))
-        g_grad_flux.add_all(k['iint/comm_flux'], deps=k['eles/gradcoru_fpts'])
-        g_grad_flux.add_all(k['bcint/comm_flux'], deps=k['eles/gradcoru_fpts'])
+        fgrads = k['eles/te_rhs'] + k['eles/gradcoru_fpts']
+        g_grad_flux.add_all(k['iint/comm_flux'], deps=fgrads)
+        g_grad_flux.add_all(k['bcint/comm_flux'], deps=fgrads)
         for l in k['eles/tdivtpcorf']:
             g_grad_flux.add(l, deps=deps(l, 'eles/tdisf_fused'))
 
@@ -623,6 +665,7 @@ class NavierStokesSystem(BaseSystem):
 
         # Graph 3: correction and physical divergence
         g_div = self.backend.graph()
+        g_div.add_all(k['eles/te_lift'])
         g_div.add_all(k['eles/tdivtconf'])
         for l in k['eles/negdivconf']:
             g_div.add(l, deps=deps(l, 'eles/tdivtconf'))
