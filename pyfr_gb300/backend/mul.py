@@ -292,12 +292,12 @@ class TensorMulKernels:
         meta['products'] = min(a.products for _, a in arglist)
         if be.mul_precision == 'tf32':
             meta['impl'] = meta['impl'].replace('bf16x3', 'tf32')
-        fn = be.lib.mul_bf16x3_apply
-        calls = [(h, C.addressof(a)) for h, a in arglist]
+        fn, n = be.lib.mul_bf16x3_apply_pieces, len(arglist)
+        hs = (C.c_void_p*n)(*(h for h, _ in arglist))
+        pas = (C.c_void_p*n)(*(C.addressof(a) for _, a in arglist))
 
         def run(stream):
-            for h, pa in calls:
-                fn(h, pa, stream)
+            fn(hs, pas, n, stream)
 
         k = Kernel(run, mats=list(ops) + list(bs) + [out] +
                    ([rowscale] if rowscale is not None else []),

@@ -509,12 +509,25 @@ class Graph:
         self.committed = True
         klist = self._topo_sort()
         self.klist = self.backend.fuse(klist, self._pgroups)
+        self._register()
+        self.stale = True
+
+    def _register(self):
         for k in self.klist:
             if hasattr(k, 'register_graph'):
                 k.register_graph(self)
             else:
                 k.graphs.add(self)
-        self.stale = True
+
+    @classmethod
+    def joined(cls, graphs):
+        """One graph of the kernels of committed graphs that run one after
+        the other: one launch, and no gap between them."""
+        g = cls(graphs[0].backend)
+        g.committed = True
+        g.klist = [k for q in graphs for k in q.klist]
+        g._register()
+        return g
 
     def run(self, stream):
         if not self.use_cuda_graph:

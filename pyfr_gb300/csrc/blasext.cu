@@ -50,6 +50,7 @@ __global__ void __launch_bounds__(BX_BLOCK)
 rkvdh2_kernel(int64_t n, int last, int errest, int first, StageCoef co,
               T *__restrict__ r1, T *__restrict__ r2, T *__restrict__ rold,
               T *__restrict__ rerr) {
+    b200::dependent_entry(co.dtp, r1, r2, rold, rerr);
     double da, db, de;
     stage_products(co, da, db, de);
     const T dta = (T)da, dtb = (T)db, dte = (T)de;
@@ -112,6 +113,7 @@ __global__ void __launch_bounds__(BX_BLOCK)
 rkmixed_kernel(int64_t n, int64_t n4, int last, int first, StageCoef co,
                double *__restrict__ acc, const float *__restrict__ rhs, float *__restrict__ u32,
                double *__restrict__ rold, double *__restrict__ rerr) {
+    b200::dependent_entry(co.dtp, acc, rhs, u32, rold, rerr);
     double da, dtb, dte;
     stage_products(co, da, dtb, dte);
     const float dta = (float)da;
@@ -359,7 +361,7 @@ int rkvdh2(int64_t n, int stage, int nstages, int errest, const double *dtp, dou
     if (errest && (!rold || !rerr))
         return b200::set_error(B200_ERR_ARG, "rkvdh2: error estimate needs rold and rerr");
     const StageCoef co{dtp, dt, stage == nstages - 1 ? 0.0 : a, b, e};
-    rkvdh2_kernel<T><<<grid_for(n), BX_BLOCK, 0, s>>>(n, stage == nstages - 1, errest, stage == 0,
+    b200::launch(rkvdh2_kernel<T>, grid_for(n), BX_BLOCK, 0, s, n, stage == nstages - 1, errest, stage == 0,
                                                       co, r1, r2, rold, rerr);
     B200_CHECK_LAUNCH("rkvdh2");
     return B200_OK;
@@ -537,11 +539,9 @@ static int rkmixed(int64_t n, int stage, int nstages, int errest, const double *
     const int64_t n4 = aligned ? n / 4 : 0;
     const StageCoef co{dtp, dt, last ? 0.0 : a, b, e};
     if (errest)
-        rkmixed_kernel<true><<<grid_for(n / 4 + 1), BX_BLOCK, 0, s>>>(
-            n, n4, last, stage == 0, co, acc, rhs, u32, rold, rerr);
+        b200::launch(rkmixed_kernel<true>, grid_for(n / 4 + 1), BX_BLOCK, 0, s, n, n4, last, stage == 0, co, acc, rhs, u32, rold, rerr);
     else
-        rkmixed_kernel<false><<<grid_for(n / 4 + 1), BX_BLOCK, 0, s>>>(
-            n, n4, last, stage == 0, co, acc, rhs, u32, rold, rerr);
+        b200::launch(rkmixed_kernel<false>, grid_for(n / 4 + 1), BX_BLOCK, 0, s, n, n4, last, stage == 0, co, acc, rhs, u32, rold, rerr);
     B200_CHECK_LAUNCH("rkmixed");
     return B200_OK;
 }

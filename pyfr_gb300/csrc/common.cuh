@@ -32,6 +32,53 @@ __device__ __forceinline__ int64_t load_ix(const void *map, int ix64, int64_t i)
                 : (int64_t)__ldg(static_cast<const int *>(map) + i);
 }
 
+// Launches by programmatic dependent launch: a kernel may be set up while the
+// one before it on the stream ends, and waits at dependent_entry until the
+// kernels before have finished and their writes are visible, which closes most
+// of the gap between short kernels (the 2-D vortex on 40 x 40 cells at p = 3,
+// FP64, 100 kernels a call: 372 -> 352 us; the largest steps are the same).
+// The kernels do not let their dependents start earlier than that: with
+// griddepcontrol.launch_dependents at the start of every kernel the same call
+// took 523 us, the waiting blocks standing in the way of running ones.  Only the
+// pieces of one large tensor-core operator do (early_dependents: their
+// operator's copy into shared memory then overlaps: a step of 12^3 hexahedra at
+// p = 4, eight pieces a right-hand side, 589 -> 536 us).
+//
+// Every kernel that is launched so calls dependent_entry first, with every
+// pointer to memory that other kernels write: no access through it can be
+// moved before the wait, whatever the qualifiers of the pointer.
+template <typename... P>
+__device__ __forceinline__ void dependent_entry(P &...p) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    ((void)([&] { asm volatile("" : "+l"(p)); }()), ...);
+}
+
+__device__ __forceinline__ void early_dependents() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
+template <typename... P, typename... A>
+inline void launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                   A &&...a) {
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c = {};
+    c.gridDim = grid;
+    c.blockDim = block;
+    c.dynamicSmemBytes = smem;
+    c.stream = st;
+    c.attrs = attr;
+    // (in captured graphs, where the chains of short kernels are: a single
+    // kernel launched from the host again and again, a 20 x 40 tensor-core
+    // apply of 24 us, takes 1.4% longer so)
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    c.numAttrs = cudaStreamIsCapturing(st, &cap) == cudaSuccess &&
+                 cap == cudaStreamCaptureStatusActive;
+    // (a failure is left for the caller's cudaGetLastError)
+    (void)cudaLaunchKernelEx(&c, kernel, static_cast<P>(a)...);
+}
+
 inline unsigned ceil_div(int64_t a, int64_t b) { return (unsigned)((a + b - 1) / b); }
 
 // FP32 <-> FP64 conversions on the integer pipes.  GB300's FP64 unit is

@@ -66,6 +66,7 @@ template <typename T, int EPI>
 __global__ void __launch_bounds__(MUL_WARPS * 32)
 mul_csr_kernel(MulHandle h, const T *__restrict__ b, int64_t ldb, T *__restrict__ c,
                int64_t ldc, int64_t ncol, T alpha, T beta, int vec) {
+    b200::dependent_entry(b, c);
     extern __shared__ __align__(16) unsigned char smem_raw[];
     T *bs = reinterpret_cast<T *>(smem_raw);   // [k][MUL_NCOL]
 
@@ -192,6 +193,7 @@ template <int EPI, int CPL>
 __global__ void __launch_bounds__(MUL_WARPS * 32)
 mul_fx_kernel(MulHandle h, const double *__restrict__ b, int64_t ldb, double *__restrict__ c,
               int64_t ldc, int64_t ncol, double alpha, double beta, int vec) {
+    b200::dependent_entry(b, c);
     using I = typename FxPair<CPL>::I;
     constexpr int NC = 32 * CPL;
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -359,13 +361,13 @@ void launch_fx(const MulHandle &h, const double *b, int64_t ldb, double *c, int6
     const unsigned grid = b200::ceil_div(ncol, 32 * CPL);
     const size_t smem = (size_t)h.k * 32 * CPL * sizeof(double);
     if (alpha == 1.0 && beta == 0.0)
-        mul_fx_kernel<EPI_SET, CPL><<<grid, MUL_WARPS * 32, smem, s>>>(h, b, ldb, c, ldc, ncol, alpha, beta, vec);
+        b200::launch(mul_fx_kernel<EPI_SET, CPL>, grid, MUL_WARPS * 32, smem, s, h, b, ldb, c, ldc, ncol, alpha, beta, vec);
     else if (alpha == 1.0 && beta == 1.0)
-        mul_fx_kernel<EPI_ADD, CPL><<<grid, MUL_WARPS * 32, smem, s>>>(h, b, ldb, c, ldc, ncol, alpha, beta, vec);
+        b200::launch(mul_fx_kernel<EPI_ADD, CPL>, grid, MUL_WARPS * 32, smem, s, h, b, ldb, c, ldc, ncol, alpha, beta, vec);
     else if (beta == 0.0)
-        mul_fx_kernel<EPI_SCALE, CPL><<<grid, MUL_WARPS * 32, smem, s>>>(h, b, ldb, c, ldc, ncol, alpha, beta, vec);
+        b200::launch(mul_fx_kernel<EPI_SCALE, CPL>, grid, MUL_WARPS * 32, smem, s, h, b, ldb, c, ldc, ncol, alpha, beta, vec);
     else
-        mul_fx_kernel<EPI_GENERAL, CPL><<<grid, MUL_WARPS * 32, smem, s>>>(h, b, ldb, c, ldc, ncol, alpha, beta, vec);
+        b200::launch(mul_fx_kernel<EPI_GENERAL, CPL>, grid, MUL_WARPS * 32, smem, s, h, b, ldb, c, ldc, ncol, alpha, beta, vec);
 }
 
 // The operator's fixed-point form (rows, entries), or false where it does
@@ -440,13 +442,13 @@ int launch_mul(const MulHandle *h, const T *b, int64_t ldb, T *c, int64_t ldc, i
         }
     }
     if (alpha == T(1) && beta == T(0))
-        mul_csr_kernel<T, EPI_SET><<<grid, MUL_WARPS * 32, smem, s>>>(*h, b, ldb, c, ldc, ncol, alpha, beta, vec);
+        b200::launch(mul_csr_kernel<T, EPI_SET>, grid, MUL_WARPS * 32, smem, s, *h, b, ldb, c, ldc, ncol, alpha, beta, vec);
     else if (alpha == T(1) && beta == T(1))
-        mul_csr_kernel<T, EPI_ADD><<<grid, MUL_WARPS * 32, smem, s>>>(*h, b, ldb, c, ldc, ncol, alpha, beta, vec);
+        b200::launch(mul_csr_kernel<T, EPI_ADD>, grid, MUL_WARPS * 32, smem, s, *h, b, ldb, c, ldc, ncol, alpha, beta, vec);
     else if (beta == T(0))
-        mul_csr_kernel<T, EPI_SCALE><<<grid, MUL_WARPS * 32, smem, s>>>(*h, b, ldb, c, ldc, ncol, alpha, beta, vec);
+        b200::launch(mul_csr_kernel<T, EPI_SCALE>, grid, MUL_WARPS * 32, smem, s, *h, b, ldb, c, ldc, ncol, alpha, beta, vec);
     else
-        mul_csr_kernel<T, EPI_GENERAL><<<grid, MUL_WARPS * 32, smem, s>>>(*h, b, ldb, c, ldc, ncol, alpha, beta, vec);
+        b200::launch(mul_csr_kernel<T, EPI_GENERAL>, grid, MUL_WARPS * 32, smem, s, *h, b, ldb, c, ldc, ncol, alpha, beta, vec);
     B200_CHECK_LAUNCH("mul_csr_kernel");
     return B200_OK;
 }

@@ -294,6 +294,7 @@ struct UmmaArgs {
     const double *rk_dtp;
     double rk_dt, rk_a, rk_b;
     int rk;
+    int early;          // let the next kernel's blocks start beside this one
 };
 
 // 32 columns of one TMEM lane quadrant (32x32b shape, 32 repetitions):
@@ -376,6 +377,11 @@ __global__ void __launch_bounds__(NTHREADS, 1) mul_umma_kernel(const __grid_cons
     const uint32_t SBO_OP = (uint32_t)p.kfull * (TF32 ? 32 : 16), LBO = 128;
     const uint32_t SBO_D = TF32 ? KC * 32 : SBO_CHUNK;
 
+    // The kernels before have finished and their writes are visible (the
+    // producer's own wait comes after its copy of the operator, which is
+    // constant); the bounded waits below count from here
+    if (warp != WARP_PROD) b200::dependent_entry();
+
     if (warp == WARP_PROD) {
         // ---- producer: operator image once, then the FP32 chunks of B ----
         if (lane == 0) bar_arrive_tx(bar(BAR_A), imgbytes);
@@ -388,6 +394,11 @@ __global__ void __launch_bounds__(NTHREADS, 1) mul_umma_kernel(const __grid_cons
                 bulk_g2s(sbase + L.a_hi + a0, p.aimg + a0, nb, bar(BAR_A));
             }
         }
+        // (the operator's copy runs beside the end of the kernels before; of
+        // several pieces of one operator the next one's does so from the
+        // start of this one)
+        if (p.early) b200::early_dependents();
+        b200::dependent_entry();
         if (lane == 0) {
             // (ring stage s and phase ph of chunk j, advanced per chunk: no
             // 64-bit divisions on the hand-off path)
@@ -1024,7 +1035,7 @@ int b200_mul_bf16x3_destroy(void *handle) {
     return B200_OK;
 }
 
-int b200_mul_bf16x3_apply(void *handle, const b200_mul_bf16x3_args_t *a, void *stream) {
+static int umma_apply(void *handle, const b200_mul_bf16x3_args_t *a, int early, void *stream) {
     UmmaHandle *h = (UmmaHandle *)handle;
     if (!h || !a || !a->err) return b200::set_error(B200_ERR_ARG, "mul_bf16x3: null handle/args");
     if (a->ncol <= 0 || a->nbatch == 0) return B200_OK;
@@ -1089,19 +1100,36 @@ int b200_mul_bf16x3_apply(void *handle, const b200_mul_bf16x3_args_t *a, void *s
     p.rk = a->rk_stage; p.rk_acc = a->rk_acc; p.rk_u = a->rk_u; p.rk_dtp = a->rk_dt_dev;
     p.rk_dt = a->rk_dt; p.rk_a = a->rk_a; p.rk_b = a->rk_b;
     p.ldc = a->ldc;
+    p.early = early;
 
     const int64_t ntiles = p.ntc * p.nbatch;
     const unsigned grid = (unsigned)(ntiles < g_sm_count ? ntiles : g_sm_count);
     const cudaStream_t st = (cudaStream_t)stream;
     if (h->tf32 && p.rk)
-        mul_umma_kernel<true, true><<<grid, NTHREADS, h->smem_bytes, st>>>(p);
+        b200::launch(mul_umma_kernel<true, true>, grid, NTHREADS, h->smem_bytes, st, p);
     else if (h->tf32)
-        mul_umma_kernel<true, false><<<grid, NTHREADS, h->smem_bytes, st>>>(p);
+        b200::launch(mul_umma_kernel<true, false>, grid, NTHREADS, h->smem_bytes, st, p);
     else if (p.rk)
-        mul_umma_kernel<false, true><<<grid, NTHREADS, h->smem_bytes, st>>>(p);
+        b200::launch(mul_umma_kernel<false, true>, grid, NTHREADS, h->smem_bytes, st, p);
     else
-        mul_umma_kernel<false, false><<<grid, NTHREADS, h->smem_bytes, st>>>(p);
+        b200::launch(mul_umma_kernel<false, false>, grid, NTHREADS, h->smem_bytes, st, p);
     B200_CHECK_LAUNCH("mul_umma_kernel");
+    return B200_OK;
+}
+
+int b200_mul_bf16x3_apply(void *handle, const b200_mul_bf16x3_args_t *a, void *stream) {
+    return umma_apply(handle, a, 0, stream);
+}
+
+int b200_mul_bf16x3_apply_pieces(void *const *handles, const b200_mul_bf16x3_args_t *const *a,
+                                 int n, void *stream) {
+    if (!handles || !a || n < 0)
+        return b200::set_error(B200_ERR_ARG, "mul_bf16x3_apply_pieces: bad arguments");
+    for (int i = 0; i < n; i++) {
+        // (every piece but the last is followed by one whose start it allows)
+        const int rc = umma_apply(handles[i], a[i], i + 1 < n, stream);
+        if (rc) return rc;
+    }
     return B200_OK;
 }
 

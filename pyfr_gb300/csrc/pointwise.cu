@@ -64,6 +64,7 @@ template <int ND, typename T, bool DIAG>
 __global__ void __launch_bounds__(PW_BLOCK)
 tflux_euler_kernel(int nupts, int64_t neles, T gamma, const T *__restrict__ u, int64_t ldu,
                    T *__restrict__ f, int64_t ldf, ElemGeom<T> geo) {
+    b200::dependent_entry(u, f);
     constexpr int NV = ND + 2;
     const int64_t e = (int64_t)blockIdx.x * PW_BLOCK + threadIdx.x;
     const int upt = blockIdx.y;
@@ -88,6 +89,7 @@ template <int ND, typename T, bool MOVING, bool DIAG>
 __global__ void __launch_bounds__(PW_BLOCK)
 tflux_euler_shift_kernel(int nupts, int64_t neles, b200::GasK<T> gas, const T *__restrict__ u,
                          int64_t ldu, T *__restrict__ f, int64_t ldf, ElemGeom<T> geo) {
+    b200::dependent_entry(u, f);
     constexpr int NV = ND + 2;
     const int64_t e = (int64_t)blockIdx.x * PW_BLOCK + threadIdx.x;
     const int upt = blockIdx.y;
@@ -166,6 +168,7 @@ __global__ void __launch_bounds__(PW_BLOCK)
 tflux_ns_kernel(int nupts, int64_t neles, b200::GasK<T> gas, const T *__restrict__ u, int64_t ldu,
                 T *__restrict__ f, int64_t ldf, T *__restrict__ gradu, int64_t ldg,
                 ElemGeom<T> geo, const T *__restrict__ av, int64_t lda, int gradwb) {
+    b200::dependent_entry(u, f, gradu, av);
     constexpr int NV = ND + 2;
     const int64_t e = (int64_t)blockIdx.x * PW_BLOCK + threadIdx.x;
     const int upt = blockIdx.y;
@@ -246,6 +249,7 @@ tflux_ns_kernel(int nupts, int64_t neles, b200::GasK<T> gas, const T *__restrict
 template <int ND, typename T>
 __global__ void __launch_bounds__(PW_BLOCK)
 gradcoru_kernel(int nupts, int64_t neles, T *__restrict__ gradu, int64_t ldg, ElemGeom<T> geo) {
+    b200::dependent_entry(gradu);
     constexpr int NV = ND + 2;
     const int64_t e = (int64_t)blockIdx.x * PW_BLOCK + threadIdx.x;
     const int upt = blockIdx.y;
@@ -274,6 +278,7 @@ template <typename T>
 __global__ void __launch_bounds__(PW_BLOCK)
 negdivconf_kernel(int nvars, int64_t neles, T *__restrict__ r, int64_t ldr,
                   const T *__restrict__ rcpdjac, int64_t ldj) {
+    b200::dependent_entry(r);
     const int64_t e = (int64_t)blockIdx.x * PW_BLOCK + threadIdx.x;
     const int upt = blockIdx.y;
     if (e >= neles) return;
@@ -440,6 +445,7 @@ template <int RS, int ND, typename T>
 __global__ void __launch_bounds__(PW_BLOCK)
 intcflux_euler_kernel(int64_t n, T gamma, T p_min, ScalView<T> vl, ScalView<T> vr, int ix64,
                       const T *__restrict__ nl, int64_t ldn, int nl_unit) {
+    b200::dependent_entry(vl.base, vr.base);
     constexpr int NV = ND + 2;
     const int64_t i = (int64_t)blockIdx.x * PW_BLOCK + threadIdx.x;
     if (i >= n) return;
@@ -472,6 +478,7 @@ template <int ND, typename T, bool MOVING>
 __global__ void __launch_bounds__(PW_BLOCK)
 intcflux_euler_shift_kernel(int64_t n, b200::GasK<T> gas, ScalView<T> vl, ScalView<T> vr,
                             int ix64, const T *__restrict__ nl, int64_t ldn, int nl_unit) {
+    b200::dependent_entry(vl.base, vr.base);
     constexpr int NV = ND + 2;
     const int64_t i = (int64_t)blockIdx.x * PW_BLOCK + threadIdx.x;
     if (i >= n) return;
@@ -552,6 +559,7 @@ intcflux_ns_kernel(int64_t n, b200::GasK<T> gas, T beta, T tau, int sides, int p
                    ScalView<T> vl, ScalView<T> vr,
                    VectView<T> gl, VectView<T> gr, int ix64, const T *__restrict__ nl,
                    int64_t ldn, int nl_unit, ScalView<T> va, FaceMetrics<T> fm) {
+    b200::dependent_entry(vl.base, vr.base, gl.base, gr.base, va.base);
     constexpr int NV = ND + 2;
     const int64_t i = (int64_t)blockIdx.x * PW_BLOCK + threadIdx.x;
     if (i >= n) return;
@@ -715,6 +723,7 @@ template <typename T>
 __global__ void __launch_bounds__(PW_BLOCK)
 intconu_kernel(int64_t n, int nvars, T beta, ScalView<T> lin, ScalView<T> rin,
                ScalView<T> lout, ScalView<T> rout, int ix64, int both) {
+    b200::dependent_entry(lin.base, rin.base, lout.base, rout.base);
     const int64_t i = (int64_t)blockIdx.x * PW_BLOCK + threadIdx.x;
     if (i >= n) return;
 
@@ -780,7 +789,7 @@ int tflux_euler(int ndims, int nupts, int64_t neles, int linear, double gamma, c
     auto geo = make_geom<T>(linear, smats, lds, nullptr, 0, verts, ldv, upts, ldup);
     dim3 grid(b200::ceil_div(neles, PW_BLOCK), nupts);
     const bool ok = with_form(ndims, linear, [&](auto nd, auto diag) {
-        tflux_euler_kernel<nd(), T, diag()><<<grid, PW_BLOCK, 0, st>>>(nupts, neles, (T)gamma, u, ldu, f, ldf, geo);
+        b200::launch(tflux_euler_kernel<nd(), T, diag()>, grid, PW_BLOCK, 0, st, nupts, neles, (T)gamma, u, ldu, f, ldf, geo);
     });
     if (!ok) return b200::set_error(B200_ERR_ARG, "tflux: ndims must be 2 or 3");
     B200_CHECK_LAUNCH("tflux_euler");
@@ -830,7 +839,7 @@ int tflux_ns(int ndims, int nupts, int64_t neles, int linear, const b200_gas_t *
                                "tflux_ns: the reference state must be at rest");
     dim3 grid(b200::ceil_div(neles, PW_BLOCK), nupts);
     const bool ok = with_form(ndims, linear, [&](auto nd, auto diag) {
-        tflux_ns_kernel<nd(), T, diag()><<<grid, PW_BLOCK, 0, st>>>(nupts, neles, g, u, ldu, f, ldf, gradu, ldg, geo, av, lda, gradwb);
+        b200::launch(tflux_ns_kernel<nd(), T, diag()>, grid, PW_BLOCK, 0, st, nupts, neles, g, u, ldu, f, ldf, gradu, ldg, geo, av, lda, gradwb);
     });
     if (!ok) return b200::set_error(B200_ERR_ARG, "tflux_ns: ndims must be 2 or 3");
     B200_CHECK_LAUNCH("tflux_ns");
@@ -847,9 +856,9 @@ int gradcoru(int ndims, int nupts, int64_t neles, int linear, T *gradu, int64_t 
     auto geo = make_geom<T>(linear, smats, lds, rcpdjac, ldr, verts, ldv, upts, ldup);
     dim3 grid(b200::ceil_div(neles, PW_BLOCK), nupts);
     if (ndims == 2)
-        gradcoru_kernel<2, T><<<grid, PW_BLOCK, 0, st>>>(nupts, neles, gradu, ldg, geo);
+        b200::launch(gradcoru_kernel<2, T>, grid, PW_BLOCK, 0, st, nupts, neles, gradu, ldg, geo);
     else if (ndims == 3)
-        gradcoru_kernel<3, T><<<grid, PW_BLOCK, 0, st>>>(nupts, neles, gradu, ldg, geo);
+        b200::launch(gradcoru_kernel<3, T>, grid, PW_BLOCK, 0, st, nupts, neles, gradu, ldg, geo);
     else
         return b200::set_error(B200_ERR_ARG, "gradcoru: ndims must be 2 or 3");
     B200_CHECK_LAUNCH("gradcoru");
@@ -868,9 +877,9 @@ int intcflux_euler(int ndims, int64_t n, int rsolver, double gamma, double p_min
     const bool ok = b200::with_rsolver(rsolver, [&](auto rsc) {
         constexpr int RS = decltype(rsc)::value;
         if (ndims == 2)
-            intcflux_euler_kernel<RS, 2, T><<<grid, PW_BLOCK, 0, st>>>(n, (T)gamma, (T)p_min, l, r, ix64, nl, ldn, nl_unit);
+            b200::launch(intcflux_euler_kernel<RS, 2, T>, grid, PW_BLOCK, 0, st, n, (T)gamma, (T)p_min, l, r, ix64, nl, ldn, nl_unit);
         else
-            intcflux_euler_kernel<RS, 3, T><<<grid, PW_BLOCK, 0, st>>>(n, (T)gamma, (T)p_min, l, r, ix64, nl, ldn, nl_unit);
+            b200::launch(intcflux_euler_kernel<RS, 3, T>, grid, PW_BLOCK, 0, st, n, (T)gamma, (T)p_min, l, r, ix64, nl, ldn, nl_unit);
     });
     if (!ok) return b200::set_error(B200_ERR_ARG, "intcflux: unknown Riemann solver %d", rsolver);
     B200_CHECK_LAUNCH("intcflux_euler");
@@ -890,9 +899,9 @@ int tflux_euler_shift(int ndims, int nupts, int64_t neles, int linear, const b20
     dim3 grid(b200::ceil_div(neles, PW_BLOCK), nupts);
     const bool ok = with_form(ndims, linear, [&](auto nd, auto diag) {
         if (g.moving)
-            tflux_euler_shift_kernel<nd(), T, true, diag()><<<grid, PW_BLOCK, 0, st>>>(nupts, neles, g, u, ldu, f, ldf, geo);
+            b200::launch(tflux_euler_shift_kernel<nd(), T, true, diag()>, grid, PW_BLOCK, 0, st, nupts, neles, g, u, ldu, f, ldf, geo);
         else
-            tflux_euler_shift_kernel<nd(), T, false, diag()><<<grid, PW_BLOCK, 0, st>>>(nupts, neles, g, u, ldu, f, ldf, geo);
+            b200::launch(tflux_euler_shift_kernel<nd(), T, false, diag()>, grid, PW_BLOCK, 0, st, nupts, neles, g, u, ldu, f, ldf, geo);
     });
     if (!ok) return b200::set_error(B200_ERR_ARG, "tflux: ndims must be 2 or 3");
     B200_CHECK_LAUNCH("tflux_euler_shift");
@@ -911,13 +920,13 @@ int intcflux_euler_shift(int ndims, int64_t n, const b200_gas_t *gas, T *ul_base
     const auto g = b200::gas_consts<T>(*reinterpret_cast<const Gas *>(gas));
     unsigned grid = b200::ceil_div(n, PW_BLOCK);
     if (ndims == 2 && g.moving)
-        intcflux_euler_shift_kernel<2, T, true><<<grid, PW_BLOCK, 0, st>>>(n, g, l, r, ix64, nl, ldn, nl_unit);
+        b200::launch(intcflux_euler_shift_kernel<2, T, true>, grid, PW_BLOCK, 0, st, n, g, l, r, ix64, nl, ldn, nl_unit);
     else if (ndims == 2)
-        intcflux_euler_shift_kernel<2, T, false><<<grid, PW_BLOCK, 0, st>>>(n, g, l, r, ix64, nl, ldn, nl_unit);
+        b200::launch(intcflux_euler_shift_kernel<2, T, false>, grid, PW_BLOCK, 0, st, n, g, l, r, ix64, nl, ldn, nl_unit);
     else if (g.moving)
-        intcflux_euler_shift_kernel<3, T, true><<<grid, PW_BLOCK, 0, st>>>(n, g, l, r, ix64, nl, ldn, nl_unit);
+        b200::launch(intcflux_euler_shift_kernel<3, T, true>, grid, PW_BLOCK, 0, st, n, g, l, r, ix64, nl, ldn, nl_unit);
     else
-        intcflux_euler_shift_kernel<3, T, false><<<grid, PW_BLOCK, 0, st>>>(n, g, l, r, ix64, nl, ldn, nl_unit);
+        b200::launch(intcflux_euler_shift_kernel<3, T, false>, grid, PW_BLOCK, 0, st, n, g, l, r, ix64, nl, ldn, nl_unit);
     B200_CHECK_LAUNCH("intcflux_euler_shift");
     return B200_OK;
 }
@@ -953,11 +962,11 @@ int intcflux_ns(int ndims, int64_t n, int rsolver, const b200_gas_t *gas, double
     const bool ok = b200::with_rsolver(rsolver, [&](auto rsc) {
         constexpr int RS = decltype(rsc)::value;
         if (ndims == 2)
-            intcflux_ns_kernel<RS, 2, T, false><<<grid, PW_BLOCK, 0, st>>>(n, g, (T)beta, (T)tau, sides, pen, l, r, gl, gr, ix64, nl, ldn, nl_unit, va, fm);
+            b200::launch(intcflux_ns_kernel<RS, 2, T, false>, grid, PW_BLOCK, 0, st, n, g, (T)beta, (T)tau, sides, pen, l, r, gl, gr, ix64, nl, ldn, nl_unit, va, fm);
         else if (!fm.m)
-            intcflux_ns_kernel<RS, 3, T, false><<<grid, PW_BLOCK, 0, st>>>(n, g, (T)beta, (T)tau, sides, pen, l, r, gl, gr, ix64, nl, ldn, nl_unit, va, fm);
+            b200::launch(intcflux_ns_kernel<RS, 3, T, false>, grid, PW_BLOCK, 0, st, n, g, (T)beta, (T)tau, sides, pen, l, r, gl, gr, ix64, nl, ldn, nl_unit, va, fm);
         else
-            intcflux_ns_kernel<RS, 3, T, true><<<grid, PW_BLOCK, 0, st>>>(n, g, (T)beta, (T)tau, sides, pen, l, r, gl, gr, ix64, nl, ldn, nl_unit, va, fm);
+            b200::launch(intcflux_ns_kernel<RS, 3, T, true>, grid, PW_BLOCK, 0, st, n, g, (T)beta, (T)tau, sides, pen, l, r, gl, gr, ix64, nl, ldn, nl_unit, va, fm);
     });
     if (!ok) return b200::set_error(B200_ERR_ARG, "intcflux: unknown Riemann solver %d", rsolver);
     B200_CHECK_LAUNCH("intcflux_ns");
@@ -973,8 +982,7 @@ int intconu(int nvars, int64_t n, double beta, const T *lin_base, const void *li
     ScalView<T> li{const_cast<T *>(lin_base), lin_map};
     ScalView<T> ri{const_cast<T *>(rin_base), rin_map};
     ScalView<T> lo{lout_base, lout_map}, ro{rout_base, rout_map};
-    intconu_kernel<T><<<b200::ceil_div(n, PW_BLOCK), PW_BLOCK, 0, st>>>(
-        n, nvars, (T)beta, li, ri, lo, ro, ix64, both);
+    b200::launch(intconu_kernel<T>, b200::ceil_div(n, PW_BLOCK), PW_BLOCK, 0, st, n, nvars, (T)beta, li, ri, lo, ro, ix64, both);
     B200_CHECK_LAUNCH("intconu");
     return B200_OK;
 }
@@ -1080,7 +1088,7 @@ int b200_negdivconf_f64(int nvars, int nupts, int64_t neles, double *r, int64_t 
                         const double *rcpdjac, int64_t ldj, void *stream) {
     if (neles <= 0 || nupts <= 0) return B200_OK;
     dim3 grid(b200::ceil_div(neles, PW_BLOCK), nupts);
-    negdivconf_kernel<double><<<grid, PW_BLOCK, 0, (cudaStream_t)stream>>>(nvars, neles, r, ldr, rcpdjac, ldj);
+    b200::launch(negdivconf_kernel<double>, grid, PW_BLOCK, 0, (cudaStream_t)stream, nvars, neles, r, ldr, rcpdjac, ldj);
     B200_CHECK_LAUNCH("negdivconf");
     return B200_OK;
 }
@@ -1089,7 +1097,7 @@ int b200_negdivconf_f32(int nvars, int nupts, int64_t neles, float *r, int64_t l
                         const float *rcpdjac, int64_t ldj, void *stream) {
     if (neles <= 0 || nupts <= 0) return B200_OK;
     dim3 grid(b200::ceil_div(neles, PW_BLOCK), nupts);
-    negdivconf_kernel<float><<<grid, PW_BLOCK, 0, (cudaStream_t)stream>>>(nvars, neles, r, ldr, rcpdjac, ldj);
+    b200::launch(negdivconf_kernel<float>, grid, PW_BLOCK, 0, (cudaStream_t)stream, nvars, neles, r, ldr, rcpdjac, ldj);
     B200_CHECK_LAUNCH("negdivconf");
     return B200_OK;
 }

@@ -180,6 +180,12 @@ struct Fx {
     __device__ __forceinline__ double value(int sc) const {
         return fixed_to_f64(hh + (w >> 31), sc);
     }
+    // The same with the conversion on the FP64 unit (kernels that leave it idle)
+    __device__ __forceinline__ double value_cvt(int sc) const {
+        const long long t = hh + (w >> 31);
+        const double y = (double)t;
+        return t == 0 ? 0.0 : __hiloint2double(__double2hiint(y) + sc * (1 << 20), __double2loint(y));
+    }
 };
 
 // The operands of a line, as the products take them
@@ -193,7 +199,7 @@ struct Operands<float, NI> {
 #pragma unroll
         for (int j = 0; j < NI; j++) x[j] = v[j];
     }
-    template <int NO>
+    template <bool CVT = false, int NO>
     __device__ __forceinline__ float row(const Mat<float, NO, NI> &m, int i) const {
         float acc = m.d[i][0] * x[0];
 #pragma unroll
@@ -221,7 +227,7 @@ struct Operands<double, NI> {
             if (wild) b[j] = make_int2(__double2hiint(v[j]), __double2loint(v[j]));
         }
     }
-    template <int NO>
+    template <bool CVT = false, int NO>
     __device__ __forceinline__ double row(const Mat<double, NO, NI> &m, int i) const {
         if (wild) {
             double y = 0.0;
@@ -235,7 +241,7 @@ struct Operands<double, NI> {
 #pragma unroll
         for (int j = 0; j < NI; j++)
             if (!absent<NO, NI>(i, j)) s.mad(m.a[i][j], b[j]);
-        return s.value(emax - m.s - 1051);
+        return CVT ? s.value_cvt(emax - m.s - 1051) : s.value(emax - m.s - 1051);
     }
 };
 
@@ -269,10 +275,10 @@ __device__ __forceinline__ void visit(const Line<T, ND, Q> &P, int l, V &&vis) {
     const int y = l % Q, z = l / Q;
 #pragma unroll
     for (int j = 0; j < Q; j++)
-        if (FLUX) vis.along(0, l * Q + j, j);
+        if constexpr (FLUX) vis.along(0, l * Q + j, j);
 #pragma unroll
     for (int e = 0; e < 2; e++)
-        if (LIFT) vis.along_end(0, l, e);
+        if constexpr (LIFT) vis.along_end(0, l, e);
 #pragma unroll
     for (int d = 1; d < ND; d++) {
         const int row = d == 1 ? y : z;
@@ -283,15 +289,15 @@ __device__ __forceinline__ void visit(const Line<T, ND, Q> &P, int l, V &&vis) {
             const int b = P.base(d, ld), st = P.stride(d);
 #pragma unroll
             for (int j = 0; j < Q; j++)
-                if (FLUX) vis.across(d, b + j * st, i, row, j);
+                if constexpr (FLUX) vis.across(d, b + j * st, i, row, j);
 #pragma unroll
             for (int e = 0; e < 2; e++)
-                if (LIFT) vis.across_end(d, ld, e, i, row);
+                if constexpr (LIFT) vis.across_end(d, ld, e, i, row);
         }
     }
 #pragma unroll
     for (int i = 0; i < Q; i++)
-        if (KEEP) vis.keep(l * Q + i, i);
+        if constexpr (KEEP) vis.keep(l * Q + i, i);
 }
 
 template <typename T, int ND, int Q, typename G>
@@ -382,8 +388,14 @@ struct FixedVisit {
         // (an absent entry is zero)
         s[i].mad(P.div.a[row][j], *reinterpret_cast<const int2 *>(g.at(d, p)));
     }
-    __device__ __forceinline__ void along_end(int, int, int) {}
-    __device__ __forceinline__ void across_end(int, int, int, int, int) {}
+    __device__ __forceinline__ void along_end(int d, int l, int e) {
+        const int2 b = *reinterpret_cast<const int2 *>(g.end_at(d, l, e));
+#pragma unroll
+        for (int i = 0; i < Q; i++) s[i].mad(P.div.a[i][Q + e], b);
+    }
+    __device__ __forceinline__ void across_end(int d, int l, int e, int i, int row) {
+        s[i].mad(P.div.a[row][Q + e], *reinterpret_cast<const int2 *>(g.end_at(d, l, e)));
+    }
     __device__ __forceinline__ void keep(int, int) {}
 };
 
@@ -413,64 +425,171 @@ __device__ __forceinline__ void div_line(const Line<double, ND, Q> &P, const G &
     for (int i = 0; i < Q; i++) v.s[i].clear();
     visit<double, ND, Q, FLUX, LIFT, KEEP>(P, l, v);
 #pragma unroll
-    for (int i = 0; i < Q; i++) y[i] = v.s[i].value(v.emax - P.div.s - 1049);
+    for (int i = 0; i < Q; i++) y[i] = v.s[i].value_cvt(v.emax - P.div.s - 1049);
 }
 
 // ---- kernels ------------------------------------------------------------------
 
-constexpr int TE_BLOCK = 256;
-
-// Elements of a block: 64 bytes of a variable's row, two sectors, so that
-// several blocks' elements fit an SM's shared memory
-template <typename T>
-constexpr int te_elems() { return 64 / (int)sizeof(T); }
-
-// u at both ends of every line.  A warp takes one line and variable of 32
-// elements; the lines of one block of elements are consecutive, so that the
-// three reads of a point are near each other in time.
+// Elements and threads of a block of the kernels that keep elements in shared
+// memory.  64 or 32 bytes of a variable's row per block (whole sectors), so
+// that the gradients of two or three blocks' elements fit an SM; the groups of
+// threads of one element (NT/E) divide the lines and points of an element into
+// nearly full rounds (p = 3 hexahedra, FP64: 48 groups for 48 lines).
 template <typename T, int ND, int Q>
-__global__ void __launch_bounds__(TE_BLOCK)
-te_interp_kernel(const __grid_constant__ Line<T, ND, Q> P, int64_t neles, int nchunk,
-                 const T *__restrict__ u, int64_t ldu, T *__restrict__ f, int64_t ldf) {
+struct Tile {
+    static constexpr int E = 64 / (int)sizeof(T) / (ND == 3 && Q == 5 ? 2 : 1);
+    static constexpr int NT = ND == 2 ? 256 : (sizeof(T) == 8 && Q == 4) ? 384 : 256;
+    static constexpr int G = NT / E, MINB = NT == 384 ? 2 : 3;
+};
+
+// Rows of a matrix from a column on; ld in bytes, below 2^32 (checked on the
+// host), so that a row's address is one multiply-add
+template <typename T>
+struct Rows {
+    T *p;
+    unsigned ld;
+    __device__ __forceinline__ T &operator()(unsigned row) const {
+        return *reinterpret_cast<T *>(
+            reinterpret_cast<uintptr_t>(p) + (unsigned long long)row * ld);
+    }
+    __device__ __forceinline__ Rows at(int64_t col) const { return Rows{p + col, ld}; }
+};
+
+// u at both ends of every line.  A warp takes a line of 32 elements, of one
+// variable (SPLIT: too few lines to fill the GPU otherwise) or of all, which
+// saves most of the index arithmetic; the lines of one block of elements are
+// consecutive, so that the three reads of a point are near each other in time.
+constexpr int TE_WARPS = 8;
+
+template <typename T, int ND, int Q, bool SPLIT>
+__global__ void __launch_bounds__(TE_WARPS * 32)
+te_interp_kernel(const __grid_constant__ Line<T, ND, Q> P, int64_t neles, unsigned nchunk,
+                 Rows<const T> u, Rows<T> f) {
+    b200::dependent_entry(u.p, f.p);
     using K = Line<T, ND, Q>;
+    constexpr int NV = K::NV, VS = SPLIT ? NV : 1;
     const int lane = threadIdx.x & 31;
-    const int64_t blk = blockIdx.x / nchunk;
-    const int t = (int)(blockIdx.x % nchunk) * (TE_BLOCK / 32) + (threadIdx.x >> 5);
-    if (t >= K::NV * ND * K::L || blk * 32 + lane >= neles) return;
-    const int v = t % K::NV, d = t / K::NV / K::L, l = t / K::NV % K::L;
+    const unsigned blk = blockIdx.x / nchunk;
+    const int t = (int)(blockIdx.x - blk * nchunk) * TE_WARPS + (threadIdx.x >> 5);
+    if (t >= VS * ND * K::L || (int64_t)blk * 32 + lane >= neles) return;
+    const int v0 = t % VS, d = t / VS / K::L, l = t / VS % K::L;
     const int p0 = K::base(d, l), st = K::stride(d);
-    const int64_t col = (blk * K::NV + v) * 32 + lane;
-    T x[Q];
+    const int64_t col = ((int64_t)blk * NV + v0) * 32 + lane;
+    const T *pu[Q];
+    T *pf[2];
 #pragma unroll
-    for (int i = 0; i < Q; i++) x[i] = u[(p0 + i * st) * ldu + col];
-    const Operands<T, Q> b(x);
+    for (int i = 0; i < Q; i++) pu[i] = &u.at(col)(p0 + i * st);
 #pragma unroll
-    for (int e = 0; e < 2; e++) f[P.fpt[d][l][e] * ldf + col] = b.row(P.interp, e);
+    for (int e = 0; e < 2; e++) pf[e] = &f.at(col)(P.fpt[d][l][e]);
+#pragma unroll
+    for (int v = 0; v < NV / VS; v++) {
+        T x[Q];
+#pragma unroll
+        for (int i = 0; i < Q; i++) x[i] = pu[i][v * 32];
+        const Operands<T, Q> b(x);
+#pragma unroll
+        for (int e = 0; e < 2; e++) pf[e][v * 32] = b.template row<true>(P.interp, e);
+    }
 }
 
 // Fluxes of one element in shared memory, component c of point p at
-// sm[(c NPS + p) E]; NPS odd, so that two neighbouring components or points lie
-// in different halves of the banks.  Ends and old values in global memory.
+// sm[(c NPS + p) E], and the common flux of flux point q at ends[(v NFS + q) E];
+// NPS and NFS odd, so that two neighbouring components or points lie in
+// different halves of the banks.
 template <typename T, int ND, int Q, int E>
 struct SmemFlux {
-    static constexpr int NPS = ipow(Q, ND) | 1;
+    static constexpr int NV = ND + 2, NPS = ipow(Q, ND) | 1,
+                         NFS = (2 * ND * ipow(Q, ND - 1)) | 1;
     const Line<T, ND, Q> &P;
-    const T *sm;            // + element
+    const T *sm, *ends;     // + element
     int v;
-    const T *fc;            // + column of the element and variable
-    int64_t ldf;
     __device__ __forceinline__ const T *at(int d, int p) const {
-        return sm + ((d * (ND + 2) + v) * NPS + p) * E;
+        return sm + ((d * NV + v) * NPS + p) * E;
+    }
+    __device__ __forceinline__ const T *end_at(int d, int l, int e) const {
+        return ends + (v * NFS + P.fpt[d][l][e]) * E;
     }
     __device__ __forceinline__ T flux(int d, int p) const { return *at(d, p); }
-    __device__ __forceinline__ int flux_hi(int d, int p) const {
-        return reinterpret_cast<const int *>(at(d, p))[1] & 0x7fffffff;
-    }
-    __device__ __forceinline__ T end(int d, int l, int e) const {
-        return fc[P.fpt[d][l][e] * ldf];
-    }
-    __device__ __forceinline__ T old(int) const { return T(0); }
+    __device__ __forceinline__ T end(int d, int l, int e) const { return *end_at(d, l, e); }
 };
+
+// x in fixed point over the largest magnitude mx of its element and variable, in
+// its own place (left as it is where that is out of range)
+__device__ __forceinline__ void fix_in_place(double &x, int mx) {
+    if (!out_of_range(mx)) *reinterpret_cast<int2 *>(&x) = split<58>(x, max(mx >> 20, 64));
+}
+__device__ __forceinline__ void fix_in_place(float &, int) {}
+
+// The divergence at the points of x-line l from the element's fluxes (and,
+// LIFT, common fluxes) in shared memory; FP64: in fixed point over mx
+template <bool LIFT, int ND, int Q, int E>
+__device__ __forceinline__ void smem_div(const Line<float, ND, Q> &P,
+                                         const SmemFlux<float, ND, Q, E> &g, int l, int,
+                                         float (&y)[Q]) {
+    SumVisit<float, ND, Q, SmemFlux<float, ND, Q, E>> f{P, g, {}};
+    visit<float, ND, Q, true, LIFT, false>(P, l, f);
+#pragma unroll
+    for (int i = 0; i < Q; i++) y[i] = f.y[i];
+}
+
+template <bool LIFT, int ND, int Q, int E>
+__device__ __forceinline__ void smem_div(const Line<double, ND, Q> &P,
+                                         const SmemFlux<double, ND, Q, E> &g, int l, int mx,
+                                         double (&y)[Q]) {
+    using G = SmemFlux<double, ND, Q, E>;
+    if (out_of_range(mx)) {
+        SumVisit<double, ND, Q, G> f{P, g, {}};
+        visit<double, ND, Q, true, LIFT, false>(P, l, f);
+#pragma unroll
+        for (int i = 0; i < Q; i++) y[i] = f.y[i];
+        return;
+    }
+    FixedVisit<ND, Q, G> f{P, g, {}};
+#pragma unroll
+    for (int i = 0; i < Q; i++) f.s[i].clear();
+    visit<double, ND, Q, true, LIFT, false>(P, l, f);
+    const int sc = max(mx >> 20, 64) - P.div.s - 1049;
+#pragma unroll
+    for (int i = 0; i < Q; i++) y[i] = f.s[i].value(sc);
+}
+
+// The same at point p alone, from the values as they are: in two dimensions
+// there are few lines for the threads of an element, and a point each, over its
+// own operands' exponent, is a shorter chain than the x-line's (40 x 40 cells at
+// p = 3, where the kernel is one chain of latencies)
+template <int ND, int Q, int E>
+__device__ __forceinline__ double smem_div_point(const Line<double, ND, Q> &P,
+                                                 const SmemFlux<double, ND, Q, E> &g, int p) {
+    double x[ND][Q + 2];
+    int row[ND], mx = 0;
+#pragma unroll
+    for (int d = 0; d < ND; d++) {
+        const int st = P.stride(d), b = p - (row[d] = p / st % Q) * st;
+        const int l = d == 0 ? p / Q : d == 1 ? p / (Q * Q) * Q + p % Q : b;
+#pragma unroll
+        for (int j = 0; j < Q + 2; j++) {
+            x[d][j] = j < Q ? g.flux(d, b + j * st) : g.end(d, l, j - Q);
+            mx = max(mx, hi_abs(x[d][j]));
+        }
+    }
+    if (out_of_range(mx)) {
+        double y = 0.0;
+#pragma unroll
+        for (int d = 0; d < ND; d++)
+#pragma unroll
+            for (int j = 0; j < Q + 2; j++)
+                if (!absent<Q, Q + 2>(row[d], j)) y = fma(P.div.d[row[d]][j], x[d][j], y);
+        return y;
+    }
+    const int emax = max(mx >> 20, 64);
+    Fx s;
+    s.clear();
+#pragma unroll
+    for (int d = 0; d < ND; d++)
+#pragma unroll
+        for (int j = 0; j < Q + 2; j++) s.mad(P.div.a[row[d]][j], split<58>(x[d][j], emax));
+    return s.value_cvt(emax - P.div.s - 1049);
+}
 
 // The gradient in physical space, (1/|J|) S^T tg
 template <int ND, typename T>
@@ -491,28 +610,56 @@ __device__ __forceinline__ void grad_to_phys(const T s[ND][ND], T rcp, const T t
     }
 }
 
+// The flux ft in reference space into the element's shared memory (sme + c NPS
+// E: component c of the point), and the largest magnitude of each variable
+template <typename T, int ND, bool DIAG, int STRIDE>
+__device__ __forceinline__ void put_tflux(T *sme, const T s[ND][ND], const T ft[ND][ND + 2],
+                                          int mx[ND + 2]) {
+#pragma unroll
+    for (int v = 0; v < ND + 2; v++)
+#pragma unroll
+        for (int i = 0; i < ND; i++) {
+            T acc = s[i][DIAG ? i : 0] * ft[DIAG ? i : 0][v];
+#pragma unroll
+            for (int k = 1; k < ND; k++)
+                if (!DIAG) acc += s[i][k] * ft[k][v];
+            sme[(i * (ND + 2) + v) * STRIDE] = acc;
+            if constexpr (sizeof(T) == 8) mx[v] = max(mx[v], hi_abs(acc));
+        }
+}
+
 // facemask: bit 2 d + end, the faces whose gradient is wanted on any element;
 // refgrad: it stays in reference space (the interface kernels transform it).
 // r may be u, and gf's first component may be c: every element's values are
 // read before they are written.
-template <typename T, int ND, int Q, bool DIAG, int E>
-__global__ void __launch_bounds__(TE_BLOCK)
+//
+// What bounds it (p = 3 hexahedra, FP64): the flux, 105 FP64 operations a point
+// on the narrow FP64 unit, and about as much issue time for the lines on the
+// integer pipes; the blocks of an SM are in different phases, so that the two
+// run side by side.
+template <typename T, int ND, int Q, bool DIAG>
+__global__ void __launch_bounds__((Tile<T, ND, Q>::NT), (Tile<T, ND, Q>::MINB))
 te_gradflux_kernel(const __grid_constant__ Line<T, ND, Q> P, int64_t neles, b200::GasK<T> gas,
-                   const T *u, int64_t ldu, const T *c, int64_t ldc, T *gf, int64_t ldg,
-                   unsigned facemask, int refgrad, ElemGeom<T> geo, T *r, int64_t ldr) {
+                   Rows<const T> u, Rows<const T> c, Rows<T> gf, unsigned facemask, int refgrad,
+                   ElemGeom<T> geo, Rows<T> r) {
+    b200::dependent_entry(u.p, c.p, gf.p, r.p);
     using K = Line<T, ND, Q>;
     constexpr int NV = K::NV, NP = K::NP, L = K::L, NFP = K::NFP, NPS = NP | 1;
-    constexpr int G = TE_BLOCK / E;
+    constexpr int E = Tile<T, ND, Q>::E, G = Tile<T, ND, Q>::G;
+    constexpr bool FIXED = sizeof(T) == 8;
+    constexpr int VU = FIXED ? 1 : NV;      // unrolling over the variables
     extern __shared__ __align__(16) unsigned char smem_raw[];
     T *sm = reinterpret_cast<T *>(smem_raw);
-
-    constexpr bool FIXED = sizeof(T) == 8;
     __shared__ int top[NV][E];      // largest flux of each variable
 
     const int el = threadIdx.x % E, grp = threadIdx.x / E;
     const int64_t e = (int64_t)blockIdx.x * E + el;
     const bool live = e < neles;
     const int64_t col0 = soa_off(live ? e : 0, 0, NV);
+    u = u.at(col0);
+    c = c.at(col0);
+    gf = gf.at(col0);
+    r = r.at(col0);
     T *const sme = sm + el;
     if (FIXED)
         for (int v = grp; v < NV; v += G) top[v][el] = 0;
@@ -526,34 +673,42 @@ te_gradflux_kernel(const __grid_constant__ Line<T, ND, Q> P, int64_t neles, b200
             sd[d] = geo.rcpdjac[e] * geo.smats[(int64_t)d * geo.lds + soa_off(e, d, ND)];
     }
     const bool scale = DIAG && !refgrad, own = DIAG || refgrad;
-    for (int t = grp; t < NV * ND * L; t += G) {
-        const int v = t % NV, d = t / NV / L, l = t / NV % L;
+    for (int t = grp; t < ND * L; t += G) {
+        const int d = t / L, l = t % L;
         const int p0 = K::base(d, l), st = K::stride(d);
-        T x[Q + 2];
-#pragma unroll
-        for (int i = 0; i < Q; i++) x[i] = live ? u[(p0 + i * st) * ldu + col0 + v * 32] : T(0);
-#pragma unroll
-        for (int i = 0; i < 2; i++)
-            x[Q + i] = live ? c[P.fpt[d][l][i] * ldc + col0 + v * 32] : T(0);
-        const Operands<T, Q + 2> b(x);
+        const int q0 = P.fpt[d][l][0], q1 = P.fpt[d][l][1];
         const T s = DIAG ? (d == 0 ? sd[0] : d == 1 ? sd[1] : sd[ND - 1]) : T(1);
+        const T *pu[Q], *pc[2] = {&c(q0), &c(q1)};
+        T *pg[2] = {&gf(d * NFP + q0), &gf(d * NFP + q1)};
 #pragma unroll
-        for (int i = 0; i < Q; i++) {
-            T y = b.row(P.grad, i);
-            if (scale) y *= s;
-            sme[((d * NV + v) * NPS + p0 + i * st) * E] = y;
-        }
-        // The derivative along the line at its ends, where the metric leaves
-        // it a component of its own.  (Where the first component's rows are
-        // those of c, this thread alone reads the value that it replaces.)
-        if (own && live) {
+        for (int i = 0; i < Q; i++) pu[i] = &u(p0 + i * st);
+        T *out = sme + (d * NV * NPS + p0) * E;
+#pragma unroll VU
+        for (int v = 0; v < NV; v++) {
+            T x[Q + 2];
 #pragma unroll
-            for (int i = 0; i < 2; i++)
-                if ((facemask >> (2 * d + i)) & 1) {
-                    const T y = b.row(P.gradend, i);
-                    gf[(int64_t)(d * NFP + P.fpt[d][l][i]) * ldg + col0 + v * 32] =
-                        scale ? s * y : y;
-                }
+            for (int i = 0; i < Q; i++) x[i] = live ? pu[i][v * 32] : T(0);
+#pragma unroll
+            for (int i = 0; i < 2; i++) x[Q + i] = live ? pc[i][v * 32] : T(0);
+            const Operands<T, Q + 2> b(x);
+#pragma unroll
+            for (int i = 0; i < Q; i++) {
+                T y = b.row(P.grad, i);
+                if (scale) y *= s;
+                out[(v * NPS + i * st) * E] = y;
+            }
+            // The derivative along the line at its ends, where the metric
+            // leaves it a component of its own.  (Where the first component's
+            // rows are those of c, this thread alone reads the value that it
+            // replaces.)
+            if (own && live) {
+#pragma unroll
+                for (int i = 0; i < 2; i++)
+                    if ((facemask >> (2 * d + i)) & 1) {
+                        const T y = b.row(P.gradend, i);
+                        pg[i][v * 32] = scale ? s * y : y;
+                    }
+            }
         }
     }
     __syncthreads();
@@ -576,28 +731,39 @@ te_gradflux_kernel(const __grid_constant__ Line<T, ND, Q> P, int64_t neles, b200
     }
 
     // The gradient at the flux points that are read
-    for (int t = grp; t < NV * ND * ND * L; t += G) {
-        const int v = t % NV, k = t / NV % ND, d = t / (NV * ND) / L, l = t / (NV * ND) % L;
+    for (int t = grp; t < ND * L; t += G) {
+        const int d = t / L, l = t % L;
         const unsigned need = (facemask >> (2 * d)) & 3;
-        if (!need || (own && k == d)) continue;
+        if (!need) continue;
         const int p0 = K::base(d, l), st = K::stride(d);
-        T x[Q];
+        const int q0 = P.fpt[d][l][0], q1 = P.fpt[d][l][1];
+#pragma unroll 1
+        for (int k = 0; k < ND; k++) {
+            if (own && k == d) continue;
+            const T *in = sme + (k * NV * NPS + p0) * E;
+            T *pg[2] = {&gf(k * NFP + q0), &gf(k * NFP + q1)};
+#pragma unroll VU
+            for (int v = 0; v < NV; v++) {
+                T x[Q];
 #pragma unroll
-        for (int i = 0; i < Q; i++) x[i] = sme[((k * NV + v) * NPS + p0 + i * st) * E];
-        const Operands<T, Q> b(x);
+                for (int i = 0; i < Q; i++) x[i] = in[(v * NPS + i * st) * E];
+                const Operands<T, Q> b(x);
 #pragma unroll
-        for (int i = 0; i < 2; i++)
-            if (live && ((need >> i) & 1))
-                gf[(int64_t)(k * NFP + P.fpt[d][l][i]) * ldg + col0 + v * 32] = b.row(P.interp, i);
+                for (int i = 0; i < 2; i++)
+                    if (live && ((need >> i) & 1)) pg[i][v * 32] = b.row(P.interp, i);
+            }
+        }
     }
     __syncthreads();
 
     // The flux in reference space, in the place of the gradient
+    int mx[NV] = {};
     for (int p = grp; p < NP; p += G) {
         T uu[NV], gr[ND][NV], ft[ND][NV], s[ND][ND] = {}, rcp = T(0);
         if (live) b200::elem_metrics<ND, T, DIAG>(geo, NP, p, e, s, rcp, !DIAG && refgrad);
+        const T *pu = &u(p);
 #pragma unroll
-        for (int v = 0; v < NV; v++) uu[v] = live ? u[p * ldu + col0 + v * 32] : T(1);
+        for (int v = 0; v < NV; v++) uu[v] = live ? pu[v * 32] : T(1);
 #pragma unroll
         for (int d = 0; d < ND; d++)
 #pragma unroll
@@ -616,158 +782,155 @@ te_gradflux_kernel(const __grid_constant__ Line<T, ND, Q> P, int64_t neles, b200
             grad_to_phys<ND, T>(s, rcp, tg, gr);
         }
         b200::ns_flux<ND, T>(uu, gr, ft, gas);
+        put_tflux<T, ND, DIAG, NPS * E>(sme + p * E, s, ft, mx);
+    }
+    // FP64: in fixed point over the largest flux of the element and variable
+    // (each value is an operand of the outputs of a line, and is split once)
+    if (FIXED) {
 #pragma unroll
-        for (int v = 0; v < NV; v++) {
-            int mx = 0;
+        for (int v = 0; v < NV; v++) atomicMax(&top[v][el], mx[v]);
+        __syncthreads();
 #pragma unroll
-            for (int i = 0; i < ND; i++) {
-                T acc = s[i][DIAG ? i : 0] * ft[DIAG ? i : 0][v];
+        for (int v = 0; v < NV; v++) mx[v] = top[v][el];
+        for (int p = grp; p < NP; p += G)
 #pragma unroll
-                for (int k = 1; k < ND; k++)
-                    if (!DIAG) acc += s[i][k] * ft[k][v];
-                sme[((i * NV + v) * NPS + p) * E] = acc;
-                if constexpr (FIXED) mx = max(mx, hi_abs(acc));
-            }
-            if constexpr (FIXED) atomicMax(&top[v][el], mx);
-        }
+            for (int k = 0; k < ND * NV; k++) fix_in_place(sme[(k * NPS + p) * E], mx[k % NV]);
     }
     __syncthreads();
-
-    // FP64: the fluxes in fixed point over the largest of the element's and
-    // variable's (each is an operand of the lines of Q points, and is split
-    // once), except where that is out of range
-    if constexpr (FIXED) {
-        for (int p = grp; p < NP; p += G) {
-#pragma unroll
-            for (int v = 0; v < NV; v++) {
-                const int mx = top[v][el];
-                if (out_of_range(mx)) continue;
-#pragma unroll
-                for (int i = 0; i < ND; i++) {
-                    double *q = &sme[((i * NV + v) * NPS + p) * E];
-                    *reinterpret_cast<int2 *>(q) = split<58>(*q, max(mx >> 20, 64));
-                }
-            }
-        }
-        __syncthreads();
-    }
 
     // The divergence along the lines of every direction
     for (int t = grp; t < NV * L; t += G) {
         const int v = t % NV, l = t / NV;
-        const SmemFlux<T, ND, Q, E> g{P, sme, v, nullptr, 0};
+        const SmemFlux<T, ND, Q, E> g{P, sme, nullptr, v};
         T y[Q];
-        bool done = false;
-        if constexpr (FIXED) {
-            const int mx = top[v][el];
-            if (!out_of_range(mx)) {
-                FixedVisit<ND, Q, SmemFlux<T, ND, Q, E>> f{P, g, {}};
-#pragma unroll
-                for (int i = 0; i < Q; i++) f.s[i].clear();
-                visit<T, ND, Q, true, false, false>(P, l, f);
-#pragma unroll
-                for (int i = 0; i < Q; i++)
-                    y[i] = f.s[i].value(max(mx >> 20, 64) - P.div.s - 1049);
-                done = true;
-            }
-        }
-        if (!done) {
-            SumVisit<T, ND, Q, SmemFlux<T, ND, Q, E>> f{P, g, {}};
-            visit<T, ND, Q, true, false, false>(P, l, f);
-#pragma unroll
-            for (int i = 0; i < Q; i++) y[i] = f.y[i];
-        }
+        smem_div<false>(P, g, l, FIXED ? top[v][el] : 0, y);
 #pragma unroll
         for (int i = 0; i < Q; i++)
-            if (live) r[(l * Q + i) * ldr + col0 + v * 32] = y[i];
+            if (live) r.at(v * 32)(l * Q + i) = y[i];
     }
 }
 
 // Euler: flux at the points, divergence, lift and scaling.  r may be u.
-template <typename T, int ND, int Q, bool DIAG, int E>
-__global__ void __launch_bounds__(TE_BLOCK)
-te_euler_kernel(const __grid_constant__ Line<T, ND, Q> P, int64_t neles, T gamma, const T *u,
-                int64_t ldu, const T *__restrict__ fc, int64_t ldf, ElemGeom<T> geo, T *r,
-                int64_t ldr) {
+template <typename T, int ND, int Q, bool DIAG>
+__global__ void __launch_bounds__((Tile<T, ND, Q>::NT), (Tile<T, ND, Q>::MINB))
+te_euler_kernel(const __grid_constant__ Line<T, ND, Q> P, int64_t neles, T gamma, Rows<const T> u,
+                Rows<const T> fc, ElemGeom<T> geo, Rows<T> r) {
+    b200::dependent_entry(u.p, fc.p, r.p);
     using K = Line<T, ND, Q>;
-    constexpr int NV = K::NV, NP = K::NP, L = K::L, NPS = NP | 1;
-    constexpr int G = TE_BLOCK / E;
+    constexpr int NV = K::NV, NP = K::NP, L = K::L, NFP = K::NFP;
+    constexpr int E = Tile<T, ND, Q>::E, G = Tile<T, ND, Q>::G;
+    using SF = SmemFlux<T, ND, Q, E>;
+    constexpr int NPS = SF::NPS, NFS = SF::NFS;
+    // (by points in two dimensions, FP64: no common exponent)
+    constexpr bool POINTS = sizeof(T) == 8 && ND == 2, FIXED = sizeof(T) == 8 && !POINTS;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     T *sm = reinterpret_cast<T *>(smem_raw);
+    __shared__ int top[NV][E];
 
     const int el = threadIdx.x % E, grp = threadIdx.x / E;
     const int64_t e = (int64_t)blockIdx.x * E + el;
     const bool live = e < neles;
     const int64_t col0 = soa_off(live ? e : 0, 0, NV);
-    T *const sme = sm + el;
+    u = u.at(col0);
+    fc = fc.at(col0);
+    r = r.at(col0);
+    T *const sme = sm + el, *const sce = sme + ND * NV * NPS * E;
+    if (FIXED) {
+        for (int v = grp; v < NV; v += G) top[v][el] = 0;
+        __syncthreads();
+    }
 
+    int mx[NV] = {};
+    // (from the last group on, so that in two dimensions other threads than
+    // the points' take the flux points)
+    for (int q = G - 1 - grp; q < NFP; q += G) {
+        const T *pf = &fc(q);
+#pragma unroll
+        for (int v = 0; v < NV; v++) {
+            const T x = live ? pf[v * 32] : T(0);
+            sce[(v * NFS + q) * E] = x;
+            if constexpr (FIXED) mx[v] = max(mx[v], hi_abs(x));
+        }
+    }
     for (int p = grp; p < NP; p += G) {
         T uu[NV], ft[ND][NV], s[ND][ND] = {}, rcp, pr, vel[ND];
         if (live) b200::elem_metrics<ND, T, DIAG>(geo, NP, p, e, s, rcp, false);
+        const T *pu = &u(p);
 #pragma unroll
-        for (int v = 0; v < NV; v++) uu[v] = live ? u[p * ldu + col0 + v * 32] : T(1);
+        for (int v = 0; v < NV; v++) uu[v] = live ? pu[v * 32] : T(1);
         b200::inviscid_flux<ND, T>(uu, ft, pr, vel, gamma);
+        put_tflux<T, ND, DIAG, NPS * E>(sme + p * E, s, ft, mx);
+    }
+    if (FIXED) {
 #pragma unroll
-        for (int i = 0; i < ND; i++)
+        for (int v = 0; v < NV; v++) atomicMax(&top[v][el], mx[v]);
+        __syncthreads();
 #pragma unroll
-            for (int v = 0; v < NV; v++) {
-                T acc = s[i][DIAG ? i : 0] * ft[DIAG ? i : 0][v];
+        for (int v = 0; v < NV; v++) mx[v] = top[v][el];
+        for (int q = G - 1 - grp; q < NFP; q += G)
 #pragma unroll
-                for (int k = 1; k < ND; k++)
-                    if (!DIAG) acc += s[i][k] * ft[k][v];
-                sme[((i * NV + v) * NPS + p) * E] = acc;
-            }
+            for (int v = 0; v < NV; v++) fix_in_place(sce[(v * NFS + q) * E], mx[v]);
+        for (int p = grp; p < NP; p += G)
+#pragma unroll
+            for (int k = 0; k < ND * NV; k++) fix_in_place(sme[(k * NPS + p) * E], mx[k % NV]);
     }
     __syncthreads();
     if (!live) return;
 
+    if constexpr (POINTS) {
+        for (int t = grp; t < NV * NP; t += G) {
+            const int v = t % NV, p = t / NV;
+            const T rj = geo.rcpdjac[(geo.linear >= b200::GEOM_PER_ELEMENT ? 0 : p * geo.ldr) + e];
+            r.at(v * 32)(p) = -rj * smem_div_point(P, SF{P, sme, sce, v}, p);
+        }
+    } else {
     for (int t = grp; t < NV * L; t += G) {
         const int v = t % NV, l = t / NV;
-        const SmemFlux<T, ND, Q, E> g{P, sme, v, fc + col0 + v * 32, ldf};
+        const SF g{P, sme, sce, v};
         T y[Q];
-        div_line<true, true, false>(P, g, l, y);
+        smem_div<true>(P, g, l, FIXED ? top[v][el] : 0, y);
 #pragma unroll
         for (int i = 0; i < Q; i++) {
             const int p = l * Q + i;
             const T rj = geo.rcpdjac[(geo.linear >= b200::GEOM_PER_ELEMENT ? 0 : p * geo.ldr) + e];
-            r[p * ldr + col0 + v * 32] = -rj * y[i];
+            r.at(v * 32)(p) = -rj * y[i];
         }
+    }
     }
 }
 
 template <typename T, int ND, int Q>
 struct GlobalEnds {
     const Line<T, ND, Q> &P;
-    const T *fc, *r;        // + column of the element and variable
-    int64_t ldf, ldr;
+    Rows<const T> fc, r;        // + column of the element and variable
     __device__ __forceinline__ T flux(int, int) const { return T(0); }
     __device__ __forceinline__ int flux_hi(int, int) const { return 0; }
-    __device__ __forceinline__ T end(int d, int l, int e) const {
-        return fc[P.fpt[d][l][e] * ldf];
-    }
-    __device__ __forceinline__ T old(int p) const { return r[p * ldr]; }
+    __device__ __forceinline__ T end(int d, int l, int e) const { return fc(P.fpt[d][l][e]); }
+    __device__ __forceinline__ T old(int p) const { return r(p); }
 };
 
 // R = -(1/|J|) (R + M3 Fc): a warp takes an x-line and variable of 32 elements
 template <typename T, int ND, int Q>
-__global__ void __launch_bounds__(TE_BLOCK)
-te_lift_kernel(const __grid_constant__ Line<T, ND, Q> P, int64_t neles, int nchunk,
-               const T *__restrict__ fc, int64_t ldf, const T *__restrict__ rcpdjac, int64_t ldj,
-               T *__restrict__ r, int64_t ldr) {
+__global__ void __launch_bounds__(TE_WARPS * 32)
+te_lift_kernel(const __grid_constant__ Line<T, ND, Q> P, int64_t neles, unsigned nchunk,
+               Rows<const T> fc, const T *__restrict__ rcpdjac, int64_t ldj, Rows<T> r) {
+    b200::dependent_entry(fc.p, r.p);
     using K = Line<T, ND, Q>;
     const int lane = threadIdx.x & 31;
-    const int64_t blk = blockIdx.x / nchunk;
-    const int t = (int)(blockIdx.x % nchunk) * (TE_BLOCK / 32) + (threadIdx.x >> 5);
-    if (t >= K::NV * K::L || blk * 32 + lane >= neles) return;
+    const unsigned blk = blockIdx.x / nchunk;
+    const int t = (int)(blockIdx.x - blk * nchunk) * TE_WARPS + (threadIdx.x >> 5);
+    const int64_t e = (int64_t)blk * 32 + lane;
+    if (t >= K::NV * K::L || e >= neles) return;
     const int v = t % K::NV, l = t / K::NV;
-    const int64_t col = (blk * K::NV + v) * 32 + lane;
-    const GlobalEnds<T, ND, Q> g{P, fc + col, r + col, ldf, ldr};
+    const int64_t col = ((int64_t)blk * K::NV + v) * 32 + lane;
+    r = r.at(col);
+    const GlobalEnds<T, ND, Q> g{P, fc.at(col), Rows<const T>{r.p, r.ld}};
     T y[Q];
     div_line<false, true, true>(P, g, l, y);
 #pragma unroll
     for (int i = 0; i < Q; i++) {
         const int p = l * Q + i;
-        r[p * ldr + col] = -rcpdjac[p * ldj + blk * 32 + lane] * y[i];
+        r(p) = -rcpdjac[p * ldj + e] * y[i];
     }
 }
 
@@ -820,23 +983,38 @@ int opt_in(Fn fn, size_t smem) {
                                                  (int)smem), "te: smem attribute");
 }
 
+// Shared memory of an element block: the fluxes, and with ends the common flux
 template <typename T, int ND, int Q>
-constexpr size_t te_smem() {
-    return (size_t)ND * (ND + 2) * (ipow(Q, ND) | 1) * te_elems<T>() * sizeof(T);
+constexpr size_t te_smem(bool ends) {
+    using SF = SmemFlux<T, ND, Q, Tile<T, ND, Q>::E>;
+    return (size_t)(ND * SF::NV * SF::NPS + (ends ? SF::NV * SF::NFS : 0)) *
+           Tile<T, ND, Q>::E * sizeof(T);
 }
 
 template <typename T>
 int te_opt_in(const TeHandle &h) {
     int rc = 0;
     with_shape(h, [&](auto nd, auto nq) {
-        constexpr int ND = nd(), Q = nq(), E = te_elems<T>();
-        constexpr size_t s = te_smem<T, ND, Q>();
-        rc = opt_in(te_gradflux_kernel<T, ND, Q, true, E>, s);
-        if (!rc) rc = opt_in(te_gradflux_kernel<T, ND, Q, false, E>, s);
-        if (!rc) rc = opt_in(te_euler_kernel<T, ND, Q, true, E>, s);
-        if (!rc) rc = opt_in(te_euler_kernel<T, ND, Q, false, E>, s);
+        constexpr int ND = nd(), Q = nq();
+        constexpr size_t s = te_smem<T, ND, Q>(false), se = te_smem<T, ND, Q>(true);
+        rc = opt_in(te_gradflux_kernel<T, ND, Q, true>, s);
+        if (!rc) rc = opt_in(te_gradflux_kernel<T, ND, Q, false>, s);
+        if (!rc) rc = opt_in(te_euler_kernel<T, ND, Q, true>, se);
+        if (!rc) rc = opt_in(te_euler_kernel<T, ND, Q, false>, se);
     });
     return rc;
+}
+
+// Rows with a leading dimension of ld values, which has to fit the kernels'
+// 32 bits of bytes
+template <typename T>
+bool rows(Rows<T> &r, T *p, int64_t ld) {
+    r = Rows<T>{p, (unsigned)(ld * (int64_t)sizeof(T))};
+    return ld >= 0 && ld * (int64_t)sizeof(T) < (1ll << 32);
+}
+
+int too_wide(const char *what) {
+    return b200::set_error(B200_ERR_UNSUPPORTED, "%s: rows of 4 GiB and more", what);
 }
 
 int check_te(const void *handle, const char *what, std::initializer_list<const void *> ptrs) {
@@ -852,11 +1030,21 @@ int te_interp(void *handle, int64_t neles, const T *u, int64_t ldu, T *f, int64_
     int rc = check_te(handle, "te_interp", {u, f});
     if (rc || neles <= 0) return rc;
     const TeHandle &h = *(const TeHandle *)handle;
+    Rows<const T> ur;
+    Rows<T> fr;
+    if (!rows(ur, u, ldu) || !rows(fr, f, ldf)) return too_wide("te_interp");
     with_shape(h, [&](auto nd, auto nq) {
-        using K = Line<T, nd(), nq()>;
-        const int nchunk = (int)b200::ceil_div(K::NV * nd() * K::L, TE_BLOCK / 32);
-        te_interp_kernel<T, nd(), nq()><<<b200::ceil_div(neles, 32) * nchunk, TE_BLOCK, 0, st>>>(
-            line_of<T, nd(), nq()>(h), neles, nchunk, u, ldu, f, ldf);
+        constexpr int ND = nd(), Q = nq();
+        using K = Line<T, ND, Q>;
+        const unsigned nblk = b200::ceil_div(neles, 32);
+        // (a warp per line and variable below 16 warps an SM)
+        const bool split = (int64_t)nblk * ND * K::L < 152 * 16;
+        const unsigned nchunk = b200::ceil_div(ND * K::L * (split ? K::NV : 1), TE_WARPS);
+        const auto P = line_of<T, ND, Q>(h);
+        if (split)
+            b200::launch(te_interp_kernel<T, ND, Q, true>, nblk * nchunk, TE_WARPS * 32, 0, st, P, neles, nchunk, ur, fr);
+        else
+            b200::launch(te_interp_kernel<T, ND, Q, false>, nblk * nchunk, TE_WARPS * 32, 0, st, P, neles, nchunk, ur, fr);
     });
     B200_CHECK_LAUNCH("te_interp");
     return B200_OK;
@@ -872,9 +1060,9 @@ int te_geom(int linear, const void *smats, const void *rcpdjac) {
 
 template <typename T>
 int te_gradflux_ns(void *handle, int64_t neles, int linear, const b200_gas_t *gas, const T *u,
-                   int64_t ldu, const T *c, int64_t ldc, T *gf, int64_t ldg, unsigned facemask, int refgrad,
-                   const T *smats, int64_t lds, const T *rcpdjac, int64_t ldj, T *r, int64_t ldr,
-                   cudaStream_t st) {
+                   int64_t ldu, const T *c, int64_t ldc, T *gf, int64_t ldg, unsigned facemask,
+                   int refgrad, const T *smats, int64_t lds, const T *rcpdjac, int64_t ldj, T *r,
+                   int64_t ldr, cudaStream_t st) {
     int rc = check_te(handle, "te_gradflux", {gas, u, c, gf, r});
     if (!rc) rc = te_geom(linear, smats, rcpdjac);
     if (rc || neles <= 0) return rc;
@@ -883,15 +1071,19 @@ int te_gradflux_ns(void *handle, int64_t neles, int linear, const b200_gas_t *ga
     if (g.shifted)
         return b200::set_error(B200_ERR_UNSUPPORTED, "te_gradflux: takes unshifted states");
     const auto geo = b200::make_geom<T>(linear, smats, lds, rcpdjac, ldj, nullptr, 0, nullptr, 0);
+    Rows<const T> ur, cr;
+    Rows<T> gr, rr;
+    if (!rows(ur, u, ldu) || !rows(cr, c, ldc) || !rows(gr, gf, ldg) || !rows(rr, r, ldr))
+        return too_wide("te_gradflux");
     with_shape(h, [&](auto nd, auto nq) {
-        constexpr int ND = nd(), Q = nq(), E = te_elems<T>();
-        const unsigned grid = b200::ceil_div(neles, E);
-        constexpr size_t s = te_smem<T, ND, Q>();
+        constexpr int ND = nd(), Q = nq(), NT = Tile<T, ND, Q>::NT;
+        const unsigned grid = b200::ceil_div(neles, Tile<T, ND, Q>::E);
+        constexpr size_t s = te_smem<T, ND, Q>(false);
         const auto P = line_of<T, ND, Q>(h);
         if (linear == b200::GEOM_DIAGONAL)
-            te_gradflux_kernel<T, ND, Q, true, E><<<grid, TE_BLOCK, s, st>>>(P, neles, g, u, ldu, c, ldc, gf, ldg, facemask, refgrad, geo, r, ldr);
+            b200::launch(te_gradflux_kernel<T, ND, Q, true>, grid, NT, s, st, P, neles, g, ur, cr, gr, facemask, refgrad, geo, rr);
         else
-            te_gradflux_kernel<T, ND, Q, false, E><<<grid, TE_BLOCK, s, st>>>(P, neles, g, u, ldu, c, ldc, gf, ldg, facemask, refgrad, geo, r, ldr);
+            b200::launch(te_gradflux_kernel<T, ND, Q, false>, grid, NT, s, st, P, neles, g, ur, cr, gr, facemask, refgrad, geo, rr);
     });
     B200_CHECK_LAUNCH("te_gradflux");
     return B200_OK;
@@ -906,15 +1098,18 @@ int te_euler(void *handle, int64_t neles, int linear, double gamma, const T *u, 
     if (rc || neles <= 0) return rc;
     const TeHandle &h = *(const TeHandle *)handle;
     const auto geo = b200::make_geom<T>(linear, smats, lds, rcpdjac, ldj, nullptr, 0, nullptr, 0);
+    Rows<const T> ur, fr;
+    Rows<T> rr;
+    if (!rows(ur, u, ldu) || !rows(fr, fc, ldf) || !rows(rr, r, ldr)) return too_wide("te_euler");
     with_shape(h, [&](auto nd, auto nq) {
-        constexpr int ND = nd(), Q = nq(), E = te_elems<T>();
-        const unsigned grid = b200::ceil_div(neles, E);
-        constexpr size_t s = te_smem<T, ND, Q>();
+        constexpr int ND = nd(), Q = nq(), NT = Tile<T, ND, Q>::NT;
+        const unsigned grid = b200::ceil_div(neles, Tile<T, ND, Q>::E);
+        constexpr size_t s = te_smem<T, ND, Q>(true);
         const auto P = line_of<T, ND, Q>(h);
         if (linear == b200::GEOM_DIAGONAL)
-            te_euler_kernel<T, ND, Q, true, E><<<grid, TE_BLOCK, s, st>>>(P, neles, (T)gamma, u, ldu, fc, ldf, geo, r, ldr);
+            b200::launch(te_euler_kernel<T, ND, Q, true>, grid, NT, s, st, P, neles, (T)gamma, ur, fr, geo, rr);
         else
-            te_euler_kernel<T, ND, Q, false, E><<<grid, TE_BLOCK, s, st>>>(P, neles, (T)gamma, u, ldu, fc, ldf, geo, r, ldr);
+            b200::launch(te_euler_kernel<T, ND, Q, false>, grid, NT, s, st, P, neles, (T)gamma, ur, fr, geo, rr);
     });
     B200_CHECK_LAUNCH("te_euler");
     return B200_OK;
@@ -926,11 +1121,14 @@ int te_lift(void *handle, int64_t neles, const T *fc, int64_t ldf, const T *rcpd
     int rc = check_te(handle, "te_lift", {fc, rcpdjac, r});
     if (rc || neles <= 0) return rc;
     const TeHandle &h = *(const TeHandle *)handle;
+    Rows<const T> fr;
+    Rows<T> rr;
+    if (!rows(fr, fc, ldf) || !rows(rr, r, ldr)) return too_wide("te_lift");
     with_shape(h, [&](auto nd, auto nq) {
-        using K = Line<T, nd(), nq()>;
-        const int nchunk = (int)b200::ceil_div(K::NV * K::L, TE_BLOCK / 32);
-        te_lift_kernel<T, nd(), nq()><<<b200::ceil_div(neles, 32) * nchunk, TE_BLOCK, 0, st>>>(
-            line_of<T, nd(), nq()>(h), neles, nchunk, fc, ldf, rcpdjac, ldj, r, ldr);
+        constexpr int ND = nd(), Q = nq();
+        using K = Line<T, ND, Q>;
+        const unsigned nchunk = b200::ceil_div(K::NV * K::L, TE_WARPS);
+        b200::launch(te_lift_kernel<T, ND, Q>, b200::ceil_div(neles, 32) * nchunk, TE_WARPS * 32, 0, st, line_of<T, ND, Q>(h), neles, nchunk, fr, rcpdjac, ldj, rr);
     });
     B200_CHECK_LAUNCH("te_lift");
     return B200_OK;

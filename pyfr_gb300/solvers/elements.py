@@ -360,12 +360,16 @@ class BaseElements:
         when its kernels are made decides.)"""
         be = self._be
         viscous = 'grad_upts' in self._scratch_bufs
-        if be.element_kernels != 'auto' or be.fuse_operators or \
+        tensor = be.mul_precision != 'native' and be.fpdtype == np.float32
+        if be.element_kernels != 'auto' or tensor or \
                 be.ref_state is not None or self.linoff or \
                 not be.precompute_metrics or \
                 getattr(self, 'antialias', False) or \
                 self._srctplargs is not None or \
                 self.cfg.get('solver', 'shock-capturing', 'none') != 'none':
+            return None
+        # (the kernels' rows are below 4 GiB)
+        if self._scal_fpts.leaddim*self._scal_fpts.itemsize >= 2**32:
             return None
         return be.tensor_elements.handle(self.basis, viscous)
 

@@ -14,7 +14,7 @@ import inspect
 
 import numpy as np
 
-from pyfr_gb300.backend.types import Kernel, NullKernel
+from pyfr_gb300.backend.types import Graph, Kernel, NullKernel
 from pyfr_gb300.solvers.elements import EulerElements, NavierStokesElements
 from pyfr_gb300.solvers.inters import (EulerBCInters, EulerIntInters,
                                        EulerMPIInters, NavierStokesBCInters,
@@ -436,8 +436,19 @@ class BaseSystem:
             self.set_time(t)
         for k in self.prepare_kernels(uinbank, t):
             k.run(self.backend.stream)
-        for g in self._rhs_graphs_cached(uinbank, foutbank):
+        for g in self._rhs_launches(uinbank, foutbank):
             self.backend.run_graph(g)
+
+    def _rhs_launches(self, uin, fout):
+        """The right-hand side's graphs as they are launched: as one, where
+        no exchange with other partitions stands between them."""
+        key = ('launches', uin, fout)
+        if key not in self._graph_cache:
+            gs = self._rhs_graphs_cached(uin, fout)
+            if not any(isinstance(g, HostStep) for g in gs):
+                gs = (Graph.joined(gs),)
+            self._graph_cache[key] = gs
+        return self._graph_cache[key]
 
     def preproc_kernels(self, uinbank):
         """Before the first step: filter, then every element's and face's
