@@ -167,6 +167,10 @@ int b200_probe_fp64_fma(int iters, double *flops_per_s, void *stream);
  * (pyfr/backends/cuda/types.py:79-116). */
 int b200_graph_begin_capture(void *stream);
 int b200_graph_end_capture(void *stream, void **gexec);
+/* While a stream is captured: the nodes that what follows on it waits for (at
+ * most max of them), and what follows made to wait for these nodes instead. */
+int b200_graph_capture_last(void *stream, void **nodes, int max, int *n);
+int b200_graph_capture_after(void *stream, void *const *nodes, int n);
 int b200_graph_launch(void *gexec, void *stream);
 int b200_graph_destroy(void *gexec);
 

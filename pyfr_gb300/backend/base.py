@@ -308,6 +308,49 @@ class B200Backend:
             if gc_was_enabled:
                 gc.enable()
 
+    def launcher(self, nodes):
+        """A function enqueueing ``nodes`` on a stream that is being
+        captured: a list of kernels, one after the other, or ``types.Nodes``,
+        each of which the graph then starts when those that it waits for
+        have finished (the capture's own dependencies are set before each
+        kernel: no other streams, no events)."""
+        if not isinstance(nodes, types.Nodes):
+            def launch(stream):
+                for k in nodes:
+                    k.run(stream)
+            return launch
+
+        last, after = self.lib.graph_capture_last, self.lib.graph_capture_after
+        items = nodes.items
+        # (a node that waits for the one before it alone follows it anyway)
+        chained = [deps == [i - 1] for i, (_, deps) in enumerate(items)]
+        used = {d for (_, deps), c in zip(items, chained) if not c
+                for d in deps}
+        ends = set(range(len(items))) - {d for _, deps in items for d in deps}
+        used |= ends
+        buf, n = (C.c_void_p*8)(), C.c_int()
+
+        def launch(stream):
+            def captured():
+                last(stream, buf, len(buf), C.byref(n))
+                return buf[:n.value]
+
+            def follow(handles):
+                after(stream, (C.c_void_p*max(len(handles), 1))(*handles),
+                      len(handles))
+
+            before, got = captured(), {}
+            for i, (k, deps) in enumerate(items):
+                if not chained[i] and i:
+                    follow(sorted({h for d in deps for h in got[d]})
+                           if deps else before)
+                k.run(stream)
+                if i in used:
+                    got[i] = captured()
+            follow(sorted({h for i in ends for h in got[i]}))
+
+        return launch
+
     def release_gexec(self, gexec):
         if gexec:
             release(self.lib.graph_destroy, gexec)

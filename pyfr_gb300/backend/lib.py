@@ -189,6 +189,8 @@ _SIGS = {
     'b200_event_create': [C.POINTER(vp)],
     'b200_event_destroy': [vp],
     'b200_event_record': [vp, vp],
+    'b200_graph_capture_last': [vp, C.POINTER(vp), i32, C.POINTER(i32)],
+    'b200_graph_capture_after': [vp, C.POINTER(vp), i32],
     'b200_event_sync': [vp],
     'b200_event_elapsed': [C.POINTER(f32), vp, vp],
     'b200_probe_fp64_fma': [i32, C.POINTER(f64), vp],

@@ -421,6 +421,24 @@ class UnorderedMetaKernel(MetaKernel):
 # Graphs
 # --------------------------------------------------------------------------
 
+class Nodes:
+    """Kernels with what each waits for: a list of (kernel, positions of
+    the nodes that have to finish before it), in an order that respects the
+    waits."""
+
+    def __init__(self):
+        self.items = []
+
+    def add(self, kern, deps=()):
+        """Append a kernel that waits for the nodes at ``deps``; returns its
+        position."""
+        deps = sorted(set(deps))
+        if deps and not 0 <= deps[0] <= deps[-1] < len(self.items):
+            raise ValueError('A node waits for one that is not before it')
+        self.items.append((kern, deps))
+        return len(self.items) - 1
+
+
 class Graph:
     """A DAG of kernels (``pyfr/backends/base/types.py:343-533``).
 
@@ -436,6 +454,7 @@ class Graph:
         self.kpdeps = {}
         self._pgroups = []
         self.klist = []
+        self._nodes = None
         self.stale = True
         self._gexec = None
         self.use_cuda_graph = backend.use_cuda_graphs
@@ -520,6 +539,17 @@ class Graph:
                 k.graphs.add(self)
 
     @classmethod
+    def of_nodes(cls, backend, nodes):
+        """A committed graph of ``Nodes``: those that do not wait for one
+        another run side by side."""
+        g = cls(backend)
+        g.committed = True
+        g.klist = [k for k, _ in nodes.items]
+        g._nodes = nodes
+        g._register()
+        return g
+
+    @classmethod
     def joined(cls, graphs):
         """One graph of the kernels of committed graphs that run one after
         the other: one launch, and no gap between them."""
@@ -538,7 +568,7 @@ class Graph:
         if self.stale or self._gexec is None:
             self.backend.release_gexec(self._gexec)
             self._gexec = self.backend.capture(
-                lambda s: [k.run(s) for k in self.klist], stream)
+                self.backend.launcher(self._nodes or self.klist), stream)
             self.stale = False
 
         self.backend.lib.graph_launch(self._gexec, stream)

@@ -57,9 +57,10 @@ __device__ __forceinline__ void early_dependents() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
+// brief: a kernel whose length the gap before it matters to
 template <typename... P, typename... A>
-inline void launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
-                   A &&...a) {
+inline void launch_if(bool brief, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem,
+                      cudaStream_t st, A &&...a) {
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
@@ -73,10 +74,19 @@ inline void launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cud
     // kernel launched from the host again and again, a 20 x 40 tensor-core
     // apply of 24 us, takes 1.4% longer so)
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    c.numAttrs = cudaStreamIsCapturing(st, &cap) == cudaSuccess &&
+    c.numAttrs = brief && cudaStreamIsCapturing(st, &cap) == cudaSuccess &&
                  cap == cudaStreamCaptureStatusActive;
     // (a failure is left for the caller's cudaGetLastError)
     (void)cudaLaunchKernelEx(&c, kernel, static_cast<P>(a)...);
+}
+
+// (beyond 32 blocks an SM nothing is gained: a step of 32^3 hexahedra is as
+// long, and its graph's instantiation up to 0.3 ms longer)
+template <typename... P, typename... A>
+inline void launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                   A &&...a) {
+    launch_if((uint64_t)grid.x * grid.y * grid.z <= 152 * 32, kernel, grid, block, smem, st,
+              static_cast<A &&>(a)...);
 }
 
 inline unsigned ceil_div(int64_t a, int64_t b) { return (unsigned)((a + b - 1) / b); }

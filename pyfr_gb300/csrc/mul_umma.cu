@@ -1105,14 +1105,15 @@ static int umma_apply(void *handle, const b200_mul_bf16x3_args_t *a, int early, 
     const int64_t ntiles = p.ntc * p.nbatch;
     const unsigned grid = (unsigned)(ntiles < g_sm_count ? ntiles : g_sm_count);
     const cudaStream_t st = (cudaStream_t)stream;
+    const bool brief = ntiles <= 8 * (int64_t)g_sm_count;
     if (h->tf32 && p.rk)
-        b200::launch(mul_umma_kernel<true, true>, grid, NTHREADS, h->smem_bytes, st, p);
+        b200::launch_if(brief, mul_umma_kernel<true, true>, grid, NTHREADS, h->smem_bytes, st, p);
     else if (h->tf32)
-        b200::launch(mul_umma_kernel<true, false>, grid, NTHREADS, h->smem_bytes, st, p);
+        b200::launch_if(brief, mul_umma_kernel<true, false>, grid, NTHREADS, h->smem_bytes, st, p);
     else if (p.rk)
-        b200::launch(mul_umma_kernel<false, true>, grid, NTHREADS, h->smem_bytes, st, p);
+        b200::launch_if(brief, mul_umma_kernel<false, true>, grid, NTHREADS, h->smem_bytes, st, p);
     else
-        b200::launch(mul_umma_kernel<false, false>, grid, NTHREADS, h->smem_bytes, st, p);
+        b200::launch_if(brief, mul_umma_kernel<false, false>, grid, NTHREADS, h->smem_bytes, st, p);
     B200_CHECK_LAUNCH("mul_umma_kernel");
     return B200_OK;
 }

@@ -320,6 +320,33 @@ int b200_graph_end_capture(void *stream, void **gexec) {
     return rc;
 }
 
+int b200_graph_capture_last(void *stream, void **nodes, int max, int *n) {
+    if (!nodes || !n || max <= 0) return set_error(B200_ERR_ARG, "capture_last: bad arguments");
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    const cudaGraphNode_t *deps = nullptr;
+    const cudaGraphEdgeData *edges = nullptr;
+    size_t nd = 0;
+    int rc = check_cuda(cudaStreamGetCaptureInfo((cudaStream_t)stream, &st, nullptr, nullptr, &deps,
+                                                 &edges, &nd), "cudaStreamGetCaptureInfo");
+    if (rc) return rc;
+    if (st != cudaStreamCaptureStatusActive)
+        return set_error(B200_ERR_STATE, "capture_last: the stream is not being captured");
+    if (nd > (size_t)max)
+        return set_error(B200_ERR_ARG, "capture_last: %d nodes, room for %d", (int)nd, max);
+    for (size_t i = 0; i < nd; i++) nodes[i] = (void *)deps[i];
+    *n = (int)nd;
+    return B200_OK;
+}
+
+int b200_graph_capture_after(void *stream, void *const *nodes, int n) {
+    if (n < 0 || (n && !nodes)) return set_error(B200_ERR_ARG, "capture_after: bad arguments");
+    return check_cuda(cudaStreamUpdateCaptureDependencies((cudaStream_t)stream,
+                                                          (cudaGraphNode_t *)nodes, nullptr,
+                                                          (size_t)n,
+                                                          cudaStreamSetCaptureDependencies),
+                      "cudaStreamUpdateCaptureDependencies");
+}
+
 int b200_graph_launch(void *gexec, void *stream) {
     return check_cuda(cudaGraphLaunch((cudaGraphExec_t)gexec, (cudaStream_t)stream),
                       "cudaGraphLaunch");

@@ -19,7 +19,7 @@ import weakref
 
 import numpy as np
 
-from pyfr_gb300.backend.types import Kernel
+from pyfr_gb300.backend.types import Kernel, Nodes
 
 RK_COEFFS = {
     'rk45': dict(
@@ -148,6 +148,10 @@ class RKVdH2Integrator:
             self._tkerns = [self.system.stage_time_kernel(ci,
                                                           dt_dev=self._dt_dev)
                             for ci in self.c]
+
+        self._plans = {}
+        if self.use_step_graph:
+            self._step_plan(0, self.dt)
 
         if self.needs_cfl:
             # pyfr/integrators/controllers.py:7-38
@@ -358,6 +362,41 @@ class RKVdH2Integrator:
         kl.extend(self.system.postproc_kernels(r2))
         return kl, ((r2, *rs) if rs else (r2,))
 
+    def _nodes_ok(self):
+        """Whether a step's kernels may run by what they wait for instead
+        of one after the other."""
+        return not (self._tdep or self.system.controlled_bcs or
+                    self.system._ef)
+
+    def step_nodes(self, idx, dt):
+        """The kernels of one step as ``Nodes`` and the resulting register
+        indices, or None where they have to run in order."""
+        if not self._nodes_ok():
+            return None
+        nodes, start = Nodes(), {}
+        tags = [f'eles/{id(e)}' for e in self.system.ele_map.values()]
+        r1, r2, rs = self._regs(idx)
+        for i in range(self.nstages):
+            ends = self.system.rhs_nodes(nodes, r2 if i else r1, r2, start)
+            if ends is None:
+                return None
+            start = {}
+            for tag, k in zip(tags, self._rk_kerns(i, r1, r2, *rs)):
+                k.bind(dt=dt)
+                start[tag] = [nodes.add(k, ends[tag])]
+            r1, r2 = r2, r1
+        return nodes, ((r2, *rs) if rs else (r2,))
+
+    def _step_plan(self, idx, dt):
+        """(a function enqueueing ``step_nodes`` under capture, the
+        resulting register indices) or None; that of the starting register
+        is made with the integrator (the step size reaches the kernels
+        through device memory)."""
+        if idx not in self._plans:
+            res = self.step_nodes(idx, dt)
+            self._plans[idx] = res and (self.backend.launcher(res[0]), res[1])
+        return self._plans[idx]
+
     def _enqueue_step(self, t, dt, idx, stream):
         """Enqueue every stage of one step; returns the register indices."""
         kl, regs = self.step_kernels(idx, dt, t)
@@ -387,11 +426,15 @@ class RKVdH2Integrator:
             self._set_dt(dt, stream)
             key = self.idxcurr
             if key not in self._step_graphs:
-                res = []
-                gexec = be.capture(
-                    lambda s: res.append(self._enqueue_step(t, dt,
-                                                            self.idxcurr, s)),
-                    stream)
+                res = self._step_plan(key, dt)
+                if res is not None:
+                    gexec = be.capture(res[0], stream)
+                    res = res[1:]
+                else:
+                    res = []
+                    gexec = be.capture(
+                        lambda s: res.append(self._enqueue_step(t, dt, key,
+                                                                s)), stream)
                 self._step_graphs[key] = (gexec, res[0])
             gexec, regs = self._step_graphs[key]
             be.lib.graph_launch(gexec, stream)
@@ -765,6 +808,19 @@ class MixedRKIntegrator(RKVdH2Integrator):
             kl.extend(post)
             kl.extend(self._ef_merge)
         return kl, ((0, 1, 2) if self.errest else (0,))
+
+    def step_nodes(self, idx, dt):
+        if not self._nodes_ok() or self.backend.fuse_stage:
+            return None
+        nodes, start = Nodes(), {}
+        tags = [f'eles/{id(e)}' for e in self.system.ele_map.values()]
+        for i in range(self.nstages):
+            ends = self.system.rhs_nodes(nodes, 0, 1, start)
+            if ends is None:
+                return None
+            start = {tag: [nodes.add(self._stage_kernel(i, j, dt), ends[tag])]
+                     for j, tag in enumerate(tags)}
+        return nodes, ((0, 1, 2) if self.errest else (0,))
 
     def _reject(self, iprev):
         self._restore_previous()

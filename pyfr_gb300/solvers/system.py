@@ -14,7 +14,7 @@ import inspect
 
 import numpy as np
 
-from pyfr_gb300.backend.types import Graph, Kernel, NullKernel
+from pyfr_gb300.backend.types import Graph, Kernel, Nodes, NullKernel
 from pyfr_gb300.solvers.elements import EulerElements, NavierStokesElements
 from pyfr_gb300.solvers.inters import (EulerBCInters, EulerIntInters,
                                        EulerMPIInters, NavierStokesBCInters,
@@ -206,6 +206,9 @@ class BaseSystem:
                 for e in self.ele_map.values()]
         self.backend.commit()
         self._graph_cache = {}
+        # (the plan of the right-hand side's launch, for the first pass)
+        if self.nrhs > 1 and self.rhs_nodes(Nodes(), 0, 1) is not None:
+            self._rhs_launches(0, 1)
 
         # Host-side geometry and gather maps were only needed to build the
         # kernels
@@ -222,7 +225,14 @@ class BaseSystem:
                  ('bcint', self._bc_inters)]
         for pn, plist in provs:
             for p in plist:
+                # (what an element type's own kernel takes the place of is
+                # not made, but for the gradients of the diagnostics)
+                skip = () if pn != 'eles' or not p.te_handle() else \
+                    set(self._general_kernels) - {'tgradpcoru_upts',
+                                                  'tgradcoru_upts'}
                 for kn, kget in p.kernels.items():
+                    if kn in skip:
+                        continue
                     params = inspect.signature(kget).parameters
                     if 'uin' in params or 'fout' in params:
                         for i in range(self.nrhs):
@@ -444,11 +454,74 @@ class BaseSystem:
         no exchange with other partitions stands between them."""
         key = ('launches', uin, fout)
         if key not in self._graph_cache:
-            gs = self._rhs_graphs_cached(uin, fout)
-            if not any(isinstance(g, HostStep) for g in gs):
-                gs = (Graph.joined(gs),)
+            nodes = Nodes()
+            if self.rhs_nodes(nodes, uin, fout) is not None:
+                gs = (Graph.of_nodes(self.backend, nodes),)
+            else:
+                gs = self._rhs_graphs_cached(uin, fout)
+                if not any(isinstance(g, HostStep) for g in gs):
+                    gs = (Graph.joined(gs),)
             self._graph_cache[key] = gs
         return self._graph_cache[key]
+
+    # Kernels that only the serial order of the graphs serves
+    _serial_kernels = ('eles/entropy_filter', 'eles/copy_soln',
+                       'iint/comm_entropy', 'bcint/comm_entropy',
+                       'vtx/vtx_zero', 'eles/qptsu', 'eles/addsrc')
+
+    def rhs_nodes(self, nodes, uin, fout, start={}):
+        """Add the kernels of a right-hand side to ``nodes`` (``Nodes``) with
+        what each waits for, so that element types run side by side, and
+        the flux beside the interfaces where it does not wait for them
+        (with three element types of a mixed mesh the kernels of one do not
+        fill the GPU).  ``start``: per element type the nodes that its first
+        kernels wait for.  Returns per element type the nodes that finish
+        its right-hand side, or None, nothing added, where the graphs'
+        order has to be kept (shock capturing, anti-aliasing, source terms,
+        partitions)."""
+        key = ('nodes', uin, fout)
+        if key not in self._graph_cache:
+            self._graph_cache[key] = self._rhs_node_list(uin, fout)
+        if self._graph_cache[key] is None:
+            return None
+        items, ends = self._graph_cache[key]
+        base = len(nodes.items)
+        for k, deps, tag in items:
+            nodes.add(k, [base + d for d in deps] +
+                      (start.get(tag, []) if tag else []))
+        return {t: [base + i for i in v] for t, v in ends.items()}
+
+    def _rhs_node_list(self, uin, fout):
+        """([(kernel, what it waits for, the element type's tag if it waits
+        for that type's start)], {tag: the nodes that finish it})."""
+        k = self._get_rhs_kernels(uin, fout)
+        if self._mpi_inters or any(k[n] for n in self._serial_kernels):
+            return None
+        items, pos = [], defaultdict(list)
+
+        def own(l, *names):
+            return [i for n in names for i in pos[n, self._ktags[l]]]
+
+        def every(*names):
+            return [i for (n, _), v in pos.items() if n in names for i in v]
+
+        def add(name, deps=None):
+            for l in k[name]:
+                tag = self._ktags[l]
+                items.append((l, [], tag) if deps is None else
+                             (l, deps(l), None))
+                pos[name, tag].append(len(items) - 1)
+
+        self._add_rhs_nodes(add, own, every)
+        return items, {f'eles/{id(e)}': self._rhs_ends(pos, f'eles/{id(e)}')
+                       for e in self.ele_map.values()}
+
+    @staticmethod
+    def _rhs_ends(pos, tag):
+        for n in ('negdivconf', 'te_lift', 'tdivtconf_cat', 'te_rhs'):
+            if pos.get((f'eles/{n}', tag)):
+                return pos[f'eles/{n}', tag]
+        raise RuntimeError('No kernel finishes the right-hand side')
 
     def preproc_kernels(self, uinbank):
         """Before the first step: filter, then every element's and face's
@@ -540,6 +613,27 @@ class EulerSystem(BaseSystem):
         g_flux_div.commit()
 
         return g_intf, g_flux_div
+
+
+    def _add_rhs_nodes(self, add, own, every):
+        comm = ('iint/comm_flux', 'bcint/comm_flux')
+        add('eles/disu')
+        for n in comm:
+            add(n, lambda l: every('eles/disu'))
+        # (the flux reads the solution alone, but beside one type's own
+        # interfaces it gains little, 2% of a step of 96 x 96 cells at p = 4,
+        # for a longer capture)
+        many = len(self.ele_map) > 1
+        add('eles/tdisf',
+            lambda l: own(l, 'eles/disu') if many else every(*comm))
+        add('eles/te_rhs', lambda l: every(*comm))
+        add('eles/tdivtconf_cat',
+            lambda l: own(l, 'eles/tdisf') + every(*comm))
+        # (which may write the input's bank)
+        add('eles/tdivtpcorf', lambda l: own(l, 'eles/tdisf', 'eles/disu'))
+        add('eles/tdivtconf',
+            lambda l: own(l, 'eles/tdivtpcorf') + every(*comm))
+        add('eles/negdivconf', lambda l: own(l, 'eles/tdivtconf'))
 
 
 class NavierStokesSystem(BaseSystem):
@@ -748,6 +842,33 @@ class NavierStokesSystem(BaseSystem):
         self._add_src(g_div, k, deps)
         g_div.commit()
         return g_grad_flux, g_div
+
+    def _add_rhs_nodes(self, add, own, every):
+        con = ('iint/con_u', 'bcint/con_u')
+        comm = ('iint/comm_flux', 'bcint/comm_flux')
+        grads = ('eles/tgradcoru_upts_cat', 'eles/tgradcoru_upts')
+        add('eles/disu')
+        add('eles/copy_fpts', lambda l: own(l, 'eles/disu'))
+        add('eles/tgradpcoru_upts', lambda l: own(l, 'eles/disu'))
+        for n in con:
+            add(n, lambda l: every('eles/disu', 'eles/copy_fpts'))
+        add('eles/te_rhs', lambda l: every(*con))
+        add('eles/tgradcoru_upts_cat',
+            lambda l: own(l, 'eles/disu') + every(*con))
+        add('eles/tgradcoru_upts',
+            lambda l: own(l, 'eles/tgradpcoru_upts') + every(*con))
+        add('eles/tdisf_fused', lambda l: own(l, *grads))
+        add('eles/gradcoru_fpts', lambda l: own(l, 'eles/tdisf_fused'))
+        for n in comm:
+            add(n, lambda l: every('eles/gradcoru_fpts', 'eles/te_rhs', *con))
+        add('eles/te_lift', lambda l: own(l, 'eles/te_rhs') + every(*comm))
+        add('eles/tdivtconf_cat',
+            lambda l: own(l, 'eles/tdisf_fused') + every(*comm))
+        add('eles/tdivtpcorf',
+            lambda l: own(l, 'eles/tdisf_fused', 'eles/disu'))
+        add('eles/tdivtconf',
+            lambda l: own(l, 'eles/tdivtpcorf') + every(*comm))
+        add('eles/negdivconf', lambda l: own(l, 'eles/tdivtconf'))
 
     def _compute_grads_graph(self, uinbank):
         key = ('grads', uinbank)
