@@ -16,12 +16,17 @@
 // walking the nonzeros of A (CSR, read through the read-only cache and
 // broadcast across the warp).  Structural zeros of A cost nothing, so the
 // sparse tensor-product operators run at their nonzero count.
+#include <algorithm>
+#include <map>
 #include <math.h>
 #include <stdlib.h>
 #include <string.h>
+#include <type_traits>
+#include <utility>
 #include <vector>
 
 #include "common.cuh"
+#include "fixedpoint.cuh"
 #include "../../include/pyfrb200.h"
 
 namespace {
@@ -40,6 +45,13 @@ struct MulHandle {
     // entry (column, high part, low part, 0)
     int4 *fxrow;     // device, m
     int4 *fxval;     // device, nnz
+    // The same by groups of up to four rows of one support (null when the
+    // rows do not fall into such groups): per group gn columns and four rows
+    // (-1: none), and (high, low part) and the value of every entry; one scale
+    int gn, ngrp, gs;
+    int *gcol, *grow;    // device, ngrp x gn and ngrp x 4
+    int2 *gval;          // device, ngrp x 4 x gn
+    double *gdbl;        // device, the same as doubles
 };
 
 template <typename T>
@@ -62,6 +74,31 @@ __device__ __forceinline__ void cp_async16(void *dst, const void *src, int bytes
                  : "memory");
 }
 
+// Stage the columns col0.. of B into bs [k][NC] (zero-filled beyond ncol); the
+// caller synchronises the block
+template <typename T, int NC>
+__device__ __forceinline__ void stage_tile(T *bs, const T *b, int64_t ldb, int k, int64_t col0,
+                                           int64_t ncol, int vec) {
+    if (vec) {
+        constexpr int VEC = 16 / sizeof(T), NV = NC / VEC;
+        for (int idx = threadIdx.x; idx < k * NV; idx += blockDim.x) {
+            const int r = idx / NV, cv = (idx % NV) * VEC;
+            const int64_t col = col0 + cv;
+            const int64_t rem = ncol - col;
+            const int bytes = rem >= VEC ? 16 : (rem > 0 ? (int)rem * (int)sizeof(T) : 0);
+            // (with nothing to read the source is any valid address)
+            cp_async16(bs + r * NC + cv, bytes ? b + r * ldb + col : b, bytes);
+        }
+        asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
+    } else {
+        for (int idx = threadIdx.x; idx < k * NC; idx += blockDim.x) {
+            int r = idx / NC, cc = idx % NC;
+            int64_t col = col0 + cc;
+            bs[idx] = (col < ncol) ? b[r * ldb + col] : T(0);
+        }
+    }
+}
+
 template <typename T, int EPI>
 __global__ void __launch_bounds__(MUL_WARPS * 32)
 mul_csr_kernel(MulHandle h, const T *__restrict__ b, int64_t ldb, T *__restrict__ c,
@@ -73,25 +110,7 @@ mul_csr_kernel(MulHandle h, const T *__restrict__ b, int64_t ldb, T *__restrict_
     const int64_t col0 = (int64_t)blockIdx.x * MUL_NCOL;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 
-    // Stage the B tile (zero-filled beyond ncol)
-    if (vec) {
-        constexpr int VEC = 16 / sizeof(T), NV = MUL_NCOL / VEC;
-        for (int idx = threadIdx.x; idx < h.k * NV; idx += blockDim.x) {
-            const int r = idx / NV, cv = (idx % NV) * VEC;
-            const int64_t col = col0 + cv;
-            const int64_t rem = ncol - col;
-            const int bytes = rem >= VEC ? 16 : (rem > 0 ? (int)rem * (int)sizeof(T) : 0);
-            // (with nothing to read the source is any valid address)
-            cp_async16(bs + r * MUL_NCOL + cv, bytes ? b + r * ldb + col : b, bytes);
-        }
-        asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;" ::: "memory");
-    } else {
-        for (int idx = threadIdx.x; idx < h.k * MUL_NCOL; idx += blockDim.x) {
-            int r = idx / MUL_NCOL, cc = idx % MUL_NCOL;
-            int64_t col = col0 + cc;
-            bs[idx] = (col < ncol) ? b[r * ldb + col] : T(0);
-        }
-    }
+    stage_tile<T, MUL_NCOL>(bs, b, ldb, h.k, col0, ncol, vec);
     __syncthreads();
 
     const T *__restrict__ av = vals<T>(h);
@@ -370,6 +389,215 @@ void launch_fx(const MulHandle &h, const double *b, int64_t ldb, double *c, int6
         b200::launch(mul_fx_kernel<EPI_GENERAL, CPL>, grid, MUL_WARPS * 32, smem, s, h, b, ldb, c, ldc, ncol, alpha, beta, vec);
 }
 
+// ---- the same by groups of rows of one support ---------------------------
+//
+// The rows of tensor-product operators come in lines: four derivatives from the
+// same four values, two face values from one line.  A group's operands are
+// loaded and split once for its rows (by the splits of fixedpoint.cuh), over
+// their own largest exponent, so that there is no pass over the column, no test
+// and no second form of an output (but for exponents out of range).  Sums: with
+// sum |ah| ~ 2^30, |al| <= 2^30 and 60 bits of B, |w| is below
+// 2^61 + N 2^59 < 2^63 for the N <= 6 taken.
+//
+// What bounds it is issue slots (the integer pipes at 53%, the FP64 unit's
+// conversions at 21%) and, in large applies, DRAM beside them: 192 x 64 gradient
+// operator of p = 3 hexahedra, 35005 columns, 25.4 us by columns (above; a
+// quarter of its rows formed twice where the values pass through zero), 22.6 us
+// by groups, its DRAM time 10.5 us; at 320 columns 21.2 -> 11.3 us, where the
+// chain of one tile is all there is.  Every other row is converted on the FP64
+// unit, the rest on the integer pipes: all on the former would take its 2 a clock
+// and SM 11.5 us of the kernel, all on the latter a third more instructions.
+//
+// Groups of pairs of values (192 x 96 and 375 x 150 lifts) are left to the FP64
+// form, which is 15-50% faster there: two products do not pay for a split.
+
+constexpr int FXG_ROWS = 4, FXG_MIN = 3, FXG_MAX = 6;
+
+template <int EPI, int CPL, int N>
+__global__ void __launch_bounds__(MUL_WARPS * 32)
+mul_fxg_kernel(MulHandle h, const double *__restrict__ b, int64_t ldb, double *__restrict__ c,
+               int64_t ldc, int64_t ncol, double alpha, double beta, int vec, int vecc) {
+    b200::dependent_entry(b, c);
+    constexpr int NC = 32 * CPL;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    double *bs = reinterpret_cast<double *>(smem_raw);   // [k][NC]
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t col0 = (int64_t)blockIdx.x * NC, col = col0 + lane * CPL;
+    stage_tile<double, NC>(bs, b, ldb, h.k, col0, ncol, vec);
+    __syncthreads();
+
+    bool ok[CPL];
+#pragma unroll
+    for (int j = 0; j < CPL; j++) ok[j] = col + j < ncol;
+    const bool pair = CPL == 2 && vecc && ok[CPL - 1];
+
+    for (int g = warp; g < h.ngrp; g += MUL_WARPS) {
+        double x[N][CPL];
+#pragma unroll
+        for (int i = 0; i < N; i++) {
+            const double *src = bs + __ldg(h.gcol + g * N + i) * NC + lane * CPL;
+            if (CPL == 2) {
+                const double2 t = *reinterpret_cast<const double2 *>(src);
+                x[i][0] = t.x;
+                x[i][CPL - 1] = t.y;
+            } else {
+                x[i][0] = src[0];
+            }
+        }
+        int emax[CPL];
+        bool wild[CPL];
+        int2 y[N][CPL];
+#pragma unroll
+        for (int j = 0; j < CPL; j++) {
+            // (1 for a subnormal without a high word: out of range)
+            int mx = 0;
+#pragma unroll
+            for (int i = 0; i < N; i++)
+                mx = max(mx, b200::hi_abs(x[i][j]) | (__double2loint(x[i][j]) != 0));
+            wild[j] = b200::out_of_range(mx);
+            emax[j] = max(mx >> 20, 64);
+#pragma unroll
+            for (int i = 0; i < N; i++) y[i][j] = b200::split<60>(x[i][j], emax[j]);
+        }
+        const bool any = __any_sync(0xffffffffu, wild[0] || wild[CPL - 1]);
+        const int4 rows = __ldg(reinterpret_cast<const int4 *>(h.grow) + g);
+        const int rr[FXG_ROWS] = {rows.x, rows.y, rows.z, rows.w};
+#pragma unroll
+        for (int q = 0; q < FXG_ROWS; q++) {
+            if (rr[q] < 0) break;
+            double *crow = c + rr[q] * ldc + col, r[CPL];
+            const int2 *av = h.gval + (g * FXG_ROWS + q) * N;
+            b200::Fx s[CPL];
+#pragma unroll
+            for (int j = 0; j < CPL; j++) s[j].clear();
+#pragma unroll
+            for (int i = 0; i < N; i++) {
+                const int2 a = __ldg(av + i);
+#pragma unroll
+                for (int j = 0; j < CPL; j++) s[j].mad(a, y[i][j]);
+            }
+#pragma unroll
+            for (int j = 0; j < CPL; j++) {
+                const int sc = emax[j] - h.gs - 1051;
+                r[j] = q % 2 ? s[j].value(sc) : s[j].value_cvt(sc);
+                // (a branch of the warp with a loop in it: as selected values
+                // these FMAs would run for every output)
+                if (any) {
+                    double f = 0.0;
+                    const double *ad = h.gdbl + (g * FXG_ROWS + q) * N;
+#pragma unroll 1
+                    for (int i = 0; i < N; i++)
+                        f = fma(__ldg(ad + i), bs[__ldg(h.gcol + g * N + i) * NC + lane * CPL + j],
+                                f);
+                    if (wild[j]) r[j] = f;
+                }
+                const double old = EPI == EPI_ADD || EPI == EPI_GENERAL
+                                       ? (ok[j] ? crow[j] : 0.0) : 0.0;
+                if (EPI == EPI_GENERAL) r[j] = alpha * r[j] + beta * old;
+                if (EPI == EPI_ADD) r[j] += old;
+                if (EPI == EPI_SCALE) r[j] *= alpha;
+            }
+            if (pair) {
+                *reinterpret_cast<double2 *>(crow) = make_double2(r[0], r[CPL - 1]);
+            } else {
+#pragma unroll
+                for (int j = 0; j < CPL; j++)
+                    if (ok[j]) crow[j] = r[j];
+            }
+        }
+    }
+}
+
+// fn(integral constants: columns per lane, group size, epilogue)
+template <typename F>
+bool with_fxg(int cpl, int n, int epi, F &&fn) {
+    auto by_epi = [&](auto c, auto g) {
+        switch (epi) {
+        case EPI_SET: fn(c, g, std::integral_constant<int, EPI_SET>()); break;
+        case EPI_ADD: fn(c, g, std::integral_constant<int, EPI_ADD>()); break;
+        case EPI_GENERAL: fn(c, g, std::integral_constant<int, EPI_GENERAL>()); break;
+        default: fn(c, g, std::integral_constant<int, EPI_SCALE>());
+        }
+    };
+    auto by_n = [&](auto c) {
+        switch (n) {
+        case 3: by_epi(c, std::integral_constant<int, 3>()); return true;
+        case 4: by_epi(c, std::integral_constant<int, 4>()); return true;
+        case 5: by_epi(c, std::integral_constant<int, 5>()); return true;
+        case 6: by_epi(c, std::integral_constant<int, 6>()); return true;
+        default: return false;
+        }
+    };
+    return cpl == 1 ? by_n(std::integral_constant<int, 1>())
+                    : by_n(std::integral_constant<int, 2>());
+}
+
+// The operator's rows in groups of one support, or false where they are not: of
+// two rows a group on average, and of one support size of FXG_MIN to FXG_MAX
+struct Groups {
+    int n = 0, s = 0;
+    std::vector<int> col, row;
+    std::vector<int2> val;
+    std::vector<double> dbl;
+};
+
+bool fx_groups(const double *a, int m, int k, Groups &g) {
+    std::map<std::vector<int>, std::vector<int>> by;
+    double top = 0.0, low = INFINITY;
+    for (int i = 0; i < m; i++) {
+        std::vector<int> sup;
+        double l1 = 0.0;
+        for (int j = 0; j < k; j++)
+            if (a[(size_t)i * k + j] != 0.0) {
+                sup.push_back(j);
+                l1 += fabs(a[(size_t)i * k + j]);
+            }
+        if (!g.n) g.n = (int)sup.size();
+        if ((int)sup.size() != g.n || g.n < FXG_MIN || g.n > FXG_MAX || !(l1 <= ldexp(1.0, 60)))
+            return false;
+        top = fmax(top, l1);
+        low = fmin(low, l1);
+        by[sup].push_back(i);
+    }
+    // (one scale: the smallest row keeps 57 of its bits)
+    if (!(low >= ldexp(1.0, -60)) || low < top / 16) return false;
+    int e;
+    frexp(top, &e);
+    g.s = 30 - e;
+    // (in the order of the first row, so that neighbouring groups write
+    // neighbouring rows)
+    std::vector<std::pair<int, const std::vector<int> *>> order;
+    for (auto &kv : by) order.push_back({kv.second[0], &kv.first});
+    std::sort(order.begin(), order.end());
+    for (auto &o : order) {
+        const std::vector<int> &rows = by[*o.second];
+        for (size_t r0 = 0; r0 < rows.size(); r0 += FXG_ROWS) {
+            g.col.insert(g.col.end(), o.second->begin(), o.second->end());
+            for (int q = 0; q < FXG_ROWS; q++) {
+                const int r = r0 + q < rows.size() ? rows[r0 + q] : -1;
+                g.row.push_back(r);
+                for (int j : *o.second) {
+                    const double x = r < 0 ? 0.0 : a[(size_t)r * k + j];
+                    const long long z = llrint(ldexp(x, g.s + 31));
+                    const long long ah = (z + (1ll << 30)) >> 31;
+                    g.val.push_back(make_int2((int)ah, (int)(z - ah * (1ll << 31))));
+                    g.dbl.push_back(x);
+                }
+            }
+        }
+    }
+    return (size_t)m >= 2 * (g.row.size() / FXG_ROWS);
+}
+
+template <typename V>
+int upload(V **dst, const std::vector<V> &src) {
+    int rc = b200::check_cuda(cudaMalloc(dst, sizeof(V) * src.size()), "mul_create");
+    if (!rc)
+        rc = b200::check_cuda(cudaMemcpy(*dst, src.data(), sizeof(V) * src.size(),
+                                         cudaMemcpyHostToDevice), "mul_create");
+    return rc;
+}
+
 // The operator's fixed-point form (rows, entries), or false where it does
 // not fit: a row of more than FX_MAXNNZ entries, or of an absolute sum
 // outside [2^-60, 2^60] (or not finite)
@@ -416,13 +644,32 @@ int launch_mul(const MulHandle *h, const T *b, int64_t ldb, T *c, int64_t ldc, i
     // 16-byte copies need a 16-byte aligned base and row stride
     const int vec = !((uintptr_t)b & 15) && !((ldb * (int64_t)sizeof(T)) & 15);
     if constexpr (sizeof(T) == 8) {
+        if (h->gval) {
+            // Groups of rows of one support, at every width: against the faster
+            // of the other two forms 21.2 -> 11.3 us at 320 columns and
+            // 74.4 -> 67.6 us at 87880 for the 192 x 64 gradient, 17.8 -> 12.4
+            // and 106 -> 88 us for the 150 x 125 interpolation at p = 4, and
+            // from 10.9 -> 7.7 to 44.4 -> 46.5 us for the 96 x 64 one.  Two
+            // columns a lane where every SM has a tile and room for two
+            const int cpl = ncol > 64 * 152 && smem <= 113 * 1024 ? 2 : 1;
+            const int vecc = !((uintptr_t)c & 15) && !(ldc & 1);
+            const int epi = alpha == 1.0 ? (beta == 0.0 ? EPI_SET : beta == 1.0 ? EPI_ADD : EPI_GENERAL)
+                                         : (beta == 0.0 ? EPI_SCALE : EPI_GENERAL);
+            with_fxg(cpl, h->gn, epi, [&](auto cp, auto gn, auto ep) {
+                b200::launch(mul_fxg_kernel<ep(), cp(), gn()>, b200::ceil_div(ncol, 32 * cp()),
+                             MUL_WARPS * 32, (size_t)h->k * 32 * cp() * sizeof(double), s, *h, b, ldb,
+                             c, ldc, ncol, alpha, beta, vec, vecc);
+            });
+            B200_CHECK_LAUNCH("mul_fxg_kernel");
+            return B200_OK;
+        }
         // (the FP64 FMAs of small outputs read B again, so C must not be B)
         const bool apart = c + (int64_t)(h->m - 1) * ldc + ncol <= b ||
                            b + (int64_t)(h->k - 1) * ldb + ncol <= c;
         // Where the FMAs bound: rows of ten entries and more at every width
         // (tetrahedra's 20 x 40 lift at 20480 columns 38.5 -> 17.4 us), rows
-        // of four and more once every SM has a tile (hexahedra's 192 x 64
-        // gradient at p = 3: 41.9 -> 25.9 us at 20480 columns, 131 -> 75 us at
+        // of four and more once every SM has a tile (hexahedra's 375 x 125
+        // gradient at p = 4: 93 -> 59 us at 20480 columns, 326 -> 222 us at
         // 87880; below 9728 columns of rows of four the FP64 form's shorter
         // chain is up to 10% faster, and for rows of two, 192 x 96, it is
         // 15-25% faster at every width).  The tile has to leave an SM room
@@ -487,6 +734,7 @@ int opt_in_smem() {
 void free_handle(MulHandle *h) {
     cudaFree(h->rowptr); cudaFree(h->colidx); cudaFree(h->val64); cudaFree(h->val32);
     cudaFree(h->fxrow); cudaFree(h->fxval);
+    cudaFree(h->gcol); cudaFree(h->grow); cudaFree(h->gval); cudaFree(h->gdbl);
     free(h);
 }
 
@@ -546,6 +794,26 @@ int b200_mul_create(const double *a, int m, int k, void **handle) {
                                                   cudaMemcpyHostToDevice), "mul_create");
         if (!rc) rc = b200::check_cuda(cudaMemcpy(h->fxval, fxval.data(), sizeof(int4) * nz,
                                                   cudaMemcpyHostToDevice), "mul_create");
+    }
+    Groups gr;
+    if (!rc && h->nnz && fx_groups(a, m, k, gr)) {
+        h->gn = gr.n;
+        h->ngrp = (int)gr.row.size() / FXG_ROWS;
+        h->gs = gr.s;
+        rc = upload(&h->gcol, gr.col);
+        if (!rc) rc = upload(&h->grow, gr.row);
+        if (!rc) rc = upload(&h->gdbl, gr.dbl);
+        if (!rc) rc = upload(&h->gval, gr.val);
+        // (opted in to the largest tile here, where no capture is open)
+        for (int cpl = 1; cpl <= 2; cpl++)
+            for (int epi : {EPI_SET, EPI_ADD, EPI_GENERAL, EPI_SCALE})
+                with_fxg(cpl, h->gn, epi, [&](auto cp, auto gn, auto ep) {
+                    if (!rc)
+                        rc = b200::check_cuda(
+                            cudaFuncSetAttribute(mul_fxg_kernel<ep(), cp(), gn()>,
+                                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                 227 * 1024), "mul: smem attribute");
+                });
     }
     if (rc) {
         free_handle(h);

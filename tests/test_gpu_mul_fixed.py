@@ -62,7 +62,7 @@ def _data(what, k, n, rng):
 @pytest.mark.parametrize('ncol', [1, 31, 64, 65, 9728, 9735, 20002])
 @pytest.mark.parametrize('kind,p', [('m0', 3), ('m3', 3), ('m4', 3),
                                     ('m132', 3), ('m4', 1), ('tet', 3),
-                                    ('wide', 0)])
+                                    ('wide', 0), ('m0', 2), ('m0', 4)])
 @pytest.mark.parametrize('what', ['smooth', 'mean', 'zeros', 'range', 'ends',
                                   'special'])
 def test_fixed_point_apply(kind, p, ncol, what):
