@@ -331,7 +331,7 @@ class TensorMulKernels:
         m, k1, k2 = args[4], args[1], args[3]
         # (plans of kernels with rings of any length)
         key = '|'.join(map(str, (be.platform_id, 'tf32' if tf32 else 'bf16',
-                                 self._products(nterms), m, k1, k2, 'r2')))
+                                 self._products(nterms), m, k1, k2, 'r3')))
         cache = _plan_cache()
         if key in cache:
             return tuple(cache[key]) if cache[key] else None

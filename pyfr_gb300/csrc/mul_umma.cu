@@ -44,7 +44,8 @@
 //   warps 0-7       read the accumulator (tcgen05.ld, one column of out per
 //                   thread, 32 operator rows per load) in two sets of four,
 //                   one warp per TMEM lane quadrant, the sets taking
-//                   alternate 32-row groups; a set scales its group by
+//                   alternate 32-row groups, or alternate tiles where the
+//                   number of groups is odd; a set scales its group by
 //                   alpha into one 128 x 32 staging tile (two per set) and
 //                   writes it with a TMA tensor store (beta = 0) or
 //                   reduce-add (beta = 1) of 512-byte rows.
@@ -57,6 +58,7 @@
 #include <cuda_bf16.h>
 #include <stdlib.h>
 #include <string.h>
+#include <type_traits>
 #include <vector>
 
 #include "common.cuh"
@@ -320,7 +322,13 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t *v) {
                  : "r"(taddr));
 }
 
-template <bool TF32, bool RK>
+// ALT: epilogue sets by tiles instead of row groups: with an odd number of
+// groups one set has a group more in every tile and the other waits for it (of
+// up to 32 rows, all the work).  Five products, 4560 tiles: 20 x 40 rows and
+// columns 51.3 -> 40.8 us, 25 x 50 51.2 -> 41.1 (with an RK stage 288 -> 170),
+// 81 x 27 59.2 -> 46.3; even numbers share the work either way.  (A template
+// argument: as a variable it cost the RK epilogue 12% in spilled registers.)
+template <bool TF32, bool RK, bool ALT>
 __global__ void __launch_bounds__(NTHREADS, 1) mul_umma_kernel(const __grid_constant__ UmmaArgs p) {
     extern __shared__ __align__(1024) unsigned char smem[];
     const Layout L = make_layout(p.npad, p.kfull, p.ns, p.eb, p.nterms);
@@ -355,7 +363,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) mul_umma_kernel(const __grid_cons
         }
         for (int s = 0; s < 2; s++) {
             bar_init(bar(BAR_ACCFULL + s), 1);
-            bar_init(bar(BAR_ACCEMPTY + s), NEPI);
+            bar_init(bar(BAR_ACCEMPTY + s), ALT ? NEPI / 2 : NEPI);
         }
         bar_init(bar(BAR_DRAIN), 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -590,7 +598,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) mul_umma_kernel(const __grid_cons
     } else {
         // ---- epilogue: TMEM -> registers -> shared memory -> TMA store ----
         // warp w reads TMEM lane quadrant w%4 (columns 32(w%4)..+31 of the
-        // tile); set h = w/4 takes the row groups g with g%2 == h.  The
+        // tile); set h = w/4 takes the row groups g with g%2 == h, or (alt) all
+        // groups of every other tile, which is then its accumulator's.  The
         // set's waits are collective (named barrier, then the abort flag)
         // so that no warp of a set is left at a barrier the others skip.
         const int quad = warp % 4, half = warp / 4;
@@ -627,6 +636,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) mul_umma_kernel(const __grid_cons
         };
         for (int64_t t = blockIdx.x; t < ntiles; t += gridDim.x, i++) {
             const int bsel = i & 1;
+            if (ALT && bsel != half) continue;
             const int64_t x0 = (t % p.ntc) * TCOLS;
             const int z = (int)(t / p.ntc);
             // Element of this thread's column (AoSoA: blocks of 32 elements
@@ -635,7 +645,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) mul_umma_kernel(const __grid_cons
             const int64_t ele = (col / (32 * p.nvars)) * 32 + col % 32;
             // The first group's scale loads are in flight during the wait
             float f[32];
-            load_scale(f, half, col, ele);
+            load_scale(f, ALT ? 0 : half, col, ele);
             // RK stage: the tile's FP64 solution rows are brought into L2
             // while its MMAs run, so that the epilogue's loads of them do
             // not wait on HBM (one bulk prefetch of up to 1 KB per row, by
@@ -643,7 +653,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) mul_umma_kernel(const __grid_cons
             if (RK && quad == 0) {
                 const int64_t nc = p.ncol - x0 < TCOLS ? p.ncol - x0 : TCOLS;
                 const uint32_t bytes = (uint32_t)(nc * 8) & ~15u;
-                for (int g = half; g < npad / 32; g += 2) {
+                for (int g = ALT ? 0 : half; g < npad / 32; g += ALT ? 1 : 2) {
                     const int row = g * 32 + lane;
                     if (row < p.m && bytes)
                         asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;"
@@ -655,8 +665,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) mul_umma_kernel(const __grid_cons
             asm volatile("bar.sync %0, %1;" :: "r"(EPI_BARRIER + half), "n"(128) : "memory");
             if (!ok || *abort_flag) break;
             asm volatile("tcgen05.fence::after_thread_sync;");
-            for (int g = half; g < npad / 32; g += 2) {
-                if (g != half) load_scale(f, g, col, ele);
+            for (int g = ALT ? 0 : half; g < npad / 32; g += ALT ? 1 : 2) {
+                if (g >= (ALT ? 1 : 2)) load_scale(f, g, col, ele);
                 uint32_t v[32];
                 const uint32_t taddr = tmem + ((uint32_t)(quad * 32) << 16) +
                                        (uint32_t)(bsel * p.accols + g * 32);
@@ -813,6 +823,21 @@ void build_block_tf32(const double *a, int m, int k, int koff, int kfull,
         }
 }
 
+// fn(the kernel of these options)
+template <typename F>
+void with_kernel(bool tf32, bool rk, bool alt, F &&fn) {
+    auto by_alt = [&](auto t, auto r) {
+        if (alt) fn(mul_umma_kernel<t(), r(), true>);
+        else fn(mul_umma_kernel<t(), r(), false>);
+    };
+    auto by_rk = [&](auto t) {
+        if (rk) by_alt(t, std::true_type());
+        else by_alt(t, std::false_type());
+    };
+    if (tf32) by_rk(std::true_type());
+    else by_rk(std::false_type());
+}
+
 int g_sm_count = 0;
 PFN_cuTensorMapEncodeTiled_v12000 g_encode_tiled = nullptr;
 
@@ -915,26 +940,13 @@ int create_impl(const double *a1, int k1, const double *a2, int k2, int m, int t
             rc0 = b200::check_cuda(
                 cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev),
                 "mul_bf16x3_create");
-        if (!rc0)
-            rc0 = b200::check_cuda(cudaFuncSetAttribute(mul_umma_kernel<false, false>,
-                                                        cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                        227 * 1024),
-                                   "mul_bf16x3: smem attribute");
-        if (!rc0)
-            rc0 = b200::check_cuda(cudaFuncSetAttribute(mul_umma_kernel<true, false>,
-                                                        cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                        227 * 1024),
-                                   "mul_tf32: smem attribute");
-        if (!rc0)
-            rc0 = b200::check_cuda(cudaFuncSetAttribute(mul_umma_kernel<false, true>,
-                                                        cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                        227 * 1024),
-                                   "mul_bf16x3 (RK stage): smem attribute");
-        if (!rc0)
-            rc0 = b200::check_cuda(cudaFuncSetAttribute(mul_umma_kernel<true, true>,
-                                                        cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                        227 * 1024),
-                                   "mul_tf32 (RK stage): smem attribute");
+        for (int v = 0; v < 8; v++)
+            with_kernel(v & 1, v & 2, v & 4, [&](auto kernel) {
+                if (!rc0)
+                    rc0 = b200::check_cuda(
+                        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             227 * 1024), "mul_bf16x3: smem attribute");
+            });
         if (!rc0) {
             void *fn = nullptr;
             cudaDriverEntryPointQueryResult q;
@@ -1106,14 +1118,9 @@ static int umma_apply(void *handle, const b200_mul_bf16x3_args_t *a, int early, 
     const unsigned grid = (unsigned)(ntiles < g_sm_count ? ntiles : g_sm_count);
     const cudaStream_t st = (cudaStream_t)stream;
     const bool brief = ntiles <= 8 * (int64_t)g_sm_count;
-    if (h->tf32 && p.rk)
-        b200::launch_if(brief, mul_umma_kernel<true, true>, grid, NTHREADS, h->smem_bytes, st, p);
-    else if (h->tf32)
-        b200::launch_if(brief, mul_umma_kernel<true, false>, grid, NTHREADS, h->smem_bytes, st, p);
-    else if (p.rk)
-        b200::launch_if(brief, mul_umma_kernel<false, true>, grid, NTHREADS, h->smem_bytes, st, p);
-    else
-        b200::launch_if(brief, mul_umma_kernel<false, false>, grid, NTHREADS, h->smem_bytes, st, p);
+    with_kernel(h->tf32, p.rk, h->npad / 32 % 2, [&](auto kernel) {
+        b200::launch_if(brief, kernel, grid, NTHREADS, h->smem_bytes, st, p);
+    });
     B200_CHECK_LAUNCH("mul_umma_kernel");
     return B200_OK;
 }

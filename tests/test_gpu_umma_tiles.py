@@ -1,0 +1,74 @@
+"""The tensor-core operator kernel where its epilogue sets take whole tiles
+(an odd number of 32-row groups) and where they share a tile's groups: against
+the FP64 product, for one, two and several tiles a CTA.
+
+Bound: the data is held in 16 significant bits (a relative residual of at most
+2^-17), the operator in 16 or 24, and three products leave out one of 2^-18:
+below 2^-15 in all, with the FP32 sums' 2^-23 a term.
+"""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _lib():
+    from pyfr_gb300.backend import B200Backend
+    from pyfr_gb300.inifile import Inifile
+
+    return B200Backend(Inifile()).lib
+
+
+def _handle(lib, a, nterms):
+    h, smem = C.c_void_p(), C.c_size_t()
+    m, k = a.shape
+    lib.mul_tc_create_terms(a.ctypes.data_as(C.POINTER(C.c_double)), k, None,
+                            0, m, 0, nterms, 0, 0, C.byref(h), C.byref(smem))
+    return h
+
+
+@pytest.mark.parametrize('rk', [False, True])
+@pytest.mark.parametrize('products', [3, 5])
+@pytest.mark.parametrize('ncol', [4, 128, 19460, 152*128*3 + 132, 100004])
+@pytest.mark.parametrize('m,k', [(1, 16), (20, 40), (32, 32), (33, 20),
+                                 (65, 27), (96, 64), (128, 33)])
+def test_epilogue_sets(m, k, ncol, products, rk):
+    import torch
+
+    from pyfr_gb300.backend.lib import MulArgs
+
+    lib = _lib()
+    rng = np.random.default_rng(m + ncol)
+    a = rng.standard_normal((m, k))
+    b = torch.from_numpy(rng.random((k, ncol)) - 0.25).float().cuda()
+    c = torch.from_numpy(rng.random((m, ncol))).float().cuda()
+    acc = c.double()
+    err = torch.zeros(1, dtype=torch.int32, device='cuda')
+    ad = torch.from_numpy(a).cuda()
+    ref, mag = ad @ b.double(), ad.abs() @ b.double().abs()
+    rb = (2.0**-15 + k*2.0**-23)*mag
+    h = _handle(lib, a, 3 if products == 5 else 2)
+
+    for beta in ([0.0] if rk else [0.0, 1.0]):
+        out = c.clone()
+        p = MulArgs(b1=b.data_ptr(), ldb1=ncol, c=out.data_ptr(), ldc=ncol,
+                    ncol=ncol, nbatch=1, alpha=1.0, beta=beta,
+                    products=products, err=err.data_ptr())
+        if rk:
+            p.rk_stage, p.rk_dt, p.rk_a, p.rk_b = 1, 0.5, 0.25, 2.0
+            p.rk_acc, p.rk_u = acc.data_ptr(), out.data_ptr()
+        torch.cuda.synchronize()
+        lib.mul_bf16x3_apply(h, C.addressof(p), None)
+        torch.cuda.synchronize()
+        assert err.item() == 0
+        if rk:
+            # acc + dt b R and fl32(acc) + dt a R
+            assert bool(((acc - (c.double() + ref)).abs() <= rb).all())
+            want, tol = c.double() + 0.125*ref, 0.125*rb
+        else:
+            want, tol = ref + beta*c.double(), rb
+        tol = tol + 2.0**-22*(want.abs() + mag)
+        assert bool(((out.double() - want).abs() <= tol).all())
+    lib.mul_bf16x3_destroy(h)
