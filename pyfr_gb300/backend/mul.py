@@ -285,6 +285,14 @@ class TensorMulKernels:
                                 ([rowscale] if rowscale is not None else []),
                                 meta)
 
+        # The first pieces of all row ranges, then the second ones: pieces of
+        # different ranges run side by side
+        levels, turn = {}, []
+        for r0, *_ in pieces:
+            turn.append(levels.get(r0, 0))
+            levels[r0] = turn[-1] + 1
+        arglist = [arglist[i] for i in np.argsort(turn, kind='stable')]
+
         be = self.backend
         for h, a in arglist:
             a.err = be.status_word

@@ -72,3 +72,49 @@ def test_epilogue_sets(m, k, ncol, products, rk):
         tol = tol + 2.0**-22*(want.abs() + mag)
         assert bool(((out.double() - want).abs() <= tol).all())
     lib.mul_bf16x3_destroy(h)
+
+
+@pytest.mark.parametrize('nbatch', [1, 3])
+@pytest.mark.parametrize('ncol', [4, 8640, 19460, 50000])
+@pytest.mark.parametrize('rows', [(192, 183), (33, 40, 64), (96, 20, 64, 64),
+                                  (20, 20, 20, 20, 20), (64, 65)])
+def test_row_ranges_side_by_side(rows, ncol, nbatch):
+    """Row ranges, each of two pieces along K (the first stored, the second
+    added), in one call against the same applies one by one: the same bits,
+    whether or not the ranges' kernels are alike."""
+    import torch
+
+    from pyfr_gb300.backend.lib import MulArgs
+
+    lib = _lib()
+    rng = np.random.default_rng(sum(rows) + ncol)
+    m, ks = sum(rows), (40, 27)
+    b = torch.from_numpy(rng.random((nbatch, sum(ks), ncol)) - 0.25)
+    b = b.float().cuda()
+    err = torch.zeros(1, dtype=torch.int32, device='cuda')
+    out = [torch.full((nbatch, m, ncol), 7.0, device='cuda') for _ in '12']
+    hs, calls = [], [[], []]
+    for k0, k, beta in ((0, ks[0], 0.0), (ks[0], ks[1], 1.0)):
+        r0 = 0
+        for r in rows:
+            h = _handle(lib, rng.standard_normal((r, k)), 2)
+            hs.append(h)
+            for o, cl in zip(out, calls):
+                cl.append(MulArgs(
+                    b1=b.data_ptr() + 4*k0*ncol, ldb1=ncol,
+                    c=o.data_ptr() + 4*r0*ncol, ldc=ncol, ncol=ncol,
+                    nbatch=nbatch, bstride1=sum(ks)*ncol, cstride=m*ncol,
+                    alpha=0.5, beta=beta, products=4, err=err.data_ptr()))
+            r0 += r
+    n = len(hs)
+    torch.cuda.synchronize()
+    for h, a in zip(hs, calls[0]):
+        lib.mul_bf16x3_apply(h, C.addressof(a), None)
+    lib.mul_bf16x3_apply_pieces((C.c_void_p*n)(*(h.value for h in hs)),
+                                (C.c_void_p*n)(*map(C.addressof, calls[1])),
+                                n, None)
+    torch.cuda.synchronize()
+    assert err.item() == 0
+    assert bool((out[0] == out[1]).all()) and bool((out[0] != 7.0).all())
+    for h in hs:
+        lib.mul_bf16x3_destroy(h)
