@@ -167,7 +167,8 @@ class PointwiseKernelProvider:
 
     # ---- element kernels ---------------------------------------------------
 
-    def _geom(self, tplargs, smats=None, rcpdjac=None, verts=None, upts=None):
+    def geometry(self, tplargs, smats=None, rcpdjac=None, verts=None,
+                 upts=None):
         linear = 'linear' in tplargs.get('ktype', 'curved')
         # The kernels rebuild metrics in place for multilinear elements
         # only; other linear shapes always read stored terms
@@ -227,7 +228,7 @@ class PointwiseKernelProvider:
     def _tflux_euler(self, tplargs, dims, extrns, u, f, smats=None,
                      verts=None, upts=None):
         nupts, neles = dims
-        lin, (sp, sl), _, (vp, vl), (upp, upl) = self._geom(
+        lin, (sp, sl), _, (vp, vl), (upp, upl) = self.geometry(
             tplargs, smats=smats, verts=verts, upts=upts)
         fn, gamma = self._fn('tflux_euler'), tplargs['c']['gamma']
         up, ul = _mat(u)
@@ -279,7 +280,7 @@ class PointwiseKernelProvider:
                              'its gradient in f')
 
         nupts, neles = dims
-        lin, (sp, sl), (rp, rl), (vp, vl), (upp, upl) = self._geom(
+        lin, (sp, sl), (rp, rl), (vp, vl), (upp, upl) = self.geometry(
             tplargs, smats, rcpdjac, verts, upts)
         gas = _gas(tplargs['c'], tplargs.get('visc_corr', 'none'),
                    self.backend.ref_state)
@@ -318,7 +319,7 @@ class PointwiseKernelProvider:
         """Per-element largest wave speed in reference space
         (pyfr/solvers/euler/kernels/wavespeed.mako:9-44)."""
         nupts, neles = dims
-        lin, (sp, sl), (rp, rl), (vp, vl), (upp, upl) = self._geom(
+        lin, (sp, sl), (rp, rl), (vp, vl), (upp, upl) = self.geometry(
             tplargs, smats, rcpdjac, verts, upts)
         gas = _gas(tplargs['c'], 'none', self.backend.ref_state)
         fn, nd = self._fn('wavespeed'), tplargs['ndims']
@@ -337,7 +338,7 @@ class PointwiseKernelProvider:
     def _gradcoru(self, tplargs, dims, extrns, gradu, smats=None,
                   rcpdjac=None, verts=None, upts=None):
         nupts, neles = dims
-        lin, (sp, sl), (rp, rl), (vp, vl), (upp, upl) = self._geom(
+        lin, (sp, sl), (rp, rl), (vp, vl), (upp, upl) = self.geometry(
             tplargs, smats, rcpdjac, verts, upts)
         fn, nd = self._fn('gradcoru'), tplargs['ndims']
         gp, gl = _mat(gradu)

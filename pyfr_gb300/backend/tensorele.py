@@ -190,11 +190,9 @@ class TensorElementKernels:
                       meta=dict(kind='te_interp', u=u, out=out))
 
     def te_gradflux(self, handle, tplargs, neles, u, comm, gradf, facemask, r,
-                    verts, upts, refgrad=False):
+                    geom, refgrad=False):
         from pyfr_gb300.backend.pointwise import _gas
-        pw = self.backend.pointwise
-        lin, (sp, sl), (rp, rl), _, _ = pw._geom(tplargs, verts=verts,
-                                                 upts=upts)
+        lin, (sp, sl), (rp, rl), _, _ = geom
         gas = _gas(tplargs['c'], tplargs.get('visc_corr', 'none'))
         fn, h = self._fn('gradflux_ns'), handle
         args = (u.data, u.leaddim, comm.data, comm.leaddim, gradf.data,
@@ -203,15 +201,13 @@ class TensorElementKernels:
         def run(stream):
             fn(h, neles, lin, C.byref(gas), *args, stream)
 
-        return Kernel(run, mats=[u, comm, gradf, r, verts, upts], misc=[gas],
+        return Kernel(run, mats=[u, comm, gradf, r], misc=[gas],
                       name='te_gradflux',
                       meta=dict(kind='te_gradflux', tplargs=tplargs, u=u, r=r,
                                 geom_mode=lin, facemask=facemask))
 
-    def te_euler(self, handle, tplargs, neles, u, fc, r, verts, upts):
-        pw = self.backend.pointwise
-        lin, (sp, sl), (rp, rl), _, _ = pw._geom(tplargs, verts=verts,
-                                                 upts=upts)
+    def te_euler(self, handle, tplargs, neles, u, fc, r, geom):
+        lin, (sp, sl), (rp, rl), _, _ = geom
         fn, h = self._fn('euler'), handle
         gamma = tplargs['c']['gamma']
         args = (u.data, u.leaddim, fc.data, fc.leaddim, sp, sl, rp, rl,
@@ -220,13 +216,12 @@ class TensorElementKernels:
         def run(stream):
             fn(h, neles, lin, gamma, *args, stream)
 
-        return Kernel(run, mats=[u, fc, r, verts, upts], name='te_euler',
+        return Kernel(run, mats=[u, fc, r], name='te_euler',
                       meta=dict(kind='te_euler', tplargs=tplargs, u=u, r=r,
                                 geom_mode=lin))
 
-    def te_lift(self, handle, tplargs, neles, fc, r, verts, upts):
-        pw = self.backend.pointwise
-        lin, _, (rp, rl), _, _ = pw._geom(tplargs, verts=verts, upts=upts)
+    def te_lift(self, handle, tplargs, neles, fc, r, geom):
+        lin, _, (rp, rl), _, _ = geom
         fn, h = self._fn('lift'), handle
         # (one 1/|J| per element: every point reads the same row)
         args = (neles, fc.data, fc.leaddim, rp, rl if lin == 0 else 0, r.data,
@@ -235,5 +230,5 @@ class TensorElementKernels:
         def run(stream):
             fn(h, *args, stream)
 
-        return Kernel(run, mats=[fc, r, verts, upts], name='te_lift',
+        return Kernel(run, mats=[fc, r], name='te_lift',
                       meta=dict(kind='te_lift', fc=fc, r=r))

@@ -791,8 +791,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) mul_umma_kernel(const __grid_cons
 // each: where a range's tiles are fewer than the SMs the others' fill them, and
 // elsewhere the ranges share their reads of B in L2.  The 375-row gradient of
 // p = 4 hexahedra, 8640 columns (68 tiles of 152 SMs), two ranges of two pieces
-// along K: four launches in turn -> two, 12.5 us less in a right-hand side of
-// 133 us.
+// along K: four launches in turn -> two, 107 -> 96 us a right-hand side.
 constexpr int MAX_SIDE = 4;
 struct UmmaSet {
     UmmaArgs p[MAX_SIDE];

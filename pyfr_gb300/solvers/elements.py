@@ -20,6 +20,7 @@ from functools import cached_property
 
 import numpy as np
 
+from pyfr_gb300.backend.pointwise import GEOM_VERTICES
 from pyfr_gb300.backend.types import NullKernel
 from pyfr_gb300.mesh import fuzzy_face_order
 from pyfr_gb300.shapes import SHAPES, adjugate_det, get_shape
@@ -371,10 +372,18 @@ class BaseElements:
         # (the kernels' rows are below 4 GiB)
         if self._scal_fpts.leaddim*self._scal_fpts.itemsize >= 2**32:
             return None
+        # (they read stored metric terms)
+        if self.te_geom()[0] == GEOM_VERTICES:
+            return None
         return be.tensor_elements.handle(self.basis, viscous)
 
-    def _te_mats(self):
-        return dict(verts=self.ploc_at('linspts', 'linear'), upts=self.upts)
+    def te_geom(self):
+        """The metric terms that the element kernels read, formed at the
+        set-up: a right-hand side's kernels are made at its first call, when
+        the host copies of a large mesh's vertices are gone."""
+        return self._cached(('te', 'geom'), lambda: self._be.pointwise.geometry(
+            dict(ktype='linear', ndims=self.ndims),
+            verts=self.ploc_at('linspts', 'linear'), upts=self.upts))
 
     def set_te_faces(self, fidxs):
         """Have the gradient formed at the flux points of these faces."""
@@ -630,7 +639,7 @@ class EulerElements(_WavespeedMixin, _DivergenceMixin, FluidElements,
             return be.kernel(
                 'te_euler', te[0], tplargs | {'ktype': 'linear'}, self.neles,
                 self.scal_upts[uin], self._scal_fpts, self.scal_upts[fout],
-                **self._te_mats()) if te else NullKernel()
+                self.te_geom()) if te else NullKernel()
         self.te_rhs = te_euler
 
 
@@ -815,7 +824,8 @@ class NavierStokesElements(_WavespeedMixin, _DivergenceMixin, FluidElements,
                 'te_gradflux', te[0], tplargs | {'ktype': 'linear-fused'},
                 self.neles, self.scal_upts[uin], self._comm_fpts,
                 self._vect_fpts, self.te_facemask, self.scal_upts[fout],
-                refgrad=not self.grad_writeback, **self._te_mats()) if te else NullKernel()
+                self.te_geom(),
+                refgrad=not self.grad_writeback) if te else NullKernel()
         self.te_rhs = te_gradflux
 
         def te_lift(fout):
@@ -823,5 +833,5 @@ class NavierStokesElements(_WavespeedMixin, _DivergenceMixin, FluidElements,
             return be.kernel(
                 'te_lift', te[0], tplargs | {'ktype': 'linear'}, self.neles,
                 self._scal_fpts, self.scal_upts[fout],
-                **self._te_mats()) if te else NullKernel()
+                self.te_geom()) if te else NullKernel()
         kernels['te_lift'] = te_lift

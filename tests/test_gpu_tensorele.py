@@ -141,3 +141,27 @@ def test_element_kernels_special_values(flow):
     assert 0 < fin.sum() < fin.size
     assert np.array_equal(np.isfinite(a), fin)
     assert np.abs(a - b)[fin].max() <= 1e-12*np.abs(b[fin]).max()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize('mesh_form', ['uniform', 'sheared', 'bent'])
+@pytest.mark.parametrize('flow', ['euler', 'ns'])
+def test_element_kernels_without_host_geometry(flow, mesh_form, monkeypatch):
+    """The set-up of a large mesh drops the host copies of its vertices, and
+    a right-hand side's kernels are made after that: the same bits as with
+    the copies kept."""
+    from pyfr_gb300.backend import base
+
+    got = []
+    for keep in (base.HOST_KEEP, 50):
+        monkeypatch.setattr(base, 'HOST_KEEP', keep)
+        s = _system(3, flow, 3, 3, 'double', mesh_form, 0.5, 'rusanov',
+                    'auto')
+        s.commit()
+        names = {k.name or '' for g in s.rhs_graphs(0, 1) for k in g.klist}
+        assert any(x.startswith('te_') for x in names)
+        s.rhs(0.0, 0, 1)
+        s.rhs(0.0, 0, 0)
+        s.backend.wait()
+        got.append([s.ele_scal_upts(i)[0] for i in (0, 1)])
+    assert all(np.array_equal(a, b) for a, b in zip(*got))
