@@ -165,6 +165,19 @@ def kernel_bytes(k, be):
         nread = nv if one else 2*nv
         nwrite = 2*nv if (t.get('both_sides') or not one) else nv
         return n*((nread + nwrite)*itemsize + 4*4)
+    if kind in ('te_interp', 'te_gradflux', 'te_lift', 'te_euler'):
+        # The element kernels: every matrix once (R, which te_lift adds to,
+        # read and written), and of the face gradients those of the faces that
+        # an interface reads (one set of metric terms per element is small)
+        def size(n, share=1):
+            return m[n].nrow*m[n].ncol*share if n in m else 0
+
+        vals = size('u') + size('out') + size('comm') + size('fc') + \
+            size('r', 2 if kind == 'te_lift' else 1)
+        if kind == 'te_gradflux':
+            nd = m['tplargs']['ndims']
+            vals += size('gradf', bin(m['facemask']).count('1')/(2*nd))
+        return int(vals)*itemsize
     if kind == 'negdivconf':
         nupts, neles = m['dims']
         nv = m['tplargs']['nvars']

@@ -203,7 +203,8 @@ class TensorElementKernels:
 
         return Kernel(run, mats=[u, comm, gradf, r], misc=[gas],
                       name='te_gradflux',
-                      meta=dict(kind='te_gradflux', tplargs=tplargs, u=u, r=r,
+                      meta=dict(kind='te_gradflux', tplargs=tplargs, u=u,
+                                comm=comm, gradf=gradf, r=r,
                                 geom_mode=lin, facemask=facemask))
 
     def te_euler(self, handle, tplargs, neles, u, fc, r, geom):
@@ -217,7 +218,7 @@ class TensorElementKernels:
             fn(h, neles, lin, gamma, *args, stream)
 
         return Kernel(run, mats=[u, fc, r], name='te_euler',
-                      meta=dict(kind='te_euler', tplargs=tplargs, u=u, r=r,
+                      meta=dict(kind='te_euler', tplargs=tplargs, u=u, fc=fc, r=r,
                                 geom_mode=lin))
 
     def te_lift(self, handle, tplargs, neles, fc, r, geom):
