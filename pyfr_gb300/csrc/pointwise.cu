@@ -961,12 +961,20 @@ int intcflux_ns(int ndims, int64_t n, int rsolver, const b200_gas_t *gas, double
     const int sides = beta == 0.5 ? 1 : beta == -0.5 ? 2 : 3, pen = tau != 0.0;
     const bool ok = b200::with_rsolver(rsolver, [&](auto rsc) {
         constexpr int RS = decltype(rsc)::value;
-        if (ndims == 2)
-            b200::launch(intcflux_ns_kernel<RS, 2, T, false>, grid, PW_BLOCK, 0, st, n, g, (T)beta, (T)tau, sides, pen, l, r, gl, gr, ix64, nl, ldn, nl_unit, va, fm);
-        else if (!fm.m)
-            b200::launch(intcflux_ns_kernel<RS, 3, T, false>, grid, PW_BLOCK, 0, st, n, g, (T)beta, (T)tau, sides, pen, l, r, gl, gr, ix64, nl, ldn, nl_unit, va, fm);
+        auto go = [&](auto nd, auto refgrad) {
+            b200::launch(intcflux_ns_kernel<RS, nd(), T, refgrad()>, grid, PW_BLOCK, 0, st, n, g, (T)beta, (T)tau, sides, pen, l, r, gl, gr, ix64, nl, ldn, nl_unit, va, fm);
+        };
+        using b2 = std::integral_constant<int, 2>;
+        using b3 = std::integral_constant<int, 3>;
+        // (gradients in reference space need the face metrics in 2-D as in 3-D)
+        if (ndims == 2 && fm.m)
+            go(b2(), std::true_type());
+        else if (ndims == 2)
+            go(b2(), std::false_type());
+        else if (fm.m)
+            go(b3(), std::true_type());
         else
-            b200::launch(intcflux_ns_kernel<RS, 3, T, true>, grid, PW_BLOCK, 0, st, n, g, (T)beta, (T)tau, sides, pen, l, r, gl, gr, ix64, nl, ldn, nl_unit, va, fm);
+            go(b3(), std::false_type());
     });
     if (!ok) return b200::set_error(B200_ERR_ARG, "intcflux: unknown Riemann solver %d", rsolver);
     B200_CHECK_LAUNCH("intcflux_ns");
