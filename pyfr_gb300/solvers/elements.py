@@ -352,13 +352,21 @@ class BaseElements:
     # set by the system
     te_facemask = 0
 
-    def te_handle(self):
-        """(handle, flux points of the lines) when this type's right-hand
-        side runs on the element kernels: tensor-product elements that are
-        all linear, in the backend's own precision (no tensor-core applies),
-        on unshifted states, with no anti-aliasing, shock capturing or
-        source terms.  None otherwise.  (The state of the system's set-up
-        when its kernels are made decides.)"""
+    # (handle, flux points of the lines) when this type's right-hand side
+    # runs on the element kernels, else None: decided once, when the system
+    # is committed, since the kernels that they take the place of are then
+    # left out (the reference state that the condition asks for is the
+    # backend's, and another integrator on it may set it later)
+    te = None
+
+    def choose_element_kernels(self):
+        self.te = self._te_handle()
+
+    def _te_handle(self):
+        """The handle for tensor-product elements that are all linear, in the
+        backend's own precision (no tensor-core applies), on unshifted
+        states, with no anti-aliasing, shock capturing or source terms.  None
+        otherwise."""
         be = self._be
         viscous = 'grad_upts' in self._scratch_bufs
         tensor = be.mul_precision != 'native' and be.fpdtype == np.float32
@@ -387,7 +395,7 @@ class BaseElements:
 
     def set_te_faces(self, fidxs):
         """Have the gradient formed at the flux points of these faces."""
-        fpt = self.te_handle()[1]
+        fpt = self.te[1]
         self.te_facemask = 0
         for d, e in np.ndindex(self.ndims, 2):
             pts = set(fpt[d, :, e].tolist())
@@ -396,9 +404,8 @@ class BaseElements:
                 self.te_facemask |= 1 << (2*d + e)
 
     def _disu_kernel(self, uin):
-        te = self.te_handle()
-        if te:
-            return self._be.kernel('te_interp', te[0], self.scal_upts[uin],
+        if self.te:
+            return self._be.kernel('te_interp', self.te[0], self.scal_upts[uin],
                                    self._scal_fpts, self.neles)
         return self._be.kernel('mul', self.opmat('M0'), self.scal_upts[uin],
                                out=self._scal_fpts)
@@ -635,11 +642,10 @@ class EulerElements(_WavespeedMixin, _DivergenceMixin, FluidElements,
         self._divergence_kernels()
 
         def te_euler(uin, fout):
-            te = self.te_handle()
             return be.kernel(
-                'te_euler', te[0], tplargs | {'ktype': 'linear'}, self.neles,
+                'te_euler', self.te[0], tplargs | {'ktype': 'linear'}, self.neles,
                 self.scal_upts[uin], self._scal_fpts, self.scal_upts[fout],
-                self.te_geom()) if te else NullKernel()
+                self.te_geom())
         self.te_rhs = te_euler
 
 
@@ -819,19 +825,17 @@ class NavierStokesElements(_WavespeedMixin, _DivergenceMixin, FluidElements,
         # (the flux at the solution points, the divergence and, at the flux
         # points, the gradient, in one kernel; then the correction)
         def te_gradflux(uin, fout):
-            te = self.te_handle()
             return be.kernel(
-                'te_gradflux', te[0], tplargs | {'ktype': 'linear-fused'},
+                'te_gradflux', self.te[0], tplargs | {'ktype': 'linear-fused'},
                 self.neles, self.scal_upts[uin], self._comm_fpts,
                 self._vect_fpts, self.te_facemask, self.scal_upts[fout],
                 self.te_geom(),
-                refgrad=not self.grad_writeback) if te else NullKernel()
+                refgrad=not self.grad_writeback)
         self.te_rhs = te_gradflux
 
         def te_lift(fout):
-            te = self.te_handle()
             return be.kernel(
-                'te_lift', te[0], tplargs | {'ktype': 'linear'}, self.neles,
+                'te_lift', self.te[0], tplargs | {'ktype': 'linear'}, self.neles,
                 self._scal_fpts, self.scal_upts[fout],
-                self.te_geom()) if te else NullKernel()
+                self.te_geom()) if self.te else NullKernel()
         kernels['te_lift'] = te_lift

@@ -149,6 +149,9 @@ class BaseSystem:
                    for et, e in self.ele_map.items())
 
     def commit(self):
+        for e in self.ele_map.values():
+            e.choose_element_kernels()
+        self._setup_gradients()
         covered = self._interfaces_cover_fpts()
         for e in self.ele_map.values():
             e.comm_covered = covered
@@ -216,6 +219,10 @@ class BaseSystem:
             e.release_host_geometry()
         self.backend.release_host_copies()
 
+    def _setup_gradients(self):
+        """Before the kernels are made: which gradients the interfaces read
+        and in which form."""
+
     def _gen_kernels(self):
         self._kernels = kernels = defaultdict(list)
         self._ktags = {}
@@ -227,7 +234,7 @@ class BaseSystem:
             for p in plist:
                 # (what an element type's own kernel takes the place of is
                 # not made, but for the gradients of the diagnostics)
-                skip = () if pn != 'eles' or not p.te_handle() else \
+                skip = () if pn != 'eles' or not p.te else \
                     set(self._general_kernels) - {'tgradpcoru_upts',
                                                   'tgradcoru_upts'}
                 for kn, kget in p.kernels.items():
@@ -265,12 +272,15 @@ class BaseSystem:
                         'gradcoru_fpts', 'tdisf', 'tdivtpcorf', 'tdivtconf',
                         'negdivconf')
 
+    # One of these finishes an element type's right-hand side
+    _last_kernels = ('negdivconf', 'te_lift', 'tdivtconf_cat', 'te_rhs')
+
     def _get_rhs_kernels(self, uinbank, foutbank):
         """The kernels of one right-hand side: for the element types that
         have one their own kernel, te_rhs, else the general ones."""
         k = self._get_kernels(uinbank, foutbank)
         for e in self.ele_map.values():
-            if not e.te_handle():
+            if not e.te:
                 continue
             tag = f'eles/{id(e)}'
             for n in self._general_kernels:
@@ -279,6 +289,11 @@ class BaseSystem:
             l = e.te_rhs(uinbank, foutbank)
             self._ktags[l] = tag
             k['eles/te_rhs'].append(l)
+        for e in self.ele_map.values():
+            tag = f'eles/{id(e)}'
+            if not any(self._ktags[l] == tag for n in self._last_kernels
+                       for l in k[f'eles/{n}']):
+                raise RuntimeError('No kernel finishes the right-hand side')
         return k
 
     def _kdeps(self, kdict, kern, *dnames):
@@ -516,12 +531,9 @@ class BaseSystem:
         return items, {f'eles/{id(e)}': self._rhs_ends(pos, f'eles/{id(e)}')
                        for e in self.ele_map.values()}
 
-    @staticmethod
-    def _rhs_ends(pos, tag):
-        for n in ('negdivconf', 'te_lift', 'tdivtconf_cat', 'te_rhs'):
-            if pos.get((f'eles/{n}', tag)):
-                return pos[f'eles/{n}', tag]
-        raise RuntimeError('No kernel finishes the right-hand side')
+    def _rhs_ends(self, pos, tag):
+        return next(pos[f'eles/{n}', tag] for n in self._last_kernels
+                    if pos.get((f'eles/{n}', tag)))
 
     def preproc_kernels(self, uinbank):
         """Before the first step: filter, then every element's and face's
@@ -643,10 +655,9 @@ class NavierStokesSystem(BaseSystem):
     mpiinterscls = NavierStokesMPIInters
     bcinterscls = NavierStokesBCInters
 
-    def commit(self):
+    def _setup_gradients(self):
         self._setup_element_kernels()
         self._setup_face_gradients()
-        super().commit()
 
     def _setup_element_kernels(self):
         """Tell the element types that run on their own kernels which
@@ -661,7 +672,7 @@ class NavierStokesSystem(BaseSystem):
                 for et, fidx, _ in s.items():
                     read[et].add(fidx)
         for et, e in self.ele_map.items():
-            if e.te_handle():
+            if e.te:
                 e.set_te_faces(read[et])
 
     def _setup_face_gradients(self):
