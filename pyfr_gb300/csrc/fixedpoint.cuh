@@ -77,6 +77,12 @@ __device__ __forceinline__ double fixed_to_f64(long long t, int sc) {
     return h == 0 ? 0.0 : __hiloint2double(hi, (int)q);
 }
 
+// The same with the conversion on the FP64 unit (kernels that leave it idle)
+__device__ __forceinline__ double fixed_to_f64_cvt(long long t, int sc) {
+    const double y = (double)t;
+    return t == 0 ? 0.0 : __hiloint2double(__double2hiint(y) + sc * (1 << 20), __double2loint(y));
+}
+
 // Sums of products of one output
 struct Fx {
     long long hh, w;
@@ -89,15 +95,11 @@ struct Fx {
         w += (long long)a.x * b.y;
         w += (long long)a.y * b.x;
     }
+    __device__ __forceinline__ long long total() const { return hh + (w >> 31); }
     // sc: emax - s - (991 + BITS)
-    __device__ __forceinline__ double value(int sc) const {
-        return fixed_to_f64(hh + (w >> 31), sc);
-    }
-    // The same with the conversion on the FP64 unit (kernels that leave it idle)
+    __device__ __forceinline__ double value(int sc) const { return fixed_to_f64(total(), sc); }
     __device__ __forceinline__ double value_cvt(int sc) const {
-        const long long t = hh + (w >> 31);
-        const double y = (double)t;
-        return t == 0 ? 0.0 : __hiloint2double(__double2hiint(y) + sc * (1 << 20), __double2loint(y));
+        return fixed_to_f64_cvt(total(), sc);
     }
 };
 

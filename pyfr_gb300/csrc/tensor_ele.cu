@@ -26,9 +26,12 @@
 // the line's own largest exponent (the arithmetic of the general apply,
 // csrc/mul.cu: IMAD.WIDE issues 56 a clock and SM where the FP64 unit issues
 // 2 FMAs; its support test is not needed, since a line is its support).
-// With B of 58 or 60 bits and A of 60 or 61 below the largest row sum the
-// result is within 2^-56 of (row sum)(largest value), an eighth of the rounding
-// of one FP64 FMA.
+// With B of 60 bits and A of 60 or 61 below the largest row sum the result is
+// within 6 2^-56 of (largest row sum)(largest value of the line), below the
+// rounding of one FP64 FMA.  The divergence at a point is the sum of a line of
+// each direction, every line over its own exponent, and the integer sums are
+// shifted to the largest of them before the one rounding to FP64: an output
+// keeps its bits however large the fluxes elsewhere in the element are.
 // The FP64 unit is left to the flux, beside which the integer work of the
 // other warps runs.
 #include <math.h>
@@ -72,10 +75,10 @@ struct Mat<float, NO, NI> {
 
 // a = (ah, al): A = (ah 2^31 + al) 2^-(s + 31), |al| <= 2^30, every row's sum of
 // |ah| below 2^30 + NI, or below 2^29 + NI (wide: rows of ND directions are
-// summed).  With B of BITS = 60 bits (58 for wide), |bh| < 2^(BITS - 31), |bl| <
-// 2^31, the cross sum of Fx stays below 2^63: 2^61 + 7 2^59 for one line of 7
-// entries, 3 2^60 + 2^60 + 22 2^57 for three of them and a kept value, and the
-// high sum below 2^60.
+// summed).  With B of BITS = 60 bits (58 where ND lines make one sum), |bh| <
+// 2^(BITS - 31), |bl| < 2^31, the cross sum of Fx stays below 2^63: 2^61 + 7 2^59
+// for one line of 7 entries, 2 2^60 + 14 2^57 for two, and the high sum below
+// 2^60, of which three still make less than the 2^61 that Fx::value takes.
 template <int NO, int NI>
 struct Mat<double, NO, NI> {
     double d[NO][NI];
@@ -188,167 +191,17 @@ struct Line {
 };
 
 // One thread's outputs of the divergence: the Q points of x-line l, from the
-// fluxes of all directions along their lines, Fc at the lines' ends and (KEEP)
-// a value already there.  Fluxes: f(d, p) gives direction d at point p; ends:
-// c(d, l, end).  The inputs are visited twice, for the largest exponent and for
-// the products, rather than held.
-template <typename T, int ND, int Q, bool FLUX, bool LIFT, bool KEEP, typename V>
-__device__ __forceinline__ void visit(const Line<T, ND, Q> &P, int l, V &&vis) {
-    const int y = l % Q, z = l / Q;
-#pragma unroll
-    for (int j = 0; j < Q; j++)
-        if constexpr (FLUX) vis.along(0, l * Q + j, j);
-#pragma unroll
-    for (int e = 0; e < 2; e++)
-        if constexpr (LIFT) vis.along_end(0, l, e);
-#pragma unroll
-    for (int d = 1; d < ND; d++) {
-        const int row = d == 1 ? y : z;
-#pragma unroll
-        for (int i = 0; i < Q; i++) {
-            // line of direction d through point i of the x-line
-            const int ld = d == 1 ? (ND == 3 ? z * Q + i : i) : y * Q + i;
-            const int b = P.base(d, ld), st = P.stride(d);
-#pragma unroll
-            for (int j = 0; j < Q; j++)
-                if constexpr (FLUX) vis.across(d, b + j * st, i, row, j);
-#pragma unroll
-            for (int e = 0; e < 2; e++)
-                if constexpr (LIFT) vis.across_end(d, ld, e, i, row);
-        }
-    }
-#pragma unroll
-    for (int i = 0; i < Q; i++)
-        if constexpr (KEEP) vis.keep(l * Q + i, i);
-}
-
-template <typename T, int ND, int Q, typename G>
-struct SumVisit {
-    const Line<T, ND, Q> &P;
-    const G &g;
-    T y[Q];
-    __device__ __forceinline__ void along(int d, int p, int j) {
-        const T x = g.flux(d, p);
-#pragma unroll
-        for (int i = 0; i < Q; i++)
-            if (!absent<Q, Q + 2>(i, j)) y[i] += P.div.d[i][j] * x;
-    }
-    __device__ __forceinline__ void along_end(int d, int l, int e) {
-        const T x = g.end(d, l, e);
-#pragma unroll
-        for (int i = 0; i < Q; i++) y[i] += P.div.d[i][Q + e] * x;
-    }
-    __device__ __forceinline__ void across(int d, int p, int i, int row, int j) {
-        if (!absent<Q, Q + 2>(row, j)) y[i] += P.div.d[row][j] * g.flux(d, p);
-    }
-    __device__ __forceinline__ void across_end(int d, int l, int e, int i, int row) {
-        y[i] += P.div.d[row][Q + e] * g.end(d, l, e);
-    }
-    __device__ __forceinline__ void keep(int p, int i) { y[i] += g.old(p); }
-};
-
-template <typename G>
-struct MaxVisit {
-    const G &g;
-    int mx;
-    __device__ __forceinline__ void along(int d, int p, int) { mx = max(mx, g.flux_hi(d, p)); }
-    __device__ __forceinline__ void along_end(int d, int l, int e) {
-        mx = max(mx, hi_abs(g.end(d, l, e)));
-    }
-    __device__ __forceinline__ void across(int d, int p, int, int, int) {
-        mx = max(mx, g.flux_hi(d, p));
-    }
-    __device__ __forceinline__ void across_end(int d, int l, int e, int, int) {
-        mx = max(mx, hi_abs(g.end(d, l, e)));
-    }
-    __device__ __forceinline__ void keep(int p, int) { mx = max(mx, hi_abs(g.old(p))); }
-};
-
-template <int ND, int Q, typename G>
-struct FxVisit {
-    const Line<double, ND, Q> &P;
-    const G &g;
-    int emax;
-    Fx s[Q];
-    __device__ __forceinline__ void along(int d, int p, int j) {
-        const int2 b = split<58>(g.flux(d, p), emax);
-#pragma unroll
-        for (int i = 0; i < Q; i++)
-            if (!absent<Q, Q + 2>(i, j)) s[i].mad(P.div.a[i][j], b);
-    }
-    __device__ __forceinline__ void along_end(int d, int l, int e) {
-        const int2 b = split<58>(g.end(d, l, e), emax);
-#pragma unroll
-        for (int i = 0; i < Q; i++) s[i].mad(P.div.a[i][Q + e], b);
-    }
-    __device__ __forceinline__ void across(int d, int p, int i, int row, int j) {
-        if (!absent<Q, Q + 2>(row, j)) s[i].mad(P.div.a[row][j], split<58>(g.flux(d, p), emax));
-    }
-    __device__ __forceinline__ void across_end(int d, int l, int e, int i, int row) {
-        s[i].mad(P.div.a[row][Q + e], split<58>(g.end(d, l, e), emax));
-    }
-    // (the coefficient one is 2^s: s is at most 29 for row sums of 1/2 and
-    // more, which te_create asks for, and positive for those it takes)
-    __device__ __forceinline__ void keep(int p, int i) {
-        s[i].mad(make_int2(1 << P.div.s, 0), split<58>(g.old(p), emax));
+// fluxes of all directions along their lines and (LIFT) the common flux at the
+// lines' ends.  Line of direction d > 0 through point i of x-line l:
+template <int ND, int Q>
+struct Cross {
+    int line, row;      // and the point's place on it
+    __device__ __forceinline__ Cross(int d, int l, int i) {
+        const int y = l % Q, z = l / Q;
+        row = d == 1 ? y : z;
+        line = d == 1 ? (ND == 3 ? z * Q + i : i) : y * Q + i;
     }
 };
-
-// Fluxes that are in fixed point already
-template <int ND, int Q, typename G>
-struct FixedVisit {
-    const Line<double, ND, Q> &P;
-    const G &g;
-    Fx s[Q];
-    __device__ __forceinline__ void along(int d, int p, int j) {
-        const int2 b = *reinterpret_cast<const int2 *>(g.at(d, p));
-#pragma unroll
-        for (int i = 0; i < Q; i++)
-            if (!absent<Q, Q + 2>(i, j)) s[i].mad(P.div.a[i][j], b);
-    }
-    __device__ __forceinline__ void across(int d, int p, int i, int row, int j) {
-        // (an absent entry is zero)
-        s[i].mad(P.div.a[row][j], *reinterpret_cast<const int2 *>(g.at(d, p)));
-    }
-    __device__ __forceinline__ void along_end(int d, int l, int e) {
-        const int2 b = *reinterpret_cast<const int2 *>(g.end_at(d, l, e));
-#pragma unroll
-        for (int i = 0; i < Q; i++) s[i].mad(P.div.a[i][Q + e], b);
-    }
-    __device__ __forceinline__ void across_end(int d, int l, int e, int i, int row) {
-        s[i].mad(P.div.a[row][Q + e], *reinterpret_cast<const int2 *>(g.end_at(d, l, e)));
-    }
-    __device__ __forceinline__ void keep(int, int) {}
-};
-
-template <bool FLUX, bool LIFT, bool KEEP, int ND, int Q, typename G>
-__device__ __forceinline__ void div_line(const Line<float, ND, Q> &P, const G &g, int l,
-                                         float (&y)[Q]) {
-    SumVisit<float, ND, Q, G> v{P, g, {}};
-    visit<float, ND, Q, FLUX, LIFT, KEEP>(P, l, v);
-#pragma unroll
-    for (int i = 0; i < Q; i++) y[i] = v.y[i];
-}
-
-template <bool FLUX, bool LIFT, bool KEEP, int ND, int Q, typename G>
-__device__ __forceinline__ void div_line(const Line<double, ND, Q> &P, const G &g, int l,
-                                         double (&y)[Q]) {
-    MaxVisit<G> m{g, 0};
-    visit<double, ND, Q, FLUX, LIFT, KEEP>(P, l, m);
-    if (out_of_range(m.mx)) {
-        SumVisit<double, ND, Q, G> v{P, g, {}};
-        visit<double, ND, Q, FLUX, LIFT, KEEP>(P, l, v);
-#pragma unroll
-        for (int i = 0; i < Q; i++) y[i] = v.y[i];
-        return;
-    }
-    FxVisit<ND, Q, G> v{P, g, max(m.mx >> 20, 64), {}};
-#pragma unroll
-    for (int i = 0; i < Q; i++) v.s[i].clear();
-    visit<double, ND, Q, FLUX, LIFT, KEEP>(P, l, v);
-#pragma unroll
-    for (int i = 0; i < Q; i++) y[i] = v.s[i].value_cvt(v.emax - P.div.s - 1049);
-}
 
 // ---- kernels ------------------------------------------------------------------
 
@@ -433,46 +286,171 @@ struct SmemFlux {
     }
     __device__ __forceinline__ T flux(int d, int p) const { return *at(d, p); }
     __device__ __forceinline__ T end(int d, int l, int e) const { return *end_at(d, l, e); }
+    // value j of line l of direction d: its points, then its ends
+    __device__ __forceinline__ const T *on(int d, int l, int j) const {
+        return j < Q ? at(d, P.base(d, l) + j * P.stride(d)) : end_at(d, l, j - Q);
+    }
 };
 
-// x in fixed point over the largest magnitude mx of its element and variable, in
-// its own place (left as it is where that is out of range)
-__device__ __forceinline__ void fix_in_place(double &x, int mx) {
-    if (!out_of_range(mx)) *reinterpret_cast<int2 *>(&x) = split<58>(x, max(mx >> 20, 64));
+// Exponents of the lines of an element in shared memory, as the products take
+// them (-1: the line's values are out of range and left as they are); the
+// variables next to each other, so that the groups of a warp, which take
+// neighbouring ones, meet no bank twice
+template <int ND, int Q, int E>
+struct LineExp {
+    static constexpr int NV = ND + 2, L = ipow(Q, ND - 1), N = ND * NV * L * E;
+    int *p;             // + element
+    __device__ __forceinline__ int &operator()(int d, int l, int v) const {
+        return p[((d * L + l) * NV + v) * E];
+    }
+};
+
+// The values of a line (LIFT: with its ends) in fixed point over their largest
+// magnitude, in their own places: every value is an operand of one line's
+// outputs alone
+template <bool LIFT, int ND, int Q, int E>
+__device__ __forceinline__ void fix_line(const SmemFlux<double, ND, Q, E> &g,
+                                         const LineExp<ND, Q, E> &ex, int d, int l) {
+    constexpr int N = LIFT ? Q + 2 : Q;
+    double x[N];
+    int mx = 0;
+#pragma unroll
+    for (int j = 0; j < N; j++) {
+        x[j] = *g.on(d, l, j);
+        mx = max(mx, hi_abs(x[j]));
+    }
+    const bool wild = out_of_range(mx);
+    const int emax = max(mx >> 20, 64);
+    ex(d, l, g.v) = wild ? -1 : emax;
+    if (wild) return;
+#pragma unroll
+    for (int j = 0; j < N; j++)
+        *reinterpret_cast<int2 *>(const_cast<double *>(g.on(d, l, j))) = split<60>(x[j], emax);
 }
-__device__ __forceinline__ void fix_in_place(float &, int) {}
+
+// All lines of the thread's element, over its G groups of threads: a line of
+// every variable a group where that fills the rounds as well (p = 3 hexahedra),
+// which saves index arithmetic, else a line and variable
+template <bool LIFT, int G, int ND, int Q, int E>
+__device__ __forceinline__ void fix_lines(SmemFlux<double, ND, Q, E> g,
+                                          const LineExp<ND, Q, E> &ex, int grp) {
+    constexpr int NV = ND + 2, L = ipow(Q, ND - 1), NL = ND * L;
+    if constexpr ((NL + G - 1) / G * NV <= (NL * NV + G - 1) / G) {
+        for (int t = grp; t < NL; t += G)
+#pragma unroll 1
+            for (g.v = 0; g.v < NV; g.v++) fix_line<LIFT>(g, ex, t / L, t % L);
+    } else {
+        for (int t = grp; t < NL * NV; t += G) {
+            g.v = t % NV;
+            fix_line<LIFT>(g, ex, t / NV / L, t / NV % L);
+        }
+    }
+}
+template <bool LIFT, int G, int ND, int Q, int E>
+__device__ __forceinline__ void fix_lines(const SmemFlux<float, ND, Q, E> &,
+                                          const LineExp<ND, Q, E> &, int) {}
 
 // The divergence at the points of x-line l from the element's fluxes (and,
-// LIFT, common fluxes) in shared memory; FP64: in fixed point over mx
+// LIFT, common fluxes) in shared memory
 template <bool LIFT, int ND, int Q, int E>
 __device__ __forceinline__ void smem_div(const Line<float, ND, Q> &P,
-                                         const SmemFlux<float, ND, Q, E> &g, int l, int,
-                                         float (&y)[Q]) {
-    SumVisit<float, ND, Q, SmemFlux<float, ND, Q, E>> f{P, g, {}};
-    visit<float, ND, Q, true, LIFT, false>(P, l, f);
+                                         const SmemFlux<float, ND, Q, E> &g,
+                                         const LineExp<ND, Q, E> &, int l, float (&y)[Q]) {
+    constexpr int N = LIFT ? Q + 2 : Q;
 #pragma unroll
-    for (int i = 0; i < Q; i++) y[i] = f.y[i];
+    for (int i = 0; i < Q; i++) y[i] = 0.0f;
+#pragma unroll
+    for (int j = 0; j < N; j++) {
+        const float x = *g.on(0, l, j);
+#pragma unroll
+        for (int i = 0; i < Q; i++)
+            if (!absent<Q, Q + 2>(i, j)) y[i] += P.div.d[i][j] * x;
+    }
+#pragma unroll
+    for (int d = 1; d < ND; d++)
+#pragma unroll
+        for (int i = 0; i < Q; i++) {
+            const Cross<ND, Q> c(d, l, i);
+#pragma unroll
+            for (int j = 0; j < N; j++)
+                if (!absent<Q, Q + 2>(c.row, j)) y[i] += P.div.d[c.row][j] * *g.on(d, c.line, j);
+        }
+}
+
+// One output whose lines are not all in range: FP64 FMAs for those that are not
+template <bool LIFT, int ND, int Q, int E>
+__device__ __noinline__ double wild_div(const Line<double, ND, Q> &P, SmemFlux<double, ND, Q, E> g,
+                                        LineExp<ND, Q, E> ex, int l, int i) {
+    constexpr int N = LIFT ? Q + 2 : Q;
+    double y = 0.0;
+#pragma unroll 1
+    for (int d = 0; d < ND; d++) {
+        const Cross<ND, Q> c(d, l, i);
+        const int line = d ? c.line : l, row = d ? c.row : i, e = ex(d, line, g.v);
+        Fx s;
+        s.clear();
+        double f = 0.0;
+#pragma unroll 1
+        for (int j = 0; j < N; j++) {
+            const double *x = g.on(d, line, j);
+            if (absent<Q, Q + 2>(row, j)) continue;
+            if (e < 0)
+                f = fma(P.div.d[row][j], *x, f);
+            else
+                s.mad(P.div.a[row][j], *reinterpret_cast<const int2 *>(x));
+        }
+        y += e < 0 ? f : s.value_cvt(e - P.div.s - 1051);
+    }
+    return y;
 }
 
 template <bool LIFT, int ND, int Q, int E>
 __device__ __forceinline__ void smem_div(const Line<double, ND, Q> &P,
-                                         const SmemFlux<double, ND, Q, E> &g, int l, int mx,
-                                         double (&y)[Q]) {
-    using G = SmemFlux<double, ND, Q, E>;
-    if (out_of_range(mx)) {
-        SumVisit<double, ND, Q, G> f{P, g, {}};
-        visit<double, ND, Q, true, LIFT, false>(P, l, f);
+                                         const SmemFlux<double, ND, Q, E> &g,
+                                         const LineExp<ND, Q, E> &ex, int l, double (&y)[Q]) {
+    constexpr int N = LIFT ? Q + 2 : Q;
+    const auto fixed = [&](int d, int line, int j) {
+        return *reinterpret_cast<const int2 *>(g.on(d, line, j));
+    };
+    Fx s[Q];
 #pragma unroll
-        for (int i = 0; i < Q; i++) y[i] = f.y[i];
-        return;
+    for (int i = 0; i < Q; i++) s[i].clear();
+#pragma unroll
+    for (int j = 0; j < N; j++) {
+        const int2 b = fixed(0, l, j);
+#pragma unroll
+        for (int i = 0; i < Q; i++)
+            if (!absent<Q, Q + 2>(i, j)) s[i].mad(P.div.a[i][j], b);
     }
-    FixedVisit<ND, Q, G> f{P, g, {}};
+    const int e0 = ex(0, l, g.v);
+    bool wild = false;
 #pragma unroll
-    for (int i = 0; i < Q; i++) f.s[i].clear();
-    visit<double, ND, Q, true, LIFT, false>(P, l, f);
-    const int sc = max(mx >> 20, 64) - P.div.s - 1049;
+    for (int i = 0; i < Q; i++) {
+        long long t[ND] = {s[i].total()};
+        int e[ND] = {e0}, top = e0, low = e0;
 #pragma unroll
-    for (int i = 0; i < Q; i++) y[i] = f.s[i].value(sc);
+        for (int d = 1; d < ND; d++) {
+            const Cross<ND, Q> c(d, l, i);
+            Fx r;
+            r.clear();
+            // (an absent entry is zero)
+#pragma unroll
+            for (int j = 0; j < N; j++) r.mad(P.div.a[c.row][j], fixed(d, c.line, j));
+            t[d] = r.total();
+            e[d] = ex(d, c.line, g.v);
+            top = max(top, e[d]);
+            low = min(low, e[d]);
+        }
+        long long sum = 0;
+#pragma unroll
+        for (int d = 0; d < ND; d++) sum += t[d] >> min(top - e[d], 63);
+        y[i] = b200::fixed_to_f64(sum, top - P.div.s - 1051);
+        wild |= low < 0;
+    }
+    if (wild) {
+#pragma unroll
+        for (int i = 0; i < Q; i++) y[i] = wild_div<LIFT>(P, g, ex, l, i);
+    }
 }
 
 // The same at point p alone, from the values as they are: in two dimensions
@@ -533,10 +511,9 @@ __device__ __forceinline__ void grad_to_phys(const T s[ND][ND], T rcp, const T t
 }
 
 // The flux ft in reference space into the element's shared memory (sme + c NPS
-// E: component c of the point), and the largest magnitude of each variable
+// E: component c of the point)
 template <typename T, int ND, bool DIAG, int STRIDE>
-__device__ __forceinline__ void put_tflux(T *sme, const T s[ND][ND], const T ft[ND][ND + 2],
-                                          int mx[ND + 2]) {
+__device__ __forceinline__ void put_tflux(T *sme, const T s[ND][ND], const T ft[ND][ND + 2]) {
 #pragma unroll
     for (int v = 0; v < ND + 2; v++)
 #pragma unroll
@@ -546,7 +523,6 @@ __device__ __forceinline__ void put_tflux(T *sme, const T s[ND][ND], const T ft[
             for (int k = 1; k < ND; k++)
                 if (!DIAG) acc += s[i][k] * ft[k][v];
             sme[(i * (ND + 2) + v) * STRIDE] = acc;
-            if constexpr (sizeof(T) == 8) mx[v] = max(mx[v], hi_abs(acc));
         }
 }
 
@@ -572,7 +548,6 @@ te_gradflux_kernel(const __grid_constant__ Line<T, ND, Q> P, int64_t neles, b200
     constexpr int VU = FIXED ? 1 : NV;      // unrolling over the variables
     extern __shared__ __align__(16) unsigned char smem_raw[];
     T *sm = reinterpret_cast<T *>(smem_raw);
-    __shared__ int top[NV][E];      // largest flux of each variable
 
     const int el = threadIdx.x % E, grp = threadIdx.x / E;
     const int64_t e = (int64_t)blockIdx.x * E + el;
@@ -583,8 +558,7 @@ te_gradflux_kernel(const __grid_constant__ Line<T, ND, Q> P, int64_t neles, b200
     gf = gf.at(col0);
     r = r.at(col0);
     T *const sme = sm + el;
-    if (FIXED)
-        for (int v = grp; v < NV; v += G) top[v][el] = 0;
+    const LineExp<ND, Q, E> ex{reinterpret_cast<int *>(sm + ND * NV * NPS * E) + el};
 
     // The corrected gradient along every line; for a diagonal metric, already
     // in physical space (unless it is wanted in reference space)
@@ -679,7 +653,6 @@ te_gradflux_kernel(const __grid_constant__ Line<T, ND, Q> P, int64_t neles, b200
     __syncthreads();
 
     // The flux in reference space, in the place of the gradient
-    int mx[NV] = {};
     for (int p = grp; p < NP; p += G) {
         T uu[NV], gr[ND][NV], ft[ND][NV], s[ND][ND] = {}, rcp = T(0);
         if (live) b200::elem_metrics<ND, T, DIAG>(geo, NP, p, e, s, rcp, !DIAG && refgrad);
@@ -704,28 +677,22 @@ te_gradflux_kernel(const __grid_constant__ Line<T, ND, Q> P, int64_t neles, b200
             grad_to_phys<ND, T>(s, rcp, tg, gr);
         }
         b200::ns_flux<ND, T>(uu, gr, ft, gas);
-        put_tflux<T, ND, DIAG, NPS * E>(sme + p * E, s, ft, mx);
-    }
-    // FP64: in fixed point over the largest flux of the element and variable
-    // (each value is an operand of the outputs of a line, and is split once)
-    if (FIXED) {
-#pragma unroll
-        for (int v = 0; v < NV; v++) atomicMax(&top[v][el], mx[v]);
-        __syncthreads();
-#pragma unroll
-        for (int v = 0; v < NV; v++) mx[v] = top[v][el];
-        for (int p = grp; p < NP; p += G)
-#pragma unroll
-            for (int k = 0; k < ND * NV; k++) fix_in_place(sme[(k * NPS + p) * E], mx[k % NV]);
+        put_tflux<T, ND, DIAG, NPS * E>(sme + p * E, s, ft);
     }
     __syncthreads();
+    // FP64: in fixed point over each line's largest flux (a value is an operand
+    // of the outputs of a line, and is split once)
+    if (FIXED) {
+        fix_lines<false, G>(SmemFlux<T, ND, Q, E>{P, sme, nullptr, 0}, ex, grp);
+        __syncthreads();
+    }
 
     // The divergence along the lines of every direction
     for (int t = grp; t < NV * L; t += G) {
         const int v = t % NV, l = t / NV;
         const SmemFlux<T, ND, Q, E> g{P, sme, nullptr, v};
         T y[Q];
-        smem_div<false>(P, g, l, FIXED ? top[v][el] : 0, y);
+        smem_div<false>(P, g, ex, l, y);
 #pragma unroll
         for (int i = 0; i < Q; i++)
             if (live) r.at(v * 32)(l * Q + i) = y[i];
@@ -743,11 +710,10 @@ te_euler_kernel(const __grid_constant__ Line<T, ND, Q> P, int64_t neles, T gamma
     constexpr int E = Tile<T, ND, Q>::E, G = Tile<T, ND, Q>::G;
     using SF = SmemFlux<T, ND, Q, E>;
     constexpr int NPS = SF::NPS, NFS = SF::NFS;
-    // (by points in two dimensions, FP64: no common exponent)
+    // (by points in two dimensions, FP64)
     constexpr bool POINTS = sizeof(T) == 8 && ND == 2, FIXED = sizeof(T) == 8 && !POINTS;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     T *sm = reinterpret_cast<T *>(smem_raw);
-    __shared__ int top[NV][E];
 
     const int el = threadIdx.x % E, grp = threadIdx.x / E;
     const int64_t e = (int64_t)blockIdx.x * E + el;
@@ -757,22 +723,15 @@ te_euler_kernel(const __grid_constant__ Line<T, ND, Q> P, int64_t neles, T gamma
     fc = fc.at(col0);
     r = r.at(col0);
     T *const sme = sm + el, *const sce = sme + ND * NV * NPS * E;
-    if (FIXED) {
-        for (int v = grp; v < NV; v += G) top[v][el] = 0;
-        __syncthreads();
-    }
+    const LineExp<ND, Q, E> ex{
+        reinterpret_cast<int *>(sm + (ND * NV * NPS + NV * NFS) * E) + el};
 
-    int mx[NV] = {};
     // (from the last group on, so that in two dimensions other threads than
     // the points' take the flux points)
     for (int q = G - 1 - grp; q < NFP; q += G) {
         const T *pf = &fc(q);
 #pragma unroll
-        for (int v = 0; v < NV; v++) {
-            const T x = live ? pf[v * 32] : T(0);
-            sce[(v * NFS + q) * E] = x;
-            if constexpr (FIXED) mx[v] = max(mx[v], hi_abs(x));
-        }
+        for (int v = 0; v < NV; v++) sce[(v * NFS + q) * E] = live ? pf[v * 32] : T(0);
     }
     for (int p = grp; p < NP; p += G) {
         T uu[NV], ft[ND][NV], s[ND][ND] = {}, rcp, pr, vel[ND];
@@ -781,22 +740,13 @@ te_euler_kernel(const __grid_constant__ Line<T, ND, Q> P, int64_t neles, T gamma
 #pragma unroll
         for (int v = 0; v < NV; v++) uu[v] = live ? pu[v * 32] : T(1);
         b200::inviscid_flux<ND, T>(uu, ft, pr, vel, gamma);
-        put_tflux<T, ND, DIAG, NPS * E>(sme + p * E, s, ft, mx);
-    }
-    if (FIXED) {
-#pragma unroll
-        for (int v = 0; v < NV; v++) atomicMax(&top[v][el], mx[v]);
-        __syncthreads();
-#pragma unroll
-        for (int v = 0; v < NV; v++) mx[v] = top[v][el];
-        for (int q = G - 1 - grp; q < NFP; q += G)
-#pragma unroll
-            for (int v = 0; v < NV; v++) fix_in_place(sce[(v * NFS + q) * E], mx[v]);
-        for (int p = grp; p < NP; p += G)
-#pragma unroll
-            for (int k = 0; k < ND * NV; k++) fix_in_place(sme[(k * NPS + p) * E], mx[k % NV]);
+        put_tflux<T, ND, DIAG, NPS * E>(sme + p * E, s, ft);
     }
     __syncthreads();
+    if (FIXED) {
+        fix_lines<true, G>(SF{P, sme, sce, 0}, ex, grp);
+        __syncthreads();
+    }
     if (!live) return;
 
     if constexpr (POINTS) {
@@ -810,7 +760,7 @@ te_euler_kernel(const __grid_constant__ Line<T, ND, Q> P, int64_t neles, T gamma
         const int v = t % NV, l = t / NV;
         const SF g{P, sme, sce, v};
         T y[Q];
-        smem_div<true>(P, g, l, FIXED ? top[v][el] : 0, y);
+        smem_div<true>(P, g, ex, l, y);
 #pragma unroll
         for (int i = 0; i < Q; i++) {
             const int p = l * Q + i;
@@ -821,15 +771,78 @@ te_euler_kernel(const __grid_constant__ Line<T, ND, Q> P, int64_t neles, T gamma
     }
 }
 
-template <typename T, int ND, int Q>
-struct GlobalEnds {
-    const Line<T, ND, Q> &P;
-    Rows<const T> fc, r;        // + column of the element and variable
-    __device__ __forceinline__ T flux(int, int) const { return T(0); }
-    __device__ __forceinline__ int flux_hi(int, int) const { return 0; }
-    __device__ __forceinline__ T end(int d, int l, int e) const { return fc(P.fpt[d][l][e]); }
-    __device__ __forceinline__ T old(int p) const { return r(p); }
-};
+// The lift at the points of x-line l from the common flux at its ends and at
+// those of the lines across it; fc(d, line, end).  FP64: the two ends of the
+// x-line over their own exponent, the others over theirs, and the two integer
+// sums shifted to the larger, so that an output has its own operands' bits
+template <int ND, int Q, typename F>
+__device__ __forceinline__ void lift_line(const Line<float, ND, Q> &P, const F &fc, int l,
+                                          float (&y)[Q]) {
+#pragma unroll
+    for (int i = 0; i < Q; i++) y[i] = 0.0f;
+#pragma unroll
+    for (int e = 0; e < 2; e++) {
+        const float x = fc(0, l, e);
+#pragma unroll
+        for (int i = 0; i < Q; i++) y[i] += P.div.d[i][Q + e] * x;
+    }
+#pragma unroll
+    for (int i = 0; i < Q; i++)
+#pragma unroll
+        for (int d = 1; d < ND; d++) {
+            const Cross<ND, Q> c(d, l, i);
+#pragma unroll
+            for (int e = 0; e < 2; e++) y[i] += P.div.d[c.row][Q + e] * fc(d, c.line, e);
+        }
+}
+
+template <int ND, int Q, typename F>
+__device__ __forceinline__ void lift_line(const Line<double, ND, Q> &P, const F &fc, int l,
+                                          double (&y)[Q]) {
+    double x[2], c[Q][ND - 1][2];
+    int row[ND - 1];
+#pragma unroll
+    for (int e = 0; e < 2; e++) x[e] = fc(0, l, e);
+#pragma unroll
+    for (int i = 0; i < Q; i++)
+#pragma unroll
+        for (int d = 1; d < ND; d++) {
+            const Cross<ND, Q> cr(d, l, i);
+            row[d - 1] = cr.row;
+#pragma unroll
+            for (int e = 0; e < 2; e++) c[i][d - 1][e] = fc(d, cr.line, e);
+        }
+
+    const int mx0 = max(hi_abs(x[0]), hi_abs(x[1])), e0 = max(mx0 >> 20, 64);
+    int2 b0[2];
+#pragma unroll
+    for (int e = 0; e < 2; e++) b0[e] = split<60>(x[e], e0);
+#pragma unroll
+    for (int i = 0; i < Q; i++) {
+        int mx = 0;
+#pragma unroll
+        for (int k = 0; k < 2 * (ND - 1); k++) mx = max(mx, hi_abs(c[i][k / 2][k % 2]));
+        if (out_of_range(mx0) || out_of_range(mx)) {
+            y[i] = fma(P.div.d[i][Q + 1], x[1], P.div.d[i][Q] * x[0]);
+#pragma unroll
+            for (int k = 0; k < 2 * (ND - 1); k++)
+                y[i] = fma(P.div.d[row[k / 2]][Q + k % 2], c[i][k / 2][k % 2], y[i]);
+            continue;
+        }
+        const int e1 = max(mx >> 20, 64), top = max(e0, e1);
+        Fx s, r;
+        s.clear();
+        r.clear();
+#pragma unroll
+        for (int e = 0; e < 2; e++) s.mad(P.div.a[i][Q + e], b0[e]);
+#pragma unroll
+        for (int k = 0; k < 2 * (ND - 1); k++)
+            r.mad(P.div.a[row[k / 2]][Q + k % 2], split<60>(c[i][k / 2][k % 2], e1));
+        y[i] = b200::fixed_to_f64_cvt((s.total() >> min(top - e0, 63)) +
+                                          (r.total() >> min(top - e1, 63)),
+                                      top - P.div.s - 1051);
+    }
+}
 
 // R = -(1/|J|) (R + M3 Fc): a warp takes an x-line and variable of 32 elements
 template <typename T, int ND, int Q>
@@ -846,13 +859,15 @@ te_lift_kernel(const __grid_constant__ Line<T, ND, Q> P, int64_t neles, unsigned
     const int v = t % K::NV, l = t / K::NV;
     const int64_t col = ((int64_t)blk * K::NV + v) * 32 + lane;
     r = r.at(col);
-    const GlobalEnds<T, ND, Q> g{P, fc.at(col), Rows<const T>{r.p, r.ld}};
-    T y[Q];
-    div_line<false, true, true>(P, g, l, y);
+    fc = fc.at(col);
+    T old[Q], y[Q];
+#pragma unroll
+    for (int i = 0; i < Q; i++) old[i] = r(l * Q + i);
+    lift_line(P, [&](int d, int line, int end) { return fc(P.fpt[d][line][end]); }, l, y);
 #pragma unroll
     for (int i = 0; i < Q; i++) {
         const int p = l * Q + i;
-        r(p) = -rcpdjac[p * ldj + e] * y[i];
+        r(p) = -rcpdjac[p * ldj + e] * (y[i] + old[i]);
     }
 }
 
@@ -905,12 +920,14 @@ int opt_in(Fn fn, size_t smem) {
                                                  (int)smem), "te: smem attribute");
 }
 
-// Shared memory of an element block: the fluxes, and with ends the common flux
+// Shared memory of an element block: the fluxes, with ends the common flux, and
+// in FP64 the lines' exponents
 template <typename T, int ND, int Q>
 constexpr size_t te_smem(bool ends) {
     using SF = SmemFlux<T, ND, Q, Tile<T, ND, Q>::E>;
-    return (size_t)(ND * SF::NV * SF::NPS + (ends ? SF::NV * SF::NFS : 0)) *
-           Tile<T, ND, Q>::E * sizeof(T);
+    constexpr int E = Tile<T, ND, Q>::E;
+    return (size_t)(ND * SF::NV * SF::NPS + (ends ? SF::NV * SF::NFS : 0)) * E * sizeof(T) +
+           (sizeof(T) == 8 ? LineExp<ND, Q, E>::N * sizeof(int) : 0);
 }
 
 template <typename T>
