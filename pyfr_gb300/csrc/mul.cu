@@ -41,10 +41,13 @@ struct MulHandle {
     double *val64;   // device, nnz
     float *val32;    // device, nnz
     // The fixed-point form of the operator (FP64 applies; null when the
-    // operator does not fit it): per row (first entry, end, scale s, 0), per
-    // entry (column, high part, low part, 0)
-    int4 *fxrow;     // device, m
-    int4 *fxval;     // device, nnz
+    // operator does not fit it): per row (first entry, end, scale s,
+    // threshold), per entry (column, high part, low part, |high part|); and, for
+    // dense rows, the magnitudes in 8 bits: per row (first word, end, threshold,
+    // 0), per word (column/4, four entries)
+    int4 *fxrow, *mgrow;     // device, m
+    int4 *fxval;             // device, nnz
+    int2 *mgval;             // device
     // The same by groups of up to four rows of one support (null when the
     // rows do not fall into such groups): per group gn columns and four rows
     // (-1: none), and (high, low part) and the value of every entry; one scale
@@ -152,35 +155,50 @@ mul_csr_kernel(MulHandle h, const T *__restrict__ b, int64_t ldb, T *__restrict_
 // dot product of doubles over a common exponent is a dot product of
 // integers, so a row of the operator times a column of B is formed as
 //
-//     B[k, n] = (bh 2^31 + bl) 2^-sb,  |bh| <= 2^30, |bl| <= 2^30
-//     A[m, k] = (ah 2^26 + al) 2^-(s + 26),  sum_k |ah| ~ 2^30, |al| <= 2^25
+//     B[k, n] = (bh 2^31 + bl) 2^-sb,  |bh| <= 2^28, |bl| <= 2^30
+//     A[m, k] = (ah 2^29 + al) 2^-(s + 29),  sum_k |ah| ~ 2^30, |al| <= 2^28
 //     hh = sum ah bh,  u = sum ah bl,  v = sum al bh    (64-bit, exact)
-//     A B = (hh + u/2^31 + v/2^26 + O(2^-2)) 2^(31 - s - sb)
+//     A B = (hh + u/2^31 + v/2^29 + ...) 2^(31 - s - sb)
 //
 // three IMAD.WIDE per nonzero, and the sum is rounded to FP64 once.  sb is
-// the column's own (its largest exponent), s the row's.  B keeps 61 bits
-// below the column's largest value and A 57 below the row's absolute sum,
-// so the result is within 1.5 2^-59 of (row sum)(column maximum), which is
-// below the rounding of an FP64 dot product unless every B value the row
-// touches is small against the column's largest.  That is tested per output
-// (the OR of the |bh| over the row's support against 2^23, the column's
-// largest being in [2^29, 2^30]): such outputs, and those of columns with
-// infinities, NaNs or exponents near the ends of the range, are formed again
-// with FP64 FMAs from global memory by the whole warp.
+// the column's own (its largest exponent), s the row's.  In units of hh the
+// result is within n/2 + 3/2 for n nonzeros, whatever their values: 1/4 of a
+// unit each for A's rounding and for the product al bl that is left out, 1/2
+// for B's truncation and 1/2 each for the roundings of u and v.  An FP64 dot
+// product is within n 2^-53 of the terms' absolute sum, so the fixed-point form
+// is as good as long as
+//     sum |ah bh| >= 2^53 (1/2 + 3/(2n)),
+// 1/13 to 1/53 of (row sum)(column maximum) for n = 15: not where large entries
+// of the row meet zeros, or where the row's support is small against the
+// column.  That is tested per output; outputs below it, and those of columns
+// with infinities, NaNs or exponents near the ends of the range, are formed
+// again with FP64 FMAs from global memory by the whole warp.  The test costs a
+// multiply-add a nonzero more (IMAD.HI), or, in wide applies of dense rows,
+// one for four, on a lower bound of the sum from the leading 8 bits of every
+// value (IDP4A, in a loop of its own, which narrow applies, one chain of
+// latencies each, are the slower for), and columns of values within a factor
+// of four of each other need none.
 //
-// Bounds: hh, u <= 2^61 by the row sums; v <= nnz 2^55, nnz <= 64 (FX_MAXNNZ),
-// so no sum overflows.
+// Bounds: hh <= 2^58 and u <= 2^60 by the row sums; v <= nnz 2^56, nnz <= 64
+// (FX_MAXNNZ), so no sum overflows.
 
-constexpr int FX_MAXNNZ = 64;
-constexpr int FX_THR = 1 << 23;
+constexpr int FX_MAXNNZ = 64, FX_TILE = 113 * 1024;
+constexpr int FX_BBITS = 59, FX_ALBITS = 29;
+// The forms of the test
+constexpr int FX_NONE = 0, FX_EACH = 1, FX_PACKED = 2;
+
+// Bytes of a tile: 8 a value and, packed, 1 of its magnitude (rows of four)
+inline size_t fx_smem(int k, int cpl, bool packed) {
+    return (size_t)(k * 8 + (packed ? (k + 3) / 4 * 4 : 0)) * 32 * cpl;
+}
 
 // Columns per lane: 2 (64 columns a CTA, 16-byte accesses) or 1
 template <int CPL>
 struct FxPair;
 template <>
-struct FxPair<1> { using I = int2; using D = double; };
+struct FxPair<1> { using I = int2; };
 template <>
-struct FxPair<2> { using I = int4; using D = double2; };
+struct FxPair<2> { using I = int4; };
 
 // The exponent field of the largest value; whether anything but zero is
 // there (hi the absolute high word, or 1 for a subnormal below it)
@@ -194,12 +212,12 @@ __device__ __forceinline__ int2 fx_split(double x, int emax) {
     const int hi = __double2hiint(x);
     const int e = (hi >> 20) & 0x7ff;
     const int d = min(emax - e, 63);
-    // 53-bit mantissa over 8 zero bits, shifted down by the exponent
-    // difference (values below 2^-61 of the largest become zero; a zero or
-    // subnormal value always does)
+    // 53-bit mantissa over zero bits, shifted down by the exponent difference
+    // (values below 2^-59 of the largest become zero; a zero or subnormal
+    // value always does)
     unsigned long long q =
         ((unsigned long long)((hi & 0xfffff) | 0x100000) << 32) | (unsigned)__double2loint(x);
-    q = (q << 8) >> d;
+    q = (q << (FX_BBITS - 53)) >> d;
     long long b = hi < 0 ? -(long long)q : (long long)q;
     b += 1ll << 30;
     int2 r;
@@ -208,7 +226,7 @@ __device__ __forceinline__ int2 fx_split(double x, int emax) {
     return r;
 }
 
-template <int EPI, int CPL>
+template <int EPI, int CPL, int TEST>
 __global__ void __launch_bounds__(MUL_WARPS * 32)
 mul_fx_kernel(MulHandle h, const double *__restrict__ b, int64_t ldb, double *__restrict__ c,
               int64_t ldc, int64_t ncol, double alpha, double beta, int vec) {
@@ -217,7 +235,12 @@ mul_fx_kernel(MulHandle h, const double *__restrict__ b, int64_t ldb, double *__
     constexpr int NC = 32 * CPL;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     I *bs = reinterpret_cast<I *>(smem_raw);             // [k][32]
-    __shared__ int cmax[MUL_WARPS][NC];
+    unsigned *mg = reinterpret_cast<unsigned *>(bs + h.k * 32);     // [(k + 3)/4][NC]
+    __shared__ int cmax[NC], cmin[NC];
+    if (threadIdx.x < NC) {
+        cmax[threadIdx.x] = 0;
+        cmin[threadIdx.x] = 0x7fffffff;
+    }
 
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t col = (int64_t)blockIdx.x * NC + lane * CPL;
@@ -227,10 +250,13 @@ mul_fx_kernel(MulHandle h, const double *__restrict__ b, int64_t ldb, double *__
     const bool full = ok[CPL - 1];
 
     // Load the tile, every warp its rows, eight rows in flight per thread;
-    // the largest magnitude of each column over the warp's rows
-    int mag[CPL];
+    // the largest and smallest magnitude of each column over the warp's rows
+    int mag[CPL], low[CPL];
 #pragma unroll
-    for (int j = 0; j < CPL; j++) mag[j] = 0;
+    for (int j = 0; j < CPL; j++) {
+        mag[j] = 0;
+        low[j] = 0x7fffffff;
+    }
     constexpr int UNR = 8;
     for (int r0 = warp; r0 < h.k; r0 += UNR * MUL_WARPS) {
         double x[UNR][CPL];
@@ -260,27 +286,38 @@ mul_fx_kernel(MulHandle h, const double *__restrict__ b, int64_t ldb, double *__
 #pragma unroll
                 for (int j = 0; j < CPL; j++) {
                     dst[j] = x[q][j];
-                    mag[j] = max(mag[j], fx_mag(x[q][j]));
+                    const int t = fx_mag(x[q][j]);
+                    mag[j] = max(mag[j], t);
+                    low[j] = min(low[j], t);
                 }
             }
         }
     }
-#pragma unroll
-    for (int j = 0; j < CPL; j++) cmax[warp][lane * CPL + j] = mag[j];
     __syncthreads();
-
-    // Column exponents; the threshold of the support test (0: a column of
-    // zeros needs none; the largest int: every output of the column by FP64)
-    int emax[CPL], thr[CPL];
 #pragma unroll
     for (int j = 0; j < CPL; j++) {
-        int mx = cmax[0][lane * CPL + j];
+        atomicMax(&cmax[lane * CPL + j], mag[j]);
+        atomicMin(&cmin[lane * CPL + j], low[j]);
+    }
+    __syncthreads();
+
+    // Column exponents; columns of which every output (wild) or none (zero) is
+    // formed by FP64; whether a column needs the test: not where its smallest
+    // value is at least a quarter of its largest, which makes sum |ah bh| at
+    // least 2^54, the threshold of one nonzero.  (The columns of a tile are
+    // mostly one variable's: those of density and energy pass.)
+    int emax[CPL];
+    bool wild[CPL], zero[CPL];
+    bool need = false;
 #pragma unroll
-        for (int w = 1; w < MUL_WARPS; w++) mx = max(mx, cmax[w][lane * CPL + j]);
+    for (int j = 0; j < CPL; j++) {
+        const int mx = cmax[lane * CPL + j], mn = cmin[lane * CPL + j];
         // (at least 64 for the splits: then zeros have an exponent
         // difference that makes them zero)
         emax[j] = max(mx >> 20, 64);
-        thr[j] = mx == 0 ? 0 : (emax[j] < 128 || emax[j] > 1900) ? 0x7fffffff : FX_THR;
+        zero[j] = mx == 0;
+        wild[j] = !zero[j] && (emax[j] < 128 || emax[j] > 1900);
+        need = need || wild[j] || (!zero[j] && mn < mx - (2 << 20));
     }
 
     // Split in place (each thread the values that it stored)
@@ -291,11 +328,17 @@ mul_fx_kernel(MulHandle h, const double *__restrict__ b, int64_t ldb, double *__
 #pragma unroll
         for (int j = 0; j < CPL; j++) t[j] = fx_split(src[j], emax[j]);
 #pragma unroll
-        for (int j = 0; j < CPL; j++) dst[j] = t[j];
+        for (int j = 0; j < CPL; j++) {
+            dst[j] = t[j];
+            // (rounded down: at most 255 2^20 of 2^28)
+            if (TEST == FX_PACKED)
+                reinterpret_cast<unsigned char *>(mg + (r / 4) * NC + lane * CPL + j)[r % 4] =
+                    (unsigned char)min(abs(t[j].x) >> 20, 255);
+        }
     }
     __syncthreads();
 
-    for (int row = warp; row < h.m; row += MUL_WARPS) {
+    const auto form = [&](int row, auto test) {
         double *crow = c + row * ldc + col;
         const int4 ri = __ldg(h.fxrow + row);
         double cin[CPL];
@@ -305,13 +348,13 @@ mul_fx_kernel(MulHandle h, const double *__restrict__ b, int64_t ldb, double *__
         }
         // (u and v start at half a unit of hh: the final shifts round)
         long long hh[CPL], u[CPL], v[CPL];
-        int m[CPL];
+        unsigned m[CPL], thr = (unsigned)ri.w;      // the test's sums
 #pragma unroll
         for (int j = 0; j < CPL; j++) {
             hh[j] = 0;
             u[j] = 1ll << 30;
-            v[j] = 1ll << 25;
-            m[j] = 0;
+            v[j] = 1ll << (FX_ALBITS - 1);
+            m[j] = zero[j] ? 1u << 30 : 0u;
         }
 #pragma unroll 4
         for (int p = ri.x; p < ri.y; p++) {
@@ -324,7 +367,19 @@ mul_fx_kernel(MulHandle h, const double *__restrict__ b, int64_t ldb, double *__
                 hh[j] += (long long)a.y * bh;
                 u[j] += (long long)a.y * bl;
                 v[j] += (long long)a.z * bh;
-                m[j] |= bh ^ (bh >> 31);
+                if (test() == FX_EACH) m[j] += __umulhi((unsigned)a.w, (unsigned)abs(bh));
+            }
+        }
+
+        if (test() == FX_PACKED) {
+            const int4 mi = __ldg(h.mgrow + row);
+            thr = (unsigned)mi.z;
+#pragma unroll 4
+            for (int p = mi.x; p < mi.y; p++) {
+                const int2 g = __ldg(h.mgval + p);
+#pragma unroll
+                for (int j = 0; j < CPL; j++)
+                    m[j] = __dp4a((unsigned)g.y, mg[g.x * NC + lane * CPL + j], m[j]);
             }
         }
 
@@ -332,17 +387,17 @@ mul_fx_kernel(MulHandle h, const double *__restrict__ b, int64_t ldb, double *__
         bool small = false;
 #pragma unroll
         for (int j = 0; j < CPL; j++) {
-            const long long t = hh[j] + (u[j] >> 31) + (v[j] >> 26);
+            const long long t = hh[j] + (u[j] >> 31) + (v[j] >> FX_ALBITS);
             r[j] = (double)t;
-            // times 2^(31 - s - sb), sb = 1083 - emax: an exponent sum, in
-            // the normal range by the limits on emax and s
+            // times 2^(31 - s - sb), sb = 1022 + FX_BBITS - emax: an exponent
+            // sum, in the normal range by the limits on emax and s
             if (t != 0)
                 r[j] = __hiloint2double(__double2hiint(r[j]) +
-                                            (emax[j] - 1052 - ri.z) * (1 << 20),
+                                            (emax[j] - (991 + FX_BBITS) - ri.z) * (1 << 20),
                                         __double2loint(r[j]));
-            small |= m[j] < thr[j];
+            small |= wild[j] || m[j] < thr;
         }
-        if (__any_sync(0xffffffffu, small)) {
+        if (test() != FX_NONE && __any_sync(0xffffffffu, small)) {
             const int p0 = __ldg(h.rowptr + row), p1 = __ldg(h.rowptr + row + 1);
             double acc[CPL];
 #pragma unroll
@@ -356,7 +411,7 @@ mul_fx_kernel(MulHandle h, const double *__restrict__ b, int64_t ldb, double *__
             }
 #pragma unroll
             for (int j = 0; j < CPL; j++)
-                if (m[j] < thr[j]) r[j] = acc[j];
+                if (wild[j] || m[j] < thr) r[j] = acc[j];
         }
 #pragma unroll
         for (int j = 0; j < CPL; j++) {
@@ -371,22 +426,31 @@ mul_fx_kernel(MulHandle h, const double *__restrict__ b, int64_t ldb, double *__
             for (int j = 0; j < CPL; j++)
                 if (ok[j]) crow[j] = r[j];
         }
-    }
+    };
+    if (__any_sync(0xffffffffu, need))
+        for (int row = warp; row < h.m; row += MUL_WARPS)
+            form(row, std::integral_constant<int, TEST>());
+    else
+        for (int row = warp; row < h.m; row += MUL_WARPS)
+            form(row, std::integral_constant<int, FX_NONE>());
 }
 
-template <int CPL>
+template <int CPL, int TEST>
 void launch_fx(const MulHandle &h, const double *b, int64_t ldb, double *c, int64_t ldc,
                int64_t ncol, double alpha, double beta, int vec, cudaStream_t s) {
     const unsigned grid = b200::ceil_div(ncol, 32 * CPL);
-    const size_t smem = (size_t)h.k * 32 * CPL * sizeof(double);
+    const size_t smem = fx_smem(h.k, CPL, TEST == FX_PACKED);
+    auto go = [&](auto epi) {
+        b200::launch(mul_fx_kernel<epi(), CPL, TEST>, grid, MUL_WARPS * 32, smem, s, h, b, ldb, c, ldc, ncol, alpha, beta, vec);
+    };
     if (alpha == 1.0 && beta == 0.0)
-        b200::launch(mul_fx_kernel<EPI_SET, CPL>, grid, MUL_WARPS * 32, smem, s, h, b, ldb, c, ldc, ncol, alpha, beta, vec);
+        go(std::integral_constant<int, EPI_SET>());
     else if (alpha == 1.0 && beta == 1.0)
-        b200::launch(mul_fx_kernel<EPI_ADD, CPL>, grid, MUL_WARPS * 32, smem, s, h, b, ldb, c, ldc, ncol, alpha, beta, vec);
+        go(std::integral_constant<int, EPI_ADD>());
     else if (beta == 0.0)
-        b200::launch(mul_fx_kernel<EPI_SCALE, CPL>, grid, MUL_WARPS * 32, smem, s, h, b, ldb, c, ldc, ncol, alpha, beta, vec);
+        go(std::integral_constant<int, EPI_SCALE>());
     else
-        b200::launch(mul_fx_kernel<EPI_GENERAL, CPL>, grid, MUL_WARPS * 32, smem, s, h, b, ldb, c, ldc, ncol, alpha, beta, vec);
+        go(std::integral_constant<int, EPI_GENERAL>());
 }
 
 // ---- the same by groups of rows of one support ---------------------------
@@ -487,8 +551,9 @@ mul_fxg_kernel(MulHandle h, const double *__restrict__ b, int64_t ldb, double *_
                     const double *ad = h.gdbl + (g * FXG_ROWS + q) * N;
 #pragma unroll 1
                     for (int i = 0; i < N; i++)
-                        f = fma(__ldg(ad + i), bs[__ldg(h.gcol + g * N + i) * NC + lane * CPL + j],
-                                f);
+                        // (a filled-up support's zero stays out of infinities)
+                        if (const double av = __ldg(ad + i); av != 0.0)
+                            f = fma(av, bs[__ldg(h.gcol + g * N + i) * NC + lane * CPL + j], f);
                     if (wild[j]) r[j] = f;
                 }
                 const double old = EPI == EPI_ADD || EPI == EPI_GENERAL
@@ -533,7 +598,17 @@ bool with_fxg(int cpl, int n, int epi, F &&fn) {
 }
 
 // The operator's rows in groups of one support, or false where they are not: of
-// two rows a group on average, and of one support size of FXG_MIN to FXG_MAX
+// two rows a group on average, of support sizes within one of each other, from
+// FXG_MIN to FXG_MAX (a smaller one is filled up with a zero entry on a column
+// that it has: the derivatives at p = 4, where the middle point's own is zero;
+// 24.5 us at 320 columns, 41 by FMAs; 117 us at 35005, by columns 114 to 172, the
+// more the smaller a line's values are against its column's), and with no entry
+// below 1/16 of the largest row's mean.  A group's sums are within (1 + N/2 + N/8)
+// 2^-57 of (largest row sum)(largest value of the support), which for such entries
+// is below 5 times the classical bound of FP64 sums, N 2^-53 of the terms' absolute
+// sum, whatever the values are (below 1 for the derivatives of p = 3 hexahedra,
+// 3.4 for the interpolation at p = 5); an entry far below the others would lose
+// the bits that it has alone where theirs meet zeros.
 struct Groups {
     int n = 0, s = 0;
     std::vector<int> col, row;
@@ -543,24 +618,29 @@ struct Groups {
 
 bool fx_groups(const double *a, int m, int k, Groups &g) {
     std::map<std::vector<int>, std::vector<int>> by;
-    double top = 0.0, low = INFINITY;
+    double top = 0.0, low = INFINITY, least = INFINITY;
+    int fewest = FXG_MAX;
     for (int i = 0; i < m; i++) {
         std::vector<int> sup;
         double l1 = 0.0;
-        for (int j = 0; j < k; j++)
-            if (a[(size_t)i * k + j] != 0.0) {
-                sup.push_back(j);
-                l1 += fabs(a[(size_t)i * k + j]);
-            }
-        if (!g.n) g.n = (int)sup.size();
-        if ((int)sup.size() != g.n || g.n < FXG_MIN || g.n > FXG_MAX || !(l1 <= ldexp(1.0, 60)))
-            return false;
+        for (int j = 0; j < k; j++) {
+            const double x = fabs(a[(size_t)i * k + j]);
+            if (x == 0.0) continue;
+            sup.push_back(j);
+            l1 += x;
+            least = fmin(least, x);
+        }
+        const int n = (int)sup.size();
+        if (n < FXG_MIN || n > FXG_MAX || !(l1 <= ldexp(1.0, 60))) return false;
+        g.n = std::max(g.n, n);
+        fewest = std::min(fewest, n);
         top = fmax(top, l1);
         low = fmin(low, l1);
         by[sup].push_back(i);
     }
+    if (g.n - fewest > 1) return false;
     // (one scale: the smallest row keeps 57 of its bits)
-    if (!(low >= ldexp(1.0, -60)) || low < top / 16) return false;
+    if (!(low >= ldexp(1.0, -60)) || low < top / 16 || 16 * g.n * least < top) return false;
     int e;
     frexp(top, &e);
     g.s = 30 - e;
@@ -572,12 +652,15 @@ bool fx_groups(const double *a, int m, int k, Groups &g) {
     for (auto &o : order) {
         const std::vector<int> &rows = by[*o.second];
         for (size_t r0 = 0; r0 < rows.size(); r0 += FXG_ROWS) {
-            g.col.insert(g.col.end(), o.second->begin(), o.second->end());
+            std::vector<int> cols = *o.second;
+            const int n = (int)cols.size();
+            cols.resize(g.n, cols[0]);
+            g.col.insert(g.col.end(), cols.begin(), cols.end());
             for (int q = 0; q < FXG_ROWS; q++) {
                 const int r = r0 + q < rows.size() ? rows[r0 + q] : -1;
                 g.row.push_back(r);
-                for (int j : *o.second) {
-                    const double x = r < 0 ? 0.0 : a[(size_t)r * k + j];
+                for (int i = 0; i < g.n; i++) {
+                    const double x = r < 0 || i >= n ? 0.0 : a[(size_t)r * k + cols[i]];
                     const long long z = llrint(ldexp(x, g.s + 31));
                     const long long ah = (z + (1ll << 30)) >> 31;
                     g.val.push_back(make_int2((int)ah, (int)(z - ah * (1ll << 31))));
@@ -602,7 +685,7 @@ int upload(V **dst, const std::vector<V> &src) {
 // not fit: a row of more than FX_MAXNNZ entries, or of an absolute sum
 // outside [2^-60, 2^60] (or not finite)
 bool fx_operator(const double *a, int m, int k, std::vector<int4> &rows,
-                 std::vector<int4> &vals) {
+                 std::vector<int4> &vals, std::vector<int4> &mgrows, std::vector<int2> &mgs) {
     for (int i = 0; i < m; i++) {
         const double *ar = a + (size_t)i * k;
         double l1 = 0.0;
@@ -621,11 +704,27 @@ bool fx_operator(const double *a, int m, int k, std::vector<int4> &rows,
         const int p0 = (int)vals.size();
         for (int j = 0; j < k; j++) {
             if (ar[j] == 0.0) continue;
-            const long long q = llrint(ldexp(ar[j], s + 26));
-            const long long ah = (q + (1ll << 25)) >> 26, al = q - ah * (1ll << 26);
-            vals.push_back(make_int4(j, (int)ah, (int)al, 0));
+            const long long q = llrint(ldexp(ar[j], s + FX_ALBITS));
+            const long long ah = (q + (1ll << (FX_ALBITS - 1))) >> FX_ALBITS,
+                            al = q - ah * (1ll << FX_ALBITS);
+            vals.push_back(make_int4(j, (int)ah, (int)al, abs((int)ah)));
         }
-        rows.push_back(make_int4(p0, (int)vals.size(), s, 0));
+        // (in units of 2^32: the high words of the products)
+        const double least = nnz ? 0.5 + 1.5 / nnz : 0.0;
+        rows.push_back(make_int4(p0, (int)vals.size(), s, (int)ceil(ldexp(least, 53 - 32))));
+        // Magnitudes |ah|/unit rounded down, the row's largest about 255; with
+        // B's, |bh| 2^-20 rounded down, the sum of the products is below
+        // sum |ah bh| 2^-20/unit, and so has to be at least
+        int top = 0;
+        for (int p = p0; p < (int)vals.size(); p++) top = std::max(top, abs(vals[p].y));
+        const int unit = top / 255 + 1, q0 = (int)mgs.size();
+        for (int p = p0; p < (int)vals.size(); p++) {
+            const int j = vals[p].x;
+            if ((int)mgs.size() == q0 || mgs.back().x != j / 4) mgs.push_back(make_int2(j / 4, 0));
+            mgs.back().y |= (int)((unsigned)(abs(vals[p].y) / unit) << (8 * (j % 4)));
+        }
+        mgrows.push_back(
+            make_int4(q0, (int)mgs.size(), (int)ceil(ldexp(least, 53 - 20) / unit), 0));
     }
     return true;
 }
@@ -667,23 +766,29 @@ int launch_mul(const MulHandle *h, const T *b, int64_t ldb, T *c, int64_t ldc, i
         const bool apart = c + (int64_t)(h->m - 1) * ldc + ncol <= b ||
                            b + (int64_t)(h->k - 1) * ldb + ncol <= c;
         // Where the FMAs bound: rows of ten entries and more at every width
-        // (tetrahedra's 20 x 40 lift at 20480 columns 38.5 -> 17.4 us), rows
-        // of four and more once every SM has a tile (hexahedra's 375 x 125
-        // gradient at p = 4: 93 -> 59 us at 20480 columns, 326 -> 222 us at
-        // 87880; below 9728 columns of rows of four the FP64 form's shorter
-        // chain is up to 10% faster, and for rows of two, 192 x 96, it is
-        // 15-25% faster at every width).  The tile has to leave an SM room
+        // (tetrahedra's 20 x 40 lift at 20480 columns 38.5 -> 17.4 us, before
+        // the test of the terms' sum), rows of four and more once every SM has
+        // a tile (hexahedra's 375 x 125 gradient at p = 4, by columns, 93 -> 59
+        // us at 20480 columns; below 9728 columns of rows of four the FP64
+        // form's shorter chain is up to 10% faster, and for rows of two,
+        // 192 x 96, it is 15-25% faster at every width).  The tile has to leave an SM room
         // for two CTAs (the 125 x 375 divergence at p = 4: 359 us against
         // 370).
         const bool many = h->nnz >= 10 * (int64_t)h->m ||
                           (h->nnz >= 4 * (int64_t)h->m && ncol > 64 * 152);
-        if (h->fxval && apart && many && smem <= 113 * 1024) {
+        if (h->fxval && apart && many && smem <= FX_TILE) {
             const int vec2 = vec && !((uintptr_t)c & 15) && !(ldc & 1);
-            // One column per lane where two would leave SMs without a tile
+            // One column per lane where two would leave SMs without a tile; the
+            // packed test of dense rows from two tiles an SM on (20 x 60
+            // divergence of p = 3 tetrahedra, columns that need the test: 17.1
+            // us by products and 17.6 packed at 9729 columns, 28.9 and 24.7
+            // at 35005, where columns that need none take 22.5)
             if (ncol <= 64 * 152)
-                launch_fx<1>(*h, b, ldb, c, ldc, ncol, alpha, beta, vec2, s);
+                launch_fx<1, FX_EACH>(*h, b, ldb, c, ldc, ncol, alpha, beta, vec2, s);
+            else if (h->mgval && ncol > 2 * 64 * 152 && fx_smem(h->k, 2, true) <= FX_TILE)
+                launch_fx<2, FX_PACKED>(*h, b, ldb, c, ldc, ncol, alpha, beta, vec2, s);
             else
-                launch_fx<2>(*h, b, ldb, c, ldc, ncol, alpha, beta, vec2, s);
+                launch_fx<2, FX_EACH>(*h, b, ldb, c, ldc, ncol, alpha, beta, vec2, s);
             B200_CHECK_LAUNCH("mul_fx_kernel");
             return B200_OK;
         }
@@ -703,16 +808,15 @@ int launch_mul(const MulHandle *h, const T *b, int64_t ldb, T *c, int64_t ldc, i
 // Opt every instantiation in to the largest tile.  Called from
 // b200_mul_create, which never runs inside a stream capture: changing a
 // function attribute while a capture is open invalidates the capture.
-template <int CPL>
+template <int CPL, int TEST>
 int opt_in_smem_fx() {
     void (*fns[4])(MulHandle, const double *, int64_t, double *, int64_t, int64_t, double,
-                   double, int) = {mul_fx_kernel<EPI_SET, CPL>, mul_fx_kernel<EPI_ADD, CPL>,
-                                   mul_fx_kernel<EPI_GENERAL, CPL>,
-                                   mul_fx_kernel<EPI_SCALE, CPL>};
-    // (less the static array of the column maxima)
+                   double, int) = {
+        mul_fx_kernel<EPI_SET, CPL, TEST>, mul_fx_kernel<EPI_ADD, CPL, TEST>,
+        mul_fx_kernel<EPI_GENERAL, CPL, TEST>, mul_fx_kernel<EPI_SCALE, CPL, TEST>};
     for (auto fn : fns) {
         cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             224 * 1024);
+                                             FX_TILE);
         if (e != cudaSuccess) return b200::check_cuda(e, "mul: smem attribute");
     }
     return B200_OK;
@@ -733,7 +837,7 @@ int opt_in_smem() {
 
 void free_handle(MulHandle *h) {
     cudaFree(h->rowptr); cudaFree(h->colidx); cudaFree(h->val64); cudaFree(h->val32);
-    cudaFree(h->fxrow); cudaFree(h->fxval);
+    cudaFree(h->fxrow); cudaFree(h->fxval); cudaFree(h->mgrow); cudaFree(h->mgval);
     cudaFree(h->gcol); cudaFree(h->grow); cudaFree(h->gval); cudaFree(h->gdbl);
     free(h);
 }
@@ -747,8 +851,9 @@ int b200_mul_create(const double *a, int m, int k, void **handle) {
         return b200::set_error(B200_ERR_ARG, "mul_create: bad arguments");
     int orc = opt_in_smem<double>();
     if (!orc) orc = opt_in_smem<float>();
-    if (!orc) orc = opt_in_smem_fx<1>();
-    if (!orc) orc = opt_in_smem_fx<2>();
+    if (!orc) orc = opt_in_smem_fx<1, FX_EACH>();
+    if (!orc) orc = opt_in_smem_fx<2, FX_EACH>();
+    if (!orc) orc = opt_in_smem_fx<2, FX_PACKED>();
     if (orc) return orc;
 
     std::vector<int> rowptr(m + 1, 0), colidx;
@@ -786,14 +891,16 @@ int b200_mul_create(const double *a, int m, int k, void **handle) {
         if (!rc) rc = b200::check_cuda(cudaMemcpy(h->val32, v32.data(), sizeof(float) * h->nnz,
                                                   cudaMemcpyHostToDevice), "mul_create");
     }
-    std::vector<int4> fxrow, fxval;
-    if (!rc && h->nnz && fx_operator(a, m, k, fxrow, fxval)) {
-        rc = b200::check_cuda(cudaMalloc(&h->fxrow, sizeof(int4) * m), "mul_create");
-        if (!rc) rc = b200::check_cuda(cudaMalloc(&h->fxval, sizeof(int4) * nz), "mul_create");
-        if (!rc) rc = b200::check_cuda(cudaMemcpy(h->fxrow, fxrow.data(), sizeof(int4) * m,
-                                                  cudaMemcpyHostToDevice), "mul_create");
-        if (!rc) rc = b200::check_cuda(cudaMemcpy(h->fxval, fxval.data(), sizeof(int4) * nz,
-                                                  cudaMemcpyHostToDevice), "mul_create");
+    std::vector<int4> fxrow, fxval, mgrow;
+    std::vector<int2> mgval;
+    if (!rc && h->nnz && fx_operator(a, m, k, fxrow, fxval, mgrow, mgval)) {
+        rc = upload(&h->fxrow, fxrow);
+        // (dense: three entries a word or more)
+        if (!rc && 3 * mgval.size() <= fxval.size()) {
+            rc = upload(&h->mgrow, mgrow);
+            if (!rc) rc = upload(&h->mgval, mgval);
+        }
+        if (!rc) rc = upload(&h->fxval, fxval);
     }
     Groups gr;
     if (!rc && h->nnz && fx_groups(a, m, k, gr)) {
