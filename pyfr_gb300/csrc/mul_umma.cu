@@ -387,8 +387,19 @@ __device__ __forceinline__ void umma_body(const UmmaArgs &p) {
 
     // The kernels before have finished and their writes are visible (the
     // producer's own wait comes after its copy of the operator, which is
-    // constant); the bounded waits below count from here
-    if (warp != WARP_PROD) b200::dependent_entry();
+    // constant, and its other reads are TMA loads); the bounded waits below
+    // count from here.  An RK stage's registers, which other kernels write, are
+    // what the epilogue reads and writes by plain accesses (the row scale is
+    // constant)
+    double *rk_acc = p.rk_acc;
+    float *rk_u = p.rk_u;
+    const double *rk_dtp = p.rk_dtp;
+    if (warp != WARP_PROD) {
+        if constexpr (RK)
+            b200::dependent_entry(rk_acc, rk_u, rk_dtp);
+        else
+            b200::dependent_entry();
+    }
 
     if (warp == WARP_PROD) {
         // ---- producer: operator image once, then the FP32 chunks of B ----
@@ -610,7 +621,7 @@ __device__ __forceinline__ void umma_body(const UmmaArgs &p) {
         double rk_dtb = 0;
         float rk_dta = 0;
         if (RK) {
-            const double h = p.rk_dtp ? *p.rk_dtp : p.rk_dt;
+            const double h = rk_dtp ? *rk_dtp : p.rk_dt;
             rk_dtb = h * p.rk_b;
             rk_dta = (float)(h * p.rk_a);
         }
@@ -657,7 +668,7 @@ __device__ __forceinline__ void umma_body(const UmmaArgs &p) {
                     const int row = g * 32 + lane;
                     if (row < p.m && bytes)
                         asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;"
-                                     :: "l"(p.rk_acc + (int64_t)row * p.ldc + x0), "r"(bytes)
+                                     :: "l"(rk_acc + (int64_t)row * p.ldc + x0), "r"(bytes)
                                      : "memory");
                 }
             }
@@ -706,19 +717,18 @@ __device__ __forceinline__ void umma_body(const UmmaArgs &p) {
                     // thread's column in place, RKB rows at a time (one warp
                     // reads 32 consecutive FP64 values per row).  Each
                     // value is read and then written by this thread only,
-                    // so the reads take the non-coherent path, and the next
-                    // rows are in flight while the current ones are
-                    // updated.
+                    // and the next rows are in flight while the current
+                    // ones are updated.
 #pragma unroll
                     for (int r = 0; r < 32; r++) f[r] *= __uint_as_float(v[r]);
                     if (col < p.ncol) {
-                        const double *acc = p.rk_acc + col;
+                        const double *acc = rk_acc + col;
                         constexpr int RKB = 4;
                         auto loadb = [&](double *t, int h2) {
 #pragma unroll
                             for (int r = 0; r < RKB; r++) {
                                 const int row = g * 32 + h2 * RKB + r;
-                                t[r] = row < p.m ? __ldg(acc + (int64_t)row * p.ldc) : 0.0;
+                                t[r] = row < p.m ? acc[(int64_t)row * p.ldc] : 0.0;
                             }
                         };
                         double t[RKB], tn[RKB];
@@ -734,9 +744,9 @@ __device__ __forceinline__ void umma_body(const UmmaArgs &p) {
                                     const float t32 = b200::narrow_f64(t[r]);
                                     const double tw = fma(rk_dtb, b200::widen_f32(rf), t[r]);
                                     const int64_t ix = (int64_t)row * p.ldc + col;
-                                    p.rk_acc[ix] = tw;
-                                    p.rk_u[ix] = p.rk == 2 ? b200::narrow_f64(tw)
-                                                           : fmaf(rk_dta, rf, t32);
+                                    rk_acc[ix] = tw;
+                                    rk_u[ix] = p.rk == 2 ? b200::narrow_f64(tw)
+                                                         : fmaf(rk_dta, rf, t32);
                                 }
                             }
 #pragma unroll
