@@ -251,7 +251,9 @@ int b200_mul_bf16x3_create_cat(const double *a1, int k1, const double *a2, int k
                                 void **handle, size_t *smem_bytes);
 int b200_mul_bf16x3_apply(void *handle, const b200_mul_bf16x3_args_t *args, void *stream);
 /* n applies one after the other (the pieces of one large operator): as n calls
- * of _apply, each one's operator copied while the one before it runs. */
+ * of _apply, each one's operator copied while the one before it runs; up to
+ * four consecutive ones of one form run side by side where none of them writes
+ * what another reads or writes. */
 int b200_mul_bf16x3_apply_pieces(void *const *handles, const b200_mul_bf16x3_args_t *const *args,
                                  int n, void *stream);
 /* TF32 variant (the second reduced contraction precision): operator

@@ -62,6 +62,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "slices.cuh"
 #include "../../include/pyfrb200.h"
 
 namespace {
@@ -1186,16 +1187,29 @@ static int umma_apply(void *handle, const b200_mul_bf16x3_args_t *a, int early, 
     return B200_OK;
 }
 
-// Whether the pieces write different rows of equally many columns and take the
-// same kernel, so that they may run side by side
+// Whether the pieces take the same kernel over equally many columns, and neither
+// writes what the other reads or writes, in any of its slices, so that they may
+// run side by side
 static bool apart(const UmmaHandle *h, const b200_mul_bf16x3_args_t *a, const UmmaHandle *g,
                   const b200_mul_bf16x3_args_t *b) {
-    if (a->ncol != b->ncol || a->nbatch != b->nbatch || a->ldc != b->ldc || a->rk_stage ||
-        b->rk_stage || a->cstride != b->cstride || h->tf32 != g->tf32 ||
-        h->npad / 32 % 2 != g->npad / 32 % 2)
+    if (a->ncol != b->ncol || a->nbatch != b->nbatch || a->rk_stage || b->rk_stage ||
+        h->tf32 != g->tf32 || h->npad / 32 % 2 != g->npad / 32 % 2)
         return false;
-    // (slices of equal stride: the rows of one slice decide)
-    return a->c + h->m * a->ldc <= b->c || b->c + g->m * b->ldc <= a->c;
+    const auto out = [](const UmmaHandle *q, const b200_mul_bf16x3_args_t *x) {
+        return b200::Slices{x->c, q->m, x->ldc, x->cstride, x->nbatch};
+    };
+    const auto clear = [&](const b200::Slices &w, const UmmaHandle *q,
+                           const b200_mul_bf16x3_args_t *x) {
+        const b200::Slices in[3] = {{x->b1, q->k1, x->ldb1, x->bstride1, x->nbatch},
+                                    {x->b2, q->k2, x->ldb2, x->bstride2, x->nbatch},
+                                    {x->rowscale, x->ldr ? q->m : 1, x->ldr ? x->ldr : x->ncol,
+                                     0, 1}};
+        for (const b200::Slices &i : in)
+            if (overlap(w, i)) return false;
+        return true;
+    };
+    const b200::Slices wa = out(h, a), wb = out(g, b);
+    return !overlap(wa, wb) && clear(wa, g, b) && clear(wb, h, a);
 }
 
 int b200_mul_bf16x3_apply(void *handle, const b200_mul_bf16x3_args_t *a, void *stream) {

@@ -118,3 +118,55 @@ def test_row_ranges_side_by_side(rows, ncol, nbatch):
     assert bool((out[0] == out[1]).all()) and bool((out[0] != 7.0).all())
     for h in hs:
         lib.mul_bf16x3_destroy(h)
+
+
+@pytest.mark.parametrize('case', ['next slice', 'chained', 'in place'])
+def test_pieces_that_share_memory(case):
+    """Pieces of which one writes what another reads or writes, in another
+    slice or as its input, in one call against the same applies one by one: the
+    same bits."""
+    import torch
+
+    from pyfr_gb300.backend.lib import MulArgs
+
+    lib = _lib()
+    rng = np.random.default_rng(8)
+    m, k, ncol, nbatch = 32, 32, 8640, 2
+    hs = [_handle(lib, rng.standard_normal((m, k)), 2) for _ in range(3)]
+    b0 = torch.from_numpy(rng.random((nbatch + 2, k, ncol)) - 0.25).float()
+    err = torch.zeros(1, dtype=torch.int32, device='cuda')
+    sz, got = m*ncol, []
+    for together in (False, True):
+        b = b0.cuda()
+        out = torch.zeros((nbatch + 2, m, ncol), device='cuda')
+
+        def args(src, dst, beta=0.0, n=nbatch):
+            return MulArgs(b1=src.data_ptr(), ldb1=ncol, c=dst.data_ptr(),
+                           ldc=ncol, ncol=ncol, nbatch=n, bstride1=sz,
+                           cstride=sz, alpha=0.5, beta=beta, products=3,
+                           err=err.data_ptr())
+        if case == 'next slice':
+            # the second adds where the first's second slice is
+            al = [args(b, out), args(b, out[1:], 1.0), args(b, out, 1.0)]
+        elif case == 'chained':
+            al = [args(b, out), args(out, out[nbatch:], 0.0),
+                  args(b, out, 1.0)]
+        else:
+            # the second writes what the first reads
+            al = [args(b, out), args(out, b), args(b, out[nbatch:])]
+        torch.cuda.synchronize()
+        if together:
+            n = len(al)
+            lib.mul_bf16x3_apply_pieces(
+                (C.c_void_p*n)(*(h.value for h in hs)),
+                (C.c_void_p*n)(*map(C.addressof, al)), n, None)
+        else:
+            for h, a in zip(hs, al):
+                lib.mul_bf16x3_apply(h, C.addressof(a), None)
+        torch.cuda.synchronize()
+        assert err.item() == 0
+        got.append((out, b))
+    assert all(bool((x == y).all()) for x, y in zip(*got))
+    assert bool((got[0][0][:nbatch] != 0).any(-1).all())
+    for h in hs:
+        lib.mul_bf16x3_destroy(h)
