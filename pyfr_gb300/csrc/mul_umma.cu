@@ -1220,10 +1220,18 @@ int b200_mul_bf16x3_apply_pieces(void *const *handles, const b200_mul_bf16x3_arg
                                  int n, void *stream) {
     if (!handles || !a || n < 0)
         return b200::set_error(B200_ERR_ARG, "mul_bf16x3_apply_pieces: bad arguments");
-    bool none = false;
+    // (a piece of no columns or slices is none, as a call of its own would be;
+    // there the others go one by one)
+    bool none, some = false;
     for (int i = 0; i < n; i++) {
         const int rc = umma_check(handles[i], a[i], none);
-        if (rc || none) return rc;
+        if (rc) return rc;
+        some = some || none;
+    }
+    if (some) {
+        for (int i = 0; i < n; i++)
+            if (const int rc = umma_apply(handles[i], a[i], 0, stream)) return rc;
+        return B200_OK;
     }
     const UmmaHandle *const *h = (const UmmaHandle *const *)handles;
     for (int i = 0; i < n;) {

@@ -120,11 +120,11 @@ def test_row_ranges_side_by_side(rows, ncol, nbatch):
         lib.mul_bf16x3_destroy(h)
 
 
-@pytest.mark.parametrize('case', ['next slice', 'chained', 'in place'])
+@pytest.mark.parametrize('case', ['next slice', 'chained', 'in place', 'empty'])
 def test_pieces_that_share_memory(case):
     """Pieces of which one writes what another reads or writes, in another
-    slice or as its input, in one call against the same applies one by one: the
-    same bits."""
+    slice or as its input, and a list with an empty piece, in one call against
+    the same applies one by one: the same bits."""
     import torch
 
     from pyfr_gb300.backend.lib import MulArgs
@@ -151,9 +151,11 @@ def test_pieces_that_share_memory(case):
         elif case == 'chained':
             al = [args(b, out), args(out, out[nbatch:], 0.0),
                   args(b, out, 1.0)]
-        else:
+        elif case == 'in place':
             # the second writes what the first reads
             al = [args(b, out), args(out, b), args(b, out[nbatch:])]
+        else:
+            al = [args(b, out), args(b, out, n=0), args(b, out[nbatch:])]
         torch.cuda.synchronize()
         if together:
             n = len(al)
