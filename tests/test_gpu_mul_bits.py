@@ -121,3 +121,52 @@ def test_terms_keep_their_bits(kind, what, ncol):
         err = np.abs(dc.cpu().numpy() - want)
         assert np.all(err <= lim), (alpha, beta, float((err/(lim + 1e-300)).max()))
     lib.mul_destroy(h)
+
+
+@pytest.mark.parametrize('ncol', [33, 200, 9731, 19461])
+@pytest.mark.parametrize('what', ['normal', 'sparse', 'exponents'])
+@pytest.mark.parametrize('kind', ['groups', 'dense', 'short'])
+def test_in_place(kind, what, ncol):
+    """An apply onto its own input, for an operator of each form (rows in
+    groups of one support; twenty entries a row, whose fixed-point form has to
+    be declined, since it reads the input again for outputs of small terms; two
+    entries a row): as the same apply to a copy, and within its bound."""
+    import torch
+
+    from pyfr_gb300.backend import B200Backend
+    from pyfr_gb300.inifile import Inifile
+
+    lib = B200Backend(Inifile()).lib
+    rng = np.random.default_rng(5)
+    m = 24
+    if kind == 'groups':
+        a = np.kron(np.eye(6), 1 + rng.random((4, 4)))
+        assert _grouped(a)
+    elif kind == 'dense':
+        a = rng.standard_normal((m, m))
+        a[:, 20:] = 0
+        a[:, :20] += np.sign(a[:, :20])
+    else:
+        a = np.kron(np.eye(12), rng.standard_normal((2, 2)))
+    a = np.ascontiguousarray(a)
+    b = _data(what, m, ncol, rng)
+    h = C.c_void_p()
+    lib.mul_create(a.ctypes.data_as(C.POINTER(C.c_double)), m, m, C.byref(h))
+    d, e = torch.from_numpy(b).cuda(), torch.from_numpy(b).cuda()
+    out = torch.empty_like(d)
+    torch.cuda.synchronize()
+    for src, dst in ((d, out), (e, e)):
+        lib.mul_f64(h, src.data_ptr(), ncol, dst.data_ptr(), ncol, ncol,
+                    C.c_double(1.0), C.c_double(0.0), None)
+    torch.cuda.synchronize()
+    lib.mul_destroy(h)
+    ref = (a.astype(np.longdouble)[:, :, None]*b).sum(1)
+    n = (a != 0).sum(1)[:, None]
+    tol = U*(n + 2)*(np.abs(a) @ np.abs(b))*(1 + 1e-9)
+    if kind == 'groups':
+        sup = np.repeat(np.abs(b).reshape(6, 4, ncol).max(1), 4, axis=0)
+        tol = np.maximum(tol, U*((1 + 5*4/8)/16*np.abs(a).sum(1).max()*sup +
+                                 np.abs(a) @ np.abs(b)))
+    for t in (out, e):
+        assert np.all(np.abs(t.cpu().numpy() - ref) <= tol)
+    assert kind == 'dense' or torch.equal(out, e)
