@@ -348,7 +348,7 @@ __global__ void errest_final_kernel(int nblk, int uniform, const double *__restr
 
 unsigned grid_for(int64_t n) {
     int64_t g = (n + BX_BLOCK - 1) / BX_BLOCK;
-    const int64_t cap = 152 * 16;
+    const int64_t cap = b200::SM_COUNT * 16;
     return (unsigned)(g < 1 ? 1 : (g > cap ? cap : g));
 }
 

@@ -32,6 +32,9 @@ __device__ __forceinline__ int64_t load_ix(const void *map, int ix64, int64_t i)
                 : (int64_t)__ldg(static_cast<const int *>(map) + i);
 }
 
+// SMs of the GPU (GB300), for the sizes at which a grid fills it
+constexpr int SM_COUNT = 152;
+
 // Launches by programmatic dependent launch: a kernel may be set up while the
 // one before it on the stream ends, and waits at dependent_entry until the
 // kernels before have finished and their writes are visible, which closes most
@@ -85,7 +88,7 @@ inline void launch_if(bool brief, void (*kernel)(P...), dim3 grid, dim3 block, s
 template <typename... P, typename... A>
 inline void launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
                    A &&...a) {
-    launch_if((uint64_t)grid.x * grid.y * grid.z <= 152 * 32, kernel, grid, block, smem, st,
+    launch_if((uint64_t)grid.x * grid.y * grid.z <= SM_COUNT * 32, kernel, grid, block, smem, st,
               static_cast<A &&>(a)...);
 }
 

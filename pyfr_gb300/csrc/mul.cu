@@ -750,7 +750,7 @@ int launch_mul(const MulHandle *h, const T *b, int64_t ldb, T *c, int64_t ldc, i
             // and 106 -> 88 us for the 150 x 125 interpolation at p = 4, and
             // from 10.9 -> 7.7 to 44.4 -> 46.5 us for the 96 x 64 one.  Two
             // columns a lane where every SM has a tile and room for two
-            const int cpl = ncol > 64 * 152 && smem <= 113 * 1024 ? 2 : 1;
+            const int cpl = ncol > 64 * b200::SM_COUNT && smem <= 113 * 1024 ? 2 : 1;
             const int vecc = !((uintptr_t)c & 15) && !(ldc & 1);
             const int epi = alpha == 1.0 ? (beta == 0.0 ? EPI_SET : beta == 1.0 ? EPI_ADD : EPI_GENERAL)
                                          : (beta == 0.0 ? EPI_SCALE : EPI_GENERAL);
@@ -775,7 +775,7 @@ int launch_mul(const MulHandle *h, const T *b, int64_t ldb, T *c, int64_t ldc, i
         // for two CTAs (the 125 x 375 divergence at p = 4: 359 us against
         // 370).
         const bool many = h->nnz >= 10 * (int64_t)h->m ||
-                          (h->nnz >= 4 * (int64_t)h->m && ncol > 64 * 152);
+                          (h->nnz >= 4 * (int64_t)h->m && ncol > 64 * b200::SM_COUNT);
         if (h->fxval && apart && many && smem <= FX_TILE) {
             const int vec2 = vec && !((uintptr_t)c & 15) && !(ldc & 1);
             // One column per lane where two would leave SMs without a tile; the
@@ -783,9 +783,9 @@ int launch_mul(const MulHandle *h, const T *b, int64_t ldb, T *c, int64_t ldc, i
             // divergence of p = 3 tetrahedra, columns that need the test: 17.1
             // us by products and 17.6 packed at 9729 columns, 28.9 and 24.7
             // at 35005, where columns that need none take 22.5)
-            if (ncol <= 64 * 152)
+            if (ncol <= 64 * b200::SM_COUNT)
                 launch_fx<1, FX_EACH>(*h, b, ldb, c, ldc, ncol, alpha, beta, vec2, s);
-            else if (h->mgval && ncol > 2 * 64 * 152 && fx_smem(h->k, 2, true) <= FX_TILE)
+            else if (h->mgval && ncol > 2 * 64 * b200::SM_COUNT && fx_smem(h->k, 2, true) <= FX_TILE)
                 launch_fx<2, FX_PACKED>(*h, b, ldb, c, ldc, ncol, alpha, beta, vec2, s);
             else
                 launch_fx<2, FX_EACH>(*h, b, ldb, c, ldc, ncol, alpha, beta, vec2, s);

@@ -977,7 +977,7 @@ int te_interp(void *handle, int64_t neles, const T *u, int64_t ldu, T *f, int64_
         using K = Line<T, ND, Q>;
         const unsigned nblk = b200::ceil_div(neles, 32);
         // (a warp per line and variable below 16 warps an SM)
-        const bool split = (int64_t)nblk * ND * K::L < 152 * 16;
+        const bool split = (int64_t)nblk * ND * K::L < b200::SM_COUNT * 16;
         const unsigned nchunk = b200::ceil_div(ND * K::L * (split ? K::NV : 1), TE_WARPS);
         const auto P = line_of<T, ND, Q>(h);
         if (split)
