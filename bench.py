@@ -194,8 +194,13 @@ def kernel_bytes(k, be):
 def kernel_flops64(k):
     """FP64 flops of one launch of an FP64 operator apply (the sparse
     kernel: one FMA per operator nonzero and column, plus one per output
-    when it accumulates into the output)."""
+    when it accumulates into the output), or of the Navier-Stokes element
+    kernel's flux on axis-aligned hexahedra (105 operations of the FP64 unit
+    a point, each counted as the FMA that it takes the place of)."""
     m = k.meta
+    if m.get('kind') == 'te_gradflux' and m['geom_mode'] == 3 and \
+            m['tplargs']['ndims'] == 3:
+        return 2*105*m['u'].nrow*m['u'].ncol//5
     if k.name != 'mul':
         return 0
     ncol, nb = m['b'].ncol, m.get('nbatch', 1)
@@ -414,8 +419,9 @@ def measure(intg, args, dist, e2e=True, profile=True):
                'avg_launch_us': round(1e3*d['ms']/d['n'], 2)}
         if be.fpdtype == np.float64 and flops:
             # The FP64 sparse applies are bound by the FP64 pipe on this
-            # GPU, not by HBM: report against the measured FMA throughput,
-            # with the HBM fraction beside it
+            # GPU, and the element kernel by it and by issue slots, not by
+            # HBM: report against the measured FMA throughput, with the HBM
+            # fraction beside it
             pk = fp64_peak(be)
             tf = flops/(d['ms']*1e-3)/1e12
             res['roofline'] = {
