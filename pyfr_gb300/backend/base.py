@@ -321,12 +321,13 @@ class B200Backend:
             return launch
 
         last, after = self.lib.graph_capture_last, self.lib.graph_capture_after
-        items = nodes.items
+        items = nodes.by_chains()
         # (a node that waits for the one before it alone follows it anyway)
-        chained = [deps == [i - 1] for i, (_, deps) in enumerate(items)]
-        used = {d for (_, deps), c in zip(items, chained) if not c
+        chained = [n > 0 and deps == [items[n - 1][1]]
+                   for n, (_, _, deps) in enumerate(items)]
+        used = {d for (_, _, deps), c in zip(items, chained) if not c
                 for d in deps}
-        ends = set(range(len(items))) - {d for _, deps in items for d in deps}
+        ends = set(range(len(items))) - {d for *_, deps in items for d in deps}
         used |= ends
         buf, n = (C.c_void_p*8)(), C.c_int()
 
@@ -340,8 +341,8 @@ class B200Backend:
                       len(handles))
 
             before, got = captured(), {}
-            for i, (k, deps) in enumerate(items):
-                if not chained[i] and i:
+            for j, (k, i, deps) in enumerate(items):
+                if j and not chained[j]:
                     follow(sorted({h for d in deps for h in got[d]})
                            if deps else before)
                 k.run(stream)
