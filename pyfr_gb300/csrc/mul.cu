@@ -466,7 +466,7 @@ void launch_fx(const MulHandle &h, const double *b, int64_t ldb, double *c, int6
 // What bounds it is issue slots (the integer pipes at 53%, the FP64 unit's
 // conversions at 21%) and, in large applies, DRAM beside them: 192 x 64 gradient
 // operator of p = 3 hexahedra, 35005 columns, 25.4 us by columns (above; a
-// quarter of its rows formed twice where the values pass through zero), 22.6 us
+// quarter of its rows formed twice where the values pass through zero), 22.0 us
 // by groups, its DRAM time 10.5 us; at 320 columns 21.2 -> 11.3 us, where the
 // chain of one tile is all there is.  Every other row is converted on the FP64
 // unit, the rest on the integer pipes: all on the former would take its 2 a clock

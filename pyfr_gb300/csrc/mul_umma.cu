@@ -34,7 +34,7 @@
 //   warp 16 lane 0  loads each 32 x 128 FP32 chunk with one 2-D tensor TMA
 //                   into a free stage;
 //   warps 8-15      split a staged chunk into BF16 hi/lo in place, in two
-//                   groups of four warps that take alternate chunks: every
+//                   groups of four warps for the even and the odd stages: every
 //                   thread reads its column of the chunk (32 values), the
 //                   group meets at a named barrier, then writes the halves
 //                   in the canonical K-major no-swizzle UMMA layout over the
