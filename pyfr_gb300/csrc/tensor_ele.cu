@@ -31,7 +31,8 @@
 // rounding of one FP64 FMA.  The divergence at a point is the sum of a line of
 // each direction, every line over its own exponent, and the integer sums are
 // shifted to the largest of them before the one rounding to FP64: an output
-// keeps its bits however large the fluxes elsewhere in the element are.
+// keeps its bits however large the fluxes elsewhere in the element are, or the
+// middle point of an odd line, which its own derivative leaves out.
 // The FP64 unit is left to the flux, beside which the integer work of the
 // other warps runs.
 #include <math.h>
@@ -113,12 +114,22 @@ void set_mat(Mat<double, NO, NI> &m, const double *a, bool wide = false) {
         }
 }
 
-// The operands of a line, as the products take them
-template <typename T, int NI>
+// The middle point of an odd line is no operand of its own derivative, which has
+// the bits of the others alone: where that point is more than four times as
+// large as they are (whether zeros or not), the line is formed by FMAs.  mx and
+// mo: the largest magnitudes of the line and of its other points.
+constexpr int middle(int q) { return q & 1 ? q / 2 : -1; }
+__device__ __forceinline__ bool lone_middle(int mx, int mo) {
+    return mo != 0 && mo < mx - (2 << 20);
+}
+
+// The operands of a line, as the products take them; MID: a point that is absent
+// from its own output
+template <typename T, int NI, int MID = -1>
 struct Operands;
 
-template <int NI>
-struct Operands<float, NI> {
+template <int NI, int MID>
+struct Operands<float, NI, MID> {
     float x[NI];
     __device__ __forceinline__ explicit Operands(const float (&v)[NI]) {
 #pragma unroll
@@ -134,16 +145,18 @@ struct Operands<float, NI> {
     }
 };
 
-template <int NI>
-struct Operands<double, NI> {
+template <int NI, int MID>
+struct Operands<double, NI, MID> {
     int2 b[NI];
     int emax;
     bool wild;
     __device__ __forceinline__ explicit Operands(const double (&v)[NI]) {
-        int mx = hi_abs(v[0]);
+        int mo = 0, mx = 0;
 #pragma unroll
-        for (int j = 1; j < NI; j++) mx = max(mx, hi_abs(v[j]));
-        wild = out_of_range(mx);
+        for (int j = 0; j < NI; j++)
+            if (j != MID) mo = max(mo, hi_abs(v[j]));
+        mx = MID < 0 ? mo : max(mo, hi_abs(v[MID < 0 ? 0 : MID]));
+        wild = out_of_range(mx) || (MID >= 0 && lone_middle(mx, mo));
         emax = max(mx >> 20, 64);
 #pragma unroll
         for (int j = 0; j < NI; j++) {
@@ -293,7 +306,7 @@ struct SmemFlux {
 };
 
 // Exponents of the lines of an element in shared memory, as the products take
-// them (-1: the line's values are out of range and left as they are); the
+// them (-1: the line is formed by FMAs, its values left as they are); the
 // variables next to each other, so that the groups of a warp, which take
 // neighbouring ones, meet no bank twice
 template <int ND, int Q, int E>
@@ -313,13 +326,14 @@ __device__ __forceinline__ void fix_line(const SmemFlux<double, ND, Q, E> &g,
                                          const LineExp<ND, Q, E> &ex, int d, int l) {
     constexpr int N = LIFT ? Q + 2 : Q;
     double x[N];
-    int mx = 0;
+    int mx = 0, mo = 0;
 #pragma unroll
     for (int j = 0; j < N; j++) {
         x[j] = *g.on(d, l, j);
         mx = max(mx, hi_abs(x[j]));
+        if (j != middle(Q)) mo = max(mo, hi_abs(x[j]));
     }
-    const bool wild = out_of_range(mx);
+    const bool wild = out_of_range(mx) || (middle(Q) >= 0 && lone_middle(mx, mo));
     const int emax = max(mx >> 20, 64);
     ex(d, l, g.v) = wild ? -1 : emax;
     if (wild) return;
@@ -377,7 +391,7 @@ __device__ __forceinline__ void smem_div(const Line<float, ND, Q> &P,
         }
 }
 
-// One output whose lines are not all in range: FP64 FMAs for those that are not
+// One output whose lines are not all in fixed point: FP64 FMAs for those that are not
 template <bool LIFT, int ND, int Q, int E>
 __device__ __noinline__ double wild_div(const Line<double, ND, Q> &P, SmemFlux<double, ND, Q, E> g,
                                         LineExp<ND, Q, E> ex, int l, int i) {
@@ -469,7 +483,7 @@ __device__ __forceinline__ double smem_div_point(const Line<double, ND, Q> &P,
 #pragma unroll
         for (int j = 0; j < Q + 2; j++) {
             x[d][j] = j < Q ? g.flux(d, b + j * st) : g.end(d, l, j - Q);
-            mx = max(mx, hi_abs(x[d][j]));
+            if (!absent<Q, Q + 2>(row[d], j)) mx = max(mx, hi_abs(x[d][j]));
         }
     }
     if (out_of_range(mx)) {
@@ -487,7 +501,10 @@ __device__ __forceinline__ double smem_div_point(const Line<double, ND, Q> &P,
 #pragma unroll
     for (int d = 0; d < ND; d++)
 #pragma unroll
-        for (int j = 0; j < Q + 2; j++) s.mad(P.div.a[row[d]][j], split<58>(x[d][j], emax));
+        for (int j = 0; j < Q + 2; j++)
+            // (an absent value may be of any size)
+            if (!absent<Q, Q + 2>(row[d], j))
+                s.mad(P.div.a[row[d]][j], split<58>(x[d][j], emax));
     return s.value_cvt(emax - P.div.s - 1049);
 }
 
@@ -586,7 +603,7 @@ te_gradflux_kernel(const __grid_constant__ Line<T, ND, Q> P, int64_t neles, b200
             for (int i = 0; i < Q; i++) x[i] = live ? pu[i][v * 32] : T(0);
 #pragma unroll
             for (int i = 0; i < 2; i++) x[Q + i] = live ? pc[i][v * 32] : T(0);
-            const Operands<T, Q + 2> b(x);
+            const Operands<T, Q + 2, middle(Q)> b(x);
 #pragma unroll
             for (int i = 0; i < Q; i++) {
                 T y = b.row(P.grad, i);
