@@ -36,6 +36,7 @@ constexpr int MUL_WARPS = 8;     // warps per CTA
 
 struct MulHandle {
     int m, k, nnz;
+    void *block;     // device memory of all that follows
     int *rowptr;     // device, m + 1
     int *colidx;     // device, nnz
     double *val64;   // device, nnz
@@ -672,14 +673,27 @@ bool fx_groups(const double *a, int m, int k, Groups &g) {
     return (size_t)m >= 2 * (g.row.size() / FXG_ROWS);
 }
 
-template <typename V>
-int upload(V **dst, const std::vector<V> &src) {
-    int rc = b200::check_cuda(cudaMalloc(dst, sizeof(V) * src.size()), "mul_create");
-    if (!rc)
-        rc = b200::check_cuda(cudaMemcpy(*dst, src.data(), sizeof(V) * src.size(),
-                                         cudaMemcpyHostToDevice), "mul_create");
-    return rc;
-}
+// An operator's arrays in one block of device memory: an allocation and a copy
+// each took most of mul_create's time
+struct Block {
+    std::vector<unsigned char> bytes;
+    std::vector<std::pair<void **, size_t>> ptrs;
+    template <typename V>
+    void add(V **dst, const std::vector<V> &src) {
+        bytes.resize((bytes.size() + 15) / 16 * 16);
+        ptrs.push_back({(void **)dst, bytes.size()});
+        const unsigned char *p = (const unsigned char *)src.data();
+        bytes.insert(bytes.end(), p, p + sizeof(V) * src.size());
+    }
+    int upload(void **block) {
+        int rc = b200::check_cuda(cudaMalloc(block, bytes.size()), "mul_create");
+        if (!rc)
+            rc = b200::check_cuda(cudaMemcpy(*block, bytes.data(), bytes.size(),
+                                             cudaMemcpyHostToDevice), "mul_create");
+        for (auto &p : ptrs) *p.first = (unsigned char *)*block + p.second;
+        return rc;
+    }
+};
 
 // The operator's fixed-point form (rows, entries), or false where it does
 // not fit: a row of more than FX_MAXNNZ entries, or of an absolute sum
@@ -836,9 +850,7 @@ int opt_in_smem() {
 }
 
 void free_handle(MulHandle *h) {
-    cudaFree(h->rowptr); cudaFree(h->colidx); cudaFree(h->val64); cudaFree(h->val32);
-    cudaFree(h->fxrow); cudaFree(h->fxval); cudaFree(h->mgrow); cudaFree(h->mgval);
-    cudaFree(h->gcol); cudaFree(h->grow); cudaFree(h->gval); cudaFree(h->gdbl);
+    cudaFree(h->block);
     free(h);
 }
 
@@ -876,41 +888,23 @@ int b200_mul_create(const double *a, int m, int k, void **handle) {
     h->m = m;
     h->k = k;
     h->nnz = (int)colidx.size();
-    size_t nz = colidx.size() ? colidx.size() : 1;
-    int rc = b200::check_cuda(cudaMalloc(&h->rowptr, sizeof(int) * (m + 1)), "mul_create");
-    if (!rc) rc = b200::check_cuda(cudaMalloc(&h->colidx, sizeof(int) * nz), "mul_create");
-    if (!rc) rc = b200::check_cuda(cudaMalloc(&h->val64, sizeof(double) * nz), "mul_create");
-    if (!rc) rc = b200::check_cuda(cudaMalloc(&h->val32, sizeof(float) * nz), "mul_create");
-    if (!rc) rc = b200::check_cuda(cudaMemcpy(h->rowptr, rowptr.data(), sizeof(int) * (m + 1),
-                                              cudaMemcpyHostToDevice), "mul_create");
-    if (!rc && h->nnz) {
-        rc = b200::check_cuda(cudaMemcpy(h->colidx, colidx.data(), sizeof(int) * h->nnz,
-                                         cudaMemcpyHostToDevice), "mul_create");
-        if (!rc) rc = b200::check_cuda(cudaMemcpy(h->val64, v64.data(), sizeof(double) * h->nnz,
-                                                  cudaMemcpyHostToDevice), "mul_create");
-        if (!rc) rc = b200::check_cuda(cudaMemcpy(h->val32, v32.data(), sizeof(float) * h->nnz,
-                                                  cudaMemcpyHostToDevice), "mul_create");
-    }
+    int rc = B200_OK;
+    Block block;
+    block.add(&h->rowptr, rowptr);
+    block.add(&h->colidx, colidx);
+    block.add(&h->val64, v64);
+    block.add(&h->val32, v32);
     std::vector<int4> fxrow, fxval, mgrow;
     std::vector<int2> mgval;
-    if (!rc && h->nnz && fx_operator(a, m, k, fxrow, fxval, mgrow, mgval)) {
-        rc = upload(&h->fxrow, fxrow);
-        // (dense: three entries a word or more)
-        if (!rc && 3 * mgval.size() <= fxval.size()) {
-            rc = upload(&h->mgrow, mgrow);
-            if (!rc) rc = upload(&h->mgval, mgval);
-        }
-        if (!rc) rc = upload(&h->fxval, fxval);
-    }
     Groups gr;
-    if (!rc && h->nnz && fx_groups(a, m, k, gr)) {
+    if (h->nnz && fx_groups(a, m, k, gr)) {
         h->gn = gr.n;
         h->ngrp = (int)gr.row.size() / FXG_ROWS;
         h->gs = gr.s;
-        rc = upload(&h->gcol, gr.col);
-        if (!rc) rc = upload(&h->grow, gr.row);
-        if (!rc) rc = upload(&h->gdbl, gr.dbl);
-        if (!rc) rc = upload(&h->gval, gr.val);
+        block.add(&h->gcol, gr.col);
+        block.add(&h->grow, gr.row);
+        block.add(&h->gdbl, gr.dbl);
+        block.add(&h->gval, gr.val);
         // (opted in to the largest tile here, where no capture is open)
         for (int cpl = 1; cpl <= 2; cpl++)
             for (int epi : {EPI_SET, EPI_ADD, EPI_GENERAL, EPI_SCALE})
@@ -921,7 +915,16 @@ int b200_mul_create(const double *a, int m, int k, void **handle) {
                                                  cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                  227 * 1024), "mul: smem attribute");
                 });
+    } else if (h->nnz && fx_operator(a, m, k, fxrow, fxval, mgrow, mgval)) {
+        block.add(&h->fxrow, fxrow);
+        block.add(&h->fxval, fxval);
+        // (dense: three entries a word or more)
+        if (3 * mgval.size() <= fxval.size()) {
+            block.add(&h->mgrow, mgrow);
+            block.add(&h->mgval, mgval);
+        }
     }
+    if (!rc) rc = block.upload(&h->block);
     if (rc) {
         free_handle(h);
         return rc;
